@@ -130,7 +130,8 @@ _SIGNATURES = {
     "bspec_moe_combine": [c_void_p, c_int, c_void_p, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_void_p, c_void_p, c_int,
                           c_void_p, c_void_p, c_longlong, c_void_p],
     "bspec_sgemm_tn_batched": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_longlong, c_longlong, c_longlong,
-                               c_longlong, c_longlong, c_longlong, c_int, c_void_p],
+                               c_longlong, c_longlong, c_longlong, c_int, c_void_p, c_void_p, c_void_p],
+    "bspec_sgemm_scratch": [c_void_p, c_void_p, c_int, c_int, c_int, c_longlong, c_longlong, c_longlong, c_longlong, c_int],
     "bspec_attention_generic": [c_void_p, c_longlong, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p,
                                 c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_int, c_longlong, c_void_p],
     "bspec_attention_bf16": [c_void_p, c_longlong, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_longlong,
@@ -159,7 +160,6 @@ _SIGNATURES = {
     "bspec_attention_prefill_tc": [c_void_p, c_longlong, c_void_p, c_void_p, c_longlong, c_void_p, c_void_p, c_void_p,
                                    c_void_p, c_void_p, c_int, c_longlong, c_int, c_int, c_int, c_int, c_int, c_float,
                                    c_int, c_int, c_void_p, c_void_p],
-    "bspec_sgemm_tn": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_longlong, c_longlong, c_longlong, c_void_p],
     "bspec_pick_slices": [c_int],
     "bspec_argmax": [c_void_p, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p],
     "bspec_sample": [c_void_p, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_ulonglong, c_void_p,
@@ -197,7 +197,7 @@ def load_library(features=None):
                     raise KernelError(f"{path} has no entry point {name}")
                 continue                              # an entry point of a feature this library was built without
             fn.argtypes = argtypes
-            fn.restype = c_longlong if name == "bspec_gemm_tc_plan" else c_int
+            fn.restype = c_longlong if name in ("bspec_gemm_tc_plan", "bspec_sgemm_scratch") else c_int
         _lib, _features = lib, want
         from . import debug
         debug.apply_environment(sys.modules[__name__], lib)
@@ -1202,7 +1202,8 @@ def _raise_status(dev, code: int) -> None:
     raise KernelError(f"a kernel on {dev} gave up a bounded wait (code {code}: GEMM 1 = stage never freed, "
                       f"2 = operands never arrived, 3 = accumulator never completed; decode attention 11/13 = stage "
                       f"never freed, 12/14 = keys never arrived; prompt attention 21/22 the same, 31-41 = a role of "
-                      f"the tensor-core prompt kernel).  The results of the steps "
+                      f"the tensor-core prompt kernel; float32 product of few rows 91 = stage never freed, 92 = operands "
+                      f"never arrived).  The results of the steps "
                       f"since the last check are not valid.")
 
 
@@ -1367,8 +1368,7 @@ def linear(x: torch.Tensor, w: torch.Tensor, out_dtype: Optional[torch.dtype] = 
     if x.dtype == torch.float32:
         assert out_dtype == torch.float32 and x.stride(1) == 1 and w.stride(1) == 1
         out = torch.empty((M, N), dtype=torch.float32, device=x.device)
-        _check(load_library().bspec_sgemm_tn(x.data_ptr(), w.data_ptr(), out.data_ptr(), M, N, K, x.stride(0),
-                                             w.stride(0), N, _stream()), "sgemm_tn")
+        _sgemm(x, w, out, M, N, K, x.stride(0), w.stride(0), 0, 0, 1)
         return out
     if (K % 8 == 0 and M > 0 and x.is_contiguous() and w.is_contiguous()
             and (TC_GEMM == "all" or (TC_GEMM == "auto" and M <= TC_GEMM_MAX_M))):
@@ -1387,10 +1387,19 @@ def linear_batched(x: torch.Tensor, w: torch.Tensor) -> torch.Tensor:
     assert w.shape == (B, N, K) and x.dtype == w.dtype and x.stride(2) == 1 and w.is_contiguous()
     if x.dtype == torch.float32:
         out = torch.empty((B, M, N), dtype=torch.float32, device=x.device)
-        _check(load_library().bspec_sgemm_tn_batched(x.data_ptr(), w.data_ptr(), out.data_ptr(), M, N, K, x.stride(1),
-                                                     K, N, x.stride(0), N * K, M * N, B, _stream()), "sgemm_tn_batched")
+        _sgemm(x, w, out, M, N, K, x.stride(1), K, x.stride(0), N * K, B)
         return out
     return torch.bmm(x, w.transpose(1, 2))
+
+def _sgemm(x, w, out, M: int, N: int, K: int, lda: int, ldw: int, sa: int, sw: int, batch: int) -> None:
+    """``batch`` float32 products, operands sa / sw numbers apart; the K slices of small tiles meet in scratch that the
+    stream's order protects."""
+    lib = load_library()
+    need = lib.bspec_sgemm_scratch(x.data_ptr(), w.data_ptr(), M, N, K, lda, ldw, sa, sw, batch)
+    scratch = torch.empty((need,), dtype=torch.float32, device=x.device) if need else None
+    _check(lib.bspec_sgemm_tn_batched(x.data_ptr(), w.data_ptr(), out.data_ptr(), M, N, K, lda, ldw, N, sa, sw, M * N, batch,
+                                      _ptr(scratch), _status_word(x.device).data_ptr(), _stream()), "sgemm_tn")
+
 
 
 # ---------------------------------------------------------------------------- latent attention

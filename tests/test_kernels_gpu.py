@@ -96,6 +96,27 @@ def test_sgemm_is_true_float32(ops, M, N, K):
     assert torch.equal(got[:1], ops.linear(a[:1].contiguous(), w))
 
 
+@pytest.mark.parametrize("N,K", [(1, 4), (17, 60), (64, 68), (130, 1020), (65, 1028), (48, 4100), (33, 1027)])
+@pytest.mark.parametrize("batch", [1, 3])
+def test_sgemm_sums_have_one_order_in_every_kernel(ops, N, K, batch):
+    """Few rows, tiles of 64 and of 128 rows, K slices in scratch, 4-byte copies (odd K): every row has the same bits in
+    all of them, and the error of sums of K / 2 terms in chains of 32."""
+    g = torch.Generator(device=DEV).manual_seed(N + K)
+    a = torch.randn(batch, 150, K, device=DEV, generator=g)
+    w = torch.randn(batch, N, K, device=DEV, generator=g)
+    whole = ops.linear_batched(a, w)
+    want = a.double() @ w.double().transpose(1, 2)
+    # a chain of 32 roundings, 16 slices per group and K / 1024 groups, each at most half a unit of the sum of magnitudes
+    bound = 2.0 ** -24 * (32 + 1 + 16 + K / 1024 + 1) * (a.abs().double() @ w.abs().double().transpose(1, 2))
+    assert bool(((whole.double() - want).abs() <= bound).all())
+    for m in (1, 2, 3, 5, 8, 9, 32, 33, 64, 65, 128, 129):
+        part = ops.linear_batched(a[:, :m].contiguous(), w)
+        assert torch.equal(part, whole[:, :m]), m
+        one = ops.linear(a[0, 150 - m:], w[0])               # the operand's last rows
+        assert torch.equal(one, whole[0, 150 - m:]), m
+    ops.check_status()
+
+
 def _rope_reference(x, pos, inv_freq, rot, interleaved):
     """float64 angle from the float32 frequencies given, float32 result."""
     ang = pos.double()[:, None] * inv_freq.double()[None, :]
