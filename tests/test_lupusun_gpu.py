@@ -236,6 +236,33 @@ def test_chunk_masked_attention_with_a_sink(ops, dtype, shape, with_sink):
     assert (got - want).abs().max() <= (2e-5 if dtype == torch.float32 else 2.5e-2)
 
 
+@pytest.mark.parametrize("Hq,G,hd,vd,ps", [(4, 1, 64, 64, 16), (3, 1, 18, 7, 5), (10, 2, 128, 96, 8), (8, 4, 256, 256, 16),
+                                           (17, 1, 16, 130, 3)])
+def test_float32_attention_rows_have_the_same_bits_in_every_portion(ops, Hq, G, hd, vd, ps):
+    """Four rows and sixteen (or eight) per block, tiles that straddle tokens, head sizes that are no whole quads, against
+    float64; a row's bits do not depend on its portion, and values that no row may see (infinite here) leave no trace."""
+    lens = [1, 33, 131, 300]
+    ks, vs, cache, ctx, tables, fill, qo = _paged(ops, torch.float32, Hq, G, hd, vd, ps, lens, lens, hd + vd)
+    cache.fill_(float("inf"))
+    fill()
+    q = torch.randn(sum(lens), Hq * hd, device=DEV, generator=torch.Generator(device=DEV).manual_seed(3))
+    whole = torch.empty(sum(lens), Hq * vd, device=DEV)
+    ops.masked_attention(q, whole, cache, ctx, tables, Hq, G, hd, vd, 0.25)
+    for e, L in enumerate(lens):
+        want = P.chunked_sink_attention(q[qo[e]:qo[e + 1]].view(L, Hq, hd).double().cpu(), ks[e].double().cpu(), vs[e].double().cpu(),
+                                        torch.full((Hq,), -1e30, dtype=F64), 0.25, 1 << 40, torch.arange(L))
+        # the bound of the test above; scores are hd products of unit normals, so a wide head's are larger
+        assert (whole[qo[e]:qo[e + 1]].view(L, Hq, vd).double().cpu() - want).abs().max() <= 2e-5 * max(1.0, hd / 64)
+    for portion in (1, 2, 9):
+        rows = torch.cat([torch.arange(max(qo[e], qo[e + 1] - portion), qo[e + 1]) for e in range(len(lens))]).to(DEV)
+        take = [min(portion, L) for L in lens]
+        ctx2 = SimpleNamespace(qo_indptr=_i32([0] + list(np.cumsum(take))), positions=ctx.positions[rows].contiguous(),
+                               n_entries=len(lens), max_q_len=max(take))
+        part = torch.empty(len(rows), Hq * vd, device=DEV)
+        ops.masked_attention(q[rows].contiguous(), part, cache, ctx2, tables, Hq, G, hd, vd, 0.25)
+        assert torch.equal(part, whole[rows]), portion
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("key", [0, 511, 512, 513, 527, 528, 1023, 1024, 1025, 1100, 1299])
 def test_one_key_decides_inside_its_chunk_and_is_unseen_outside(ops, dtype, key):
