@@ -8,14 +8,15 @@
 //                     portion come from the request's state), unit length of every q and k head (q also times a
 //                     scale), beta = sigmoid(b), g = exp(-exp(A_log) softplus(a + dt_bias))
 //   delta_recurrence  per (request, head, 32 or 8 value columns): the token loop over the portion with the state in
-//                     registers (a column of S is spread over four lanes), state read at the start and written at
-//                     the end; the request's blocks also move the convolutions' inputs on
+//                     registers (a column of S is spread over four or sixteen lanes), state read at the start and
+//                     written at the end; the request's blocks also move the convolutions' inputs on.  Steps with a
+//                     portion of eight tokens or more take delta_tiles_prepare and delta_tiles instead, which
+//                     multiply the rule out over tiles
 //   gated_rmsnorm     per (token, head): o / rms(o) * w * silu(gate), with options other mixers use
 //
 // The order of every sum depends on the sizes alone, not on how a request was cut into portions or on what else is
 // in the step.
-#include "common.cuh"
-#include <cuda_pipeline.h>
+#include "state_tiles.cuh"
 #include <math.h>
 using namespace bspec;
 
@@ -96,8 +97,8 @@ delta_prepare_kernel(const float* __restrict__ proj, int ld, int b_off, int a_of
 // lanes and a block holds 8 columns, which makes four times as many warps with dependent chains a quarter as long.  Per token both read-outs are taken from the state before the write,
 //     a = S^T k,  b = S^T q,  u = beta (v - g a),  o = g b + u (k . q),  S <- g S + k u^T,
 // which is the rule above with o = (g S + k u^T)^T q multiplied out: one pass over the registers for the three sums
-// (reduced over the column's lanes together), one for the update.  The 16-lane form takes two tokens per pass.  The next tile of tokens is copied into the
-// other half of the staging buffers while the current one is worked on.
+// (reduced over the column's lanes together), one for the update.  The next tile of tokens is copied into the other half
+// of the staging buffers while the current one is worked on.
 template <int R, int COLS, int LANES>
 __global__ void __launch_bounds__(COLS * LANES)
 delta_recurrence_kernel(const float* __restrict__ mix, const float* __restrict__ gates, const float* __restrict__ proj,
@@ -112,7 +113,6 @@ delta_recurrence_kernel(const float* __restrict__ mix, const float* __restrict__
   __shared__ __align__(16) float ks[2][TILE][DP];
   __shared__ float vs[2][TILE][COLS];
   __shared__ float bg[2][TILE][2];
-  __shared__ float sc[TILE / 2][4];                // products between the two tokens of every pair of the tile
   const int e = blockIdx.z, h = blockIdx.y;
   const int q_begin = qo_indptr[e], n = qo_indptr[e + 1] - q_begin;
   const int C = 2 * Gk * dim + H * vdim;
@@ -223,84 +223,10 @@ delta_recurrence_kernel(const float* __restrict__ mix, const float* __restrict__
         qd[c] = *reinterpret_cast<const float4*>(&qs[buf][tt][row]);
       }
     };
-    if constexpr (LANES == 16) {
-      // The long chain of one prompt: two tokens per pass.  With a = S^T k and b = S^T q of BOTH tokens taken from
-      // the state before either write, and the tokens' mutual products (the same for every column, formed once
-      // per tile below),
-      //   u1 = beta1 (v1 - g1 a1)                    o1 = g1 b1 + u1 (k1.q1)
-      //   u2 = beta2 (v2 - g2 (g1 a2 + u1 (k1.k2)))  o2 = g2 (g1 b2 + u1 (k1.q2)) + u2 (k2.q2)
-      //   S <- g1 g2 S + g2 u1 k1 + u2 k2,
-      // which is the rule applied twice, multiplied out: one round of reductions and one pass over the registers
-      // for two tokens.
-      {
-        const int pr = min((int)(threadIdx.x >> 4), TILE / 2 - 1), sub = threadIdx.x & 15;
-        const float *k1 = ks[buf][2 * pr], *q1 = qs[buf][2 * pr], *k2 = ks[buf][2 * pr + 1], *q2 = qs[buf][2 * pr + 1];
-        float x0 = 0.f, x1 = 0.f, x2 = 0.f, x3 = 0.f;
-        for (int d = sub; d < dimp; d += 16) {
-          x0 += k1[d] * q1[d]; x1 += k1[d] * k2[d]; x2 += k1[d] * q2[d]; x3 += k2[d] * q2[d];
-        }
-#pragma unroll
-        for (int o = 1; o < 16; o <<= 1) {
-          x0 += __shfl_xor_sync(0xffffffffu, x0, o); x1 += __shfl_xor_sync(0xffffffffu, x1, o);
-          x2 += __shfl_xor_sync(0xffffffffu, x2, o); x3 += __shfl_xor_sync(0xffffffffu, x3, o);
-        }
-        if (sub == 0 && (int)(threadIdx.x >> 4) < TILE / 2 && 2 * pr + 1 < nt) {
-          sc[pr][0] = x0; sc[pr][1] = x1; sc[pr][2] = x2; sc[pr][3] = x3;
-        }
-      }
-      __syncthreads();
-      const int np = nt >> 1;
-      float4 k1n[R / 4], q1n[R / 4], k2n[R / 4], q2n[R / 4];
-      if (np > 0) { fetch(0, k1n, q1n); fetch(1, k2n, q2n); }
-      for (int pp = 0; pp < np; ++pp) {
-        float4 k1[R / 4], q1[R / 4], k2[R / 4], q2[R / 4];
-#pragma unroll
-        for (int c = 0; c < R / 4; ++c) { k1[c] = k1n[c]; q1[c] = q1n[c]; k2[c] = k2n[c]; q2[c] = q2n[c]; }
-        const int t1 = 2 * pp, t2 = 2 * pp + 1;
-        const float beta1 = bg[buf][t1][0], g1 = bg[buf][t1][1], v1 = vs[buf][t1][col];
-        const float beta2 = bg[buf][t2][0], g2 = bg[buf][t2][1], v2 = vs[buf][t2][col];
-        const float kq11 = sc[pp][0], kk12 = sc[pp][1], kq12 = sc[pp][2], kq22 = sc[pp][3];
-        float a1 = 0.f, b1 = 0.f, a2 = 0.f, b2 = 0.f;
-#pragma unroll
-        for (int c = 0; c < R / 4; ++c) {
-          a1 += s[4 * c] * k1[c].x; a1 += s[4 * c + 1] * k1[c].y; a1 += s[4 * c + 2] * k1[c].z; a1 += s[4 * c + 3] * k1[c].w;
-          b1 += s[4 * c] * q1[c].x; b1 += s[4 * c + 1] * q1[c].y; b1 += s[4 * c + 2] * q1[c].z; b1 += s[4 * c + 3] * q1[c].w;
-          a2 += s[4 * c] * k2[c].x; a2 += s[4 * c + 1] * k2[c].y; a2 += s[4 * c + 2] * k2[c].z; a2 += s[4 * c + 3] * k2[c].w;
-          b2 += s[4 * c] * q2[c].x; b2 += s[4 * c + 1] * q2[c].y; b2 += s[4 * c + 2] * q2[c].z; b2 += s[4 * c + 3] * q2[c].w;
-        }
-        if (pp + 1 < np) { fetch(2 * pp + 2, k1n, q1n); fetch(2 * pp + 3, k2n, q2n); }
-#pragma unroll
-        for (int o = 1; o < LANES; o <<= 1) {
-          a1 += __shfl_xor_sync(0xffffffffu, a1, o); b1 += __shfl_xor_sync(0xffffffffu, b1, o);
-          a2 += __shfl_xor_sync(0xffffffffu, a2, o); b2 += __shfl_xor_sync(0xffffffffu, b2, o);
-        }
-        const float u1 = beta1 * (v1 - g1 * a1);
-        const float u2 = beta2 * (v2 - g2 * (g1 * a2 + u1 * kk12));
-        if (live && r == 0) {
-          float* op = out + (size_t)(q_begin + t0 + t1) * H * vdim + h * vdim + j;
-          op[0] = g1 * b1 + u1 * kq11;
-          op[(size_t)H * vdim] = g2 * (g1 * b2 + u1 * kq12) + u2 * kq22;
-        }
-        const float c0 = g1 * g2, c1 = g2 * u1;
-#pragma unroll
-        for (int c = 0; c < R / 4; ++c) {
-          s[4 * c] = fmaf(k2[c].x, u2, fmaf(k1[c].x, c1, c0 * s[4 * c]));
-          s[4 * c + 1] = fmaf(k2[c].y, u2, fmaf(k1[c].y, c1, c0 * s[4 * c + 1]));
-          s[4 * c + 2] = fmaf(k2[c].z, u2, fmaf(k1[c].z, c1, c0 * s[4 * c + 2]));
-          s[4 * c + 3] = fmaf(k2[c].w, u2, fmaf(k1[c].w, c1, c0 * s[4 * c + 3]));
-        }
-      }
-      if (nt & 1) {                                 // the portion's last token
-        float4 kr[R / 4], qr[R / 4];
-        fetch(nt - 1, kr, qr);
-        one_token(nt - 1, kr, qr);
-      }
-    } else {
-      for (int tt = 0; tt < nt; ++tt) {
-        float4 kr[R / 4], qr[R / 4];
-        fetch(tt, kr, qr);
-        one_token(tt, kr, qr);
-      }
+    for (int tt = 0; tt < nt; ++tt) {
+      float4 kr[R / 4], qr[R / 4];
+      fetch(tt, kr, qr);
+      one_token(tt, kr, qr);
     }
   }
   bspec::pdl_launch_dependents();
@@ -311,6 +237,144 @@ delta_recurrence_kernel(const float* __restrict__ mix, const float* __restrict__
       if (row < dimp) *reinterpret_cast<float4*>(sp + row) = make_float4(s[4 * c], s[4 * c + 1], s[4 * c + 2], s[4 * c + 3]);
     }
   }
+}
+
+// ---------------------------------------------------------------- portions of whole tiles
+// A token at a time is a chain of dependent latencies: the sums, their reduction over the column's lanes, u, the update
+// (with two tokens per pass 366 ns a token, 753 us for portions of 333, 826 and 2,048 tokens, 16 heads of 128 x 128).  The rule
+// applied B = 8 times and multiplied out needs one such chain for the tile.  With c_t = g_1 .. g_t and
+// y(s, t) = g_(s+1) .. g_t, both from the state S before the tile,
+//     x_t = beta_t (v_t - c_t S^T k_t),      u = T x,   T = (I + L)^-1,  L_ts = beta_t y(s, t) (k_s . k_t)  for s < t,
+//     o_t = c_t S^T q_t + sum_s<=t y(s, t) (k_s . q_t) u_s,                S <- c_B S + sum_s y(s, B) k_s u_s^T.
+// T's numbers stay within [-1, 1] (below the diagonal -beta_t k_t . (product of contractions) k_s), so the explicit
+// inverse loses no more than the substitution would.  T, and with it the factors of x in o and in the update, are the
+// same for every value column: delta_tiles_prepare forms them once per (tile, head).  Tokens that a last tile lacks count
+// as k = q = v = 0, beta = 0, g = 1.  In the terms of state_tiles: F = y(t, B) T_ts, P = sum_r y(r, t) (k_r . q_t) T_rs,
+// d = beta c_t, e = beta.
+__global__ void __launch_bounds__(128)
+delta_tiles_prepare_kernel(const float* __restrict__ mix, const float* __restrict__ gates, const int* __restrict__ qo_indptr,
+                           float* __restrict__ coef, int H, int Gk, int dim, int vdim) {
+  bspec::pdl_prologue(60);
+  __shared__ float qs[ST_B][MAX_DIM + 8], ks[ST_B][MAX_DIM + 8];        // (rows eight banks apart)
+  __shared__ float dots[ST_B][ST_B], y[ST_B][ST_B], be[ST_B], g[ST_B], low[ST_B][ST_B], inv[ST_B][ST_B];
+  const int i = blockIdx.x, h = blockIdx.y, e = blockIdx.z;
+  const int q_begin = qo_indptr[e], n = qo_indptr[e + 1] - q_begin;
+  if (i * ST_B >= n) return;
+  const int cnt = min(ST_B, n - i * ST_B), C = 2 * Gk * dim + H * vdim, kh = h / (H / Gk);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+#pragma unroll
+  for (int u = 0; u < ST_B / 4; ++u) {
+    const int t = warp + 4 * u;
+    const float* row = mix + (size_t)(q_begin + i * ST_B + min(t, cnt - 1)) * C;
+    for (int d = lane; d < dim; d += 32) {
+      qs[t][d] = t < cnt ? row[kh * dim + d] : 0.f;
+      ks[t][d] = t < cnt ? row[(Gk + kh) * dim + d] : 0.f;
+    }
+  }
+  if (tid < ST_B) {
+    const float* gr = gates + (size_t)(q_begin + i * ST_B + min(tid, cnt - 1)) * 2 * H + h;
+    be[tid] = tid < cnt ? gr[0] : 0.f;
+    g[tid] = tid < cnt ? gr[H] : 1.f;
+  }
+  __syncthreads();
+  // dots[t][s]: k_s . q_t for s <= t, k_s . k_t for s > t; a warp takes two t, eight lanes a dot (four s at a time)
+#pragma unroll
+  for (int u = 0; u < ST_B / 2; ++u) {
+    const int t = 2 * warp + u / 2, s_ = 4 * (u & 1) + lane / 8;
+    const float *kk = ks[s_], *other = s_ <= t ? qs[t] : ks[t];
+    float a = 0.f;
+    for (int d = lane % 8; d < dim; d += 8) a = fmaf(kk[d], other[d], a);
+#pragma unroll
+    for (int o = 1; o < 8; o <<= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+    if (lane % 8 == 0) dots[t][s_] = a;
+  }
+  const int ct = (tid / ST_B) % ST_B, cs = tid % ST_B;         // the cell of this thread (tid < 64)
+  __syncthreads();
+  if (tid < ST_B * ST_B) {
+    float a = 1.f;                                             // y(s, t)
+#pragma unroll
+    for (int r = 1; r < ST_B; ++r) a *= r > cs && r <= ct ? g[r] : 1.f;
+    y[cs][ct] = a;
+    low[ct][cs] = cs < ct ? be[ct] * a * dots[cs][ct] : 0.f;
+  }
+  __syncthreads();
+  if (tid < ST_B) {                                            // column tid of T
+    float col[ST_B];
+#pragma unroll
+    for (int t = 0; t < ST_B; ++t) {
+      float a = t == tid ? 1.f : 0.f;
+#pragma unroll
+      for (int r = 0; r < t; ++r) a = r >= tid && t > tid ? fmaf(-low[t][r], col[r], a) : a;
+      col[t] = a;
+      inv[t][tid] = a;
+    }
+  }
+  __syncthreads();
+  float* co = coef + (state_tile_slot(q_begin, e, i) * H + h) * ST_CO + ct * ST_ROW;
+  if (tid < ST_B * ST_B) {
+    float a = 0.f;
+#pragma unroll
+    for (int r = 0; r < ST_B; ++r) a = r >= cs && r <= ct ? fmaf(y[r][ct] * dots[ct][r], inv[r][cs], a) : a;
+    co[cs] = cs <= ct ? y[ct][ST_B - 1] * inv[ct][cs] : 0.f;
+    co[ST_B + cs] = a;
+    if (cs == 0) {
+      const float c = g[0] * y[0][ct];
+      co[16] = be[ct] * c;
+      co[17] = be[ct];
+      co[18] = c;
+      co[19] = g[0] * y[0][ST_B - 1];
+    }
+  }
+}
+
+template <int R>
+__global__ void __launch_bounds__(ST_THREADS)
+delta_tiles_kernel(const float* __restrict__ mix, const float* __restrict__ proj, const float* __restrict__ coef, int ld,
+                   float* __restrict__ state, long long state_stride, long long tail_off, const int* __restrict__ qo_indptr,
+                   const int* __restrict__ state_slots, float* __restrict__ out, int H, int Gk, int dim, int vdim, int taps) {
+  bspec::pdl_prologue_late(61);
+  const int dimp = (dim + 3) & ~3;                             // a column of S is kept padded to whole float4s; the pad stays 0
+  const int e = blockIdx.z, h = blockIdx.y;
+  const int q_begin = qo_indptr[e], n = qo_indptr[e + 1] - q_begin;
+  const int C = 2 * Gk * dim + H * vdim;
+  float* srow = state + (size_t)state_slots[e] * state_stride;
+  if (n <= 0) return;
+  if (taps > 1) {                                              // as in delta_recurrence_kernel
+    float* tail = srow + tail_off;
+    const int share = blockIdx.y * gridDim.x + blockIdx.x, shares = gridDim.y * gridDim.x;
+    for (int c = share * ST_THREADS + threadIdx.x; c < C; c += shares * ST_THREADS)
+      for (int s = 0; s < taps - 1; ++s) {
+        const int rel = n + s - (taps - 1);
+        tail[(size_t)s * C + c] = rel >= 0 ? proj[(size_t)(q_begin + rel) * ld + c] : tail[(size_t)(s + n) * C + c];
+      }
+  }
+  const int kh = h / (H / Gk);
+  const float* row = mix + (size_t)q_begin * C;
+  StateTiles p;
+  p.q = row + kh * dim, p.k = row + (Gk + kh) * dim, p.v = row + 2 * Gk * dim + h * vdim;
+  p.q_stride = p.k_stride = p.v_stride = C;
+  p.coef = coef + (state_tile_slot(q_begin, e, 0) * H + h) * ST_CO, p.coef_stride = (long long)H * ST_CO;
+  p.s = srow + (size_t)h * vdim * dimp, p.s_stride = p.s_rows = dimp;
+  p.out = out + (size_t)q_begin * H * vdim + (size_t)h * vdim, p.out_stride = (long long)H * vdim;
+  p.n = n, p.dim = dim, p.vdim = vdim, p.j0 = blockIdx.x * ST_COLS;
+  state_tiles<R, true>(p, [](float x) { return x; });
+}
+
+template <int R>
+int launch_delta_tiles(dim3 grid, cudaStream_t stream, const float* mix, const float* proj, const float* coef, int ld, float* state,
+                       long long state_stride, long long tail_off, const int* qo_indptr, const int* state_slots, float* out, int H,
+                       int Gk, int dim, int vdim, int taps) {
+  static bool set[bspec::kMaxDevices] = {};
+  bool& done = set[bspec::current_device()];
+  if (!done) {
+    const cudaError_t err = cudaFuncSetAttribute(delta_tiles_kernel<R>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                 (int)state_tiles_smem(16 * R));
+    if (err != cudaSuccess) return (int)err;
+    done = true;
+  }
+  BSPEC_LAUNCH_SERIALIZED((delta_tiles_kernel<R>), grid, ST_THREADS, state_tiles_smem(16 * R), stream, mix, proj, coef, ld, state,
+                          state_stride, tail_off, qo_indptr, state_slots, out, H, Gk, dim, vdim, taps);
+  return BSPEC_LAUNCH_CHECK();
 }
 
 // out[t, h*V + j] = x / sqrt(mean_j x^2 + eps) * w[j] * act(gate[t, h*V + j]) * out_scale with x = o[t, h, j], or
@@ -478,13 +542,30 @@ BSPEC_API int bspec_delta_prepare(const float* proj, int n, int ld, int b_off, i
   return BSPEC_LAUNCH_CHECK();
 }
 
+// Floats of scratch for a step of n tokens whose longest portion has max_q_len: the tiles' coefficients, or 0 where the
+// portions are shorter than a tile and go token by token.
+BSPEC_API long long bspec_delta_scratch(int n, int n_entries, int max_q_len, int H) {
+  return max_q_len >= ST_B ? bspec::state_tile_slots(n, n_entries) * H * ST_CO : 0;
+}
+
 BSPEC_API int bspec_delta_recurrence(const float* mix, const float* gates, const float* proj, int ld, float* state,
                                      long long state_stride, long long tail_off, const int* qo_indptr,
-                                     const int* state_slots, float* out, int n_entries, int H, int Gk, int dim,
-                                     int vdim, int taps, cudaStream_t stream) {
+                                     const int* state_slots, float* out, int n_entries, int max_q_len, int H, int Gk,
+                                     int dim, int vdim, int taps, float* scratch, cudaStream_t stream) {
   if (n_entries <= 0) return 0;
   if (dim <= 0 || dim > MAX_DIM || H % Gk != 0 || n_entries > 65535 || H > 65535)
     return (int)cudaErrorInvalidValue;
+  if (scratch != nullptr) {
+    BSPEC_LAUNCH(delta_tiles_prepare_kernel, dim3((max_q_len + ST_B - 1) / ST_B, H, n_entries), 128, 0, stream, mix, gates,
+                 qo_indptr, scratch, H, Gk, dim, vdim);
+    const int err = BSPEC_LAUNCH_CHECK();
+    if (err != 0) return err;
+    const dim3 tiles((vdim + ST_COLS - 1) / ST_COLS, H, n_entries);
+    return dim <= 128 ? launch_delta_tiles<8>(tiles, stream, mix, proj, scratch, ld, state, state_stride, tail_off, qo_indptr,
+                                              state_slots, out, H, Gk, dim, vdim, taps)
+                      : launch_delta_tiles<16>(tiles, stream, mix, proj, scratch, ld, state, state_stride, tail_off, qo_indptr,
+                                              state_slots, out, H, Gk, dim, vdim, taps);
+  }
   // 32 value columns of 4 lanes per block; 8 columns of 16 lanes when that would leave most of the device idle
   const bool narrow = (long long)((vdim + 31) / 32) * H * n_entries < 2ll * bspec::sm_count();
   const int cols = narrow ? 8 : 32;

@@ -13,7 +13,7 @@
 // A step holds portions of several requests (qo_indptr, state_slots); a portion of one token is a decode step.  Every
 // sum runs in an order fixed by the sizes alone, so a position's result does not depend on how the request was cut
 // or on what else is in the step.
-#include "common.cuh"
+#include "state_tiles.cuh"
 #include <math.h>
 using namespace bspec;
 
@@ -214,6 +214,131 @@ lightning_recurrence_kernel(const float* __restrict__ proj, long long ld, int q_
       if (i < dim) sp[i] = s[m];
     }
   }
+}
+
+// ---------------------------------------------------------------- lightning attention, portions of whole tiles
+// The token loop above is bound by its four-token passes' shared-memory loads and latencies (270 ns a token: 553 us for 2,048
+// tokens, 16 heads of 128 x 128).  Eight tokens at a time (state_tiles.cuh): x = v, F = diag(d^(B-1-t)), P_ts = d^(t-s)
+// (k_s . q_t), c_t = d^(t+1).  A tile of ``cnt`` < 8 tokens counts the others as zeros without decay.  The preparation
+// kernel, one block per (tile, head), also leaves q and k as the recurrence wants them (silu, scale, rotation), which every
+// block of a head would repeat otherwise: qk [n][H][q: dim | k: dim].
+__global__ void __launch_bounds__(128)
+lightning_tiles_prepare_kernel(const float* __restrict__ proj, long long ld, int q_off, int k_off, const float* __restrict__ decay,
+                               const int* __restrict__ qo_indptr, float* __restrict__ qk, float* __restrict__ coef, int H, int dim,
+                               int act, float k_scale, const float* __restrict__ inv_freq, int rot, const int* __restrict__ positions) {
+  bspec::pdl_prologue(65);
+  __shared__ float qs[ST_B][264], ks[ST_B][264], dots[ST_B][ST_B];      // (rows eight banks apart)
+  const int i = blockIdx.x, h = blockIdx.y, e = blockIdx.z;
+  const int q_begin = qo_indptr[e], n = qo_indptr[e + 1] - q_begin;
+  if (i * ST_B >= n) return;
+  const int cnt = min(ST_B, n - i * ST_B), t0 = q_begin + i * ST_B;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+#pragma unroll
+  for (int u = 0; u < ST_B / 4; ++u) {
+    const int t = warp + 4 * u;
+    const float* row = proj + (size_t)(t0 + min(t, cnt - 1)) * ld + (size_t)h * dim;
+    for (int d = lane; d < dim; d += 32) {
+      const float q = row[q_off + d], k = row[k_off + d];
+      qs[t][d] = t < cnt ? (act ? silu_f(q) : q) : 0.f;
+      ks[t][d] = t < cnt ? (act ? silu_f(k) : k) * k_scale : 0.f;
+    }
+  }
+  __syncthreads();
+  if (rot > 0) {
+    const int half = rot / 2;
+    for (int x = tid; x < cnt * half; x += 128) {
+      const int t = x / half, d = x - t * half;
+      float sn, c;
+      rotation_sincos(positions[t0 + t], inv_freq, half, d, &sn, &c);
+      const float qu = qs[t][d], qv = qs[t][d + half], ku = ks[t][d], kv = ks[t][d + half];
+      qs[t][d] = qu * c - qv * sn;
+      qs[t][d + half] = qv * c + qu * sn;
+      ks[t][d] = ku * c - kv * sn;
+      ks[t][d + half] = kv * c + ku * sn;
+    }
+    __syncthreads();
+  }
+#pragma unroll
+  for (int u = 0; u < ST_B / 4; ++u) {
+    const int t = warp + 4 * u;
+    float* row = qk + ((size_t)(t0 + t) * H + h) * 2 * dim;
+    for (int d = lane; t < cnt && d < dim; d += 32) {
+      row[d] = qs[t][d];
+      row[dim + d] = ks[t][d];
+    }
+  }
+  // a warp takes two t, eight lanes a dot (four s at a time)
+#pragma unroll
+  for (int u = 0; u < ST_B / 2; ++u) {
+    const int t = 2 * warp + u / 2, s = 4 * (u & 1) + lane / 8;
+    float a = 0.f;
+    for (int d = lane % 8; d < dim; d += 8) a = fmaf(ks[s][d], qs[t][d], a);
+#pragma unroll
+    for (int o = 1; o < 8; o <<= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+    if (lane % 8 == 0) dots[t][s] = a;
+  }
+  __syncthreads();
+  float* co = coef + (state_tile_slot(q_begin, e, i) * H + h) * ST_CO;
+  if (tid < ST_B * ST_B) {
+    const int t = tid / ST_B, s = tid % ST_B;
+    const float d = decay[h];
+    float pw[ST_B + 1];                                        // d^0 .. d^8
+    pw[0] = 1.f;
+#pragma unroll
+    for (int u = 0; u < ST_B; ++u) pw[u + 1] = pw[u] * d;
+    auto power = [&](int u) {
+      float v = 1.f;
+#pragma unroll
+      for (int x = 1; x <= ST_B; ++x) v = u == x ? pw[x] : v;
+      return v;
+    };
+    co[t * ST_ROW + s] = s == t && t < cnt ? power(cnt - 1 - t) : 0.f;
+    co[t * ST_ROW + ST_B + s] = s <= t ? power(t - s) * dots[t][s] : 0.f;
+    if (s == 0) {
+      co[t * ST_ROW + 16] = 0.f;
+      co[t * ST_ROW + 17] = 1.f;
+      co[t * ST_ROW + 18] = power(t + 1);
+      co[t * ST_ROW + 19] = power(cnt);
+    }
+  }
+}
+
+template <int R>
+__global__ void __launch_bounds__(ST_THREADS)
+lightning_tiles_kernel(const float* __restrict__ proj, long long ld, int v_off, const float* __restrict__ qk,
+                       const float* __restrict__ coef, float* __restrict__ state, long long state_stride,
+                       const int* __restrict__ qo_indptr, const int* __restrict__ state_slots, float* __restrict__ out, int H, int dim,
+                       int vdim, int act) {
+  bspec::pdl_prologue_late(65);
+  const int e = blockIdx.z, h = blockIdx.y;
+  const int q_begin = qo_indptr[e], n = qo_indptr[e + 1] - q_begin;
+  if (n <= 0) return;
+  StateTiles p;
+  p.q = qk + ((size_t)q_begin * H + h) * 2 * dim, p.k = p.q + dim;
+  p.q_stride = p.k_stride = (long long)H * 2 * dim;
+  p.v = proj + (size_t)q_begin * ld + v_off + (size_t)h * vdim, p.v_stride = ld;
+  p.coef = coef + (state_tile_slot(q_begin, e, 0) * H + h) * ST_CO, p.coef_stride = (long long)H * ST_CO;
+  p.s = state + (size_t)state_slots[e] * state_stride + (size_t)h * vdim * dim, p.s_stride = p.s_rows = dim;
+  p.out = out + (size_t)q_begin * H * vdim + (size_t)h * vdim, p.out_stride = (long long)H * vdim;
+  p.n = n, p.dim = dim, p.vdim = vdim, p.j0 = blockIdx.x * ST_COLS;
+  state_tiles<R, false>(p, [act](float x) { return act ? silu_f(x) : x; });
+}
+
+template <int R>
+int launch_lightning_tiles(dim3 grid, cudaStream_t stream, const float* proj, long long ld, int v_off, const float* qk, const float* coef,
+                           float* state, long long state_stride, const int* qo_indptr, const int* state_slots, float* out, int H,
+                           int dim, int vdim, int act) {
+  static bool set[bspec::kMaxDevices] = {};
+  bool& done = set[bspec::current_device()];
+  if (!done) {
+    const cudaError_t err = cudaFuncSetAttribute(lightning_tiles_kernel<R>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                 (int)state_tiles_smem(16 * R));
+    if (err != cudaSuccess) return (int)err;
+    done = true;
+  }
+  BSPEC_LAUNCH_SERIALIZED((lightning_tiles_kernel<R>), grid, ST_THREADS, state_tiles_smem(16 * R), stream, proj, ld, v_off, qk, coef,
+                          state, state_stride, qo_indptr, state_slots, out, H, dim, vdim, act);
+  return BSPEC_LAUNCH_CHECK();
 }
 
 // ---------------------------------------------------------------- selective scan
@@ -431,16 +556,34 @@ selective_scan_kernel(const float* __restrict__ xz, long long ld, const float* _
 }
 }  // namespace
 
+// Floats of scratch for a step of n tokens whose longest portion has max_q_len: 0 where the portions are shorter than a tile.
+BSPEC_API long long bspec_lightning_scratch(int n, int n_entries, int max_q_len, int H, int dim) {
+  return max_q_len >= ST_B ? bspec::state_tile_slots(n, n_entries) * H * ST_CO + (long long)n * H * 2 * dim : 0;
+}
+
 BSPEC_API int bspec_lightning_recurrence(const float* proj, long long ld, int q_off, int k_off, int v_off,
                                          const float* decay, float* state, long long state_stride,
-                                         const int* qo_indptr, const int* state_slots, float* out, int n_entries, int H,
-                                         int dim, int vdim, int act, float k_scale, const float* inv_freq, int rot,
-                                         const int* positions, cudaStream_t stream) {
+                                         const int* qo_indptr, const int* state_slots, float* out, int n, int n_entries,
+                                         int max_q_len, int H, int dim, int vdim, int act, float k_scale,
+                                         const float* inv_freq, int rot, const int* positions, float* scratch,
+                                         cudaStream_t stream) {
   if (n_entries <= 0) return 0;
   if (rot < 0 || rot > dim || rot % 2 || (rot > 0 && (inv_freq == nullptr || positions == nullptr)))
     return (int)cudaErrorInvalidValue;
   if (dim <= 0 || dim > 256 || vdim <= 0 || H <= 0 || H > 65535 || n_entries > 65535)
     return (int)cudaErrorInvalidValue;
+  if (scratch != nullptr) {
+    float* qk = scratch + bspec::state_tile_slots(n, n_entries) * H * ST_CO;
+    BSPEC_LAUNCH(lightning_tiles_prepare_kernel, dim3((max_q_len + ST_B - 1) / ST_B, H, n_entries), 128, 0, stream, proj, ld, q_off,
+                 k_off, decay, qo_indptr, qk, scratch, H, dim, act, k_scale, inv_freq, rot, positions);
+    const int err = BSPEC_LAUNCH_CHECK();
+    if (err != 0) return err;
+    const dim3 tiles((vdim + ST_COLS - 1) / ST_COLS, H, n_entries);
+    return dim <= 128 ? launch_lightning_tiles<8>(tiles, stream, proj, ld, v_off, qk, scratch, state, state_stride, qo_indptr,
+                                                  state_slots, out, H, dim, vdim, act)
+                      : launch_lightning_tiles<16>(tiles, stream, proj, ld, v_off, qk, scratch, state, state_stride, qo_indptr,
+                                                  state_slots, out, H, dim, vdim, act);
+  }
   const dim3 grid((vdim + LT_COLS - 1) / LT_COLS, H, n_entries);
   // few blocks (a lone prompt): 32 lanes per column, so that an SM holds 16 warps of its one block; many blocks
   // (a decode batch): 8 lanes with more rows each, and the SMs fill with blocks

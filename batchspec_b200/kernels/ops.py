@@ -51,8 +51,9 @@ _SIGNATURES = {
     "bspec_scale": [c_void_p, c_longlong, c_float, c_void_p],
     "bspec_gate_mul": [c_void_p, c_void_p, c_longlong, c_void_p, c_longlong, c_int, c_int, c_int, c_float, c_void_p],
     "bspec_lightning_recurrence": [c_void_p, c_longlong, c_int, c_int, c_int, c_void_p, c_void_p, c_longlong, c_void_p,
-                                   c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_float, c_void_p, c_int,
-                                   c_void_p, c_void_p],
+                                   c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_void_p,
+                                   c_int, c_void_p, c_void_p, c_void_p],
+    "bspec_lightning_scratch": [c_int, c_int, c_int, c_int, c_int],
     "bspec_branch_join": [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p,
                           c_float, c_void_p, c_longlong, c_int, c_int, c_void_p, c_void_p, c_float, c_void_p, c_int, c_int,
                           c_longlong, c_int, c_void_p],
@@ -77,7 +78,8 @@ _SIGNATURES = {
                             c_longlong, c_longlong, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int,
                             c_int, c_int, c_int, c_float, c_float, c_void_p],
     "bspec_delta_recurrence": [c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_longlong, c_longlong, c_void_p,
-                               c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p],
+                               c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p],
+    "bspec_delta_scratch": [c_int, c_int, c_int, c_int],
     "bspec_gated_rmsnorm": [c_void_p, c_void_p, c_longlong, c_void_p, c_int, c_void_p, c_int, c_longlong, c_int, c_int, c_int,
                             c_float, c_int, c_void_p, c_float, c_void_p],
     "bspec_state_space": [c_void_p, c_longlong, c_void_p, c_void_p, c_longlong, c_void_p, c_void_p, c_void_p, c_void_p,
@@ -197,7 +199,7 @@ def load_library(features=None):
                     raise KernelError(f"{path} has no entry point {name}")
                 continue                              # an entry point of a feature this library was built without
             fn.argtypes = argtypes
-            fn.restype = c_longlong if name in ("bspec_gemm_tc_plan", "bspec_sgemm_scratch") else c_int
+            fn.restype = c_longlong if name == "bspec_gemm_tc_plan" or name.endswith("_scratch") else c_int
         _lib, _features = lib, want
         from . import debug
         debug.apply_environment(sys.modules[__name__], lib)
@@ -999,10 +1001,16 @@ def delta_recurrence(mix: torch.Tensor, gates: torch.Tensor, proj: torch.Tensor,
     n = mix.shape[0]
     assert state.stride(0) % 4 == 0 and dim <= 256 and tail_off >= n_heads * v_dim * (-(-dim // 4) * 4)
     out = torch.empty((n, n_heads * v_dim), dtype=torch.float32, device=mix.device)
-    _check(load_library().bspec_delta_recurrence(
+    lib = load_library()
+    longest = getattr(ctx, "max_q_len", n)                    # (an upper bound will do)
+    need = lib.bspec_delta_scratch(n, ctx.n_entries, longest, n_heads)
+    scratch = torch.empty((need,), dtype=torch.float32, device=mix.device) if need else None
+    _check(lib.bspec_delta_recurrence(
         mix.data_ptr(), gates.data_ptr(), proj.data_ptr(), proj.shape[1], state.data_ptr(), state.stride(0),
-        int(tail_off), ctx.qo_indptr.data_ptr(), ctx.state_slots.data_ptr(), out.data_ptr(), ctx.n_entries, n_heads,
-        n_kv_heads, dim, v_dim, taps, _stream()), "delta_recurrence")
+        int(tail_off), ctx.qo_indptr.data_ptr(), ctx.state_slots.data_ptr(), out.data_ptr(), ctx.n_entries,
+        longest, n_heads, n_kv_heads, dim, v_dim, taps, _ptr(scratch), _stream()), "delta_recurrence")
+    if need:
+        count_launches(1)
     return out
 
 
@@ -1106,11 +1114,18 @@ def lightning_recurrence(proj: torch.Tensor, q_off: int, k_off: int, v_off: int,
     assert max(q_off, k_off) + n_heads * dim <= ld and v_off + n_heads * v_dim <= ld and activation in ("silu", None)
     assert not rotary_dim or (inv_freq.dtype == torch.float32 and inv_freq.shape == (2, rotary_dim // 2) and rotary_dim <= dim)
     out = torch.empty((n, n_heads * v_dim), dtype=torch.float32, device=proj.device)
-    _check(load_library().bspec_lightning_recurrence(
+    lib = load_library()
+    longest = getattr(ctx, "max_q_len", n)                    # (an upper bound will do)
+    need = lib.bspec_lightning_scratch(n, ctx.n_entries, longest, n_heads, dim)
+    scratch = torch.empty((need,), dtype=torch.float32, device=proj.device) if need else None
+    _check(lib.bspec_lightning_recurrence(
         proj.data_ptr(), proj.stride(0), int(q_off), int(k_off), int(v_off), decay.data_ptr(), state.data_ptr(),
-        state.stride(0), ctx.qo_indptr.data_ptr(), ctx.state_slots.data_ptr(), out.data_ptr(), ctx.n_entries, n_heads,
-        dim, v_dim, int(activation == "silu"), float(k_scale), _ptr(inv_freq) if rotary_dim else None, int(rotary_dim),
-        ctx.positions.data_ptr() if rotary_dim else None, _stream()), "lightning_recurrence")
+        state.stride(0), ctx.qo_indptr.data_ptr(), ctx.state_slots.data_ptr(), out.data_ptr(), n, ctx.n_entries, longest,
+        n_heads, dim, v_dim, int(activation == "silu"), float(k_scale), _ptr(inv_freq) if rotary_dim else None,
+        int(rotary_dim), ctx.positions.data_ptr() if rotary_dim else None, _ptr(scratch), _stream()),
+        "lightning_recurrence")
+    if need:
+        count_launches(1)
     return out
 
 

@@ -474,6 +474,50 @@ def test_delta_rule_recurrence_with_many_requests(ops, Hh, G, dk, dv, n_req):
         assert (torch.cat(got[i]).double().cpu() - want).abs().max() <= 2e-4 * max(1.0, want.abs().max().item()), i
 
 
+@pytest.mark.parametrize("lens", [[8], [7, 8], [1, 9, 16, 17], [200, 3, 64]])
+@pytest.mark.parametrize("Hh,G,dk,dv", [(2, 1, 128, 40), (3, 3, 6, 16), (4, 2, 256, 17)])
+def test_delta_rule_tiles(ops, Hh, G, dk, dv, lens):
+    """Portions with whole tiles of eight tokens, partial ones and none, keys that repeat (the tile's inverse at its largest),
+    gates at 0 and 1, two portions one after the other, against the plain recurrence; a request's last token being
+    infinite changes nothing before it."""
+    C = 2 * G * dk + Hh * dv
+    dimp = -(-dk // 4) * 4
+    gen = torch.Generator(device=DEV).manual_seed(dk + sum(lens))
+    n, E = sum(lens), len(lens)
+    state = torch.zeros(E, Hh * dv * dimp, device=DEV)
+    qo = [0] + list(np.cumsum(lens))
+    ctx = SimpleNamespace(qo_indptr=_i32(qo), n_entries=E, max_q_len=max(lens), state_slots=_i32(range(E)))
+    outs, mixes, gate = [], [], []
+    for part in range(2):
+        k = torch.randn(n, G, dk, device=DEV, generator=gen)
+        if part:
+            k[1:] = k[:1].clone()                                  # one key for all tokens
+        k /= k.norm(dim=-1, keepdim=True)
+        qv = torch.randn(n, G * dk + Hh * dv, device=DEV, generator=gen) * 0.5
+        mix = torch.cat([qv[:, :G * dk], k.reshape(n, -1), qv[:, G * dk:]], 1).contiguous()
+        gates = torch.rand(n, 2 * Hh, device=DEV, generator=gen)
+        gates[::5, :Hh], gates[1::5, :Hh], gates[2::7, Hh:], gates[3::7, Hh:] = 1.0, 0.0, 1.0, 0.0
+        before = state.clone()
+        outs.append(ops.delta_recurrence(mix, gates, mix, state, state.shape[1], ctx, Hh, G, dk, dv, 1))
+        mixes.append(mix)
+        gate.append(gates)
+        spoilt = mix.clone()
+        spoilt[[e - 1 for e in qo[1:]]] = float("inf")
+        other = ops.delta_recurrence(spoilt, gates, spoilt, before, state.shape[1], ctx, Hh, G, dk, dv, 1)
+        keep = torch.ones(n, dtype=torch.bool, device=DEV)
+        keep[[e - 1 for e in qo[1:]]] = False
+        assert torch.equal(other[keep], outs[-1][keep])
+    for e in range(E):
+        def whole(parts):
+            return torch.cat([p[qo[e]:qo[e + 1]] for p in parts]).double().cpu()
+        m, g = whole(mixes), whole(gate)
+        T = m.shape[0]
+        q, k = (m[:, a:a + G * dk].view(T, G, dk).repeat_interleave(Hh // G, dim=1) for a in (0, G * dk))
+        want = P.gated_delta_rule(q, k, m[:, 2 * G * dk:].view(T, Hh, dv), g[:, :Hh], g[:, Hh:]).reshape(T, -1)
+        # the bound of the tests above
+        assert (whole(outs) - want).abs().max() <= 2e-4 * max(1.0, want.abs().max().item()), e
+
+
 # ------------------------------------------------------------------------------------------- the engine
 
 @pytest.mark.parametrize("dtype", DTYPES)
