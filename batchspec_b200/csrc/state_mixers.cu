@@ -431,14 +431,26 @@ constexpr int SC_MAX_N = 256;
 // the recurrence runs over the current batch, and softplus and silu are taken once per batch outside the chain, so
 // what is left per token is one exponential and two multiply-adds per state.  Every token's arithmetic is the same
 // wherever it falls in a batch, so a position's result does not depend on where a portion was cut.
-template <typename T, int NPL, int LN>
+//
+// A chain of 2,048 tokens takes 605 us whatever the device has free (4,096 channels of 16 states: 32 to 128 blocks).  So
+// long portions of few requests go in segments of SC_SEG tokens, all at once: MODE 1 runs every segment from a zero state
+// and leaves its end state and the sum of its dt; scan_segments_kernel carries the state from segment to segment,
+// S <- exp(A sum dt) S + end, leaving the state before each; MODE 2 runs every segment again from there and writes the
+// outputs.  Twice the arithmetic, but on all SMs.  MODE 0: the portion from end to end.
+constexpr int SC_SEG = 64, SC_SEG_MIN = 256, SC_SEG_ENTRIES = 4;
+
+// Where segment i of entry e has its state: segments of different entries never meet.
+__device__ __forceinline__ size_t scan_segment_slot(int q_begin, int e, int i) { return (size_t)(q_begin / SC_SEG + e + i); }
+
+template <typename T, int NPL, int LN, int MODE>
 __global__ void __launch_bounds__(SC_THREADS)
 selective_scan_kernel(const float* __restrict__ xz, long long ld, const float* __restrict__ xc,
                       const float* __restrict__ dt_raw, const float* __restrict__ bc, long long ld_bc,
                       const float* __restrict__ a2t, const void* __restrict__ dvec, const void* __restrict__ dt_bias,
                       int w_dtype, float* __restrict__ state, long long state_stride, long long tail_off,
                       const int* __restrict__ qo_indptr, const int* __restrict__ state_slots, T* __restrict__ out,
-                      long long out_stride, float out_scale, int inner, int N, int taps) {
+                      long long out_stride, float out_scale, int inner, int N, int taps, float* __restrict__ part,
+                      float* __restrict__ dt_sum) {
   bspec::pdl_prologue_late(67);
   constexpr int NS = NPL * LN;                               // states this instance covers (N <= NS)
   constexpr int BCR = SC_TT * 2 * NS / SC_THREADS;           // staged B and C values per thread and batch
@@ -449,8 +461,18 @@ selective_scan_kernel(const float* __restrict__ xz, long long ld, const float* _
   const int c = blockIdx.x * (SC_THREADS / LN) + threadIdx.x / LN;
   const bool live = c < inner;
   const int cc = live ? c : 0;
-  const int t0 = qo_indptr[e], nt = qo_indptr[e + 1] - t0;
+  int t0 = qo_indptr[e], nt = qo_indptr[e + 1] - t0;
   float* sp = state + (size_t)state_slots[e] * state_stride;
+  if constexpr (MODE != 0) {
+    const int seg = blockIdx.z;
+    if (seg * SC_SEG >= nt) return;
+    const size_t slot = scan_segment_slot(t0, e, seg);
+    sp = part + slot * N * inner;
+    dt_sum += slot * inner;
+    t0 += seg * SC_SEG;
+    nt = min(SC_SEG, nt - seg * SC_SEG);
+  }
+  float total = 0.f;
   float xn[SC_TT], dn[SC_TT], zn[SC_TT], bn[BCR];
   auto fetch = [&](int base) {
     const int cnt = min(SC_TT, nt - base);
@@ -460,7 +482,7 @@ selective_scan_kernel(const float* __restrict__ xz, long long ld, const float* _
       const size_t t = (size_t)(t0 + base + tt);
       xn[tt] = xc[t * inner + cc];
       dn[tt] = dt_raw[t * inner + cc];
-      zn[tt] = xz[t * ld + inner + cc];
+      zn[tt] = MODE == 1 ? 0.f : xz[t * ld + inner + cc];
     }
 #pragma unroll
     for (int u = 0; u < BCR; ++u) {
@@ -477,7 +499,7 @@ selective_scan_kernel(const float* __restrict__ xz, long long ld, const float* _
   for (int m = 0; m < NPL; ++m) {
     const int n = lane + LN * m;
     const bool has = live && n < N;
-    s[m] = has ? sp[(size_t)n * inner + cc] : 0.f;
+    s[m] = has && MODE != 1 ? sp[(size_t)n * inner + cc] : 0.f;
     a2[m] = has ? a2t[(size_t)n * inner + cc] : 0.f;
   }
   const float dskip = load_as_f32(dvec, w_dtype, cc), dtb = load_as_f32(dt_bias, w_dtype, cc);
@@ -495,7 +517,8 @@ selective_scan_kernel(const float* __restrict__ xz, long long ld, const float* _
       if (tt >= cnt) break;
       xv[tt] = xn[tt];
       dv[tt] = softplus_f(dn[tt] + dtb);
-      gv[tt] = silu_f(zn[tt]) * out_scale;
+      if (MODE != 1) gv[tt] = silu_f(zn[tt]) * out_scale;
+      if (MODE == 1) total += dv[tt];
     }
     __syncthreads();
     if (base + SC_TT < nt) fetch(base + SC_TT);
@@ -526,7 +549,7 @@ selective_scan_kernel(const float* __restrict__ xz, long long ld, const float* _
       }
 #pragma unroll
       for (int o = 1; o < LN; o <<= 1) y += __shfl_xor_sync(0xffffffffu, y, o);
-      if (live && lane == 0)
+      if (MODE != 1 && live && lane == 0)
         out[(size_t)(t0 + base + tt) * out_stride + cc] = from_f32<T>(__fmul_rn(__fmaf_rn(dskip, xt, y), gt));
     };
     if (cnt == SC_TT) {
@@ -539,18 +562,62 @@ selective_scan_kernel(const float* __restrict__ xz, long long ld, const float* _
     }
   }
   bspec::pdl_launch_dependents();
-  if (!live) return;
+  if (!live || MODE == 2) return;
 #pragma unroll
   for (int m = 0; m < NPL; ++m) {
     const int n = lane + LN * m;
     if (n < N) sp[(size_t)n * inner + cc] = s[m];
   }
-  if (lane == 0) {
+  if (MODE == 1 && lane == 0) dt_sum[cc] = total;
+  if (MODE == 0 && lane == 0) {
     // the convolution's last taps-1 inputs, oldest first: rows of this portion, and before them what the state held
     float* tail = sp + tail_off;
     for (int u = 0; u < taps - 1; ++u) {
       const int rel = nt - (taps - 1) + u;
       tail[(size_t)u * inner + cc] = rel >= 0 ? xz[(size_t)(t0 + rel) * ld + cc] : tail[(size_t)(u + nt) * inner + cc];
+    }
+  }
+}
+
+// One thread per (channel, state): the state carried over the portion's segments; part[segment] takes the state before it.
+// The blocks of state 0 also keep the convolution's last taps - 1 inputs.
+__global__ void __launch_bounds__(128)
+scan_segments_kernel(const float* __restrict__ xz, long long ld, const float* __restrict__ a2t, float* __restrict__ state,
+                     long long state_stride, long long tail_off, const int* __restrict__ qo_indptr,
+                     const int* __restrict__ state_slots, int inner, int N, int taps, float* __restrict__ part,
+                     const float* __restrict__ dt_sum) {
+  bspec::pdl_prologue(67);
+  const int e = blockIdx.z, n = blockIdx.y, c = blockIdx.x * 128 + threadIdx.x;
+  const int t0 = qo_indptr[e], nt = qo_indptr[e + 1] - t0;
+  if (c >= inner || nt <= 0) return;
+  float* sp = state + (size_t)state_slots[e] * state_stride;
+  const int segs = (nt + SC_SEG - 1) / SC_SEG;
+  const size_t first = scan_segment_slot(t0, e, 0), step = (size_t)N * inner;
+  float* pp = part + first * step + (size_t)n * inner + c;
+  const float* dp = dt_sum + first * inner + c;
+  const float a2 = a2t[(size_t)n * inner + c];
+  float s = sp[(size_t)n * inner + c];
+  for (int i0 = 0; i0 < segs; i0 += 8) {                       // eight segments' numbers asked for at a time
+    float end[8], dts[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      const bool ok = i0 + u < segs;
+      end[u] = ok ? pp[(i0 + u) * step] : 0.f;
+      dts[u] = ok ? dp[(size_t)(i0 + u) * inner] : 0.f;
+    }
+#pragma unroll
+    for (int u = 0; u < 8; ++u)
+      if (i0 + u < segs) {
+        pp[(i0 + u) * step] = s;
+        s = scan_update(s, __fmul_rn(dts[u], a2), end[u]);
+      }
+  }
+  sp[(size_t)n * inner + c] = s;
+  if (n == 0) {
+    float* tail = sp + tail_off;
+    for (int u = 0; u < taps - 1; ++u) {
+      const int rel = nt - (taps - 1) + u;
+      tail[(size_t)u * inner + c] = rel >= 0 ? xz[(size_t)(t0 + rel) * ld + c] : tail[(size_t)(u + nt) * inner + c];
     }
   }
 }
@@ -633,21 +700,41 @@ BSPEC_API int bspec_scan_conv(const float* xz, long long ld, const void* conv, c
   return BSPEC_LAUNCH_CHECK();
 }
 
+// Floats of scratch for a step of n tokens: 0 where the portions go from end to end.  In segments where the longest chain is
+// long and the requests are so few that twice the arithmetic spread over the device takes less time than that chain (one
+// request of 2,048 tokens about a fifth of its time; it grows with the requests, the chain does not).
+BSPEC_API long long bspec_scan_scratch(int n, int n_entries, int max_q_len, int inner, int N) {
+  if (max_q_len < SC_SEG_MIN || n_entries > SC_SEG_ENTRIES || N > 65535) return 0;
+  return (long long)(n / SC_SEG + n_entries + 1) * (N + 1) * inner;
+}
+
 BSPEC_API int bspec_selective_scan(const float* xz, long long ld, const float* xc, const float* dt_raw, const float* bc,
                                    long long ld_bc, const float* a2t, const void* dvec, const void* dt_bias,
                                    int w_dtype, float* state, long long state_stride, long long tail_off,
                                    const int* qo_indptr, const int* state_slots, void* out, int out_dtype,
-                                   long long out_stride, float out_scale, int n_entries, int inner, int N, int taps,
-                                   cudaStream_t stream) {
+                                   long long out_stride, float out_scale, int n, int n_entries, int max_q_len, int inner,
+                                   int N, int taps, float* scratch, cudaStream_t stream) {
   if (n_entries <= 0) return 0;
   if (inner <= 0 || N <= 0 || N > SC_MAX_N || taps < 1 || n_entries > 65535) return (int)cudaErrorInvalidValue;
   // few channels x requests: more lanes per channel, so that a lone prompt's chain is shorter and more SMs take part
-  const bool few = (long long)((inner + SC_THREADS - 1) / SC_THREADS) * n_entries < 148;
+  const bool few = scratch == nullptr && (long long)((inner + SC_THREADS - 1) / SC_THREADS) * n_entries < 148;
+  const int segs = scratch != nullptr ? (max_q_len + SC_SEG - 1) / SC_SEG : 1;
+  if (segs > 65535) return (int)cudaErrorInvalidConfiguration;
+  float* dt_sum = scratch != nullptr ? scratch + (size_t)(n / SC_SEG + n_entries + 1) * N * inner : nullptr;
+#define LSM(T, NPL, LN, MODE)                                                                                        \
+  BSPEC_LAUNCH_SERIALIZED((selective_scan_kernel<T, NPL, LN, MODE>),                                                 \
+                          dim3((inner + SC_THREADS / LN - 1) / (SC_THREADS / LN), n_entries, segs), SC_THREADS, 0,   \
+                          stream, xz, ld, xc, dt_raw, bc, ld_bc, a2t, dvec, dt_bias, w_dtype, state, state_stride,   \
+                          tail_off, qo_indptr, state_slots, (T*)out, out_stride, out_scale, inner, N, taps, scratch, \
+                          dt_sum)
 #define LS(T, NPL, LN)                                                                                               \
-  BSPEC_LAUNCH_SERIALIZED((selective_scan_kernel<T, NPL, LN>),                                                       \
-                          dim3((inner + SC_THREADS / LN - 1) / (SC_THREADS / LN), n_entries), SC_THREADS, 0, stream, \
-                          xz, ld, xc, dt_raw, bc, ld_bc, a2t, dvec, dt_bias, w_dtype, state, state_stride, tail_off, \
-                          qo_indptr, state_slots, (T*)out, out_stride, out_scale, inner, N, taps)
+  do {                                                                                                               \
+    if (scratch == nullptr) { LSM(T, NPL, LN, 0); break; }                                                           \
+    LSM(float, NPL, LN, 1);                                                                                          \
+    BSPEC_LAUNCH(scan_segments_kernel, dim3((inner + 127) / 128, N, n_entries), 128, 0, stream, xz, ld, a2t, state,  \
+                 state_stride, tail_off, qo_indptr, state_slots, inner, N, taps, scratch, dt_sum);                   \
+    LSM(T, NPL, LN, 2);                                                                                              \
+  } while (0)
 #define LSN(T)                                                                                                       \
   do {                                                                                                               \
     if (few) {                                                                                                       \
@@ -661,6 +748,7 @@ BSPEC_API int bspec_selective_scan(const float* xz, long long ld, const float* x
   if (out_dtype == BSPEC_F32) LSN(float); else LSN(__nv_bfloat16);
 #undef LSN
 #undef LS
+#undef LSM
   return BSPEC_LAUNCH_CHECK();
 }
 

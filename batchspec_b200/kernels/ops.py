@@ -63,7 +63,8 @@ _SIGNATURES = {
                         c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p],
     "bspec_selective_scan": [c_void_p, c_longlong, c_void_p, c_void_p, c_void_p, c_longlong, c_void_p, c_void_p,
                              c_void_p, c_int, c_void_p, c_longlong, c_longlong, c_void_p, c_void_p, c_void_p, c_int,
-                             c_longlong, c_float, c_int, c_int, c_int, c_int, c_void_p],
+                             c_longlong, c_float, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p],
+    "bspec_scan_scratch": [c_int, c_int, c_int, c_int, c_int],
     "bspec_silu_mul": [c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p],
     "bspec_relu_mul": [c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p],
     "bspec_qkv_prepare": [c_void_p, c_longlong, c_int, c_int, c_int, c_int, c_int, c_void_p, c_int, c_void_p, c_int, c_int, c_float,
@@ -1181,11 +1182,18 @@ def selective_scan(xz: torch.Tensor, xc: torch.Tensor, dt_raw: torch.Tensor, bc:
     assert d_skip.dtype == dt_bias.dtype and d_skip.numel() == dt_bias.numel() == inner
     assert state.dtype == f32 and tail_off >= n_state * inner and tail_off + (taps - 1) * inner <= state.shape[1]
     assert out.shape == (n, inner) and out.stride(1) == 1
-    _check(load_library().bspec_selective_scan(
+    lib = load_library()
+    longest = getattr(ctx, "max_q_len", n)                    # (an upper bound will do)
+    need = lib.bspec_scan_scratch(n, ctx.n_entries, longest, inner, n_state)
+    scratch = torch.empty((need,), dtype=f32, device=xz.device) if need else None
+    _check(lib.bspec_selective_scan(
         xz.data_ptr(), xz.stride(0), xc.data_ptr(), dt_raw.data_ptr(), bc.data_ptr(), bc.stride(0),
         decay_table.data_ptr(), d_skip.data_ptr(), dt_bias.data_ptr(), _dtype_code(d_skip.dtype), state.data_ptr(), state.stride(0),
         int(tail_off), ctx.qo_indptr.data_ptr(), ctx.state_slots.data_ptr(), out.data_ptr(), _dtype_code(out.dtype),
-        out.stride(0), float(out_scale), ctx.n_entries, inner, n_state, taps, _stream()), "selective_scan")
+        out.stride(0), float(out_scale), n, ctx.n_entries, longest, inner, n_state, taps, _ptr(scratch), _stream()),
+        "selective_scan")
+    if need:
+        count_launches(2)
 
 
 # ---------------------------------------------------------------------------- matrix products

@@ -591,6 +591,42 @@ def test_interleaved_rotation_and_append_from_wider_rows(ops, dtype, Hq, G, hd, 
     assert int((cache != 0).sum()) <= n * entry
 
 
+@pytest.mark.parametrize("lens", [[256], [255, 257, 1, 64], [1000, 3]])
+@pytest.mark.parametrize("inner,N,taps", [(64, 16, 4), (130, 5, 1), (33, 40, 3)])
+def test_selective_scan_in_segments(ops, inner, N, taps, lens):
+    """Portions long enough to run in segments at once (whole ones, partial ones, requests of a token beside them), from a
+    state that is not zero, against the recurrence in float64; states and the convolution's inputs are left as the
+    end-to-end form leaves them."""
+    gen = torch.Generator(device=DEV).manual_seed(inner + sum(lens))
+    n, E = sum(lens), len(lens)
+    rand = lambda *shape: torch.randn(*shape, device=DEV, generator=gen)
+    xz, xc, dt_raw, bc = rand(n, 2 * inner + 3), rand(n, inner), rand(n, inner) - 2, rand(n, 2 * N)
+    a_log, d_skip, dt_bias = rand(inner, N), rand(inner), rand(inner)
+    tail_off = N * inner
+    state = rand(E + 1, tail_off + (taps - 1) * inner)
+    before = state.clone()
+    slots = list(range(E, 0, -1))
+    qo = [0] + list(np.cumsum(lens))
+    out = torch.empty(n, inner, device=DEV)
+    ctx = SimpleNamespace(qo_indptr=_i32(qo), n_entries=E, max_q_len=max(lens), state_slots=_i32(slots))
+    ops.selective_scan(xz, xc, dt_raw, bc, a_log, d_skip, dt_bias, state, tail_off, ctx, out, 0.5, inner, N, taps)
+    assert torch.equal(state[0], before[0])
+    for e in range(E):
+        rows = slice(qo[e], qo[e + 1])
+        x, z, b = xc[rows].double(), xz[rows, inner:2 * inner].double(), bc[rows].double()
+        dt = torch.nn.functional.softplus(dt_raw[rows].double() + dt_bias.double(), threshold=60)
+        A, S = -torch.exp(a_log.double()), before[slots[e], :tail_off].view(N, inner).t().double()
+        want = torch.empty(lens[e], inner, device=DEV, dtype=torch.float64)
+        for t in range(lens[e]):
+            S = torch.exp(dt[t, :, None] * A) * S + (dt[t] * x[t])[:, None] * b[t, None, :N]
+            want[t] = (S @ b[t, N:] + d_skip.double() * x[t]) * torch.nn.functional.silu(z[t]) * 0.5
+        assert (out[rows].double() - want).abs().max() <= 2e-5 * max(1.0, want.abs().max().item()), e
+        got = state[slots[e], :tail_off].view(N, inner).t().double()
+        assert (got - S).abs().max() <= 2e-5 * max(1.0, S.abs().max().item()), e
+        kept = torch.cat([before[slots[e], tail_off:].view(taps - 1, inner), xz[rows, :inner]])[lens[e]:]
+        assert torch.equal(state[slots[e], tail_off:].view(taps - 1, inner), kept), e
+
+
 # ------------------------------------------------------------------------------------------- whole models
 
 @pytest.mark.parametrize("dtype", DTYPES)
