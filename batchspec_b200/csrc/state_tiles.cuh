@@ -41,8 +41,8 @@ struct StateTiles {
 // The sums lie in rows of 16 floats without padding: the half warps write to different halves of the banks (row t ^ g), the
 // quads of a row are turned by the row's number, so that neither the writes nor the 16-byte reads collide.  Tokens are
 // staged 16 at a time, the next stage under the current one.  2,048 tokens of 16 heads of 128 x 128 on a B200, with the
-// preparation: 341 us (delta rule; 753 us for it beside two shorter requests before, 515 us now) and 339 us (lightning
-// attention; 553 us before).  Eight warps of two columns each took 333 us alone but 544 us beside the two.
+// preparation: 261 us (delta rule; 435 us beside requests of 333 and 826 tokens, 753 us token by token) and 263 us (lightning
+// attention; 553 us).  Eight warps of two columns each took as long alone and a tenth more beside the two.
 template <int R, bool RK, typename Act>
 __device__ __forceinline__ void state_tiles(const StateTiles& p, Act act) {
   constexpr int NT = ST_THREADS, DP = 16 * R;
@@ -63,8 +63,35 @@ __device__ __forceinline__ void state_tiles(const StateTiles& p, Act act) {
   }
   // rows of q and k start on 16-byte boundaries
   const bool vec = ((dim | (int)p.q_stride | (int)p.k_stride) & 3) == 0 && (((uintptr_t)p.q | (uintptr_t)p.k) & 15) == 0;
+  // this thread's first copies of a whole stage: token warp of q and k, token tid / 16 of v, a quad of the coefficients
+  const float *q_src = p.q + warp * p.q_stride + 4 * lane, *k_src = p.k + warp * p.k_stride + 4 * lane;
+  const int v_tok = tid / ST_COLS, v_col = p.j0 + tid % ST_COLS;
+  const float* v_src = p.v + v_tok * p.v_stride + v_col;
+  const int c_half = tid / (ST_CO / 4), c_off = tid % (ST_CO / 4) * 4;
   auto stage = [&](int t0, int buf) {                          // tokens t0 .. t0 + STAGE - 1 of the portion, zeros past its end
     const int nt = min(ST_STAGE, n - t0);
+    if (vec && nt == ST_STAGE) {                               // (the general form below took a sixth of the kernel's time)
+      const float *qr = q_src + t0 * p.q_stride, *kr = k_src + t0 * p.k_stride, *vr = v_src + t0 * p.v_stride;
+      float *qd = qs + (buf * ST_STAGE + warp) * DP + 4 * lane, *kd = ks + (buf * ST_STAGE + warp) * DP + 4 * lane;
+#pragma unroll
+      for (int i = 0; i < ST_STAGE / (NT / 32); ++i)
+#pragma unroll
+        for (int d = 0; d < DP; d += 128)
+          if (d + 4 * lane < dim) {
+            __pipeline_memcpy_async(qd + i * (NT / 32) * DP + d, qr + i * (NT / 32) * p.q_stride + d, 16);
+            __pipeline_memcpy_async(kd + i * (NT / 32) * DP + d, kr + i * (NT / 32) * p.k_stride + d, 16);
+          }
+#pragma unroll
+      for (int i = 0; i < ST_STAGE * ST_COLS / NT; ++i) {
+        float* vd = vs + buf * ST_STAGE * ST_COLS + tid + i * NT;
+        if (v_col < p.vdim) __pipeline_memcpy_async(vd, vr + i * (NT / ST_COLS) * p.v_stride, 4);
+        else *vd = 0.f;
+      }
+      if (c_half < ST_STAGE / ST_B)
+        __pipeline_memcpy_async(cs + (buf * (ST_STAGE / ST_B) + c_half) * ST_CO + c_off, p.coef + (t0 / ST_B + c_half) * p.coef_stride + c_off, 16);
+      __pipeline_commit();
+      return;
+    }
     for (int tt = warp; tt < ST_STAGE; tt += NT / 32) {
       const float *qr = p.q + (t0 + min(tt, nt - 1)) * p.q_stride, *kr = p.k + (t0 + min(tt, nt - 1)) * p.k_stride;
       float *qd = qs + (buf * ST_STAGE + tt) * DP, *kd = ks + (buf * ST_STAGE + tt) * DP;
@@ -122,7 +149,7 @@ __device__ __forceinline__ void state_tiles(const StateTiles& p, Act act) {
     __pipeline_wait_prior(0);
     __syncthreads();                                           // the stage is there, and every thread is done with the other half
     if (t0 + ST_STAGE < n) stage(t0 + ST_STAGE, buf ^ 1);
-#pragma unroll 1
+#pragma unroll
     for (int half = 0; half < ST_STAGE / ST_B && t0 + half * ST_B < n; ++half) {
       const float* kt = ks + (buf * ST_STAGE + half * ST_B) * DP + 4 * r16;
       const float* qt = qs + (buf * ST_STAGE + half * ST_B) * DP + 4 * r16;
