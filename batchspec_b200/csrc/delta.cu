@@ -90,6 +90,77 @@ delta_prepare_kernel(const float* __restrict__ proj, int ld, int b_off, int a_of
   }
 }
 
+// The same for four taps and heads of up to 128 numbers that start on 16-byte boundaries: a lane holds four channels of the
+// warp's head with their weights, and the inputs of TT consecutive tokens and the three before them, so that an input is
+// read once for four uses.  Bound by memory: 3,207 tokens of 4,096 channels 92 -> 46 us, 2,048 of them 74 -> 45 us on a B200
+// (the bytes need 16 and 10).
+template <int TT>
+__global__ void __launch_bounds__(DP_WARPS * 32)
+delta_prepare4_kernel(const float* __restrict__ proj, int n, int ld, int b_off, int a_off, const void* __restrict__ conv,
+                      const void* __restrict__ a_log, const void* __restrict__ dt_bias, int w_dtype,
+                      const float* __restrict__ state, long long state_stride, long long tail_off,
+                      const int* __restrict__ qo_indptr, const int* __restrict__ tok_entry,
+                      const int* __restrict__ state_slots, float* __restrict__ mix, float* __restrict__ gates, int H,
+                      int Gk, int dim, int vdim, float q_scale, float unit_eps) {
+  bspec::pdl_prologue(60);
+  const int t0 = blockIdx.x * TT, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (blockIdx.y == 0) {
+    for (int x = threadIdx.x; x < min(TT, n - t0) * H; x += blockDim.x) {
+      const int t = t0 + x / H, h = x % H;
+      const float b = proj[(size_t)t * ld + b_off + h], a = proj[(size_t)t * ld + a_off + h];
+      gates[(size_t)t * 2 * H + h] = 1.f / (1.f + expf(-b));
+      const float rate = expf(load_as_f32(a_log, w_dtype, h)) * softplus_f(a + load_as_f32(dt_bias, w_dtype, h));
+      gates[(size_t)t * 2 * H + H + h] = expf(-rate);
+    }
+  }
+  const int slot = blockIdx.y * DP_WARPS + warp;
+  if (slot >= 2 * Gk + H) return;
+  const bool is_v = slot >= 2 * Gk;
+  const int C = 2 * Gk * dim + H * vdim;
+  const int c = (is_v ? 2 * Gk * dim + (slot - 2 * Gk) * vdim : slot * dim) + 4 * lane;
+  const bool on = 4 * lane < (is_v ? vdim : dim);
+  float w[4][4], x[TT + 3][4];                     // x[u]: the input of token t0 + u - 3
+  auto row4 = [](const float* p, float (&f)[4]) {
+    const float4 v = *reinterpret_cast<const float4*>(p);
+    f[0] = v.x; f[1] = v.y; f[2] = v.z; f[3] = v.w;
+  };
+#pragma unroll
+  for (int u = 0; u < TT + 3; ++u) {
+    const int t = t0 + u - 3;
+    x[u][0] = x[u][1] = x[u][2] = x[u][3] = 0.f;
+    if (on && t >= 0 && t < n) row4(proj + (size_t)t * ld + c, x[u]);
+  }
+#pragma unroll
+  for (int q = 0; q < 4; ++q)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) w[q][j] = on ? load_as_f32(conv, w_dtype, (size_t)(c + q) * 4 + j) : 0.f;
+#pragma unroll
+  for (int u = 0; u < TT; ++u) {
+    const int t = t0 + u;
+    if (t >= n) break;
+    const int e = tok_entry[t], i = t - qo_indptr[e];
+    float y[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {                  // oldest input first
+      float v[4] = {x[u + j][0], x[u + j][1], x[u + j][2], x[u + j][3]};
+      if (i < 3 - j) {
+        v[0] = v[1] = v[2] = v[3] = 0.f;
+        if (on) row4(state + (size_t)state_slots[e] * state_stride + tail_off + (size_t)(i + j) * C + c, v);
+      }
+#pragma unroll
+      for (int q = 0; q < 4; ++q) y[q] += w[q][j] * v[q];
+    }
+#pragma unroll
+    for (int q = 0; q < 4; ++q) y[q] = silu_f(y[q]);
+    float r = 1.f;
+    if (!is_v) {
+      const float ss = warp_sum(y[0] * y[0] + y[1] * y[1] + y[2] * y[2] + y[3] * y[3]);
+      r = (slot < Gk ? q_scale : 1.f) / sqrtf(ss + unit_eps);
+    }
+    if (on) *reinterpret_cast<float4*>(mix + (size_t)t * C + c) = make_float4(y[0] * r, y[1] * r, y[2] * r, y[3] * r);
+  }
+}
+
 // LANES: lanes that share one column of S; R: floats of the column that one lane holds (a multiple of 4, dim <=
 // LANES R); COLS: value columns of a block.  Lane r holds rows 4 LANES c + 4 r + {0..3} for c < R / 4, so that the
 // lanes of a column read contiguous bytes of state at a time.  Many short columns per block (LANES 4, COLS 32) when
@@ -536,6 +607,15 @@ BSPEC_API int bspec_delta_prepare(const float* proj, int n, int ld, int b_off, i
   if (dim > 256) return (int)cudaErrorInvalidValue;
   const dim3 grid(n, (2 * Gk + H + DP_WARPS - 1) / DP_WARPS);
   if (grid.y > 65535) return (int)cudaErrorInvalidConfiguration;
+  // Eight tokens per warp where that leaves two blocks an SM; fewer tokens (decode steps) keep a warp per token and head.
+  if (taps == 4 && dim <= 128 && vdim <= 128 && ((dim | vdim | ld) & 3) == 0 && ((state_stride | tail_off) & 3) == 0 &&
+      ((reinterpret_cast<uintptr_t>(proj) | reinterpret_cast<uintptr_t>(state) | reinterpret_cast<uintptr_t>(mix)) & 15) == 0 &&
+      (long long)(n / 8) * grid.y >= 2ll * bspec::sm_count()) {
+    BSPEC_LAUNCH((delta_prepare4_kernel<8>), dim3((n + 7) / 8, grid.y), DP_WARPS * 32, 0, stream, proj, n, ld, b_off, a_off, conv,
+                 a_log, dt_bias, w_dtype, state, state_stride, tail_off, qo_indptr, tok_entry, state_slots, mix, gates, H, Gk, dim,
+                 vdim, q_scale, unit_eps);
+    return BSPEC_LAUNCH_CHECK();
+  }
   BSPEC_LAUNCH(delta_prepare_kernel, grid, DP_WARPS * 32, 0, stream, proj, ld, b_off, a_off, conv, a_log, dt_bias, w_dtype,
                state, state_stride, tail_off, qo_indptr, tok_entry, state_slots, mix, gates, H, Gk, dim, vdim, taps,
                q_scale, unit_eps);

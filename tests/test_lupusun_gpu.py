@@ -474,6 +474,40 @@ def test_delta_rule_recurrence_with_many_requests(ops, Hh, G, dk, dv, n_req):
         assert (torch.cat(got[i]).double().cpu() - want).abs().max() <= 2e-4 * max(1.0, want.abs().max().item()), i
 
 
+@pytest.mark.parametrize("Hh,G,dk,dv", [(16, 8, 128, 64), (8, 4, 36, 100)])
+def test_delta_prepare_takes_tokens_eight_at_a_time(ops, Hh, G, dk, dv):
+    """Enough tokens that a warp takes eight of them, requests of 1 to 60 that begin anywhere in the eight, against the plain
+    convolution after the state's inputs, and against every request alone (a warp per token)."""
+    taps, C = 4, 2 * G * dk + Hh * dv
+    ld = C + 2 * Hh
+    gen = torch.Generator(device=DEV).manual_seed(dk)
+    lens = [1 + (11 * i) % 60 for i in range(40)]
+    n, E = sum(lens), len(lens)
+    assert (n // 8) * -(-(2 * G + Hh) // 4) >= 2 * ops.sm_count()
+    proj, conv = torch.randn(n, ld, device=DEV, generator=gen), torch.randn(C, taps, device=DEV, generator=gen)
+    a_log, dt_bias = torch.randn(Hh, device=DEV, generator=gen), torch.randn(Hh, device=DEV, generator=gen)
+    state = torch.randn(E, (taps - 1) * C, device=DEV, generator=gen)
+    qo = [0] + list(np.cumsum(lens))
+
+    def run(first, last):
+        ctx = SimpleNamespace(qo_indptr=_i32([q - qo[first] for q in qo[first:last + 1]]), n_entries=last - first,
+                              tok_entry=torch.cat([torch.full((k,), i) for i, k in enumerate(lens[first:last])]).to(DEV, torch.int32),
+                              state_slots=_i32(range(first, last)))
+        return ops.delta_prepare(proj[qo[first]:qo[last]].contiguous(), C, C + Hh, conv, a_log, dt_bias, state, 0, ctx, Hh, G, dk, dv,
+                                 taps, dk ** -0.5, 1e-6)
+    mix, gates = run(0, E)
+    for e in (0, 1, 7, 20, E - 1):
+        m, g = run(e, e + 1)
+        rows = slice(qo[e], qo[e + 1])
+        assert torch.equal(g, gates[rows])
+        x = torch.cat([state[e].view(taps - 1, C), proj[rows, :C]]).double().cpu()
+        y = P.silu(P.short_conv(x, conv.double().cpu())[taps - 1:])
+        q, k = (P.unit(y[:, i * G * dk:(i + 1) * G * dk].reshape(-1, G, dk)).reshape(-1, G * dk) for i in (0, 1))
+        want = torch.cat([q * dk ** -0.5, k, y[:, 2 * G * dk:]], 1)
+        for got in (m, mix[rows]):
+            assert (got.double().cpu() - want).abs().max() <= 2e-6 * max(1.0, want.abs().max().item())
+
+
 @pytest.mark.parametrize("lens", [[8], [7, 8], [1, 9, 16, 17], [200, 3, 64]])
 @pytest.mark.parametrize("Hh,G,dk,dv", [(2, 1, 128, 40), (3, 3, 6, 16), (4, 2, 256, 17)])
 def test_delta_rule_tiles(ops, Hh, G, dk, dv, lens):
