@@ -54,16 +54,20 @@ __device__ __forceinline__ void mma_bf16(float (&d)[4], const uint32_t (&a)[4], 
                : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
-__host__ __device__ inline size_t smem_bytes(int D, int BM, int stages = 2) {
+// ``shares``: score tiles in shared memory, 1 or (kernels that divide the numbers of an entry) one per warp of a row group.
+__host__ __device__ inline size_t smem_bytes(int D, int BM, int stages = 2, int shares = 1) {
   const int DP = D + 8;
-  return (size_t)(BM + stages * BN) * DP * 2 + (size_t)BM * (BN + 8) * 4 + 2 * (size_t)BM * (BN + 8) * 2 + 3 * BM * 4;
+  return (size_t)(BM + stages * BN) * DP * 2 + (size_t)shares * BM * (BN + 8) * 4 + 2 * (size_t)BM * (BN + 8) * 2 + 3 * BM * 4;
 }
 
 // RG row groups x CH column groups of warps; NT: n-tiles (of 8 columns) of the output one warp may own,
 // R / (8 CH) <= NT.
 // ST: tiles of entries in shared memory: 2 (the next one arrives under the current one's products) or 1 (two CTAs
 // share an SM instead and cover each other's loads).
-template <int RG, int CH, int NT, int ST = 2>
+// DS: the CH warps of a row group divide the numbers of an entry between them instead of the keys.  A warp then multiplies
+// all 32 keys of the tile with a CH-th of the R + P numbers, 3 fragment loads for 4 products instead of 2 for 1, and leaves
+// a share of the scores that the softmax adds up in the warps' order.
+template <int RG, int CH, int NT, int ST = 2, bool DS = false>
 __global__ void __launch_bounds__(32 * RG * CH)
 latent_attn_mma_kernel(const __nv_bfloat16* __restrict__ ql, long long ql_row, long long ql_head,
                        const __nv_bfloat16* __restrict__ qr, long long qr_row, long long qr_head,
@@ -84,7 +88,7 @@ latent_attn_mma_kernel(const __nv_bfloat16* __restrict__ ql, long long ql_row, l
   __nv_bfloat16* Qs = reinterpret_cast<__nv_bfloat16*>(smem_raw);
   __nv_bfloat16* Ks = Qs + (size_t)BM * DP;
   float* Ss = reinterpret_cast<float*>(Ks + (size_t)ST * BN * DP);
-  __nv_bfloat16* Ph = reinterpret_cast<__nv_bfloat16*>(Ss + (size_t)BM * SP);
+  __nv_bfloat16* Ph = reinterpret_cast<__nv_bfloat16*>(Ss + (size_t)(DS ? CH : 1) * BM * SP);
   __nv_bfloat16* Pl = Ph + (size_t)BM * PP;
   float* row_m = reinterpret_cast<float*>(Pl + (size_t)BM * PP);
   float* row_l = row_m + BM;
@@ -200,6 +204,8 @@ latent_attn_mma_kernel(const __nv_bfloat16* __restrict__ ql, long long ql_row, l
   const uint32_t qa_s = smem_addr(Qs + (size_t)(16 * rg + 8 * (mat & 1) + r8) * DP + 8 * (mat >> 1));
   const uint32_t kb_s = KW == 16 ? smem_addr(Ks + (size_t)(KW * ch + 8 * (mat >> 1) + r8) * DP + 8 * (mat & 1))
                                  : smem_addr(Ks + (size_t)(KW * ch + r8) * DP + 8 * (mat & 1));
+  // DS: both halves of the tile's keys, 16 rows apart
+  const uint32_t kd_s = smem_addr(Ks + (size_t)(8 * (mat >> 1) + r8) * DP + 8 * (mat & 1));
   const uint32_t ph_s = smem_addr(Ph + (size_t)(16 * rg + 8 * (mat & 1) + r8) * PP + 8 * (mat >> 1));
   const uint32_t pl_s = smem_addr(Pl + (size_t)(16 * rg + 8 * (mat & 1) + r8) * PP + 8 * (mat >> 1));
   const uint32_t vt_s = smem_addr(Ks + (size_t)(8 * (mat & 1) + r8) * DP + col0 + 8 * (mat >> 1));
@@ -211,6 +217,11 @@ latent_attn_mma_kernel(const __nv_bfloat16* __restrict__ ql, long long ql_row, l
     row_pos[half] = row < rows_total ? pos0 + (int)(row / H) : -1;
     row_lo[half] = window > 0 ? row_pos[half] - window + 1 : 0;         // the first key the row sees
   }
+
+  // the same for this thread's softmax row
+  const long long soft_row = row0 + srow;
+  const int soft_pos = soft_row < rows_total ? pos0 + (int)(soft_row / H) : -1;
+  const int soft_lo = window > 0 ? soft_pos - window + 1 : 0;
 
   long long ahead = lookup(t_begin);
   if (t_begin < t_end) load_tile(0, ahead);
@@ -225,8 +236,43 @@ latent_attn_mma_kernel(const __nv_bfloat16* __restrict__ ql, long long ql_row, l
       cp_async_commit();
       ahead = lookup(tile + 2);
     }
-    // ---- S: this warp's 16 rows x KW keys, two accumulator sets over alternating k steps
-    {
+    if constexpr (DS) {
+      // ---- S: this warp's 16 rows x 32 keys over its share of the numbers, fragments fetched one k step ahead
+      float s[4][4];
+#pragma unroll
+      for (int y = 0; y < 4; ++y) s[y][0] = s[y][1] = s[y][2] = s[y][3] = 0.f;
+      const uint32_t kb = kd_s + (uint32_t)buf * (uint32_t)(BN * DP * 2);
+      const int nks = D / 16, k_begin = nks * ch / CH, k_end = nks * (ch + 1) / CH;
+      uint32_t fa[2][4], f0[2][4], f1[2][4];
+      auto fetch = [&](int slot, int k) {
+        ldsm_x4(fa[slot], qa_s + 32u * k);
+        ldsm_x4(f0[slot], kb + 32u * k);
+        ldsm_x4(f1[slot], kb + 32u * k + (uint32_t)(16 * DP * 2));
+      };
+      auto mul = [&](int slot) {
+        mma_bf16(s[0], fa[slot], f0[slot][0], f0[slot][1]);
+        mma_bf16(s[1], fa[slot], f0[slot][2], f0[slot][3]);
+        mma_bf16(s[2], fa[slot], f1[slot][0], f1[slot][1]);
+        mma_bf16(s[3], fa[slot], f1[slot][2], f1[slot][3]);
+      };
+      if (k_begin < k_end) fetch(0, k_begin);
+      int k = k_begin;
+      for (; k + 2 <= k_end; k += 2) {
+        fetch(1, k + 1);
+        mul(0);
+        if (k + 2 < k_end) fetch(0, k + 2);
+        mul(1);
+      }
+      if (k < k_end) mul(0);
+      float* share = Ss + (size_t)ch * BM * SP;
+#pragma unroll
+      for (int nt = 0; nt < 4; ++nt)
+#pragma unroll
+        for (int half = 0; half < 2; ++half)
+          *reinterpret_cast<float2*>(share + (16 * rg + qrow + 8 * half) * SP + 8 * nt + qcol) =
+              make_float2(s[nt][2 * half], s[nt][2 * half + 1]);
+    } else {
+      // ---- S: this warp's 16 rows x KW keys, two accumulator sets over alternating k steps
       constexpr int NS = KW / 8;
       float s[4][NS][4];
 #pragma unroll
@@ -300,6 +346,20 @@ latent_attn_mma_kernel(const __nv_bfloat16* __restrict__ ql, long long ql_row, l
       for (int j = 0; j < KPT; j += 4) {
         const float4 x = *reinterpret_cast<const float4*>(Ss + srow * SP + KPT * spart + j);
         v[j] = x.x; v[j + 1] = x.y; v[j + 2] = x.z; v[j + 3] = x.w;
+      }
+      if constexpr (DS) {                          // the other shares, then scale and mask
+#pragma unroll
+        for (int w = 1; w < CH; ++w)
+#pragma unroll
+          for (int j = 0; j < KPT; j += 4) {
+            const float4 x = *reinterpret_cast<const float4*>(Ss + (size_t)w * BM * SP + srow * SP + KPT * spart + j);
+            v[j] += x.x; v[j + 1] += x.y; v[j + 2] += x.z; v[j + 3] += x.w;
+          }
+#pragma unroll
+        for (int j = 0; j < KPT; ++j) {
+          const int key = tile * BN + KPT * spart + j;
+          v[j] = key <= soft_pos && key >= soft_lo ? v[j] * scale : -INFINITY;
+        }
       }
 #pragma unroll
       for (int j = 0; j < KPT; ++j) mx = fmaxf(mx, v[j]);
@@ -533,7 +593,12 @@ BSPEC_API int bspec_latent_attention_mma(const void* ql, long long ql_row, long 
   if ((long long)max_q_len * H > 2147483647ll || n_entries > 65535 || n_splits > 64) return (int)cudaErrorInvalidConfiguration;
   dim3 grid((unsigned)row_tiles, n_entries, n_splits);
   const bool one_stage = small_pair || (BM < 64 && decode_stages() == 1);
-  const size_t smem = smem_bytes(R + P, BM, one_stage ? 1 : 2);
+  // Shares of the numbers of an entry on 16-row tiles, where as many CTAs still share an SM with the larger score tiles (a
+  // decode step of 64 requests through four layers, 16 heads, latent 512 + 64: 769 -> 738 us).  With 32 rows, prompt
+  // portions, the warps wait for the products rather than for their operands: 2,048 tokens 4.17 -> 4.77 ms.
+  auto per_sm = [](size_t bytes) { return (int)((227 * 1024) / (bytes + 1024)); };
+  const bool divide = one_stage && BM == 16 && min(4, per_sm(smem_bytes(R + P, BM, 1, 4))) >= min(4, per_sm(smem_bytes(R + P, BM, 1)));
+  const size_t smem = smem_bytes(R + P, BM, one_stage ? 1 : 2, divide ? 4 : 1);
 #define LM(RG, CH, N)                                                                                                \
   do {                                                                                                               \
     cudaFuncSetAttribute(latent_attn_mma_kernel<RG, CH, N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
@@ -542,14 +607,15 @@ BSPEC_API int bspec_latent_attention_mma(const void* ql, long long ql_row, long 
                  (const __nv_bfloat16*)cache, qo_indptr, positions, kv_indptr, kv_indices, H, R, P, page_size,       \
                  scale, n_splits, o_part, ml_part, n_pages, inv_freq, magnitude, window, sink); \
   } while (0)
-#define LM1(RG, CH, N)                                                                                               \
+#define LMS(RG, CH, N, DS)                                                                                           \
   do {                                                                                                               \
-    cudaFuncSetAttribute(latent_attn_mma_kernel<RG, CH, N, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
-    BSPEC_LAUNCH((latent_attn_mma_kernel<RG, CH, N, 1>), grid, 32 * RG * CH, smem, stream, (const __nv_bfloat16*)ql, \
+    cudaFuncSetAttribute(latent_attn_mma_kernel<RG, CH, N, 1, DS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
+    BSPEC_LAUNCH((latent_attn_mma_kernel<RG, CH, N, 1, DS>), grid, 32 * RG * CH, smem, stream, (const __nv_bfloat16*)ql, \
                  ql_row, ql_head, (const __nv_bfloat16*)qr, qr_row, qr_head, (__nv_bfloat16*)out, o_row, o_head,     \
                  (const __nv_bfloat16*)cache, qo_indptr, positions, kv_indptr, kv_indices, H, R, P, page_size,       \
                  scale, n_splits, o_part, ml_part, n_pages, inv_freq, magnitude, window, sink); \
   } while (0)
+#define LM1(RG, CH, N) LMS(RG, CH, N, false)
   if (small_pair) {
     const int ntw = R / 32;
     if (ntw <= 4) LM1(2, 4, 4); else if (ntw <= 8) LM1(2, 4, 8); else LM1(2, 4, 16);
@@ -562,7 +628,8 @@ BSPEC_API int bspec_latent_attention_mma(const void* ql, long long ql_row, long 
     if (ntw <= 8) LM(4, 2, 8); else if (ntw <= 16) LM(4, 2, 16); else LM(4, 2, 32);
   } else if (one_stage) {
     const int ntw = R / 32;
-    if (BM == 16) { if (ntw <= 4) LM1(1, 4, 4); else if (ntw <= 8) LM1(1, 4, 8); else LM1(1, 4, 16); }
+    if (BM == 16 && divide) { if (ntw <= 4) LMS(1, 4, 4, true); else if (ntw <= 8) LMS(1, 4, 8, true); else LMS(1, 4, 16, true); }
+    else if (BM == 16) { if (ntw <= 4) LM1(1, 4, 4); else if (ntw <= 8) LM1(1, 4, 8); else LM1(1, 4, 16); }
     else { if (ntw <= 4) LM1(2, 4, 4); else if (ntw <= 8) LM1(2, 4, 8); else LM1(2, 4, 16); }
   } else {
     const int ntw = R / 32;
@@ -570,6 +637,7 @@ BSPEC_API int bspec_latent_attention_mma(const void* ql, long long ql_row, long 
     else { if (ntw <= 4) LM(2, 4, 4); else if (ntw <= 8) LM(2, 4, 8); else LM(2, 4, 16); }
   }
 #undef LM1
+#undef LMS
 #undef LM
   int err = BSPEC_LAUNCH_CHECK();
   if (err != 0 || n_splits == 1) return err;
