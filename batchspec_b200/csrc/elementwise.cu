@@ -692,6 +692,26 @@ BSPEC_API int bspec_relu_squared(void* x, int dtype, long long total, cudaStream
 }
 
 // ---------------------------------------------------------------- soft cap in place:  cap * tanh(x / cap)
+// Bound by memory: four quads per thread are on their way before the first is worked on (a number at a time took 148 us
+// for 2,048 x 32,000, where the bytes need 80; whole scoring passes of that size are 61 us shorter).  Lengths and pointers that
+// are no whole quads take the kernel of single numbers.
+__global__ void __launch_bounds__(256)
+tanh_softcap_vec_kernel(float4* __restrict__ x, size_t quads, float cap) {
+  bspec::pdl_prologue(17);
+  const size_t step = (size_t)gridDim.x * 256;
+  for (size_t i = (size_t)blockIdx.x * 256 + threadIdx.x; i < quads; i += 4 * step) {
+    float4 v[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+      if (i + u * step < quads) v[u] = x[i + u * step];
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+      if (i + u * step < quads)
+        x[i + u * step] = make_float4(cap * tanhf(v[u].x / cap), cap * tanhf(v[u].y / cap), cap * tanhf(v[u].z / cap),
+                                      cap * tanhf(v[u].w / cap));
+  }
+}
+
 __global__ void tanh_softcap_kernel(float* __restrict__ x, size_t total, float cap) {
   bspec::pdl_prologue(17);
   for (size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x; idx < total; idx += (size_t)gridDim.x * blockDim.x)
@@ -701,8 +721,14 @@ __global__ void tanh_softcap_kernel(float* __restrict__ x, size_t total, float c
 BSPEC_API int bspec_tanh_softcap(float* x, long long total, float cap, cudaStream_t stream) {
   if (total <= 0) return 0;
   const int threads = 256;
-  size_t want = ((size_t)total + threads - 1) / threads;
   const size_t cap_blocks = (size_t)bspec::sm_count() * 32;
+  if (total % 4 == 0 && ((uintptr_t)x & 15) == 0) {
+    const size_t want = ((size_t)total / 4 + threads - 1) / threads;
+    BSPEC_LAUNCH((tanh_softcap_vec_kernel), (int)(want > cap_blocks ? cap_blocks : want), threads, 0, stream, (float4*)x,
+                 (size_t)total / 4, cap);
+    return BSPEC_LAUNCH_CHECK();
+  }
+  size_t want = ((size_t)total + threads - 1) / threads;
   BSPEC_LAUNCH((tanh_softcap_kernel), (int)(want > cap_blocks ? cap_blocks : want), threads, 0, stream, x, (size_t)total, cap);
   return BSPEC_LAUNCH_CHECK();
 }

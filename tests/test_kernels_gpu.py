@@ -117,6 +117,20 @@ def test_sgemm_sums_have_one_order_in_every_kernel(ops, N, K, batch):
     ops.check_status()
 
 
+@pytest.mark.parametrize("total", [4, 1028, 148 * 32 * 256 * 4 + 4, 148 * 32 * 256 * 20 + 8])
+def test_tanh_softcap_in_quads_and_one_by_one(ops, total):
+    """Four numbers at a time, less and more than a thread's four quads, against the kernel of single numbers, which takes
+    what begins off a 16-byte boundary."""
+    x = torch.randn(total + 1, device=DEV, generator=torch.Generator(device=DEV).manual_seed(total % 97)) * 90
+    quads, single = x[:total].clone(), x.clone()
+    single[1:].copy_(x[:total])
+    ops.tanh_softcap_(quads, 30.0)
+    ops.tanh_softcap_(single[1:], 30.0)
+    assert torch.equal(quads, single[1:]) and single[0] == x[0]
+    # tanhf (2 units), the quotient, the product
+    assert (quads.double() - 30.0 * torch.tanh(x[:total].double() / 30.0)).abs().max() <= 30.0 * 2.0 ** -21
+
+
 def _rope_reference(x, pos, inv_freq, rot, interleaved):
     """float64 angle from the float32 frequencies given, float32 result."""
     ang = pos.double()[:, None] * inv_freq.double()[None, :]
