@@ -9,9 +9,9 @@
 //                     scale), beta = sigmoid(b), g = exp(-exp(A_log) softplus(a + dt_bias))
 //   delta_recurrence  per (request, head, 32 or 8 value columns): the token loop over the portion with the state in
 //                     registers (a column of S is spread over four or sixteen lanes), state read at the start and
-//                     written at the end; the request's blocks also move the convolutions' inputs on.  Steps with a
-//                     portion of eight tokens or more take delta_tiles_prepare and delta_tiles instead, which
-//                     multiply the rule out over tiles
+//                     written at the end; the request's blocks also move the convolutions' inputs on.  Long portions
+//                     (ST_FROM tokens and more) take delta_tiles_prepare and delta_tiles instead, which multiply the
+//                     rule out over tiles of eight tokens
 //   gated_rmsnorm     per (token, head): o / rms(o) * w * silu(gate), with options other mixers use
 //
 // The order of every sum depends on the sizes alone, not on how a request was cut into portions or on what else is
@@ -168,14 +168,14 @@ delta_prepare4_kernel(const float* __restrict__ proj, int n, int ld, int b_off, 
 // lanes and a block holds 8 columns, which makes four times as many warps with dependent chains a quarter as long.  Per token both read-outs are taken from the state before the write,
 //     a = S^T k,  b = S^T q,  u = beta (v - g a),  o = g b + u (k . q),  S <- g S + k u^T,
 // which is the rule above with o = (g S + k u^T)^T q multiplied out: one pass over the registers for the three sums
-// (reduced over the column's lanes together), one for the update.  The next tile of tokens is copied into the other half
-// of the staging buffers while the current one is worked on.
+// (reduced over the column's lanes together), one for the update.  The 16-lane form takes two tokens per pass.  The next tile of
+// tokens is copied into the other half of the staging buffers while the current one is worked on.
 template <int R, int COLS, int LANES>
 __global__ void __launch_bounds__(COLS * LANES)
 delta_recurrence_kernel(const float* __restrict__ mix, const float* __restrict__ gates, const float* __restrict__ proj,
                         int ld, float* __restrict__ state, long long state_stride, long long tail_off,
                         const int* __restrict__ qo_indptr, const int* __restrict__ state_slots,
-                        float* __restrict__ out, int H, int Gk, int dim, int vdim, int taps) {
+                        float* __restrict__ out, int H, int Gk, int dim, int vdim, int taps, int below) {
   bspec::pdl_prologue_late(61);
   constexpr int NT = COLS * LANES, DP = LANES * R;
   constexpr int TILE = DP > 128 ? 8 : 16;          // tokens whose q, k, v, beta, g are staged in shared memory at a time
@@ -184,11 +184,12 @@ delta_recurrence_kernel(const float* __restrict__ mix, const float* __restrict__
   __shared__ __align__(16) float ks[2][TILE][DP];
   __shared__ float vs[2][TILE][COLS];
   __shared__ float bg[2][TILE][2];
+  __shared__ float sc[TILE / 2][4];                // products between the two tokens of every pair of the tile
   const int e = blockIdx.z, h = blockIdx.y;
   const int q_begin = qo_indptr[e], n = qo_indptr[e + 1] - q_begin;
   const int C = 2 * Gk * dim + H * vdim;
   float* srow = state + (size_t)state_slots[e] * state_stride;
-  if (n <= 0) return;
+  if (n <= 0 || n >= below) return;                // nothing, or the portion goes by tiles
   if (taps > 1) {
     // the convolutions' inputs: slot s holds the input at index n + s - (taps - 1) of this portion, or what an
     // older slot held; ascending s, so that a slot is read before it is overwritten.  The request's blocks share
@@ -294,10 +295,84 @@ delta_recurrence_kernel(const float* __restrict__ mix, const float* __restrict__
         qd[c] = *reinterpret_cast<const float4*>(&qs[buf][tt][row]);
       }
     };
-    for (int tt = 0; tt < nt; ++tt) {
-      float4 kr[R / 4], qr[R / 4];
-      fetch(tt, kr, qr);
-      one_token(tt, kr, qr);
+    if constexpr (LANES == 16) {
+      // The long chain of one prompt: two tokens per pass.  With a = S^T k and b = S^T q of BOTH tokens taken from
+      // the state before either write, and the tokens' mutual products (the same for every column, formed once
+      // per tile below),
+      //   u1 = beta1 (v1 - g1 a1)                    o1 = g1 b1 + u1 (k1.q1)
+      //   u2 = beta2 (v2 - g2 (g1 a2 + u1 (k1.k2)))  o2 = g2 (g1 b2 + u1 (k1.q2)) + u2 (k2.q2)
+      //   S <- g1 g2 S + g2 u1 k1 + u2 k2,
+      // which is the rule applied twice, multiplied out: one round of reductions and one pass over the registers
+      // for two tokens.
+      {
+        const int pr = min((int)(threadIdx.x >> 4), TILE / 2 - 1), sub = threadIdx.x & 15;
+        const float *k1 = ks[buf][2 * pr], *q1 = qs[buf][2 * pr], *k2 = ks[buf][2 * pr + 1], *q2 = qs[buf][2 * pr + 1];
+        float x0 = 0.f, x1 = 0.f, x2 = 0.f, x3 = 0.f;
+        for (int d = sub; d < dimp; d += 16) {
+          x0 += k1[d] * q1[d]; x1 += k1[d] * k2[d]; x2 += k1[d] * q2[d]; x3 += k2[d] * q2[d];
+        }
+#pragma unroll
+        for (int o = 1; o < 16; o <<= 1) {
+          x0 += __shfl_xor_sync(0xffffffffu, x0, o); x1 += __shfl_xor_sync(0xffffffffu, x1, o);
+          x2 += __shfl_xor_sync(0xffffffffu, x2, o); x3 += __shfl_xor_sync(0xffffffffu, x3, o);
+        }
+        if (sub == 0 && (int)(threadIdx.x >> 4) < TILE / 2 && 2 * pr + 1 < nt) {
+          sc[pr][0] = x0; sc[pr][1] = x1; sc[pr][2] = x2; sc[pr][3] = x3;
+        }
+      }
+      __syncthreads();
+      const int np = nt >> 1;
+      float4 k1n[R / 4], q1n[R / 4], k2n[R / 4], q2n[R / 4];
+      if (np > 0) { fetch(0, k1n, q1n); fetch(1, k2n, q2n); }
+      for (int pp = 0; pp < np; ++pp) {
+        float4 k1[R / 4], q1[R / 4], k2[R / 4], q2[R / 4];
+#pragma unroll
+        for (int c = 0; c < R / 4; ++c) { k1[c] = k1n[c]; q1[c] = q1n[c]; k2[c] = k2n[c]; q2[c] = q2n[c]; }
+        const int t1 = 2 * pp, t2 = 2 * pp + 1;
+        const float beta1 = bg[buf][t1][0], g1 = bg[buf][t1][1], v1 = vs[buf][t1][col];
+        const float beta2 = bg[buf][t2][0], g2 = bg[buf][t2][1], v2 = vs[buf][t2][col];
+        const float kq11 = sc[pp][0], kk12 = sc[pp][1], kq12 = sc[pp][2], kq22 = sc[pp][3];
+        float a1 = 0.f, b1 = 0.f, a2 = 0.f, b2 = 0.f;
+#pragma unroll
+        for (int c = 0; c < R / 4; ++c) {
+          a1 += s[4 * c] * k1[c].x; a1 += s[4 * c + 1] * k1[c].y; a1 += s[4 * c + 2] * k1[c].z; a1 += s[4 * c + 3] * k1[c].w;
+          b1 += s[4 * c] * q1[c].x; b1 += s[4 * c + 1] * q1[c].y; b1 += s[4 * c + 2] * q1[c].z; b1 += s[4 * c + 3] * q1[c].w;
+          a2 += s[4 * c] * k2[c].x; a2 += s[4 * c + 1] * k2[c].y; a2 += s[4 * c + 2] * k2[c].z; a2 += s[4 * c + 3] * k2[c].w;
+          b2 += s[4 * c] * q2[c].x; b2 += s[4 * c + 1] * q2[c].y; b2 += s[4 * c + 2] * q2[c].z; b2 += s[4 * c + 3] * q2[c].w;
+        }
+        if (pp + 1 < np) { fetch(2 * pp + 2, k1n, q1n); fetch(2 * pp + 3, k2n, q2n); }
+#pragma unroll
+        for (int o = 1; o < LANES; o <<= 1) {
+          a1 += __shfl_xor_sync(0xffffffffu, a1, o); b1 += __shfl_xor_sync(0xffffffffu, b1, o);
+          a2 += __shfl_xor_sync(0xffffffffu, a2, o); b2 += __shfl_xor_sync(0xffffffffu, b2, o);
+        }
+        const float u1 = beta1 * (v1 - g1 * a1);
+        const float u2 = beta2 * (v2 - g2 * (g1 * a2 + u1 * kk12));
+        if (live && r == 0) {
+          float* op = out + (size_t)(q_begin + t0 + t1) * H * vdim + h * vdim + j;
+          op[0] = g1 * b1 + u1 * kq11;
+          op[(size_t)H * vdim] = g2 * (g1 * b2 + u1 * kq12) + u2 * kq22;
+        }
+        const float c0 = g1 * g2, c1 = g2 * u1;
+#pragma unroll
+        for (int c = 0; c < R / 4; ++c) {
+          s[4 * c] = fmaf(k2[c].x, u2, fmaf(k1[c].x, c1, c0 * s[4 * c]));
+          s[4 * c + 1] = fmaf(k2[c].y, u2, fmaf(k1[c].y, c1, c0 * s[4 * c + 1]));
+          s[4 * c + 2] = fmaf(k2[c].z, u2, fmaf(k1[c].z, c1, c0 * s[4 * c + 2]));
+          s[4 * c + 3] = fmaf(k2[c].w, u2, fmaf(k1[c].w, c1, c0 * s[4 * c + 3]));
+        }
+      }
+      if (nt & 1) {                                 // the portion's last token
+        float4 kr[R / 4], qr[R / 4];
+        fetch(nt - 1, kr, qr);
+        one_token(nt - 1, kr, qr);
+      }
+    } else {
+      for (int tt = 0; tt < nt; ++tt) {
+        float4 kr[R / 4], qr[R / 4];
+        fetch(tt, kr, qr);
+        one_token(tt, kr, qr);
+      }
     }
   }
   bspec::pdl_launch_dependents();
@@ -330,7 +405,7 @@ delta_tiles_prepare_kernel(const float* __restrict__ mix, const float* __restric
   __shared__ float dots[ST_B][ST_B], y[ST_B][ST_B], be[ST_B], g[ST_B], low[ST_B][ST_B], inv[ST_B][ST_B];
   const int i = blockIdx.x, h = blockIdx.y, e = blockIdx.z;
   const int q_begin = qo_indptr[e], n = qo_indptr[e + 1] - q_begin;
-  if (i * ST_B >= n) return;
+  if (n < ST_FROM || i * ST_B >= n) return;
   const int cnt = min(ST_B, n - i * ST_B), C = 2 * Gk * dim + H * vdim, kh = h / (H / Gk);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 #pragma unroll
@@ -409,7 +484,7 @@ delta_tiles_kernel(const float* __restrict__ mix, const float* __restrict__ proj
   const int q_begin = qo_indptr[e], n = qo_indptr[e + 1] - q_begin;
   const int C = 2 * Gk * dim + H * vdim;
   float* srow = state + (size_t)state_slots[e] * state_stride;
-  if (n <= 0) return;
+  if (n < ST_FROM) return;
   if (taps > 1) {                                              // as in delta_recurrence_kernel
     float* tail = srow + tail_off;
     const int share = blockIdx.y * gridDim.x + blockIdx.x, shares = gridDim.y * gridDim.x;
@@ -622,15 +697,15 @@ BSPEC_API int bspec_delta_prepare(const float* proj, int n, int ld, int b_off, i
   return BSPEC_LAUNCH_CHECK();
 }
 
-// Floats of scratch for a step of n tokens whose longest portion has max_q_len: the tiles' coefficients, or 0 where the
-// portions are shorter than a tile and go token by token.
+// Floats of scratch for a step of n tokens whose longest portion has max_q_len: the tiles' coefficients, or 0 where no
+// portion goes by tiles.
 BSPEC_API long long bspec_delta_scratch(int n, int n_entries, int max_q_len, int H) {
-  return max_q_len >= ST_B ? bspec::state_tile_slots(n, n_entries) * H * ST_CO : 0;
+  return max_q_len >= ST_FROM ? bspec::state_tile_slots(n, n_entries) * H * ST_CO : 0;
 }
 
 BSPEC_API int bspec_delta_recurrence(const float* mix, const float* gates, const float* proj, int ld, float* state,
                                      long long state_stride, long long tail_off, const int* qo_indptr,
-                                     const int* state_slots, float* out, int n_entries, int max_q_len, int H, int Gk,
+                                     const int* state_slots, float* out, int n_entries, int min_q_len, int max_q_len, int H, int Gk,
                                      int dim, int vdim, int taps, float* scratch, cudaStream_t stream) {
   if (n_entries <= 0) return 0;
   if (dim <= 0 || dim > MAX_DIM || H % Gk != 0 || n_entries > 65535 || H > 65535)
@@ -641,11 +716,13 @@ BSPEC_API int bspec_delta_recurrence(const float* mix, const float* gates, const
     const int err = BSPEC_LAUNCH_CHECK();
     if (err != 0) return err;
     const dim3 tiles((vdim + ST_COLS - 1) / ST_COLS, H, n_entries);
-    return dim <= 128 ? launch_delta_tiles<8>(tiles, stream, mix, proj, scratch, ld, state, state_stride, tail_off, qo_indptr,
+    const int tiled = dim <= 128 ? launch_delta_tiles<8>(tiles, stream, mix, proj, scratch, ld, state, state_stride, tail_off, qo_indptr,
                                               state_slots, out, H, Gk, dim, vdim, taps)
                       : launch_delta_tiles<16>(tiles, stream, mix, proj, scratch, ld, state, state_stride, tail_off, qo_indptr,
                                               state_slots, out, H, Gk, dim, vdim, taps);
+    if (tiled != 0 || min_q_len >= ST_FROM) return tiled;
   }
+  const int below = scratch != nullptr ? ST_FROM : 0x7fffffff;           // the portions left for the token loop
   // 32 value columns of 4 lanes per block; 8 columns of 16 lanes when that would leave most of the device idle
   const bool narrow = (long long)((vdim + 31) / 32) * H * n_entries < 2ll * bspec::sm_count();
   const int cols = narrow ? 8 : 32;
@@ -654,10 +731,10 @@ BSPEC_API int bspec_delta_recurrence(const float* mix, const float* gates, const
   do {                                                                                                             \
     if (narrow)                                                                                                    \
       BSPEC_LAUNCH_SERIALIZED((delta_recurrence_kernel<R16, 8, 16>), grid, 8 * 16, 0, stream, mix, gates, proj, ld, state, \
-                   state_stride, tail_off, qo_indptr, state_slots, out, H, Gk, dim, vdim, taps);                   \
+                   state_stride, tail_off, qo_indptr, state_slots, out, H, Gk, dim, vdim, taps, below);            \
     else                                                                                                           \
       BSPEC_LAUNCH_SERIALIZED((delta_recurrence_kernel<R4, 32, 4>), grid, 32 * 4, 0, stream, mix, gates, proj, ld, state,     \
-                   state_stride, tail_off, qo_indptr, state_slots, out, H, Gk, dim, vdim, taps);                   \
+                   state_stride, tail_off, qo_indptr, state_slots, out, H, Gk, dim, vdim, taps, below);            \
   } while (0)
   if (dim <= 32) LR(8, 4); else if (dim <= 64) LR(16, 4); else if (dim <= 128) LR(32, 8); else LR(64, 16);
 #undef LR

@@ -63,7 +63,7 @@ lightning_recurrence_kernel(const float* __restrict__ proj, long long ld, int q_
                             const float* __restrict__ decay, float* __restrict__ state, long long state_stride,
                             const int* __restrict__ qo_indptr, const int* __restrict__ state_slots,
                             float* __restrict__ out, int H, int dim, int vdim, int act, float k_scale,
-                            const float* __restrict__ inv_freq, int rot, const int* __restrict__ positions) {
+                            const float* __restrict__ inv_freq, int rot, const int* __restrict__ positions, int below) {
   bspec::pdl_prologue_late(65);
   constexpr int LT_THREADS = LT_COLS * L;
   constexpr int DM = L * NR;                                // rows of S this instance holds (dim <= DM)
@@ -77,6 +77,7 @@ lightning_recurrence_kernel(const float* __restrict__ proj, long long ld, int q_
   const int j = blockIdx.x * LT_COLS + col;                 // value column of the head
   const bool live = j < vdim;
   const int t0 = qo_indptr[e], nt = qo_indptr[e + 1] - t0;
+  if (nt >= below) return;                                  // the portion goes by tiles
   const float d = decay[h];
   float* sp = state + (size_t)state_slots[e] * state_stride + ((size_t)h * vdim + (live ? j : 0)) * dim;
   float qn[NR], kn[NR], vn[VR];
@@ -230,7 +231,7 @@ lightning_tiles_prepare_kernel(const float* __restrict__ proj, long long ld, int
   __shared__ float qs[ST_B][264], ks[ST_B][264], dots[ST_B][ST_B];      // (rows eight banks apart)
   const int i = blockIdx.x, h = blockIdx.y, e = blockIdx.z;
   const int q_begin = qo_indptr[e], n = qo_indptr[e + 1] - q_begin;
-  if (i * ST_B >= n) return;
+  if (n < ST_FROM || i * ST_B >= n) return;
   const int cnt = min(ST_B, n - i * ST_B), t0 = q_begin + i * ST_B;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 #pragma unroll
@@ -312,7 +313,7 @@ lightning_tiles_kernel(const float* __restrict__ proj, long long ld, int v_off, 
   bspec::pdl_prologue_late(65);
   const int e = blockIdx.z, h = blockIdx.y;
   const int q_begin = qo_indptr[e], n = qo_indptr[e + 1] - q_begin;
-  if (n <= 0) return;
+  if (n < ST_FROM) return;
   StateTiles p;
   p.q = qk + ((size_t)q_begin * H + h) * 2 * dim, p.k = p.q + dim;
   p.q_stride = p.k_stride = (long long)H * 2 * dim;
@@ -437,7 +438,7 @@ constexpr int SC_MAX_N = 256;
 // and leaves its end state and the sum of its dt; scan_segments_kernel carries the state from segment to segment,
 // S <- exp(A sum dt) S + end, leaving the state before each; MODE 2 runs every segment again from there and writes the
 // outputs.  Twice the arithmetic, but on all SMs.  MODE 0: the portion from end to end.
-constexpr int SC_SEG = 64, SC_SEG_MIN = 256, SC_SEG_ENTRIES = 4;
+constexpr int SC_SEG = 64, SC_SEG_MIN = 512, SC_SEG_ENTRIES = 4, SC_SEG_MAX_N = 32;
 
 // Where segment i of entry e has its state: segments of different entries never meet.
 __device__ __forceinline__ size_t scan_segment_slot(int q_begin, int e, int i) { return (size_t)(q_begin / SC_SEG + e + i); }
@@ -623,15 +624,15 @@ scan_segments_kernel(const float* __restrict__ xz, long long ld, const float* __
 }
 }  // namespace
 
-// Floats of scratch for a step of n tokens whose longest portion has max_q_len: 0 where the portions are shorter than a tile.
+// Floats of scratch for a step of n tokens whose longest portion has max_q_len: 0 where none goes by tiles.
 BSPEC_API long long bspec_lightning_scratch(int n, int n_entries, int max_q_len, int H, int dim) {
-  return max_q_len >= ST_B ? bspec::state_tile_slots(n, n_entries) * H * ST_CO + (long long)n * H * 2 * dim : 0;
+  return max_q_len >= ST_FROM ? bspec::state_tile_slots(n, n_entries) * H * ST_CO + (long long)n * H * 2 * dim : 0;
 }
 
 BSPEC_API int bspec_lightning_recurrence(const float* proj, long long ld, int q_off, int k_off, int v_off,
                                          const float* decay, float* state, long long state_stride,
                                          const int* qo_indptr, const int* state_slots, float* out, int n, int n_entries,
-                                         int max_q_len, int H, int dim, int vdim, int act, float k_scale,
+                                         int min_q_len, int max_q_len, int H, int dim, int vdim, int act, float k_scale,
                                          const float* inv_freq, int rot, const int* positions, float* scratch,
                                          cudaStream_t stream) {
   if (n_entries <= 0) return 0;
@@ -646,11 +647,13 @@ BSPEC_API int bspec_lightning_recurrence(const float* proj, long long ld, int q_
     const int err = BSPEC_LAUNCH_CHECK();
     if (err != 0) return err;
     const dim3 tiles((vdim + ST_COLS - 1) / ST_COLS, H, n_entries);
-    return dim <= 128 ? launch_lightning_tiles<8>(tiles, stream, proj, ld, v_off, qk, scratch, state, state_stride, qo_indptr,
+    const int tiled = dim <= 128 ? launch_lightning_tiles<8>(tiles, stream, proj, ld, v_off, qk, scratch, state, state_stride, qo_indptr,
                                                   state_slots, out, H, dim, vdim, act)
                       : launch_lightning_tiles<16>(tiles, stream, proj, ld, v_off, qk, scratch, state, state_stride, qo_indptr,
                                                   state_slots, out, H, dim, vdim, act);
+    if (tiled != 0 || min_q_len >= ST_FROM) return tiled;
   }
+  const int below = scratch != nullptr ? ST_FROM : 0x7fffffff;           // the portions left for the token loop
   const dim3 grid((vdim + LT_COLS - 1) / LT_COLS, H, n_entries);
   // few blocks (a lone prompt): 32 lanes per column, so that an SM holds 16 warps of its one block; many blocks
   // (a decode batch): 8 lanes with more rows each, and the SMs fill with blocks
@@ -658,7 +661,7 @@ BSPEC_API int bspec_lightning_recurrence(const float* proj, long long ld, int q_
 #define LL(NR, L)                                                                                                  \
   BSPEC_LAUNCH_SERIALIZED((lightning_recurrence_kernel<NR, L>), grid, LT_COLS * L, 0, stream, proj, ld, q_off,     \
                           k_off, v_off, decay, state, state_stride, qo_indptr, state_slots, out, H, dim, vdim, act,   \
-                          k_scale, inv_freq, rot, positions)
+                          k_scale, inv_freq, rot, positions, below)
   if (dim <= 32) LL(4, 8);
   else if (dim <= 64) { if (few) LL(4, 16); else LL(8, 8); }
   else if (dim <= 128) { if (few) LL(4, 32); else LL(16, 8); }
@@ -701,10 +704,11 @@ BSPEC_API int bspec_scan_conv(const float* xz, long long ld, const void* conv, c
 }
 
 // Floats of scratch for a step of n tokens: 0 where the portions go from end to end.  In segments where the longest chain is
-// long and the requests are so few that twice the arithmetic spread over the device takes less time than that chain (one
-// request of 2,048 tokens about a fifth of its time; it grows with the requests, the chain does not).
+// long and the requests are so few that twice the arithmetic spread over the device takes less time than that chain.
+// Measured with 4,096 channels of 16 states, end to end / in segments, us: 1 x 256 tokens 83 / 91, 4 x 300 169 / 176,
+// 1 x 2,048 609 / 259.  More than 32 states spread over several lanes of a channel and go from end to end.
 BSPEC_API long long bspec_scan_scratch(int n, int n_entries, int max_q_len, int inner, int N) {
-  if (max_q_len < SC_SEG_MIN || n_entries > SC_SEG_ENTRIES || N > 65535) return 0;
+  if (max_q_len < SC_SEG_MIN || n_entries > SC_SEG_ENTRIES || N > SC_SEG_MAX_N) return 0;
   return (long long)(n / SC_SEG + n_entries + 1) * (N + 1) * inner;
 }
 
@@ -727,17 +731,19 @@ BSPEC_API int bspec_selective_scan(const float* xz, long long ld, const float* x
                           stream, xz, ld, xc, dt_raw, bc, ld_bc, a2t, dvec, dt_bias, w_dtype, state, state_stride,   \
                           tail_off, qo_indptr, state_slots, (T*)out, out_stride, out_scale, inner, N, taps, scratch, \
                           dt_sum)
-#define LS(T, NPL, LN)                                                                                               \
+#define LS(T, NPL, LN) LSM(T, NPL, LN, 0)
+#define LSS(T, NPL)                                                                                                  \
   do {                                                                                                               \
-    if (scratch == nullptr) { LSM(T, NPL, LN, 0); break; }                                                           \
-    LSM(float, NPL, LN, 1);                                                                                          \
+    LSM(float, NPL, 1, 1);                                                                                           \
     BSPEC_LAUNCH(scan_segments_kernel, dim3((inner + 127) / 128, N, n_entries), 128, 0, stream, xz, ld, a2t, state,  \
                  state_stride, tail_off, qo_indptr, state_slots, inner, N, taps, scratch, dt_sum);                   \
-    LSM(T, NPL, LN, 2);                                                                                              \
+    LSM(T, NPL, 1, 2);                                                                                               \
   } while (0)
 #define LSN(T)                                                                                                       \
   do {                                                                                                               \
-    if (few) {                                                                                                       \
+    if (scratch != nullptr) {                                                                                        \
+      if (N <= 16) LSS(T, 16); else LSS(T, 32);                                                                      \
+    } else if (few) {                                                                                                       \
       if (N <= 16) LS(T, 4, 4); else if (N <= 32) LS(T, 8, 4); else if (N <= 64) LS(T, 8, 8);                        \
       else if (N <= 128) LS(T, 16, 8); else LS(T, 32, 8);                                                            \
     } else {                                                                                                         \
@@ -748,6 +754,7 @@ BSPEC_API int bspec_selective_scan(const float* xz, long long ld, const float* x
   if (out_dtype == BSPEC_F32) LSN(float); else LSN(__nv_bfloat16);
 #undef LSN
 #undef LS
+#undef LSS
 #undef LSM
   return BSPEC_LAUNCH_CHECK();
 }

@@ -11,6 +11,11 @@ namespace bspec {
 
 // tokens of a tile; floats of a token's row of coefficients [F_t 8 | P_t 8 | d_t, e_t, c_t, c_B]; floats of a tile's
 constexpr int ST_B = 8, ST_ROW = 20, ST_CO = ST_B * ST_ROW;
+// A step's portions of at least ST_FROM tokens go by tiles, the others token by token.  Measured with 16 heads of 128 x 128, by
+// tokens / by tiles with the preparation, us: delta rule 4 x 8 tokens 15 / 19, 128 x 9 135 / 245, 64 x 16 107 / 118,
+// 1 x 64 23.5 / 21.3, 32 x 64 183 / 177, 1 x 256 75 / 44, 8 x 2,048 1,559 / 1,263; lightning attention 4 x 8 13 / 22, 128 x 9
+// 170 / 232, 64 x 16 135 / 116, 1 x 64 22.5 / 23.3, 32 x 64 254 / 173, 1 x 256 72 / 44, 8 x 2,048 2,126 / 1,226.
+constexpr int ST_FROM = 64;
 constexpr int ST_COLS = 16, ST_STAGE = 16, ST_THREADS = 128;
 
 // Where tile i of entry e has its coefficients (times heads): tiles of different entries never meet.

@@ -51,7 +51,7 @@ _SIGNATURES = {
     "bspec_scale": [c_void_p, c_longlong, c_float, c_void_p],
     "bspec_gate_mul": [c_void_p, c_void_p, c_longlong, c_void_p, c_longlong, c_int, c_int, c_int, c_float, c_void_p],
     "bspec_lightning_recurrence": [c_void_p, c_longlong, c_int, c_int, c_int, c_void_p, c_void_p, c_longlong, c_void_p,
-                                   c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_void_p,
+                                   c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_void_p,
                                    c_int, c_void_p, c_void_p, c_void_p],
     "bspec_lightning_scratch": [c_int, c_int, c_int, c_int, c_int],
     "bspec_branch_join": [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p,
@@ -79,7 +79,7 @@ _SIGNATURES = {
                             c_longlong, c_longlong, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int,
                             c_int, c_int, c_int, c_float, c_float, c_void_p],
     "bspec_delta_recurrence": [c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_longlong, c_longlong, c_void_p,
-                               c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p],
+                               c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p],
     "bspec_delta_scratch": [c_int, c_int, c_int, c_int],
     "bspec_gated_rmsnorm": [c_void_p, c_void_p, c_longlong, c_void_p, c_int, c_void_p, c_int, c_longlong, c_int, c_int, c_int,
                             c_float, c_int, c_void_p, c_float, c_void_p],
@@ -992,6 +992,11 @@ def delta_prepare(proj: torch.Tensor, b_off: int, a_off: int, conv: torch.Tensor
     return mix, gates
 
 
+def _portion_bounds(ctx, n: int):
+    """Bounds of the step's portions: none is shorter than the first or longer than the second."""
+    return getattr(ctx, "extras", {}).get("min_q_len", 1), getattr(ctx, "max_q_len", n)
+
+
 def delta_recurrence(mix: torch.Tensor, gates: torch.Tensor, proj: torch.Tensor, state: torch.Tensor, tail_off: int,
                      ctx, n_heads: int, n_kv_heads: int, dim: int, v_dim: int, taps: int) -> torch.Tensor:
     """The gated delta rule over every entry's portion, per head: S <- g S; u = beta (v - S^T k); S <- S + k u^T;
@@ -1003,13 +1008,13 @@ def delta_recurrence(mix: torch.Tensor, gates: torch.Tensor, proj: torch.Tensor,
     assert state.stride(0) % 4 == 0 and dim <= 256 and tail_off >= n_heads * v_dim * (-(-dim // 4) * 4)
     out = torch.empty((n, n_heads * v_dim), dtype=torch.float32, device=mix.device)
     lib = load_library()
-    longest = getattr(ctx, "max_q_len", n)                    # (an upper bound will do)
+    shortest, longest = _portion_bounds(ctx, n)
     need = lib.bspec_delta_scratch(n, ctx.n_entries, longest, n_heads)
     scratch = torch.empty((need,), dtype=torch.float32, device=mix.device) if need else None
     _check(lib.bspec_delta_recurrence(
         mix.data_ptr(), gates.data_ptr(), proj.data_ptr(), proj.shape[1], state.data_ptr(), state.stride(0),
         int(tail_off), ctx.qo_indptr.data_ptr(), ctx.state_slots.data_ptr(), out.data_ptr(), ctx.n_entries,
-        longest, n_heads, n_kv_heads, dim, v_dim, taps, _ptr(scratch), _stream()), "delta_recurrence")
+        shortest, longest, n_heads, n_kv_heads, dim, v_dim, taps, _ptr(scratch), _stream()), "delta_recurrence")
     if need:
         count_launches(1)
     return out
@@ -1116,12 +1121,12 @@ def lightning_recurrence(proj: torch.Tensor, q_off: int, k_off: int, v_off: int,
     assert not rotary_dim or (inv_freq.dtype == torch.float32 and inv_freq.shape == (2, rotary_dim // 2) and rotary_dim <= dim)
     out = torch.empty((n, n_heads * v_dim), dtype=torch.float32, device=proj.device)
     lib = load_library()
-    longest = getattr(ctx, "max_q_len", n)                    # (an upper bound will do)
+    shortest, longest = _portion_bounds(ctx, n)
     need = lib.bspec_lightning_scratch(n, ctx.n_entries, longest, n_heads, dim)
     scratch = torch.empty((need,), dtype=torch.float32, device=proj.device) if need else None
     _check(lib.bspec_lightning_recurrence(
         proj.data_ptr(), proj.stride(0), int(q_off), int(k_off), int(v_off), decay.data_ptr(), state.data_ptr(),
-        state.stride(0), ctx.qo_indptr.data_ptr(), ctx.state_slots.data_ptr(), out.data_ptr(), n, ctx.n_entries, longest,
+        state.stride(0), ctx.qo_indptr.data_ptr(), ctx.state_slots.data_ptr(), out.data_ptr(), n, ctx.n_entries, shortest, longest,
         n_heads, dim, v_dim, int(activation == "silu"), float(k_scale), _ptr(inv_freq) if rotary_dim else None,
         int(rotary_dim), ctx.positions.data_ptr() if rotary_dim else None, _ptr(scratch), _stream()),
         "lightning_recurrence")

@@ -591,7 +591,46 @@ def test_interleaved_rotation_and_append_from_wider_rows(ops, dtype, Hq, G, hd, 
     assert int((cache != 0).sum()) <= n * entry
 
 
-@pytest.mark.parametrize("lens", [[256], [255, 257, 1, 64], [1000, 3]])
+@pytest.mark.parametrize("Hh,dk,dv,act,scale", [(2, 128, 33, "silu", 1.0), (3, 20, 7, None, 0.25), (1, 256, 16, "silu", 1.0),
+                                                (4, 64, 64, None, 0.125), (2, 6, 130, "silu", 0.5)])
+def test_lightning_attention_by_tiles(ops, Hh, dk, dv, act, scale):
+    """Portions long enough to go by tiles (whole and partial last ones) beside ones that go token by token, states carried
+    between them, against the plain recurrence; a request's last token being infinite changes nothing before it."""
+    steps = [dict(a=70, b=1, c=5), dict(a=64, c=63), dict(a=1, b=200, c=65)]
+    gen = torch.Generator(device=DEV).manual_seed(dk + dv)
+    ld = 2 * Hh * dk + Hh * dv + 1
+    k_off, v_off = Hh * dk, 2 * Hh * dk + 1
+    decay = torch.tensor([0.5, 0.99, 1.0, 0.9][:Hh], device=DEV)
+    state = torch.zeros(5, Hh * dv * dk, device=DEV)
+    slots = {"a": 2, "b": 0, "c": 4}
+    proj = {r: torch.randn(sum(s.get(r, 0) for s in steps), ld, device=DEV, generator=gen) for r in slots}
+
+    def run(x, ctx):
+        before = state.clone()
+        o = ops.lightning_recurrence(x, 0, k_off, v_off, decay, state, ctx, Hh, dk, dv, act, scale)
+        last = (ctx.qo_indptr[1:] - 1).long()
+        spoilt = x.clone()
+        spoilt[last] = float("inf")
+        other = ops.lightning_recurrence(spoilt, 0, k_off, v_off, decay, before, ctx, Hh, dk, dv, act, scale)
+        keep = torch.ones(len(x), dtype=torch.bool, device=DEV)
+        keep[last] = False
+        assert torch.equal(other[keep], o[keep])
+        return o
+
+    got = _feed(steps, slots, proj, run)
+    f = P.silu if act else (lambda t: t)
+    for r in slots:
+        x = proj[r].double().cpu()
+        T = x.shape[0]
+        q, k = f(x[:, :Hh * dk]).view(T, Hh, dk), f(x[:, k_off:k_off + Hh * dk]).view(T, Hh, dk) * scale
+        want = P.decaying_linear_attention(q, k, f(x[:, v_off:v_off + Hh * dv]).view(T, Hh, dv), decay.double().cpu().tolist())
+        want = want.reshape(T, Hh * dv)
+        # the bound of the test above
+        assert (got[r] - want).abs().max() <= 2e-5 * max(1.0, want.abs().max().item()), r
+    assert not state[1].any() and not state[3].any()
+
+
+@pytest.mark.parametrize("lens", [[512], [511, 513, 1, 64], [1000, 3]])
 @pytest.mark.parametrize("inner,N,taps", [(64, 16, 4), (130, 5, 1), (33, 40, 3)])
 def test_selective_scan_in_segments(ops, inner, N, taps, lens):
     """Portions long enough to run in segments at once (whole ones, partial ones, requests of a token beside them), from a
