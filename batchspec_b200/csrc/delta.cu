@@ -700,7 +700,10 @@ BSPEC_API int bspec_delta_prepare(const float* proj, int n, int ld, int b_off, i
 // Floats of scratch for a step of n tokens whose longest portion has max_q_len: the tiles' coefficients, or 0 where no
 // portion goes by tiles.
 BSPEC_API long long bspec_delta_scratch(int n, int n_entries, int max_q_len, int H) {
-  return max_q_len >= ST_FROM ? bspec::state_tile_slots(n, n_entries) * H * ST_CO : 0;
+  // many requests fill the device token by token, and the second kernel for the short ones comes on top: 512 tokens beside 63
+  // decoded ones 182 us by tokens, 193 by tiles; 2,048 beside 24 668 and 488
+  if (max_q_len < ST_FROM || (n_entries > 32 && max_q_len < 1024)) return 0;
+  return bspec::state_tile_slots(n, n_entries) * H * ST_CO;
 }
 
 BSPEC_API int bspec_delta_recurrence(const float* mix, const float* gates, const float* proj, int ld, float* state,
