@@ -203,7 +203,8 @@ sgemm_join_kernel(const float* __restrict__ part, float* __restrict__ C, int M, 
 
 // ------------------------------------------------------------------------------------------------ few rows
 // A block owns tiles of 16 rows of W (16 output numbers of MT tokens) one after the other; a stage is 512 k of them and of
-// the tokens, fetched by a producer warp that runs ahead across tiles and, for W, ahead of the kernel before: W by one
+// the tokens, fetched by a producer warp that runs ahead across tiles and, where W is a parameter (``w_ahead``: nothing on the
+// stream before this kernel writes it), ahead of the end of the kernel before: W by one
 // bulk copy per row, the tokens by 16-byte copies (a bulk copy costs an SM about 40 clocks whatever its size, which bound
 // the kernel when the tokens' 256-byte slices were such copies: 347 us against 20x at 128,256 x 2,048 and 8 tokens).  Rows
 // and slices are padded by 4 floats: a quarter warp's 16-byte loads fall into different banks.  64 consumer threads:
@@ -225,7 +226,7 @@ __device__ __forceinline__ void bulk_copy(void* dst, const void* src, uint32_t b
 template <int MT>
 __global__ void __launch_bounds__(ROW_THREADS)
 sgemm_rows_kernel(const float* __restrict__ A, const float* __restrict__ W, float* __restrict__ C, int M, int N, int K,
-                  long long lda, long long ldw, long long ldc, long long sa, long long sw, long long sc, int* status) {
+                  long long lda, long long ldw, long long ldc, long long sa, long long sw, long long sc, int w_ahead, int* status) {
   constexpr int STAGES = rows_stages(MT), SF = rows_stage_floats(MT);
   extern __shared__ __align__(128) float smem_f[];
   float* red = smem_f + STAGES * SF;                                  // [2][SL][RT][MT] slice values
@@ -265,7 +266,8 @@ sgemm_rows_kernel(const float* __restrict__ A, const float* __restrict__ W, floa
       }
       asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(s32(full + s)) : "memory");
     };
-    // the first stages' weights do not depend on the kernel before this one
+    // the first stages' weights need not wait for the kernel before this one, unless it may be writing them
+    if (!w_ahead) bspec::pdl_wait();
     int pre = 0;
     for (int tile = blockIdx.x; tile < tiles && pre < STAGES; tile += gridDim.x)
       for (int kc = 0; kc < kcs && pre < STAGES; ++kc) weights(tile, kc, pre++);
@@ -360,7 +362,7 @@ sgemm_rows_kernel(const float* __restrict__ A, const float* __restrict__ W, floa
 
 template <int MT>
 int launch_rows(const float* A, const float* W, float* C, int M, int N, int K, long long lda, long long ldw, long long ldc,
-                long long sa, long long sw, long long sc, int batch, int* status, cudaStream_t stream) {
+                long long sa, long long sw, long long sc, int batch, int w_ahead, int* status, cudaStream_t stream) {
   static bool set[bspec::kMaxDevices] = {};
   bool& done = set[bspec::current_device()];
   if (!done) {
@@ -371,7 +373,7 @@ int launch_rows(const float* A, const float* W, float* C, int M, int N, int K, l
   const int tiles = (N + RT - 1) / RT * ((M + MT - 1) / MT);
   const int fit = max(1, 2 * bspec::sm_count() / batch);
   BSPEC_LAUNCH((sgemm_rows_kernel<MT>), dim3(min(tiles, fit), 1, batch), ROW_THREADS, rows_smem(MT), stream, A, W, C, M, N, K, lda,
-               ldw, ldc, sa, sw, sc, status);
+               ldw, ldc, sa, sw, sc, w_ahead, status);
   return BSPEC_LAUNCH_CHECK();
 }
 
@@ -425,16 +427,17 @@ BSPEC_API long long bspec_sgemm_scratch(const float* A, const float* W, int M, i
 }
 
 // `batch` products C_b = A_b * W_b^T whose operands lie sa / sw / sc elements apart.  ``scratch``: bspec_sgemm_scratch
-// floats; ``status``: the device's status word (0 unless a bounded wait ran out).
+// floats; ``w_ahead``: W is complete whatever still runs on the stream (a parameter), so it may be read before the kernel
+// before this one ends; ``status``: the device's status word (0 unless a bounded wait ran out).
 BSPEC_API int bspec_sgemm_tn_batched(const float* A, const float* W, float* C, int M, int N, int K, long long lda,
                                      long long ldw, long long ldc, long long sa, long long sw, long long sc, int batch,
-                                     float* scratch, int* status, cudaStream_t stream) {
+                                     float* scratch, int w_ahead, int* status, cudaStream_t stream) {
   if (M <= 0 || N <= 0 || batch <= 0) return 0;
   if (batch > 65535) return (int)cudaErrorInvalidConfiguration;
   const bool vec = rows_of_16_bytes(A, W, K, lda, ldw, sa, sw);
   if (M <= ROWS_MAX_M && K > 0 && vec) {
     auto fn = M == 1 ? launch_rows<1> : (M == 2 ? launch_rows<2> : (M <= 4 ? launch_rows<4> : launch_rows<8>));
-    return fn(A, W, C, M, N, K, lda, ldw, ldc, sa, sw, sc, batch, status, stream);
+    return fn(A, W, C, M, N, K, lda, ldw, ldc, sa, sw, sc, batch, w_ahead, status, stream);
   }
   const int groups = (K + GROUP - 1) / GROUP, splits = K > 0 && scratch != nullptr ? tile_splits(M, N, K, batch) : 1;
   auto fn = M > 64 ? (vec ? launch_tile<128, true> : launch_tile<128, false>) : (vec ? launch_tile<64, true> : launch_tile<64, false>);

@@ -50,6 +50,7 @@ struct GemmParams {
                          // 3: relu(gate) * up
   float glu_alpha, glu_limit;
   int act;               // a plain activation on every output (no gate): 0 none, 1 the square of relu, 2 the exact gelu
+  int w_ahead;           // 1: W is a parameter and may be read before the kernel before this one has ended
   int prefetch_kb;       // K blocks of weights (beyond the stages) to pull into the L2 before waiting on the predecessor
   // fused q/k/v projection (rope_freq != nullptr): tile t of W is head t (q heads, then k heads, then v heads)
   const float* rope_freq;    // [2][64] frequencies as two floats each (see elementwise.cu, rope_sincos)
@@ -140,8 +141,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   if (warp == 0) {
     if (lane == 0) {
       int armed = 0;
-      // The weights do not depend on the kernel before this one: fetch them for the first stages at once, and
-      // only then wait for that kernel to finish before touching the activations it wrote.
+      // Weights that are parameters do not depend on the kernel before this one: fetch them for the first stages at once,
+      // and only then wait for that kernel to finish before touching the activations it wrote.
+      if (!p.w_ahead) bspec::pdl_wait();
       const int pre = min(nkb, p.stages);
       for (int i = 0; i < pre; ++i) {
         unsigned char* a_dst = smem + (size_t)i * stage_bytes;
@@ -453,7 +455,7 @@ struct RopeEpilogue {
 
 static int launch_gemm(const void* X, const void* W, void* C, int M, int N, int K, int out_f32, int glu, int* status,
                        int sm_count, const RopeEpilogue* rope, cudaStream_t stream, float glu_alpha = 1.f,
-                       float glu_limit = 0.f, int act = 0) {
+                       float glu_limit = 0.f, int act = 0, int w_ahead = 1) {
   int plan[5];
   if (bspec_gemm_tc_plan(M, N, K, sm_count, plan) < 0) return (int)cudaErrorInvalidValue;
   if (glu && (N % 16 != 0)) return (int)cudaErrorInvalidValue;
@@ -463,6 +465,7 @@ static int launch_gemm(const void* X, const void* W, void* C, int M, int N, int 
   p.glu_alpha = glu_alpha; p.glu_limit = glu_limit;
   if (act && (glu || rope != nullptr)) return (int)cudaErrorInvalidValue;
   p.act = act;
+  p.w_ahead = w_ahead;
   p.swap = plan[0]; p.bn = plan[1]; p.splits = plan[2]; p.stages = plan[3];
   p.rope_freq = nullptr; p.positions = p.tok_entry = p.kv_indptr = p.kv_indices = nullptr; p.cache = nullptr;
   p.Hq = p.Hkv = p.page_size = p.interleaved = p.write_kv = 0;
@@ -487,7 +490,7 @@ static int launch_gemm(const void* X, const void* W, void* C, int M, int N, int 
     const long long per_kb = ctas * (p.swap ? TM : p.bn) * BK * 2;
     long long pf = per_kb > 0 ? (48ll << 20) / per_kb : 0;
     if (pf > p.kblocks_per_split) pf = p.kblocks_per_split;
-    p.prefetch_kb = bspec::pdl_enabled() ? (int)pf : 0;
+    p.prefetch_kb = bspec::pdl_enabled() && w_ahead ? (int)pf : 0;
   }
   CUtensorMap map_a, map_b;
   const void* a_ptr = p.swap ? W : X;
@@ -524,12 +527,14 @@ static int launch_gemm(const void* X, const void* W, void* C, int M, int N, int 
   return BSPEC_LAUNCH_CHECK();
 }
 
-// C = X W^T.  `status`: one int on the device, 0 unless a bounded wait ran out.
+// C = X W^T.  `status`: one int on the device, 0 unless a bounded wait ran out.  `w_ahead` 1: W is complete whatever still
+// runs on the stream (a parameter), and its first tiles are read before the kernel before this one ends; the entry points
+// with an epilogue, whose W are parameters by their layout, always do that.
 // glu != 0: the rows of W come in groups of 16 (8 gate rows, then the 8 matching up rows; N a multiple of 16) and
 // C is [M, N/2] = silu(gate) * up (glu 1), relu(gate) * up (glu 3) or gelu(gate) * up in the tanh form (glu 4).
 BSPEC_API int bspec_gemm_tc(const void* X, const void* W, void* C, int M, int N, int K, int out_f32, int glu,
-                            int* status, int sm_count, cudaStream_t stream) {
-  return launch_gemm(X, W, C, M, N, K, out_f32, glu, status, sm_count, nullptr, stream);
+                            int w_ahead, int* status, int sm_count, cudaStream_t stream) {
+  return launch_gemm(X, W, C, M, N, K, out_f32, glu, status, sm_count, nullptr, stream, 1.f, 0.f, 0, w_ahead);
 }
 
 // C = act(X W^T) with a plain activation on every output: act 1 = the square of relu, 2 = the exact (erf) gelu.

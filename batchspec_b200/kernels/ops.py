@@ -133,7 +133,7 @@ _SIGNATURES = {
     "bspec_moe_combine": [c_void_p, c_int, c_void_p, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_void_p, c_void_p, c_int,
                           c_void_p, c_void_p, c_longlong, c_void_p],
     "bspec_sgemm_tn_batched": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_longlong, c_longlong, c_longlong,
-                               c_longlong, c_longlong, c_longlong, c_int, c_void_p, c_void_p, c_void_p],
+                               c_longlong, c_longlong, c_longlong, c_int, c_void_p, c_int, c_void_p, c_void_p],
     "bspec_sgemm_scratch": [c_void_p, c_void_p, c_int, c_int, c_int, c_longlong, c_longlong, c_longlong, c_longlong, c_int],
     "bspec_attention_generic": [c_void_p, c_longlong, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p,
                                 c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_int, c_longlong, c_void_p],
@@ -153,7 +153,7 @@ _SIGNATURES = {
                                           c_int, c_float, c_int, c_int, c_void_p, c_void_p, c_float, c_void_p, c_int, c_void_p,
                                           c_void_p, c_void_p, c_longlong, c_void_p],
     "bspec_gemm_tc_plan": [c_int, c_int, c_int, c_int, c_void_p],
-    "bspec_gemm_tc": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p, c_int, c_void_p],
+    "bspec_gemm_tc": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_int, c_void_p],
     "bspec_gemm_tc_act": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p, c_int, c_void_p],
     "bspec_gemm_tc_clamped_glu": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_float, c_float, c_void_p, c_int,
                                   c_void_p],
@@ -604,7 +604,7 @@ def interleave_gate_up(gate: torch.Tensor, up: torch.Tensor, group: int = GLU_GR
 def linear_glu(x: torch.Tensor, w13: torch.Tensor, group: int = GLU_GROUP, activation: str = "silu") -> torch.Tensor:
     """act(x Wg^T) * (x Wu^T), act = silu, relu or gelu_tanh, for bfloat16 with ``w13`` interleaved by
     ``interleave_gate_up``: one kernel with the activation in the GEMM's epilogue for decode-sized steps, vendor GEMM +
-    activation kernel otherwise."""
+    activation kernel otherwise.  ``w13`` is a parameter in the sense of ``linear``."""
     epilogue, kernel = GATED_ACTIVATIONS[activation]
     _require_cuda(x, w13)
     M, K = x.shape
@@ -614,10 +614,10 @@ def linear_glu(x: torch.Tensor, w13: torch.Tensor, group: int = GLU_GROUP, activ
             and x.is_contiguous() and (TC_GEMM == "all" or (TC_GEMM == "auto" and M <= TC_GEMM_MAX_M))):
         out = torch.empty((M, inter), dtype=x.dtype, device=x.device)
         _check(load_library().bspec_gemm_tc(x.data_ptr(), w13.data_ptr(), out.data_ptr(), M, N, K, 0,
-                                            epilogue,
+                                            epilogue, 1,
                                             _status_word(x.device).data_ptr(), sm_count(x.device), _stream()), "gemm_tc_glu")
         return out
-    u = linear(x, w13)
+    u = linear(x, w13, w_is_parameter=True)
     out = torch.empty((M, inter), dtype=x.dtype, device=x.device)
     kernel(u, out, group)
     return out
@@ -626,7 +626,7 @@ def linear_glu(x: torch.Tensor, w13: torch.Tensor, group: int = GLU_GROUP, activ
 def linear_clamped_glu(x: torch.Tensor, w13: torch.Tensor, alpha: float, limit: float, group: int = GLU_GROUP) -> torch.Tensor:
     """g sigmoid(alpha g) (u + 1) with g = min(x Wg^T, limit), u = clamp(x Wu^T, -limit, limit), for ``w13`` interleaved
     by ``interleave_gate_up``: one kernel with the activation in the product's epilogue for decode-sized bfloat16
-    steps, else product + activation kernel."""
+    steps, else product + activation kernel.  ``w13`` is a parameter in the sense of ``linear``."""
     _require_cuda(x, w13)
     M, K = x.shape
     N = w13.shape[0]
@@ -638,7 +638,7 @@ def linear_clamped_glu(x: torch.Tensor, w13: torch.Tensor, alpha: float, limit: 
                                                         float(alpha), float(limit), _status_word(x.device).data_ptr(),
                                                         sm_count(x.device), _stream()), "gemm_tc_clamped_glu")
         return out
-    clamped_glu(linear(x, w13), out, alpha, limit, group)
+    clamped_glu(linear(x, w13, w_is_parameter=True), out, alpha, limit, group)
     return out
 
 
@@ -1321,8 +1321,9 @@ def raise_if_gave_up() -> None:
             _raise_status(dev, code)
 
 
-def gemm_tc(x: torch.Tensor, w: torch.Tensor, out_dtype: torch.dtype) -> torch.Tensor:
-    """x [M, K] @ w[N, K]^T on the tcgen05 kernel (bfloat16 operands, float32 accumulation)."""
+def gemm_tc(x: torch.Tensor, w: torch.Tensor, out_dtype: torch.dtype, w_is_parameter: bool = False) -> torch.Tensor:
+    """x [M, K] @ w[N, K]^T on the tcgen05 kernel (bfloat16 operands, float32 accumulation).  ``w_is_parameter`` as in
+    ``linear``."""
     lib = load_library()
     M, K = x.shape
     N = w.shape[0]
@@ -1331,7 +1332,7 @@ def gemm_tc(x: torch.Tensor, w: torch.Tensor, out_dtype: torch.dtype) -> torch.T
         raise KernelError(f"gemm_tc: sizes M={M} N={N} K={K} are not supported (K must be a multiple of 8)")
     out = torch.empty((M, N), dtype=out_dtype, device=x.device)
     _check(lib.bspec_gemm_tc(x.data_ptr(), w.data_ptr(), out.data_ptr(), M, N, K, int(out_dtype == torch.float32), 0,
-                             _status_word(x.device).data_ptr(), sm_count(x.device), _stream()), "gemm_tc")
+                             int(w_is_parameter), _status_word(x.device).data_ptr(), sm_count(x.device), _stream()), "gemm_tc")
     return out
 
 
@@ -1341,7 +1342,7 @@ PLAIN_ACTIVATIONS = {"relu2": (1, relu_squared_), "gelu": (2, gelu_erf_)}     # 
 def linear_act(x: torch.Tensor, w: torch.Tensor, activation: str) -> torch.Tensor:
     """act(x w^T) with a plain activation on every output (``PLAIN_ACTIVATIONS``): one kernel with the activation in
     the tcgen05 product's epilogue for decode-sized bfloat16 steps when the epilogue knows it, else the product and
-    the in-place activation kernel."""
+    the in-place activation kernel.  ``w`` is a parameter in the sense of ``linear``."""
     epilogue, kernel = PLAIN_ACTIVATIONS[activation]
     _require_cuda(x, w)
     M, K = x.shape
@@ -1353,7 +1354,7 @@ def linear_act(x: torch.Tensor, w: torch.Tensor, activation: str) -> torch.Tenso
                                                 _status_word(x.device).data_ptr(), sm_count(x.device), _stream()),
                "gemm_tc_act")
         return out
-    return kernel(linear(x, w))
+    return kernel(linear(x, w, w_is_parameter=True))
 
 
 FUSE_QKV_ROPE = True       # decode-sized steps: rotary encoding and the cache append in the q/k/v product's epilogue
@@ -1367,7 +1368,7 @@ def linear_qkv_rope(x: torch.Tensor, wqkv: torch.Tensor, n_heads: int, n_kv_head
     pages done in the product's epilogue, for bfloat16 steps of at most ``TC_GEMM_MAX_M`` tokens and heads of
     128 rotated over their whole width.  Returns [M, (Hq + 2 Hkv) * 128] whose q columns hold the rotated queries
     (its k and v columns are not written), or None when the sizes are not these: the caller then runs the product,
-    ``rope_kv_append`` and so on one after the other."""
+    ``rope_kv_append`` and so on one after the other.  ``wqkv`` is a parameter in the sense of ``linear``."""
     M, K = x.shape
     N = wqkv.shape[0]
     if not (FUSE_QKV_ROPE and TC_GEMM != "none" and x.dtype == torch.bfloat16
@@ -1386,8 +1387,11 @@ def linear_qkv_rope(x: torch.Tensor, wqkv: torch.Tensor, n_heads: int, n_kv_head
     return out
 
 
-def linear(x: torch.Tensor, w: torch.Tensor, out_dtype: Optional[torch.dtype] = None) -> torch.Tensor:
-    """x [M, K] @ w[N, K]^T -> [M, N] in ``out_dtype`` (default: x's dtype)."""
+def linear(x: torch.Tensor, w: torch.Tensor, out_dtype: Optional[torch.dtype] = None,
+           w_is_parameter: bool = False) -> torch.Tensor:
+    """x [M, K] @ w[N, K]^T -> [M, N] in ``out_dtype`` (default: x's dtype).  ``w_is_parameter``: nothing that still runs on
+    the stream writes ``w``, so that a product of few rows may read it while the kernel before is at work (the kernels
+    of this package let their successor start early; ``x`` is always waited for)."""
     _require_cuda(x, w)
     out_dtype = out_dtype or x.dtype
     M, K = x.shape
@@ -1396,38 +1400,39 @@ def linear(x: torch.Tensor, w: torch.Tensor, out_dtype: Optional[torch.dtype] = 
     if x.dtype == torch.float32:
         assert out_dtype == torch.float32 and x.stride(1) == 1 and w.stride(1) == 1
         out = torch.empty((M, N), dtype=torch.float32, device=x.device)
-        _sgemm(x, w, out, M, N, K, x.stride(0), w.stride(0), 0, 0, 1)
+        _sgemm(x, w, out, M, N, K, x.stride(0), w.stride(0), 0, 0, 1, w_is_parameter)
         return out
     if (K % 8 == 0 and M > 0 and x.is_contiguous() and w.is_contiguous()
             and (TC_GEMM == "all" or (TC_GEMM == "auto" and M <= TC_GEMM_MAX_M))):
-        return gemm_tc(x, w, out_dtype)
+        return gemm_tc(x, w, out_dtype, w_is_parameter)
     if out_dtype == x.dtype:
         return torch.mm(x, w.t())
     return torch.mm(x, w.t(), out_dtype=out_dtype)
 
 
-def linear_batched(x: torch.Tensor, w: torch.Tensor) -> torch.Tensor:
+def linear_batched(x: torch.Tensor, w: torch.Tensor, w_is_parameter: bool = False) -> torch.Tensor:
     """x [B, M, K] (rows and batches may be strided, K dense) times w [B, N, K]^T -> [B, M, N] contiguous: one product
-    per head.  bfloat16 on the vendor library's batched product, float32 on this package's FFMA kernel."""
+    per head.  bfloat16 on the vendor library's batched product, float32 on this package's FFMA kernels.
+    ``w_is_parameter`` as in ``linear``."""
     _require_cuda(x, w)
     B, M, K = x.shape
     N = w.shape[1]
     assert w.shape == (B, N, K) and x.dtype == w.dtype and x.stride(2) == 1 and w.is_contiguous()
     if x.dtype == torch.float32:
         out = torch.empty((B, M, N), dtype=torch.float32, device=x.device)
-        _sgemm(x, w, out, M, N, K, x.stride(1), K, x.stride(0), N * K, B)
+        _sgemm(x, w, out, M, N, K, x.stride(1), K, x.stride(0), N * K, B, w_is_parameter)
         return out
     return torch.bmm(x, w.transpose(1, 2))
 
-def _sgemm(x, w, out, M: int, N: int, K: int, lda: int, ldw: int, sa: int, sw: int, batch: int) -> None:
+
+def _sgemm(x, w, out, M: int, N: int, K: int, lda: int, ldw: int, sa: int, sw: int, batch: int, w_is_parameter: bool) -> None:
     """``batch`` float32 products, operands sa / sw numbers apart; the K slices of small tiles meet in scratch that the
     stream's order protects."""
     lib = load_library()
     need = lib.bspec_sgemm_scratch(x.data_ptr(), w.data_ptr(), M, N, K, lda, ldw, sa, sw, batch)
     scratch = torch.empty((need,), dtype=torch.float32, device=x.device) if need else None
     _check(lib.bspec_sgemm_tn_batched(x.data_ptr(), w.data_ptr(), out.data_ptr(), M, N, K, lda, ldw, N, sa, sw, M * N, batch,
-                                      _ptr(scratch), _status_word(x.device).data_ptr(), _stream()), "sgemm_tn")
-
+                                      _ptr(scratch), int(w_is_parameter), _status_word(x.device).data_ptr(), _stream()), "sgemm_tn")
 
 
 # ---------------------------------------------------------------------------- latent attention

@@ -213,7 +213,7 @@ class DecoderModel:
                 ops.gather_rows_add(resid, pending, ctx.logit_rows, picked, scale, vec)
             z = self.final_norm.forward(picked, None)
         with bucket("lm_head"):
-            logits = ops.linear(z, self.head, out_dtype=torch.float32)
+            logits = ops.linear(z, self.head, out_dtype=torch.float32, w_is_parameter=True)
         if self.logits_part is not None:
             self.logits_part.forward(logits, ctx)
         return logits

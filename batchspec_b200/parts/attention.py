@@ -67,7 +67,7 @@ class Attention(Mixer):
                                           tables.page_size, write_kv=cache.owner)
         if qkv is None:
             with bucket("attn.qkv_proj"):
-                qkv = ops.linear(x, self.wqkv)
+                qkv = ops.linear(x, self.wqkv, w_is_parameter=True)
             if table is None:
                 q = qkv[:, :Hq * hd].view(n, Hq, hd)
                 k = qkv[:, Hq * hd:(Hq + Hkv) * hd].view(n, Hkv, hd)
@@ -83,4 +83,4 @@ class Attention(Mixer):
         with bucket("attn.compute"):
             ops.paged_attention(qkv, out, cache.kv, ctx, tables, Hq, Hkv, hd, self.scale, self.window)
         with bucket("attn.o_proj"):
-            return ops.linear(out, self.wo)
+            return ops.linear(out, self.wo, w_is_parameter=True)

@@ -67,7 +67,7 @@ class GatedDeltaRule(Mixer):
         H, G, dk, dv = self.n_heads, self.n_kv_heads, self.head_dim, self.v_dim
         state = cache.state
         with bucket("delta.in_proj"):
-            proj = ops.linear(x, self.w_in, out_dtype=torch.float32)
+            proj = ops.linear(x, self.w_in, out_dtype=torch.float32, w_is_parameter=True)
         with bucket("delta.prepare"):
             mix, gates = ops.delta_prepare(proj, self.b_off, self.a_off, self.conv, self.a_log, self.dt_bias, state,
                                            self.tail_off, ctx, H, G, dk, dv, self.taps, dk ** -0.5, self.unit_eps)
@@ -76,4 +76,4 @@ class GatedDeltaRule(Mixer):
         with bucket("delta.out_norm"):
             y = ops.gated_rmsnorm(o, proj[:, self.g_off:self.g_off + H * dv], self.norm, self.eps, H, dv, x.dtype)
         with bucket("delta.o_proj"):
-            return ops.linear(y, self.w_o)
+            return ops.linear(y, self.w_o, w_is_parameter=True)

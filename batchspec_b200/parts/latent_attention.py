@@ -101,22 +101,22 @@ class LatentAttention(Mixer):
         tables = ctx.tables[cache.group]
         pos = self.position
         with bucket("attn.down_proj"):
-            down = ops.linear(x, self.w_down, out_dtype=torch.float32)
+            down = ops.linear(x, self.w_down, out_dtype=torch.float32, w_is_parameter=True)
         with bucket("attn.latent_prepare"):
             cq = ops.latent_prepare(down, 0, self.q_rank, self.q_rank, R, P, self.n_q, self.n_kv, self.eps,
                                     pos.inv_freq, pos.magnitude, ctx.positions, ctx.tok_entry, tables.kv_indptr,
                                     tables.kv_indices, cache.kv, tables.page_size, write_kv=cache.owner)
         with bucket("attn.q_proj"):
-            q = ops.linear(cq, self.w_uq).view(n, H, dh + P)
+            q = ops.linear(cq, self.w_uq, w_is_parameter=True).view(n, H, dh + P)
         q_rot = q[:, :, dh:]                      # rotated on its way into the attention kernel
         with bucket("attn.absorb"):
-            q_lat = ops.linear_batched(q[:, :, :dh].transpose(0, 1), self.w_uk_t)          # [H, n, R]
+            q_lat = ops.linear_batched(q[:, :, :dh].transpose(0, 1), self.w_uk_t, w_is_parameter=True)          # [H, n, R]
         o_lat = torch.empty((H, n, R), dtype=x.dtype, device=x.device)
         with bucket("attn.compute"):
             ops.latent_attention(q_lat, q_rot, o_lat, cache.kv, ctx, tables, H, R, P, self.scale,
                                  rotate=(pos.inv_freq, pos.magnitude), window=self.window, sink=self.sinks)
         with bucket("attn.v_proj"):
-            v = ops.linear_batched(o_lat, self.w_uv)                                        # [H, n, v_dim]
+            v = ops.linear_batched(o_lat, self.w_uv, w_is_parameter=True)                                        # [H, n, v_dim]
         heads = torch.empty((n, H * self.v_dim), dtype=x.dtype, device=x.device)
         with bucket("attn.gate"):
             if self.gated:
@@ -125,4 +125,4 @@ class LatentAttention(Mixer):
                 gate = self.open_gate.expand(n, H)                  # every row reads the same logits (row stride 0)
             ops.gate_heads(v, gate, heads)
         with bucket("attn.o_proj"):
-            return ops.linear(heads, self.w_o)
+            return ops.linear(heads, self.w_o, w_is_parameter=True)

@@ -56,11 +56,11 @@ class LightningAttention(Mixer):
     def forward(self, x, ctx, cache):
         H, dk, dv = self.n_heads, self.head_dim, self.v_dim
         with bucket("lightning.in_proj"):
-            proj = ops.linear(x, self.w_in, out_dtype=torch.float32)
+            proj = ops.linear(x, self.w_in, out_dtype=torch.float32, w_is_parameter=True)
         with bucket("lightning.recurrence"):
             o = ops.lightning_recurrence(proj, 0, self.k_off, self.v_off, self.decay, cache.state, ctx, H, dk, dv)
         with bucket("lightning.out_norm"):
             y = ops.gated_rmsnorm(o, proj[:, self.g_off:self.g_off + H * dv], self.norm, self.eps, 1, H * dv, x.dtype,
                                   gate_act="sigmoid")
         with bucket("lightning.o_proj"):
-            return ops.linear(y, self.w_o)
+            return ops.linear(y, self.w_o, w_is_parameter=True)

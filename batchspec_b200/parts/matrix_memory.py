@@ -64,7 +64,7 @@ class MatrixMemory(Mixer):
     def forward(self, x, ctx, cache):
         y = self.pre_projection(x, ctx, cache)
         with bucket("matrix_memory.o_proj"):
-            return ops.linear(y, self.wo)
+            return ops.linear(y, self.wo, w_is_parameter=True)
 
     def pre_projection(self, x, ctx, cache, out=None, out_scale: float = 1.0):
         """The normed and gated heads [n, H v_dim] in the run dtype, times ``out_scale``; written into ``out`` (a view of
@@ -74,7 +74,7 @@ class MatrixMemory(Mixer):
         g_off = v_off + H * dv
         i_off = g_off + H * dv
         with bucket("matrix_memory.in_proj"):
-            proj = ops.linear(x, self.w_in, out_dtype=torch.float32)
+            proj = ops.linear(x, self.w_in, out_dtype=torch.float32, w_is_parameter=True)
         with bucket("matrix_memory.recurrence"):
             o, den = ops.matrix_memory(proj, 0, k_off, v_off, i_off, i_off + H, self.i_bias, self.f_bias, self.gate_cap,
                                        dk ** -0.5, cache.state, self.m_off, ctx, H, dk, dv)

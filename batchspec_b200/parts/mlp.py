@@ -47,12 +47,12 @@ class SwiGLU(FeedForward):
                 m = ops.linear_glu(x, self.w13, self.group, self.activation)
         else:
             with bucket("mlp.gate_up_proj"):
-                u = ops.linear(x, self.w13)
+                u = ops.linear(x, self.w13, w_is_parameter=True)
             m = torch.empty((x.shape[0], self.intermediate), dtype=x.dtype, device=x.device)
             with bucket("mlp.act"):
                 ops.GATED_ACTIVATIONS[self.activation][1](u, m)
         with bucket("mlp.down_proj"):
-            return ops.linear(m, self.w2)
+            return ops.linear(m, self.w2, w_is_parameter=True)
 
 
 @register_part(FEED_FORWARDS, "clamped_glu")
@@ -88,12 +88,12 @@ class ClampedGLU(FeedForward):
                 m = ops.linear_clamped_glu(x, self.w13, self.alpha, self.limit, self.group)
         else:
             with bucket("mlp.gate_up_proj"):
-                u = ops.linear(x, self.w13)
+                u = ops.linear(x, self.w13, w_is_parameter=True)
             m = torch.empty((x.shape[0], self.intermediate), dtype=x.dtype, device=x.device)
             with bucket("mlp.act"):
                 ops.clamped_glu(u, m, self.alpha, self.limit)
         with bucket("mlp.down_proj"):
-            return ops.linear(m, self.w2)
+            return ops.linear(m, self.w2, w_is_parameter=True)
 
 
 @register_part(FEED_FORWARDS, "mlp")
@@ -121,4 +121,4 @@ class PlainMLP(FeedForward):
         with bucket("mlp.up_proj"):
             u = ops.linear_act(x, self.w1, self.activation)
         with bucket("mlp.down_proj"):
-            return ops.linear(u, self.w2)
+            return ops.linear(u, self.w2, w_is_parameter=True)

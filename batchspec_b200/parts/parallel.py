@@ -79,4 +79,4 @@ class ParallelMixer(Mixer):
         self.left.pre_projection(x, ctx, cache, both[:, :wl], self.left_scale)
         self.right.pre_projection(x, ctx, cache, both[:, wl:], self.right_scale)
         with bucket("parallel.o_proj"):
-            return ops.linear(both, self.wo)
+            return ops.linear(both, self.wo, w_is_parameter=True)

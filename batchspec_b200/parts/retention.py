@@ -55,7 +55,7 @@ class Retention(Mixer):
         H, dk, dv = self.n_heads, self.head_dim, self.v_dim
         k_off, v_off, g_off = H * dk, 2 * H * dk, 2 * H * dk + H * dv
         with bucket("retention.in_proj"):
-            proj = ops.linear(x, self.w_in, out_dtype=torch.float32)
+            proj = ops.linear(x, self.w_in, out_dtype=torch.float32, w_is_parameter=True)
         pos = self.position
         rot = getattr(pos, "rotary_dim", 0)
         inside = rot > 0 and ctx.max_q_len == 1 and not pos.interleaved and pos.magnitude == 1.0
@@ -69,4 +69,4 @@ class Retention(Mixer):
         with bucket("retention.out_norm"):
             y = ops.gated_rmsnorm(o, proj[:, g_off:g_off + H * dv], None, self.eps, H, dv, x.dtype)
         with bucket("retention.o_proj"):
-            return ops.linear(y, self.wo)
+            return ops.linear(y, self.wo, w_is_parameter=True)

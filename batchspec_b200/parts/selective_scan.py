@@ -66,7 +66,7 @@ class SelectiveScan(Mixer):
     def forward(self, x, ctx, cache):
         y = self.pre_projection(x, ctx, cache)
         with bucket("scan.o_proj"):
-            return ops.linear(y, self.wo)
+            return ops.linear(y, self.wo, w_is_parameter=True)
 
     def pre_projection(self, x, ctx, cache, out=None, out_scale: float = 1.0):
         """y * silu(z) [n, inner] in the run dtype, times ``out_scale``; written into ``out`` (a view of columns of
@@ -75,14 +75,14 @@ class SelectiveScan(Mixer):
         if out is None:
             out = torch.empty((n, self.inner), dtype=x.dtype, device=x.device)
         with bucket("scan.in_proj"):
-            xz = ops.linear(x, self.w_in, out_dtype=torch.float32)
+            xz = ops.linear(x, self.w_in, out_dtype=torch.float32, w_is_parameter=True)
         with bucket("scan.conv"):
             xc, xr = ops.scan_conv(xz, self.conv, self.conv_bias, cache.state, self.tail_off, ctx, self.inner,
                                    self.taps, x.dtype)
         with bucket("scan.x_proj"):
-            dt_low = ops.linear(xr, self.w_x_dt)
-            bc = ops.linear(xr, self.w_x_bc, out_dtype=torch.float32)
-            dt_raw = ops.linear(dt_low, self.w_dt, out_dtype=torch.float32)
+            dt_low = ops.linear(xr, self.w_x_dt, w_is_parameter=True)
+            bc = ops.linear(xr, self.w_x_bc, out_dtype=torch.float32, w_is_parameter=True)
+            dt_raw = ops.linear(dt_low, self.w_dt, out_dtype=torch.float32, w_is_parameter=True)
         with bucket("scan.recurrence"):
             ops.selective_scan(xz, xc, dt_raw, bc, self.a_log, self.d_skip, self.dt_bias, cache.state, self.tail_off,
                                ctx, out, out_scale, self.inner, self.n_state, self.taps, self.decay_table)

@@ -160,7 +160,7 @@ class SinkAttention(Mixer):
     def forward(self, x, ctx, cache):
         out = self.pre_projection(x, ctx, cache)
         with bucket("attn.o_proj"):
-            return ops.linear(out, self.wo)
+            return ops.linear(out, self.wo, w_is_parameter=True)
 
     def pre_projection(self, x, ctx, cache, out=None, out_scale: float = 1.0):
         """The attended (and gated) heads [n, H * v_dim] in the run dtype, times ``out_scale``; written into ``out``
@@ -173,7 +173,7 @@ class SinkAttention(Mixer):
         before = (-self.keep, cache.kv, tables) if self.keep else pooled         # what is seen before the window
         one_each = ctx.max_q_len == 1             # a token that completes a block finds the block's others in the cache
         with bucket("attn.qkv_proj"):
-            proj = ops.linear(x, self.wqkv, out_dtype=torch.float32)
+            proj = ops.linear(x, self.wqkv, out_dtype=torch.float32, w_is_parameter=True)
         qkv = proj[:, :self.qkv_width]
         gate = proj[:, self.qkv_width:] if self.gate else None
         with bucket("attn.rope"):

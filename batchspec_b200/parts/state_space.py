@@ -68,14 +68,14 @@ class StateSpace(Mixer):
     def forward(self, x, ctx, cache):
         y = self.pre_projection(x, ctx, cache)
         with bucket("state_space.o_proj"):
-            return ops.linear(y, self.wo)
+            return ops.linear(y, self.wo, w_is_parameter=True)
 
     def pre_projection(self, x, ctx, cache, out=None, out_scale: float = 1.0):
         """The normed rows [n, inner] in the run dtype, times ``out_scale``; written into ``out`` (a view of columns of
         wider rows) when given."""
         I, C = self.inner, self.channels
         with bucket("state_space.in_proj"):
-            proj = ops.linear(x, self.w_in, out_dtype=torch.float32)
+            proj = ops.linear(x, self.w_in, out_dtype=torch.float32, w_is_parameter=True)
         xbc, dt = proj[:, I:I + C], proj[:, I + C:]
         with bucket("state_space.conv"):
             conv, _ = ops.scan_conv(xbc, self.conv, self.conv_bias, cache.state, self.tail_off, ctx, C, self.taps)

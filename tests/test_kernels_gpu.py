@@ -117,6 +117,32 @@ def test_sgemm_sums_have_one_order_in_every_kernel(ops, N, K, batch):
     ops.check_status()
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("M", [1, 8, 32])
+def test_a_product_may_be_the_second_operand_of_the_next(ops, dtype, M):
+    """The kernels of this package let their successor start while they still write, so a product whose W the kernel
+    before forms has to wait for it.  Against the same product after a synchronisation."""
+    g = torch.Generator(device=DEV).manual_seed(M)
+    a = torch.randn(2304, 2048, device=DEV, generator=g).to(dtype)
+    b = torch.randn(1024, 2048, device=DEV, generator=g).to(dtype)
+    x = torch.randn(M, 1024, device=DEV, generator=g).to(dtype)
+    first = ops.linear if dtype == torch.float32 else lambda p, q: ops.gemm_tc(p, q, dtype)
+    second = ops.linear if dtype == torch.float32 or M <= 8 else lambda p, q: ops.gemm_tc(p, q, dtype)
+    for _ in range(3):
+        w = first(a, b)
+        got = second(x, w)
+        torch.cuda.synchronize()
+        assert torch.equal(got, second(x, w.clone()))
+        if dtype == torch.float32:
+            xb = x.view(M, 4, 256).transpose(0, 1)
+            k = first(a, b).view(4, 2304, 256)
+            got = ops.linear_batched(xb, k)
+            torch.cuda.synchronize()
+            assert torch.equal(got, ops.linear_batched(xb, k.clone()))
+        assert torch.equal(ops.linear(x, w, w_is_parameter=True), ops.linear(x, w))      # (w has long been written)
+    ops.check_status()
+
+
 @pytest.mark.parametrize("total", [4, 1028, 148 * 32 * 256 * 4 + 4, 148 * 32 * 256 * 20 + 8])
 def test_tanh_softcap_in_quads_and_one_by_one(ops, total):
     """Four numbers at a time, less and more than a thread's four quads, against the kernel of single numbers, which takes
