@@ -581,6 +581,9 @@ selective_scan_kernel(const float* __restrict__ xz, long long ld, const float* _
 }
 
 // One thread per (channel, state): the state carried over the portion's segments; part[segment] takes the state before it.
+// A segment's exponent is the sum of its tokens': near zero, where 1 - exp(x) is what matters, the state moves by the small
+// difference as in scan_update; where most of the state is gone, exp(x) S + end is the form without cancellation (s + (end - s)
+// would leave a rounding of the state before, whole, in the state after).
 // The blocks of state 0 also keep the convolution's last taps - 1 inputs.
 __global__ void __launch_bounds__(128)
 scan_segments_kernel(const float* __restrict__ xz, long long ld, const float* __restrict__ a2t, float* __restrict__ state,
@@ -610,7 +613,8 @@ scan_segments_kernel(const float* __restrict__ xz, long long ld, const float* __
     for (int u = 0; u < 8; ++u)
       if (i0 + u < segs) {
         pp[(i0 + u) * step] = s;
-        s = scan_update(s, __fmul_rn(dts[u], a2), end[u]);
+        const float x = __fmul_rn(dts[u], a2);
+        s = x > -0.5f ? scan_update(s, x, end[u]) : __fmaf_rn(expf(x), s, end[u]);
       }
   }
   sp[(size_t)n * inner + c] = s;

@@ -666,6 +666,35 @@ def test_selective_scan_in_segments(ops, inner, N, taps, lens):
         assert torch.equal(state[slots[e], tail_off:].view(taps - 1, inner), kept), e
 
 
+@pytest.mark.parametrize("N", [16, 32])
+@pytest.mark.parametrize("size", [1e4, 1e5])
+def test_a_state_that_is_gone_leaves_no_rounding_behind_in_segments(ops, N, size):
+    """A start state, and a burst of inputs at a segment's end, far larger than what follows, with decays of exp(-0.5) a
+    token: from the second segment after them on the outputs and the state are held to what is there then."""
+    inner, n = 64, 700
+    gen = torch.Generator(device=DEV).manual_seed(N)
+    rand = lambda *shape: torch.randn(*shape, device=DEV, generator=gen)
+    xz, xc, bc = rand(n, 2 * inner), rand(n, inner), rand(n, 2 * N)
+    xc[318:320] *= size
+    dt_raw = torch.full((n, inner), 0.5, device=DEV).expm1().log()                # softplus of it is 0.5
+    a_log, d_skip, dt_bias = 0.05 * rand(inner, N), rand(inner), torch.zeros(inner, device=DEV)
+    state = rand(1, N * inner) * size
+    before = state.clone()
+    out = torch.empty(n, inner, device=DEV)
+    ctx = SimpleNamespace(qo_indptr=_i32([0, n]), n_entries=1, max_q_len=n, state_slots=_i32([0]))
+    ops.selective_scan(xz, xc, dt_raw, bc, a_log, d_skip, dt_bias, state, N * inner, ctx, out, 1.0, inner, N, 1)
+    x, z, b = xc.double(), xz[:, inner:].double(), bc.double()
+    dt = torch.nn.functional.softplus(dt_raw.double())
+    A, S = -torch.exp(a_log.double()), before.view(N, inner).t().double()
+    want = torch.empty(n, inner, device=DEV, dtype=torch.float64)
+    for t in range(n):
+        S = torch.exp(dt[t, :, None] * A) * S + (dt[t] * x[t])[:, None] * b[t, None, :N]
+        want[t] = (S @ b[t, N:] + d_skip.double() * x[t]) * torch.nn.functional.silu(z[t])
+    for rows in (slice(64, 318), slice(384, n)):                                   # (a token loop is at 1e-6 of these rows)
+        assert (out[rows].double() - want[rows]).abs().max() <= 1e-5 * want[rows].abs().max(), rows
+    assert (state.view(N, inner).t().double() - S).abs().max() <= 1e-5 * S.abs().max()
+
+
 # ------------------------------------------------------------------------------------------- whole models
 
 @pytest.mark.parametrize("dtype", DTYPES)
