@@ -187,7 +187,7 @@ attn_generic_kernel(const T* __restrict__ q, long long q_row_stride, T* __restri
           if (biased) x = __fsub_rn(x, __fmul_rn(slopes[kvh * G + (row0 + r) % G], (float)(seen[r].y - key)));
         }
         const float top = fmaxf(m[r], warp_max(x));
-        const float p = on ? expf(x - top) : 0.f;
+        const float p = x == -INFINITY ? 0.f : expf(x - top);             // (unseen, or a score of -inf in a chunk of nothing else)
         const float corr = m[r] == top ? 1.f : expf(m[r] - top);          // (also where the row sees nothing yet)
         l[r] = fmaf(l[r], corr, p);
         if (corr != 1.f) {

@@ -263,6 +263,31 @@ def test_float32_attention_rows_have_the_same_bits_in_every_portion(ops, Hq, G, 
         assert torch.equal(part, whole[rows]), portion
 
 
+@pytest.mark.parametrize("chunks", [(0,), (1,), (0, 2, 3), (1, 9)])
+@pytest.mark.parametrize("Hq,G,hd", [(4, 4, 16), (8, 1, 64), (2, 1, 256)])
+def test_keys_whose_scores_are_minus_infinity_count_nothing(ops, Hq, G, hd, chunks):
+    """Scores that overflow to -inf in whole chunks of 32 keys, the first and the only chunks of a warp among them: the
+    softmax over the other keys, as in float64."""
+    L, ps = 330, 16
+    ks, vs, cache, ctx, tables, fill, qo = _paged(ops, torch.float32, Hq, G, hd, hd, ps, [5], [L], hd)
+    q = torch.randn(5, Hq, hd, device=DEV, generator=torch.Generator(device=DEV).manual_seed(3))
+    q[:, :, 0] = 3e30
+    ks[0][:, :, 0] = 0
+    gone = torch.zeros(L, dtype=torch.bool)
+    for c in chunks:
+        gone[32 * c:32 * c + 32] = True
+    ks[0][gone.to(DEV), :, 0] = -3e30
+    fill()
+    out = torch.empty(5, Hq * hd, device=DEV)
+    ops.masked_attention(q.view(5, Hq * hd), out, cache, ctx, tables, Hq, G, hd, hd, 0.25)
+    k = ks[0].double().repeat_interleave(Hq // G, 1)
+    v = vs[0].double().repeat_interleave(Hq // G, 1)
+    s = torch.einsum("qhd,khd->hqk", q.double(), k) * 0.25
+    hide = gone.to(DEV)[None, :] | (torch.arange(L, device=DEV)[None, :] > torch.arange(L - 5, L, device=DEV)[:, None])
+    want = torch.einsum("hqk,khd->qhd", s.masked_fill(hide, -math.inf).softmax(-1), v)
+    assert (out.view(5, Hq, hd).double() - want).abs().max() <= 2e-5 * max(1.0, hd / 64)     # the bound of the test above
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("key", [0, 511, 512, 513, 527, 528, 1023, 1024, 1025, 1100, 1299])
 def test_one_key_decides_inside_its_chunk_and_is_unseen_outside(ops, dtype, key):
