@@ -184,7 +184,8 @@ attn_generic_kernel(const T* __restrict__ q, long long q_row_stride, T* __restri
         if (on) {
           x = s[r] * scale;
           if (softcap > 0.f) x = softcap * tanhf(x / softcap);
-          if (biased) x = __fsub_rn(x, __fmul_rn(slopes[kvh * G + (row0 + r) % G], (float)(seen[r].y - key)));
+          // one rounding, fused by name so that every instance has the same bits
+          if (biased) x = __fmaf_rn(-slopes[kvh * G + (row0 + r) % G], (float)(seen[r].y - key), x);
         }
         const float top = fmaxf(m[r], warp_max(x));
         const float p = x == -INFINITY ? 0.f : expf(x - top);             // (unseen, or a score of -inf in a chunk of nothing else)

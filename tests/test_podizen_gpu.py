@@ -279,6 +279,34 @@ def _attention_case(ops, dtype, Hq, G, hd, vd, ps, q_lens, kv_lens, window, pool
     return got, want
 
 
+@pytest.mark.parametrize("Hq,G,hd", [(4, 1, 16), (3, 3, 64), (2, 1, 256)])
+def test_a_distance_bias_is_taken_off_in_one_rounding(ops, Hq, G, hd):
+    """Scores up to 30,000 that the bias takes down to [0, 1]: the product slope * distance alone would be off by up to 1e-3,
+    the fused operation is exact to the last digits of what is left."""
+    L, ps, n = 300, 16, 3
+    i32 = lambda x: torch.tensor(list(x), dtype=torch.int32, device=DEV)
+    g = torch.Generator(device=DEV).manual_seed(hd)
+    slope = torch.full((Hq,), 100.3, device=DEV)
+    dist = torch.arange(L - 1, -1, -1, device=DEV)
+    k, v = torch.zeros(L, G, hd, device=DEV), torch.randn(L, G, hd, device=DEV, generator=g)
+    k[:, :, 0] = (slope[0].double() * dist + torch.rand(L, device=DEV, generator=g).double()).float()[:, None]
+    q = torch.zeros(n, Hq, hd, device=DEV)
+    q[:, :, 0] = 1
+    pages = torch.zeros(-(-L // ps), 2, G, ps, hd, device=DEV)
+    for p in range(L):
+        pages[p // ps, 0, :, p % ps], pages[p // ps, 1, :, p % ps] = k[p], v[p]
+    tables = SimpleNamespace(kv_indptr=i32([0, len(pages)]), kv_indices=i32(range(len(pages))), page_size=ps)
+    ctx = SimpleNamespace(qo_indptr=i32([0, n]), positions=i32(range(L - n, L)), n_entries=1, max_q_len=n)
+    out = torch.empty(n, Hq * hd, device=DEV)
+    ops.masked_attention(q.view(n, -1), out, pages.view(len(pages), -1), ctx, tables, Hq, G, hd, hd, 1.0, slopes=slope)
+    for t in range(n):
+        pos = L - n + t
+        away = (pos - torch.arange(pos + 1, device=DEV)).double()
+        p = (k[:pos + 1, :, 0].double() - slope[0].double() * away[:, None]).softmax(0)
+        want = torch.einsum("jg,jgd->gd", p, v[:pos + 1].double()).repeat_interleave(Hq // G, 0)
+        assert (out[t].view(Hq, hd).double() - want).abs().max() <= 3e-6       # 300 weights and sums of float32
+
+
 BIAS_SHAPES = [
     # Hq, G, hd, vd, page, q_lens, kv_lens, window
     (3, 3, 16, 16, 4, [5, 1, 2], [5, 9, 30], 7),
