@@ -405,7 +405,7 @@ int tile_splits(int M, int N, int K, int batch) {
   if (groups == 1 || tiles >= 4ll * slots || (long long)groups * M * N * batch > SCRATCH_FLOATS) return 1;
   int best = 1;
   double best_cost = 1e30;
-  for (int s = 1; s <= groups; ++s) {
+  for (int s = 1; s <= groups && (long long)s * batch <= 65535; ++s) {       // (batch x splits is a grid's z)
     const int per = (groups + s - 1) / s;
     const double waves = (double)((tiles * s + slots - 1) / slots);
     const double cost = waves * per + (s > 1 ? 0.25 : 0.0);          // the join: a pass over the groups' sums

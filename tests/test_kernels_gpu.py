@@ -117,6 +117,16 @@ def test_sgemm_sums_have_one_order_in_every_kernel(ops, N, K, batch):
     ops.check_status()
 
 
+def test_sgemm_takes_many_products_of_long_sums(ops):
+    """2,000 products of one output column and 64 groups of k: as many K slices as a grid's z still takes."""
+    B, M, K = 2000, 33, 65536
+    g = torch.Generator(device=DEV).manual_seed(5)
+    a, w = torch.randn(M, K, device=DEV, generator=g), torch.randn(B, 1, K, device=DEV, generator=g)
+    got = ops.linear_batched(a.expand(B, M, K), w)
+    for b in (0, 1, 999, B - 1):
+        assert torch.equal(got[b], ops.linear(a, w[b]))
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("M", [1, 8, 32])
 def test_a_product_may_be_the_second_operand_of_the_next(ops, dtype, M):
