@@ -11,7 +11,8 @@
 // Two kernels:
 //   sgemm_rows_kernel  few rows (decode steps): bound by reading W once.  W streams through a ring of shared-memory
 //                      stages by bulk copies, a thread owns one output number and one slice at a time.
-//   sgemm_tile_kernel  everything else: bound by the multiply-adds.  BM x 64 tiles, 8 x 4 outputs per thread.
+//   sgemm_tile_kernel  everything else: bound by the multiply-adds.  BM x 64 tiles, 8 x 4 outputs per thread; 32 x 32 tiles
+//                      where those would leave most of the device idle.
 #include "tma.cuh"
 
 using namespace bspec;
@@ -43,7 +44,7 @@ __device__ __forceinline__ bool sync_and(bool ok) {
 }
 
 // ------------------------------------------------------------------------------------------------ tiles
-// A thread holds rows tm + (BM/8) i and columns tn + 16 j, 8 x 4 outputs.  Both operands lie K-major in shared memory as
+// A thread holds rows tm + (BM/8) i and columns tn + 16 j, TI x TJ = 8 x 4 outputs (32 x 32 tiles: 4 x 2 on 128 threads).  Both operands lie K-major in shared memory as
 // they do in global memory (rows of 32 k and 4 floats of padding): a 16-byte load is two packed operands and nothing is
 // transposed or duplicated.  A warp is 8 x 4 threads, placed so that neighbours share a row of A and neighbours of
 // neighbours a row of W: both loads then take two passes of shared memory instead of four.  The group's running sum waits
@@ -51,9 +52,12 @@ __device__ __forceinline__ bool sync_and(bool ok) {
 // Bound by the arithmetic.  968 x 16,384 x 2,048 on a B200: 1,684 us, 38.6 TFLOP/s (64 x 64 tiles of scalar multiply-adds
 // with synchronous loads before: about 14.6 in a whole prompt); 8 x 8 outputs per thread and one block per SM: 1,784 us;
 // scalar multiply-adds instead of packed ones: 2,047 us.
-constexpr int BN = 64, BK = 32, LDT = BK + 4;
+constexpr int BK = 32, LDT = BK + 4;
 
-constexpr int tile_smem(int bm) { return (2 * (bm + BN) * LDT + bm * BN) * 4; }
+template <int BM> struct Tile {
+  static constexpr int TI = BM == 32 ? 4 : 8, TJ = BM == 32 ? 2 : 4, BN = 16 * TJ, RM = BM / TI, NT = 16 * RM;
+  static constexpr int SMEM = (2 * (BM + BN) * LDT + BM * BN) * 4, PER_SM = BM == 128 ? 2 : 4;
+};
 
 // 16 (VEC) or 4 bytes from global to shared memory, zeros where ``ok`` is false
 template <bool VEC>
@@ -68,16 +72,16 @@ __device__ __forceinline__ void copy_or_zero(float* dst, const float* src, bool 
 // groups s, s + 1, .. of its share; with ``splits`` > 1 group g leaves its sum in part[(z * groups + g) * M * N], which
 // sgemm_join_kernel adds up, else C takes the groups one after the other.
 template <int BM, bool VEC>
-__global__ void __launch_bounds__(BM * 2, BM == 128 ? 2 : 4)
+__global__ void __launch_bounds__(Tile<BM>::NT, Tile<BM>::PER_SM)
 sgemm_tile_kernel(const float* __restrict__ A, const float* __restrict__ W, float* __restrict__ C, float* __restrict__ part,
                   int M, int N, int K, long long lda, long long ldw, long long ldc, long long sa, long long sw, long long sc,
                   int splits) {
   bspec::pdl_prologue(10);
   extern __shared__ __align__(16) float smem_f[];
-  constexpr int NT = BM * 2, RM = BM / 8;
+  constexpr int NT = Tile<BM>::NT, RM = Tile<BM>::RM, BN = Tile<BM>::BN, TI = Tile<BM>::TI, TJ = Tile<BM>::TJ;
   float* as = smem_f;                               // [2][BM][LDT]
   float* ws = as + 2 * BM * LDT;                    // [2][BN][LDT]
-  float* gsum = ws + 2 * BN * LDT;                  // [8][NT][4]: outputs (i, 0..3) of every thread at row i
+  float* gsum = ws + 2 * BN * LDT;                  // [TI][NT][TJ]: outputs (i, 0 .. TJ - 1) of every thread at row i
   const int z = blockIdx.z / splits, split = blockIdx.z % splits;
   A += (size_t)z * sa;
   W += (size_t)z * sw;
@@ -119,11 +123,11 @@ sgemm_tile_kernel(const float* __restrict__ A, const float* __restrict__ W, floa
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
 
-  unsigned long long acc[8][4];
+  unsigned long long acc[TI][TJ];
 #pragma unroll
-  for (int i = 0; i < 8; ++i)
+  for (int i = 0; i < TI; ++i)
 #pragma unroll
-    for (int j = 0; j < 4; ++j) acc[i][j] = 0ull;
+    for (int j = 0; j < TJ; ++j) acc[i][j] = 0ull;
   if (t_begin < t_end) load(t_begin, 0);
   for (int t = t_begin; t < t_end; ++t) {
     const int buf = (t - t_begin) & 1;
@@ -138,32 +142,43 @@ sgemm_tile_kernel(const float* __restrict__ A, const float* __restrict__ W, floa
     const float* w_ = ws + (size_t)(buf * BN + tn) * LDT;
 #pragma unroll
     for (int k = 0; k < BK; k += 4) {
-      ulonglong2 b[4];
+      ulonglong2 b[TJ];
 #pragma unroll
-      for (int j = 0; j < 4; ++j) b[j] = *reinterpret_cast<const ulonglong2*>(w_ + 16 * j * LDT + k);
+      for (int j = 0; j < TJ; ++j) b[j] = *reinterpret_cast<const ulonglong2*>(w_ + 16 * j * LDT + k);
 #pragma unroll
-      for (int i = 0; i < 8; ++i) {
+      for (int i = 0; i < TI; ++i) {
         const ulonglong2 a = *reinterpret_cast<const ulonglong2*>(a_ + RM * i * LDT + k);
 #pragma unroll
-        for (int j = 0; j < 4; ++j) fma2(acc[i][j], a.x, b[j].x);
+        for (int j = 0; j < TJ; ++j) fma2(acc[i][j], a.x, b[j].x);
 #pragma unroll
-        for (int j = 0; j < 4; ++j) fma2(acc[i][j], a.y, b[j].y);
+        for (int j = 0; j < TJ; ++j) fma2(acc[i][j], a.y, b[j].y);
       }
     }
     const int done = (t + 1) * BK;
     if (done % SLICE == 0 || t + 1 == t_end) {
       const bool first = (t * BK) % GROUP < SLICE;                    // the group's first slice
 #pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        float4* at = reinterpret_cast<float4*>(gsum) + i * NT + tid;
+      for (int i = 0; i < TI; ++i) {
         unsigned long long* q = acc[i];
-        float4 v = make_float4(fold2(q[0]), fold2(q[1]), fold2(q[2]), fold2(q[3]));
-        if (!first) {
-          const float4 o = *at;
-          v = make_float4(o.x + v.x, o.y + v.y, o.z + v.z, o.w + v.w);
+        if constexpr (TJ == 4) {
+          float4* at = reinterpret_cast<float4*>(gsum) + i * NT + tid;
+          float4 v = make_float4(fold2(q[0]), fold2(q[1]), fold2(q[2]), fold2(q[3]));
+          if (!first) {
+            const float4 o = *at;
+            v = make_float4(o.x + v.x, o.y + v.y, o.z + v.z, o.w + v.w);
+          }
+          *at = v;
+        } else {
+          float2* at = reinterpret_cast<float2*>(gsum) + i * NT + tid;
+          float2 v = make_float2(fold2(q[0]), fold2(q[1]));
+          if (!first) {
+            const float2 o = *at;
+            v = make_float2(o.x + v.x, o.y + v.y);
+          }
+          *at = v;
         }
-        *at = v;
-        q[0] = q[1] = q[2] = q[3] = 0ull;
+#pragma unroll
+        for (int j = 0; j < TJ; ++j) q[j] = 0ull;
       }
       if (done % GROUP == 0 || t + 1 == t_end) {
         __syncthreads();
@@ -178,7 +193,7 @@ sgemm_tile_kernel(const float* __restrict__ A, const float* __restrict__ W, floa
             // the output's place: row index ri of thread row tmi, column index cj of thread column tni
             const int ri = (i / BN) / RM, tmi = (i / BN) % RM, cj = (i % BN) / 16, tni = i % 16;
             const int owner = (tmi / 8 * 4 + tni / 4) * 32 + (tni & 1) + (tni & 2) * 2 + (tmi & 1) * 2 + (tmi & 6) * 4;
-            const float v = gsum[(ri * NT + owner) * 4 + cj];
+            const float v = gsum[(ri * NT + owner) * TJ + cj];
             *at = set ? v : *at + v;
           }
         }
@@ -383,13 +398,13 @@ int launch_tile(const float* A, const float* W, float* C, float* part, int M, in
   static bool set[bspec::kMaxDevices] = {};
   bool& done = set[bspec::current_device()];
   if (!done) {
-    const cudaError_t e = cudaFuncSetAttribute(sgemm_tile_kernel<BM, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, tile_smem(BM));
+    const cudaError_t e = cudaFuncSetAttribute(sgemm_tile_kernel<BM, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, Tile<BM>::SMEM);
     if (e != cudaSuccess) return (int)e;
     done = true;
   }
-  const dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM, batch * splits);
+  const dim3 grid((N + Tile<BM>::BN - 1) / Tile<BM>::BN, (M + BM - 1) / BM, batch * splits);
   if (grid.y > 65535 || grid.z > 65535) return (int)cudaErrorInvalidConfiguration;
-  BSPEC_LAUNCH((sgemm_tile_kernel<BM, VEC>), grid, BM * 2, tile_smem(BM), stream, A, W, C, part, M, N, K, lda, ldw, ldc, sa, sw, sc,
+  BSPEC_LAUNCH((sgemm_tile_kernel<BM, VEC>), grid, Tile<BM>::NT, Tile<BM>::SMEM, stream, A, W, C, part, M, N, K, lda, ldw, ldc, sa, sw, sc,
                splits);
   return BSPEC_LAUNCH_CHECK();
 }
@@ -398,10 +413,11 @@ constexpr int ROWS_MAX_M = 32;          // most rows of the kernel for few rows
 constexpr long long SCRATCH_FLOATS = 64ll << 20;
 
 // How many blocks along K the tile kernel takes: whole groups each, so that the last wave of blocks is well filled.
+template <int BM>
 int tile_splits(int M, int N, int K, int batch) {
-  const int bm = M > 64 ? 128 : 64, slots = bspec::sm_count() * (bm == 128 ? 2 : 4);
+  const int slots = bspec::sm_count() * Tile<BM>::PER_SM;
   const int groups = (K + GROUP - 1) / GROUP;
-  const long long tiles = (long long)((M + bm - 1) / bm) * ((N + BN - 1) / BN) * batch;
+  const long long tiles = (long long)((M + BM - 1) / BM) * ((N + Tile<BM>::BN - 1) / Tile<BM>::BN) * batch;
   if (groups == 1 || tiles >= 4ll * slots || (long long)groups * M * N * batch > SCRATCH_FLOATS) return 1;
   int best = 1;
   double best_cost = 1e30;
@@ -414,6 +430,18 @@ int tile_splits(int M, int N, int K, int batch) {
   return best;
 }
 
+struct TilePlan {
+  int bm, splits;
+};
+
+// Rows of a tile and blocks along K.  Where the large tiles' blocks are fewer than the SMs, each of them works alone on its SM
+// and a product takes the time of one: 32 x 32 tiles then.
+TilePlan tile_plan(int M, int N, int K, int batch) {
+  const int bm = M > 64 ? 128 : 64, splits = bm == 128 ? tile_splits<128>(M, N, K, batch) : tile_splits<64>(M, N, K, batch);
+  const long long blocks = (long long)((M + bm - 1) / bm) * ((N + 63) / 64) * batch * splits;
+  return blocks < bspec::sm_count() ? TilePlan{32, tile_splits<32>(M, N, K, batch)} : TilePlan{bm, splits};
+}
+
 bool rows_of_16_bytes(const float* A, const float* W, int K, long long lda, long long ldw, long long sa, long long sw) {
   return ((K | lda | ldw | sa | sw) & 3) == 0 && (((uintptr_t)A | (uintptr_t)W) & 15) == 0;
 }
@@ -423,7 +451,7 @@ bool rows_of_16_bytes(const float* A, const float* W, int K, long long lda, long
 BSPEC_API long long bspec_sgemm_scratch(const float* A, const float* W, int M, int N, int K, long long lda, long long ldw,
                                         long long sa, long long sw, int batch) {
   if (M <= 0 || N <= 0 || K <= 0 || batch <= 0 || (M <= ROWS_MAX_M && rows_of_16_bytes(A, W, K, lda, ldw, sa, sw))) return 0;
-  return tile_splits(M, N, K, batch) > 1 ? (long long)((K + GROUP - 1) / GROUP) * M * N * batch : 0;
+  return tile_plan(M, N, K, batch).splits > 1 ? (long long)((K + GROUP - 1) / GROUP) * M * N * batch : 0;
 }
 
 // `batch` products C_b = A_b * W_b^T whose operands lie sa / sw / sc elements apart.  ``scratch``: bspec_sgemm_scratch
@@ -439,8 +467,10 @@ BSPEC_API int bspec_sgemm_tn_batched(const float* A, const float* W, float* C, i
     auto fn = M == 1 ? launch_rows<1> : (M == 2 ? launch_rows<2> : (M <= 4 ? launch_rows<4> : launch_rows<8>));
     return fn(A, W, C, M, N, K, lda, ldw, ldc, sa, sw, sc, batch, w_ahead, status, stream);
   }
-  const int groups = (K + GROUP - 1) / GROUP, splits = K > 0 && scratch != nullptr ? tile_splits(M, N, K, batch) : 1;
-  auto fn = M > 64 ? (vec ? launch_tile<128, true> : launch_tile<128, false>) : (vec ? launch_tile<64, true> : launch_tile<64, false>);
+  const TilePlan plan = tile_plan(M, N, K, batch);
+  const int groups = (K + GROUP - 1) / GROUP, splits = K > 0 && scratch != nullptr ? plan.splits : 1;
+  auto fn = plan.bm == 128 ? (vec ? launch_tile<128, true> : launch_tile<128, false>)
+            : (plan.bm == 64 ? (vec ? launch_tile<64, true> : launch_tile<64, false>) : (vec ? launch_tile<32, true> : launch_tile<32, false>));
   const int err = fn(A, W, C, scratch, M, N, K, lda, ldw, ldc, sa, sw, sc, batch, splits, stream);
   if (err != 0 || splits == 1) return err;
   const long long blocks = ((long long)M * N + 255) / 256;

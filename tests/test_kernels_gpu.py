@@ -96,11 +96,12 @@ def test_sgemm_is_true_float32(ops, M, N, K):
     assert torch.equal(got[:1], ops.linear(a[:1].contiguous(), w))
 
 
-@pytest.mark.parametrize("N,K", [(1, 4), (17, 60), (64, 68), (130, 1020), (65, 1028), (48, 4100), (33, 1027)])
+@pytest.mark.parametrize("N,K", [(1, 4), (17, 60), (64, 68), (130, 1020), (65, 1028), (48, 4100), (33, 1027), (2500, 2052),
+                                 (9617, 516), (9617, 2052), (9617, 1027)])
 @pytest.mark.parametrize("batch", [1, 3])
 def test_sgemm_sums_have_one_order_in_every_kernel(ops, N, K, batch):
-    """Few rows, tiles of 64 and of 128 rows, K slices in scratch, 4-byte copies (odd K): every row has the same bits in
-    all of them, and the error of sums of K / 2 terms in chains of 32."""
+    """Few rows (one tile of W per block, and many: 9,617 columns), tiles of 32, 64 and 128 rows, K slices in scratch, 4-byte
+    copies (odd K): every row has the same bits in all of them, and the error of sums of K / 2 terms in chains of 32."""
     g = torch.Generator(device=DEV).manual_seed(N + K)
     a = torch.randn(batch, 150, K, device=DEV, generator=g)
     w = torch.randn(batch, N, K, device=DEV, generator=g)
