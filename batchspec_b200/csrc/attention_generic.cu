@@ -3,7 +3,7 @@
 // storage, float32 arithmetic throughout.  A block holds R consecutive (query token, query head of the group) rows of one
 // request and kv head.  Keys are visited in chunks of 32 that start at multiples of 32 of the key index; chunk c goes to
 // warp c % W, which keeps a running softmax of its chunks for every row, and the warps' results are joined in their order
-// at the end.  So the order of every sum depends only on the query's own position (and the head sizes, which choose W),
+// at the end.  (attn_row_kernel below: one warp per row, which takes the W shares of the chunks one after the other.)  So the order of every sum depends only on the query's own position (and the head sizes, which choose W),
 // not on how the request was cut into steps or on what else is in the batch: a key that a row does not see adds an
 // exact nothing.
 //
@@ -52,6 +52,39 @@ template <int ND> struct Shape { static constexpr int W = ND == 8 ? 4 : 8, LDK =
 constexpr int attn_smem(int nd, int r) {
   const int w = nd == 8 ? 4 : 8;
   return (w * 32 * (32 * nd + 4) + r * 32 * nd + w * r * 32 + 2 * w * r) * 4 + w * 32 * 16 + r * 8 * 2;
+}
+
+// One row's results, ``n`` shares in their order: part[w * part_step + d] with maximum and sum at ml[w * ml_step].  ``gp``: one
+// gate logit per output number, or (gate_per_head) one per head.
+template <typename T, int ND>
+__device__ __forceinline__ void join_row(const float* part, int part_step, const float* ml, int ml_step, int n,
+                                         const float* __restrict__ sink, T* __restrict__ op, int vd,
+                                         const float* __restrict__ gp, int gate_per_head, float out_scale) {
+  const int lane = threadIdx.x & 31;
+  float top = sink != nullptr ? *sink : -INFINITY;
+  for (int w = 0; w < n; ++w) top = fmaxf(top, ml[w * ml_step]);
+  float sum = 0.f, o[ND];
+#pragma unroll
+  for (int i = 0; i < ND; ++i) o[i] = 0.f;
+  for (int w = 0; w < n; ++w) {
+    const float mw = ml[w * ml_step], lw = ml[w * ml_step + 1];
+    if (mw == -INFINITY && lw == 0.f) continue;             // the share has no key for this row
+    const float f = expf(mw - top);
+    sum = fmaf(lw, f, sum);
+#pragma unroll
+    for (int i = 0; i < ND; ++i) o[i] = fmaf(part[(size_t)w * part_step + lane + 32 * i], f, o[i]);
+  }
+  if (sink != nullptr) sum += expf(*sink - top);            // one more term of the denominator only
+  const float inv = 1.f / sum;
+#pragma unroll
+  for (int i = 0; i < ND; ++i) {
+    const int d = lane + 32 * i;
+    if (d < vd) {
+      float x = o[i] * inv;
+      if (gp != nullptr) x = x / (1.f + expf(-gp[gate_per_head ? 0 : d]));
+      op[d] = from_f32<T>(x * out_scale);
+    }
+  }
 }
 
 template <typename T, int ND, int R>
@@ -252,34 +285,124 @@ attn_generic_kernel(const T* __restrict__ q, long long q_row_stride, T* __restri
   __syncthreads();
   for (int r = warp; r < nr; r += W) {
     const int t = q_begin + (row0 + r) / G, h = kvh * G + (row0 + r) % G;
-    float top = sink != nullptr ? sink[h] : -INFINITY;
-    for (int w = 0; w < W; ++w) top = fmaxf(top, ml[(w * R + r) * 2]);
-    float sum = 0.f, o[ND];
+    join_row<T, ND>(part + (size_t)r * D, R * D, ml + 2 * r, 2 * R, W, sink != nullptr ? sink + h : nullptr,
+                    out + (size_t)t * out_stride + (size_t)h * vd, vd,
+                    gate != nullptr ? gate + (size_t)t * gate_stride + (size_t)h * (gate_per_head ? 1 : vd) : nullptr, gate_per_head,
+                    out_scale);
+  }
+}
+
+// One warp per (query token, query head) row, for short requests and for many rows with keys of their own (by_rows):
+// nothing is shared or staged, a lane reads its key itself, so a block needs a few KB instead of the 70 to 140 that keep one to
+// three blocks on an SM above, and little code.  A warp takes the shares of the chunks one after the other, each from an empty
+// softmax, and joins them as the kernel above does: a row has the same bits in both.
+constexpr int ROW_WARPS = 4;
+
+constexpr int attn_row_smem(int nd, int warps) { return warps * (32 * nd + (nd == 8 ? 4 : 8) * (32 * nd + 2)) * 4; }
+
+template <typename T, int ND>
+__global__ void __launch_bounds__(ROW_WARPS * 32)
+attn_row_kernel(const T* __restrict__ q, long long q_row_stride, T* __restrict__ out,
+                const T* __restrict__ cache, const int* __restrict__ qo_indptr,
+                const int* __restrict__ positions, const int* __restrict__ kv_indptr,
+                const int* __restrict__ kv_indices, int Hq, int Hkv, int hd, int page_size, float scale,
+                int window, long long n_pages, int vd, int chunk, const float* __restrict__ sink,
+                float softcap, int v_is_k, const float* __restrict__ gate, long long gate_stride,
+                long long out_stride, float out_scale, int gate_per_head, const float* __restrict__ slopes,
+                int pool, const T* __restrict__ pool_cache, const int* __restrict__ pool_indptr,
+                const int* __restrict__ pool_indices, long long pool_pages) {
+  bspec::pdl_prologue(7);
+  constexpr int W = Shape<ND>::W, D = 32 * ND;
+  extern __shared__ __align__(16) float smem_f[];
+  const int e = blockIdx.y, kvh = blockIdx.z, G = Hq / Hkv, warps = blockDim.x >> 5;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int q_begin = qo_indptr[e], rows = (qo_indptr[e + 1] - q_begin) * G;
+  const int row = (int)(gridDim.x - 1 - blockIdx.x) * warps + warp;
+  if (row >= rows) return;
+  const int t = q_begin + row / G, h = kvh * G + row % G;
+  float* qs = smem_f + warp * (D + W * (D + 2));
+  float* part = qs + D;                                     // [W][D]
+  float* ml = part + W * D;                                 // [W][2]
+  const T* qp = q + (size_t)t * q_row_stride + (size_t)h * hd;
+  for (int d = lane; d < hd; d += 32) qs[d] = to_f32(qp[d]);
+  const int pos = positions[t], *table = kv_indices + kv_indptr[e];
+  int lo = window > 0 ? max(0, pos - window + 1) : 0;
+  if (chunk > 0) lo = max(lo, (pos / chunk) * chunk);
+  const int before = pool != 0 ? bspec::pooled_seen(pos, window, pool) : 0;
+  const size_t k_elems = (size_t)Hkv * page_size * hd;
+  const size_t page_elems = k_elems + (v_is_k ? (size_t)0 : (size_t)Hkv * page_size * vd);
+  const float slope = slopes != nullptr ? slopes[h] : 0.f;
+  float acc[ND], m, l;                                      // l: this lane's keys only
+  __syncwarp();
+  auto visit = [&](int share, int lo_, int hi_, const int* tab, const T* base, long long pages, bool biased) {
+    if (hi_ < lo_) return;
+    const bool vec = ((hd | (int)page_elems) & 3) == 0 && ((uintptr_t)base & (4 * sizeof(T) - 1)) == 0;     // keys start on whole quads
+    for (int c = lo_ / 32 + (share + W - lo_ / 32 % W) % W; c <= hi_ / 32; c += W) {
+      const int key = 32 * c + lane;
+      bool on = key >= lo_ && key <= hi_;
+      if (on && !bspec::in_range(tab[key / page_size], pages, 107)) on = false;
+      long long vo = -1;
+      float x = -INFINITY;
+      if (on) {
+        const size_t page = (size_t)tab[key / page_size] * page_elems;
+        const size_t at = (size_t)kvh * page_size + (size_t)(key % page_size);
+        const T* kp = base + page + at * hd;
+        vo = (long long)(page + (v_is_k ? at * hd : k_elems + at * vd));
+        float dot = 0.f;
+        if (vec) {
+#pragma unroll 4
+          for (int d = 0; d < hd; d += 4) {
+            const float4 k4 = load4(kp + d), q4 = *reinterpret_cast<const float4*>(qs + d);
+            dot = fmaf(q4.x, k4.x, dot);
+            dot = fmaf(q4.y, k4.y, dot);
+            dot = fmaf(q4.z, k4.z, dot);
+            dot = fmaf(q4.w, k4.w, dot);
+          }
+        } else {
+          for (int d = 0; d < hd; ++d) dot = fmaf(qs[d], to_f32(kp[d]), dot);
+        }
+        x = dot * scale;
+        if (softcap > 0.f) x = softcap * tanhf(x / softcap);
+        if (biased) x = __fmaf_rn(-slope, (float)(pos - key), x);
+      }
+      const float top = fmaxf(m, warp_max(x));
+      const float p = x == -INFINITY ? 0.f : expf(x - top);
+      const float corr = m == top ? 1.f : expf(m - top);
+      l = fmaf(l, corr, p);
+      if (corr != 1.f) {
 #pragma unroll
-    for (int i = 0; i < ND; ++i) o[i] = 0.f;
-    for (int w = 0; w < W; ++w) {
-      const float mw = ml[(w * R + r) * 2], lw = ml[(w * R + r) * 2 + 1];
-      if (mw == -INFINITY && lw == 0.f) continue;           // the warp had no key for this row
-      const float f = expf(mw - top);
-      sum = fmaf(lw, f, sum);
+        for (int i = 0; i < ND; ++i) acc[i] *= corr;
+      }
+      m = top;
+      const int last = min(31, hi_ - 32 * c);
+#pragma unroll 4
+      for (int k = 0; k <= last; ++k) {
+        const float pk = __shfl_sync(0xffffffffu, p, k);
+        const long long at = __shfl_sync(0xffffffffu, vo, k);
+        if (pk != 0.f) {                                    // an unseen key's value may be anything
 #pragma unroll
-      for (int i = 0; i < ND; ++i) o[i] = fmaf(part[(size_t)(w * R + r) * D + lane + 32 * i], f, o[i]);
-    }
-    if (sink != nullptr) sum += expf(sink[h] - top);        // one more term of the denominator only
-    const float inv = 1.f / sum;
-    T* op = out + (size_t)t * out_stride + (size_t)h * vd;
-    // one gate logit per output number, or (gate_per_head) one per head: row [Hq] instead of [Hq * vd]
-    const float* gp = gate != nullptr ? gate + (size_t)t * gate_stride + (size_t)h * (gate_per_head ? 1 : vd) : nullptr;
-#pragma unroll
-    for (int i = 0; i < ND; ++i) {
-      const int d = lane + 32 * i;
-      if (d < vd) {
-        float x = o[i] * inv;
-        if (gp != nullptr) x = x / (1.f + expf(-gp[gate_per_head ? 0 : d]));
-        op[d] = from_f32<T>(x * out_scale);
+          for (int i = 0; i < ND; ++i)
+            if (lane + 32 * i < vd) acc[i] = fmaf(pk, to_f32(base[at + lane + 32 * i]), acc[i]);
+        }
       }
     }
+  };
+  const int last_share = min(W - 1, max(pos, before - 1) / 32);             // the shares behind it have no chunk
+  for (int share = 0; share <= last_share; ++share) {
+    m = -INFINITY, l = 0.f;
+#pragma unroll
+    for (int i = 0; i < ND; ++i) acc[i] = 0.f;
+    if (pool < 0) visit(share, 0, before - 1, table, cache, n_pages, slopes != nullptr);
+    if (pool > 0) visit(share, 0, before - 1, pool_indices + pool_indptr[e], pool_cache, pool_pages, false);
+    visit(share, lo, pos, table, cache, n_pages, slopes != nullptr);
+    const float sum = warp_sum(l);
+    if (lane == 0) ml[2 * share] = m, ml[2 * share + 1] = sum;
+#pragma unroll
+    for (int i = 0; i < ND; ++i) part[share * D + lane + 32 * i] = acc[i];
   }
+  __syncwarp();
+  join_row<T, ND>(part, D, ml, 2, last_share + 1, sink != nullptr ? sink + h : nullptr, out + (size_t)t * out_stride + (size_t)h * vd, vd,
+                  gate != nullptr ? gate + (size_t)t * gate_stride + (size_t)h * (gate_per_head ? 1 : vd) : nullptr, gate_per_head, out_scale);
 }
 
 template <typename T, int ND, int R, typename... Args>
@@ -297,11 +420,50 @@ int launch_shape(int n_entries, int max_rows, int Hkv, cudaStream_t stream, Args
   return BSPEC_LAUNCH_CHECK();
 }
 
+template <typename T, int ND, typename... Args>
+int launch_rows(int n_entries, int max_rows, int Hkv, cudaStream_t stream, Args... args) {
+  const int warps = min(ROW_WARPS, max_rows);
+  const dim3 grid((max_rows + warps - 1) / warps, n_entries, Hkv);
+  if (grid.y > 65535 || grid.z > 65535) return (int)cudaErrorInvalidConfiguration;
+  BSPEC_LAUNCH((attn_row_kernel<T, ND>), grid, warps * 32, attn_row_smem(ND, warps), stream, args...);
+  return BSPEC_LAUNCH_CHECK();
+}
+
 // R by the rows of the longest portion: 4 for decode steps of groups of up to four heads (a row that is not there costs as
 // much as one that is), else 16 (8 where heads of more than 128 numbers would not leave the registers for it).
+constexpr int rows_of_block(int width, int max_rows) { return max_rows <= 4 ? 4 : (width <= 128 ? 16 : 8); }
+
+// Whether a row's keys are so few, or the rows so many, that a warp per row is faster.  ``keys``: no request has more (0: not
+// known, or a captured step's bound).  us, blocks of R rows / a warp per row; heads are query heads / kv heads x size, float32
+// unless said:
+//   prompts of up to 32 keys: 7 tokens 32/8 x 64 16 / 6, 24/8 x 128 22 / 8; 64 requests of 20 tokens 260 / 65 and 279 / 73;
+//   prompts of up to 64 keys that fill the device: 200 of 60 tokens 2,873 / 1,394 (one of 61 tokens 17 / 26: not);
+//   decode up to 64 keys where the device is filled twice: 300 requests of 50 keys 24/8 x 128 372 / 113, 12/2 x 64 69 / 31, 16/1 x 256
+//   131 / 113; 64 of 30 keys 24/8 x 128 54 / 26 (32/8 x 64, filled 1.7 times, 18 / 19: not);
+//   decode up to 32 keys: groups of more than four heads, R = 16 for them, 64 requests of 30 keys 5/1 x 64 16 / 12, 64/4 x 128
+//   47 / 32 (16/1 x 256, R = 8, 29 / 36: not); rows with keys of their own, 32/32 x 96 176 / 23; bfloat16, whose keys a block
+//   stages through registers, 32/8 x 64 24 / 20, 16/1 x 256 38 / 35 (4/1 x 16 9.4 / 10.1: not);
+//   decode at any length where the device is filled often and most rows of a block are not there: one row of four, 64 requests of
+//   1,000 keys 32/32 x 96 1,162 / 736, bfloat16 1,716 / 647 (8/8 x 128, filled 3.5 times, 341 / 746: not); two of four in bfloat16.
+bool by_rows(bool bf16, int width, int n_entries, int max_rows, int max_q_len, int Hkv, int keys) {
+  const int R = rows_of_block(width, max_rows), nd = width <= 64 ? 2 : (width <= 128 ? 4 : 8), G = max_rows / max_q_len;
+  const double full = bspec::sm_count() * (double)((227 * 1024) / (attn_smem(nd, R) + 1024));
+  const double waves = (double)((max_rows + R - 1) / R) * n_entries * Hkv / full;
+  const bool few = keys > 0 && keys <= 32, some = keys > 0 && keys <= 64;
+  if (max_q_len > 1) return few || (some && waves >= (width > 64 ? 2 : 1.5));
+  if (few && ((G > 4 && width <= 128) || (G == 1 && (width > 64 || waves >= 1)) || (bf16 && width >= 32))) return true;
+  return (some && waves >= 2) || (G == 1 && waves >= (width > 64 ? 5 : 8)) || (G == 2 && bf16 && width > 64 && waves >= 8);
+}
+
 template <typename T, typename... Args>
-int launch_sizes(int width, int n_entries, int max_rows, int Hkv, cudaStream_t stream, Args... args) {
-  if (max_rows <= 4) {
+int launch_sizes(int width, int n_entries, int max_rows, int max_q_len, int Hkv, int max_kv_len, cudaStream_t stream, Args... args) {
+  if (by_rows(sizeof(T) == 2, width, n_entries, max_rows, max_q_len, Hkv, max_kv_len)) {
+    if (width <= 64) return launch_rows<T, 2>(n_entries, max_rows, Hkv, stream, args...);
+    if (width <= 128) return launch_rows<T, 4>(n_entries, max_rows, Hkv, stream, args...);
+    return launch_rows<T, 8>(n_entries, max_rows, Hkv, stream, args...);
+  }
+  const int R = rows_of_block(width, max_rows);
+  if (R == 4) {
     if (width <= 64) return launch_shape<T, 2, 4>(n_entries, max_rows, Hkv, stream, args...);
     if (width <= 128) return launch_shape<T, 4, 4>(n_entries, max_rows, Hkv, stream, args...);
     return launch_shape<T, 8, 4>(n_entries, max_rows, Hkv, stream, args...);
@@ -321,7 +483,7 @@ static int launch_attention_generic(const void* q, long long q_row_stride, void*
                                     const float* sink, float softcap, int v_is_k, const float* gate,
                                     long long gate_stride, long long out_stride, float out_scale, int gate_per_head,
                                     const float* slopes, int pool, const void* pool_cache, const int* pool_indptr,
-                                    const int* pool_indices, long long pool_pages, cudaStream_t stream) {
+                                    const int* pool_indices, long long pool_pages, int max_kv_len, cudaStream_t stream) {
   if (n_entries <= 0 || max_q_len <= 0) return 0;
   if ((pool != 0 && window <= 0) || (pool > 0 && (v_is_k || pool_cache == nullptr || pool_indptr == nullptr)))
     return (int)cudaErrorInvalidValue;
@@ -331,11 +493,11 @@ static int launch_attention_generic(const void* q, long long q_row_stride, void*
   if (max_rows > (1 << 30)) return (int)cudaErrorInvalidConfiguration;
   const int width = hd > vd ? hd : vd;
   if (dtype == BSPEC_F32)
-    return launch_sizes<float>(width, n_entries, (int)max_rows, Hkv, stream, (const float*)q, q_row_stride, (float*)out,
+    return launch_sizes<float>(width, n_entries, (int)max_rows, max_q_len, Hkv, max_kv_len, stream, (const float*)q, q_row_stride, (float*)out,
                                (const float*)cache, qo_indptr, positions, kv_indptr, kv_indices, Hq, Hkv, hd, page_size, scale,
                                window, n_pages, vd, chunk, sink, softcap, v_is_k, gate, gate_stride, out_stride, out_scale,
                                gate_per_head, slopes, pool, (const float*)pool_cache, pool_indptr, pool_indices, pool_pages);
-  return launch_sizes<__nv_bfloat16>(width, n_entries, (int)max_rows, Hkv, stream, (const __nv_bfloat16*)q, q_row_stride,
+  return launch_sizes<__nv_bfloat16>(width, n_entries, (int)max_rows, max_q_len, Hkv, max_kv_len, stream, (const __nv_bfloat16*)q, q_row_stride,
                                      (__nv_bfloat16*)out, (const __nv_bfloat16*)cache, qo_indptr, positions, kv_indptr, kv_indices,
                                      Hq, Hkv, hd, page_size, scale, window, n_pages, vd, chunk, sink, softcap, v_is_k, gate,
                                      gate_stride, out_stride, out_scale, gate_per_head, slopes, pool, (const __nv_bfloat16*)pool_cache,
@@ -350,13 +512,13 @@ BSPEC_API int bspec_attention_generic(const void* q, long long q_row_stride, voi
   return launch_attention_generic(q, q_row_stride, out, cache, dtype, qo_indptr, positions, kv_indptr, kv_indices,
                                   n_entries, max_q_len, Hq, Hkv, hd, page_size, scale, window, n_pages, hd, 0, nullptr,
                                   0.f, 0, nullptr, 0, (long long)Hq * hd, 1.f, 0, nullptr, 0, nullptr, nullptr, nullptr,
-                                  0, stream);
+                                  0, 0, stream);
 }
 
 // The same with values of their own size ``vd``, a chunk mask (0: none), a sink per query head (null: none), a soft
 // cap on the scores (0: none), values that are the keys, a sigmoid gate on the output (per number, or per head), an
 // output scale and stride, a distance bias (slopes per query head, null: none) and pooled blocks or kept first tokens
-// before the window (pool > 0 or < 0; 0: none).
+// before the window (pool > 0 or < 0; 0: none).  ``max_kv_len``: no request has more keys (0: not known).
 BSPEC_API int bspec_attention_masked(const void* q, long long q_row_stride, void* out, const void* cache, int dtype,
                                      const int* qo_indptr, const int* positions, const int* kv_indptr,
                                      const int* kv_indices, int n_entries, int max_q_len, int Hq, int Hkv, int hd,
@@ -365,11 +527,11 @@ BSPEC_API int bspec_attention_masked(const void* q, long long q_row_stride, void
                                      long long gate_stride, long long out_stride, float out_scale,
                                      int gate_per_head, const float* slopes, int pool, const void* pool_cache,
                                      const int* pool_indptr, const int* pool_indices, long long pool_pages,
-                                     cudaStream_t stream) {
+                                     int max_kv_len, cudaStream_t stream) {
   return launch_attention_generic(q, q_row_stride, out, cache, dtype, qo_indptr, positions, kv_indptr, kv_indices,
                                   n_entries, max_q_len, Hq, Hkv, hd, page_size, scale, window, n_pages, vd, chunk, sink,
                                   softcap, v_is_k, gate, gate_stride, out_stride, out_scale, gate_per_head, slopes, pool,
-                                  pool_cache, pool_indptr, pool_indices, pool_pages, stream);
+                                  pool_cache, pool_indptr, pool_indices, pool_pages, max_kv_len, stream);
 }
 
 // ---------------------------------------------------------------- q/k/v preparation

@@ -74,7 +74,7 @@ _SIGNATURES = {
     "bspec_attention_masked": [c_void_p, c_longlong, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p,
                                c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_int, c_int, c_void_p,
                                c_longlong, c_float, c_int, c_void_p, c_longlong, c_longlong, c_float, c_int, c_void_p,
-                               c_int, c_void_p, c_void_p, c_void_p, c_longlong, c_void_p],
+                               c_int, c_void_p, c_void_p, c_void_p, c_longlong, c_int, c_void_p],
     "bspec_delta_prepare": [c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_int, c_void_p,
                             c_longlong, c_longlong, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int,
                             c_int, c_int, c_int, c_float, c_float, c_void_p],
@@ -871,7 +871,7 @@ def paged_attention(qkv: torch.Tensor, out: torch.Tensor, cache: torch.Tensor, c
         ctx.qo_indptr.data_ptr(), ctx.positions.data_ptr(), tables.kv_indptr.data_ptr(), tables.kv_indices.data_ptr(),
         ctx.n_entries, ctx.max_q_len, n_heads, n_kv_heads, head_dim, head_dim, tables.page_size, float(scale),
         int(window), int(chunk), _ptr(sink), cache.shape[0], float(softcap), 0, None, 0, out.stride(0), 1.0, 0, _ptr(slopes),
-        *_pool_args(pooled, cache, tables.page_size), _stream()), "attention_generic")
+        *_pool_args(pooled, cache, tables.page_size), getattr(ctx, "max_kv_len", 0), _stream()), "attention_generic")
 
 
 def qkv_prepare(qkv: torch.Tensor, n_heads: int, n_kv_heads: int, head_dim: int, v_dim: int,
@@ -963,7 +963,7 @@ def masked_attention(q: torch.Tensor, out: torch.Tensor, cache: torch.Tensor, ct
         ctx.max_q_len, n_heads, n_kv_heads, head_dim, v_dim, tables.page_size, float(scale), int(window), int(chunk),
         _ptr(sink), cache.shape[0], float(softcap), int(bool(values_are_keys)), _ptr(gate),
         gate.stride(0) if gate is not None else 0, out.stride(0), float(out_scale), int(bool(gate_per_head)), _ptr(slopes),
-        *_pool_args(pooled, cache, tables.page_size), _stream()), "attention_masked")
+        *_pool_args(pooled, cache, tables.page_size), getattr(ctx, "max_kv_len", 0), _stream()), "attention_masked")
 
 
 # ---------------------------------------------------------------------------- gated delta rule

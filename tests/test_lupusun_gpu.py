@@ -263,6 +263,28 @@ def test_float32_attention_rows_have_the_same_bits_in_every_portion(ops, Hq, G, 
         assert torch.equal(part, whole[rows]), portion
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("Hq,G,hd,n_req", [(32, 32, 64, 40), (48, 48, 128, 200), (16, 4, 96, 300), (6, 6, 256, 250), (20, 1, 40, 60)])
+def test_attention_rows_have_the_same_bits_in_full_and_idle_grids(ops, dtype, Hq, G, hd, n_req):
+    """Decode steps of many requests, of which the smallest and the largest take a warp per row, against each request alone,
+    with its number of keys known (short ones: a warp per row), not known, a bound far above, and too small, which is no error."""
+    ps = 16
+    lens = [1 + (29 * i) % 300 for i in range(n_req)]
+    ks, vs, cache, ctx, tables, fill, qo = _paged(ops, dtype, Hq, G, hd, hd, ps, [1] * n_req, lens, hd)
+    cache.normal_(generator=torch.Generator(device=DEV).manual_seed(9))
+    q = torch.randn(n_req, Hq * hd, device=DEV, generator=torch.Generator(device=DEV).manual_seed(3)).to(dtype)
+    out = torch.empty(n_req, Hq * hd, device=DEV, dtype=dtype)
+    ops.masked_attention(q, out, cache, ctx, tables, Hq, G, hd, hd, 0.1)
+    for e in (0, 1, 7, n_req // 2, n_req - 1):
+        one = SimpleNamespace(qo_indptr=_i32([0, 1]), positions=ctx.positions[e:e + 1], n_entries=1, max_q_len=1)
+        tab = SimpleNamespace(kv_indptr=tables.kv_indptr[e:e + 2].contiguous(), kv_indices=tables.kv_indices, page_size=ps)
+        got = torch.empty(1, Hq * hd, device=DEV, dtype=dtype)
+        for bound in (0, lens[e], 4096, max(1, lens[e] // 3)):
+            one.max_kv_len = bound
+            ops.masked_attention(q[e:e + 1], got, cache, one, tab, Hq, G, hd, hd, 0.1)
+            assert torch.equal(got[0], out[e]), (e, bound)
+
+
 @pytest.mark.parametrize("chunks", [(0,), (1,), (0, 2, 3), (1, 9)])
 @pytest.mark.parametrize("Hq,G,hd", [(4, 4, 16), (8, 1, 64), (2, 1, 256)])
 def test_keys_whose_scores_are_minus_infinity_count_nothing(ops, Hq, G, hd, chunks):
