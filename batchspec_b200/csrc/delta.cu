@@ -399,13 +399,13 @@ delta_recurrence_kernel(const float* __restrict__ mix, const float* __restrict__
 // d = beta c_t, e = beta.
 __global__ void __launch_bounds__(128)
 delta_tiles_prepare_kernel(const float* __restrict__ mix, const float* __restrict__ gates, const int* __restrict__ qo_indptr,
-                           float* __restrict__ coef, int H, int Gk, int dim, int vdim) {
+                           int n_entries, float* __restrict__ coef, int H, int Gk, int dim, int vdim) {
   bspec::pdl_prologue(60);
   __shared__ float qs[ST_B][MAX_DIM + 8], ks[ST_B][MAX_DIM + 8];        // (rows eight banks apart)
   __shared__ float dots[ST_B][ST_B], y[ST_B][ST_B], be[ST_B], g[ST_B], low[ST_B][ST_B], inv[ST_B][ST_B];
-  const int i = blockIdx.x, h = blockIdx.y, e = blockIdx.z;
-  const int q_begin = qo_indptr[e], n = qo_indptr[e + 1] - q_begin;
-  if (n < ST_FROM || i * ST_B >= n) return;
+  const int h = blockIdx.y, e = state_tile_entry(qo_indptr, n_entries, blockIdx.x);
+  const int q_begin = qo_indptr[e], n = qo_indptr[e + 1] - q_begin, i = blockIdx.x - (int)state_tile_slot(q_begin, e, 0);
+  if (n < ST_FROM || i * ST_B >= n) return;                    // (i >= 0: the first entry's slots begin at 0)
   const int cnt = min(ST_B, n - i * ST_B), C = 2 * Gk * dim + H * vdim, kh = h / (H / Gk);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 #pragma unroll
@@ -708,14 +708,14 @@ BSPEC_API long long bspec_delta_scratch(int n, int n_entries, int max_q_len, int
 
 BSPEC_API int bspec_delta_recurrence(const float* mix, const float* gates, const float* proj, int ld, float* state,
                                      long long state_stride, long long tail_off, const int* qo_indptr,
-                                     const int* state_slots, float* out, int n_entries, int min_q_len, int max_q_len, int H, int Gk,
+                                     const int* state_slots, float* out, int n, int n_entries, int min_q_len, int H, int Gk,
                                      int dim, int vdim, int taps, float* scratch, cudaStream_t stream) {
   if (n_entries <= 0) return 0;
   if (dim <= 0 || dim > MAX_DIM || H % Gk != 0 || n_entries > 65535 || H > 65535)
     return (int)cudaErrorInvalidValue;
   if (scratch != nullptr) {
-    BSPEC_LAUNCH(delta_tiles_prepare_kernel, dim3((max_q_len + ST_B - 1) / ST_B, H, n_entries), 128, 0, stream, mix, gates,
-                 qo_indptr, scratch, H, Gk, dim, vdim);
+    BSPEC_LAUNCH(delta_tiles_prepare_kernel, dim3((unsigned)bspec::state_tile_slots(n, n_entries), H), 128, 0, stream, mix, gates,
+                 qo_indptr, n_entries, scratch, H, Gk, dim, vdim);
     const int err = BSPEC_LAUNCH_CHECK();
     if (err != 0) return err;
     const dim3 tiles((vdim + ST_COLS - 1) / ST_COLS, H, n_entries);

@@ -225,13 +225,13 @@ lightning_recurrence_kernel(const float* __restrict__ proj, long long ld, int q_
 // block of a head would repeat otherwise: qk [n][H][q: dim | k: dim].
 __global__ void __launch_bounds__(128)
 lightning_tiles_prepare_kernel(const float* __restrict__ proj, long long ld, int q_off, int k_off, const float* __restrict__ decay,
-                               const int* __restrict__ qo_indptr, float* __restrict__ qk, float* __restrict__ coef, int H, int dim,
-                               int act, float k_scale, const float* __restrict__ inv_freq, int rot, const int* __restrict__ positions) {
+                               const int* __restrict__ qo_indptr, int n_entries, float* __restrict__ qk, float* __restrict__ coef,
+                               int H, int dim, int act, float k_scale, const float* __restrict__ inv_freq, int rot, const int* __restrict__ positions) {
   bspec::pdl_prologue(65);
   __shared__ float qs[ST_B][264], ks[ST_B][264], dots[ST_B][ST_B];      // (rows eight banks apart)
-  const int i = blockIdx.x, h = blockIdx.y, e = blockIdx.z;
-  const int q_begin = qo_indptr[e], n = qo_indptr[e + 1] - q_begin;
-  if (n < ST_FROM || i * ST_B >= n) return;
+  const int h = blockIdx.y, e = state_tile_entry(qo_indptr, n_entries, blockIdx.x);
+  const int q_begin = qo_indptr[e], n = qo_indptr[e + 1] - q_begin, i = blockIdx.x - (int)state_tile_slot(q_begin, e, 0);
+  if (n < ST_FROM || i * ST_B >= n) return;                    // (i >= 0: the first entry's slots begin at 0)
   const int cnt = min(ST_B, n - i * ST_B), t0 = q_begin + i * ST_B;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 #pragma unroll
@@ -636,7 +636,7 @@ BSPEC_API long long bspec_lightning_scratch(int n, int n_entries, int max_q_len,
 BSPEC_API int bspec_lightning_recurrence(const float* proj, long long ld, int q_off, int k_off, int v_off,
                                          const float* decay, float* state, long long state_stride,
                                          const int* qo_indptr, const int* state_slots, float* out, int n, int n_entries,
-                                         int min_q_len, int max_q_len, int H, int dim, int vdim, int act, float k_scale,
+                                         int min_q_len, int H, int dim, int vdim, int act, float k_scale,
                                          const float* inv_freq, int rot, const int* positions, float* scratch,
                                          cudaStream_t stream) {
   if (n_entries <= 0) return 0;
@@ -646,8 +646,8 @@ BSPEC_API int bspec_lightning_recurrence(const float* proj, long long ld, int q_
     return (int)cudaErrorInvalidValue;
   if (scratch != nullptr) {
     float* qk = scratch + bspec::state_tile_slots(n, n_entries) * H * ST_CO;
-    BSPEC_LAUNCH(lightning_tiles_prepare_kernel, dim3((max_q_len + ST_B - 1) / ST_B, H, n_entries), 128, 0, stream, proj, ld, q_off,
-                 k_off, decay, qo_indptr, qk, scratch, H, dim, act, k_scale, inv_freq, rot, positions);
+    BSPEC_LAUNCH(lightning_tiles_prepare_kernel, dim3((unsigned)bspec::state_tile_slots(n, n_entries), H), 128, 0, stream, proj, ld,
+                 q_off, k_off, decay, qo_indptr, n_entries, qk, scratch, H, dim, act, k_scale, inv_freq, rot, positions);
     const int err = BSPEC_LAUNCH_CHECK();
     if (err != 0) return err;
     const dim3 tiles((vdim + ST_COLS - 1) / ST_COLS, H, n_entries);

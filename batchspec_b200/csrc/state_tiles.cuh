@@ -22,6 +22,22 @@ constexpr int ST_COLS = 16, ST_STAGE = 16, ST_THREADS = 128;
 __device__ __forceinline__ size_t state_tile_slot(int q_begin, int e, int i) { return (size_t)(q_begin / ST_B + e + i); }
 inline long long state_tile_slots(int n, int n_entries) { return n / ST_B + n_entries + 1; }
 
+// The entry whose slots hold ``slot``: the last one that begins at or before it.  (The preparation kernels' grids go over the
+// slots: over the tiles of the longest portion times the requests, a portion of 8,192 tokens beside 63 decoded ones was a
+// million blocks with 16,384 tiles to form.)  A warp looks at 32 entries at a time.
+__device__ __forceinline__ int state_tile_entry(const int* __restrict__ qo_indptr, int n_entries, int slot) {
+  const int lane = threadIdx.x & 31;
+  int first = 0, count = n_entries;                            // the answer is one of ``count`` entries from ``first`` on
+  while (count > 1) {
+    const int step = (count + 31) / 32, e = first + lane * step;
+    const unsigned before = __ballot_sync(0xffffffffu, lane * step < count && (int)state_tile_slot(qo_indptr[min(e, n_entries - 1)], e, 0) <= slot);
+    const int k = max(0, 31 - __clz(before));
+    first += k * step;
+    count = min(step, count - k * step);
+  }
+  return first;
+}
+
 constexpr size_t state_tiles_smem(int dp) {
   return (size_t)(2 * ST_STAGE * (2 * dp + ST_COLS) + 2 * (ST_STAGE / ST_B) * ST_CO + 4 * 64 * 16 + 4 * 32) * 4;
 }

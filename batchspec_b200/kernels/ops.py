@@ -51,7 +51,7 @@ _SIGNATURES = {
     "bspec_scale": [c_void_p, c_longlong, c_float, c_void_p],
     "bspec_gate_mul": [c_void_p, c_void_p, c_longlong, c_void_p, c_longlong, c_int, c_int, c_int, c_float, c_void_p],
     "bspec_lightning_recurrence": [c_void_p, c_longlong, c_int, c_int, c_int, c_void_p, c_void_p, c_longlong, c_void_p,
-                                   c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_void_p,
+                                   c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_void_p,
                                    c_int, c_void_p, c_void_p, c_void_p],
     "bspec_lightning_scratch": [c_int, c_int, c_int, c_int, c_int],
     "bspec_branch_join": [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p,
@@ -1013,8 +1013,8 @@ def delta_recurrence(mix: torch.Tensor, gates: torch.Tensor, proj: torch.Tensor,
     scratch = torch.empty((need,), dtype=torch.float32, device=mix.device) if need else None
     _check(lib.bspec_delta_recurrence(
         mix.data_ptr(), gates.data_ptr(), proj.data_ptr(), proj.shape[1], state.data_ptr(), state.stride(0),
-        int(tail_off), ctx.qo_indptr.data_ptr(), ctx.state_slots.data_ptr(), out.data_ptr(), ctx.n_entries,
-        shortest, longest, n_heads, n_kv_heads, dim, v_dim, taps, _ptr(scratch), _stream()), "delta_recurrence")
+        int(tail_off), ctx.qo_indptr.data_ptr(), ctx.state_slots.data_ptr(), out.data_ptr(), n, ctx.n_entries,
+        shortest, n_heads, n_kv_heads, dim, v_dim, taps, _ptr(scratch), _stream()), "delta_recurrence")
     if need:
         count_launches(1)
     return out
@@ -1126,7 +1126,7 @@ def lightning_recurrence(proj: torch.Tensor, q_off: int, k_off: int, v_off: int,
     scratch = torch.empty((need,), dtype=torch.float32, device=proj.device) if need else None
     _check(lib.bspec_lightning_recurrence(
         proj.data_ptr(), proj.stride(0), int(q_off), int(k_off), int(v_off), decay.data_ptr(), state.data_ptr(),
-        state.stride(0), ctx.qo_indptr.data_ptr(), ctx.state_slots.data_ptr(), out.data_ptr(), n, ctx.n_entries, shortest, longest,
+        state.stride(0), ctx.qo_indptr.data_ptr(), ctx.state_slots.data_ptr(), out.data_ptr(), n, ctx.n_entries, shortest,
         n_heads, dim, v_dim, int(activation == "silu"), float(k_scale), _ptr(inv_freq) if rotary_dim else None,
         int(rotary_dim), ctx.positions.data_ptr() if rotary_dim else None, _ptr(scratch), _stream()),
         "lightning_recurrence")

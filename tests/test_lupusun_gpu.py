@@ -555,7 +555,7 @@ def test_delta_prepare_takes_tokens_eight_at_a_time(ops, Hh, G, dk, dv):
             assert (got.double().cpu() - want).abs().max() <= 2e-6 * max(1.0, want.abs().max().item())
 
 
-@pytest.mark.parametrize("lens", [[64], [63, 71], [1, 9, 65, 80], [200, 3, 64]])
+@pytest.mark.parametrize("lens", [[64], [63, 71], [1, 9, 65, 80], [200, 3, 64], [1] * 20 + [1030] + [3] * 15 + [70, 2]])
 @pytest.mark.parametrize("Hh,G,dk,dv", [(2, 1, 128, 40), (3, 3, 6, 16), (4, 2, 256, 17)])
 def test_delta_rule_tiles(ops, Hh, G, dk, dv, lens):
     """Portions of whole and partial tiles of eight tokens beside shorter ones that go token by token, keys that repeat (the tile's inverse at its largest),

@@ -591,6 +591,29 @@ def test_interleaved_rotation_and_append_from_wider_rows(ops, dtype, Hq, G, hd, 
     assert int((cache != 0).sum()) <= n * entry
 
 
+@pytest.mark.parametrize("first", [1, 36, 1100])
+def test_tiles_are_found_among_many_requests(ops, first):
+    """Long portions behind ``first`` decoded tokens, so that a tile's request is looked for among up to 1,104, against the same
+    portions alone."""
+    Hh, dk, dv = 2, 64, 16
+    lens = [1] * first + [90, 7, 64, 1]
+    n, ld = sum(lens), Hh * (2 * dk + dv)
+    gen = torch.Generator(device=DEV).manual_seed(first)
+    proj, decay = torch.randn(n, ld, device=DEV, generator=gen), torch.tensor([0.9, 0.99], device=DEV)
+    qo = [0] + list(np.cumsum(lens))
+
+    def run(first_entry, last):
+        state = torch.zeros(last - first_entry, Hh * dk * dv, device=DEV)
+        ctx = SimpleNamespace(qo_indptr=_i32([q - qo[first_entry] for q in qo[first_entry:last + 1]]), n_entries=last - first_entry,
+                              max_q_len=max(lens[first_entry:last]), state_slots=_i32(range(last - first_entry)))
+        return ops.lightning_recurrence(proj[qo[first_entry]:qo[last]], 0, Hh * dk, 2 * Hh * dk, decay, state, ctx, Hh, dk, dv, None), state
+
+    out, state = run(0, len(lens))
+    for e in range(first, first + 4):
+        o, s = run(e, e + 1)
+        assert (out[qo[e]:qo[e + 1]] - o).abs().max() <= 2e-5 * o.abs().max() and (state[e] - s[0]).abs().max() <= 2e-5 * s.abs().max()
+
+
 @pytest.mark.parametrize("Hh,dk,dv,act,scale", [(2, 128, 33, "silu", 1.0), (3, 20, 7, None, 0.25), (1, 256, 16, "silu", 1.0),
                                                 (4, 64, 64, None, 0.125), (2, 6, 130, "silu", 0.5)])
 def test_lightning_attention_by_tiles(ops, Hh, dk, dv, act, scale):
