@@ -9,8 +9,8 @@
 //                     scale), beta = sigmoid(b), g = exp(-exp(A_log) softplus(a + dt_bias))
 //   delta_recurrence  per (request, head, 32 or 8 value columns): the token loop over the portion with the state in
 //                     registers (a column of S is spread over four or sixteen lanes), state read at the start and
-//                     written at the end; the request's blocks also move the convolutions' inputs on.  Long portions
-//                     (ST_FROM tokens and more) take delta_tiles_prepare and delta_tiles instead, which multiply the
+//                     written at the end; the request's blocks also move the convolutions' inputs on.  Where that is faster, portions
+//                     of ST_FROM tokens and more take delta_tiles_prepare and delta_tiles instead, which multiply the
 //                     rule out over tiles of eight tokens
 //   gated_rmsnorm     per (token, head): o / rms(o) * w * silu(gate), with options other mixers use
 //
@@ -697,12 +697,15 @@ BSPEC_API int bspec_delta_prepare(const float* proj, int n, int ld, int b_off, i
   return BSPEC_LAUNCH_CHECK();
 }
 
-// Floats of scratch for a step of n tokens whose longest portion has max_q_len: the tiles' coefficients, or 0 where no
+// Floats of scratch for a step of n tokens in portions of min_q_len to max_q_len: the tiles' coefficients, or 0 where no
 // portion goes by tiles.
-BSPEC_API long long bspec_delta_scratch(int n, int n_entries, int max_q_len, int H) {
-  // many requests fill the device token by token, and the second kernel for the short ones comes on top: 512 tokens beside 63
-  // decoded ones 182 us by tokens, 193 by tiles; 2,048 beside 24 668 and 488
-  if (max_q_len < ST_FROM || (n_entries > 32 && max_q_len < 1024)) return 0;
+BSPEC_API long long bspec_delta_scratch(int n, int n_entries, int min_q_len, int max_q_len, int H, int dim, int vdim) {
+  if (n <= 0 || n_entries <= 0 || H <= 0 || dim <= 0 || vdim <= 0) return 0;
+  // (the token loop's blocks of 8 columns, chosen where 32 would leave SMs idle, do less per microsecond)
+  const bool narrow = (long long)((vdim + 31) / 32) * H * n_entries < 2ll * bspec::sm_count();
+  const bspec::TokenCost tokens = {dim <= 64 ? 0.165 : (dim <= 128 ? 0.225 : 0.38), (narrow ? 0.9e-6 : 0.34e-6) * (dim <= 32 ? 1.8 : 1.0)};
+  const bspec::TokenCost tiles = {dim <= 128 ? 0.118 : 0.2, dim <= 128 ? 6.2e-4 : 1.13e-3};
+  if (!bspec::tiles_pay(n, n_entries, min_q_len, max_q_len, H, dim, vdim, tokens, tiles)) return 0;
   return bspec::state_tile_slots(n, n_entries) * H * ST_CO;
 }
 

@@ -628,9 +628,17 @@ scan_segments_kernel(const float* __restrict__ xz, long long ld, const float* __
 }
 }  // namespace
 
-// Floats of scratch for a step of n tokens whose longest portion has max_q_len: 0 where none goes by tiles.
-BSPEC_API long long bspec_lightning_scratch(int n, int n_entries, int max_q_len, int H, int dim) {
-  return max_q_len >= ST_FROM ? bspec::state_tile_slots(n, n_entries) * H * ST_CO + (long long)n * H * 2 * dim : 0;
+// Floats of scratch for a step of n tokens in portions of min_q_len to max_q_len: the tiles' coefficients and prepared q and k
+// (as large as the step's q and k columns), or 0 where no portion goes by tiles.
+BSPEC_API long long bspec_lightning_scratch(int n, int n_entries, int min_q_len, int max_q_len, int H, int dim, int vdim) {
+  if (n <= 0 || n_entries <= 0 || H <= 0 || dim <= 0 || vdim <= 0) return 0;
+  // (the token loop's time per unit of work falls with the blocks that share the device)
+  const long long blocks = (long long)((vdim + LT_COLS - 1) / LT_COLS) * H * n_entries, sms = bspec::sm_count();
+  const double rate = (blocks < 3 * sms ? 1.0e-6 : (blocks < 6 * sms ? 0.66e-6 : 0.45e-6)) * (dim <= 32 ? 1.42 : 1.0);
+  const bspec::TokenCost tokens = {dim <= 32 ? 0.165 : (dim <= 64 ? 0.19 : (dim <= 128 ? 0.25 : 0.38)), rate};
+  const bspec::TokenCost tiles = {dim <= 128 ? 0.115 : 0.165, dim <= 128 ? 6.0e-4 : 9e-4};
+  if (!bspec::tiles_pay(n, n_entries, min_q_len, max_q_len, H, dim, vdim, tokens, tiles)) return 0;
+  return bspec::state_tile_slots(n, n_entries) * H * ST_CO + (long long)n * H * 2 * dim;
 }
 
 BSPEC_API int bspec_lightning_recurrence(const float* proj, long long ld, int q_off, int k_off, int v_off,

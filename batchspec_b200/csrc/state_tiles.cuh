@@ -11,10 +11,7 @@ namespace bspec {
 
 // tokens of a tile; floats of a token's row of coefficients [F_t 8 | P_t 8 | d_t, e_t, c_t, c_B]; floats of a tile's
 constexpr int ST_B = 8, ST_ROW = 20, ST_CO = ST_B * ST_ROW;
-// A step's portions of at least ST_FROM tokens go by tiles, the others token by token.  Measured with 16 heads of 128 x 128, by
-// tokens / by tiles with the preparation, us: delta rule 4 x 8 tokens 15 / 19, 128 x 9 135 / 245, 64 x 16 107 / 118,
-// 1 x 64 23.5 / 21.3, 32 x 64 183 / 177, 1 x 256 75 / 44, 8 x 2,048 1,559 / 1,263; lightning attention 4 x 8 13 / 22, 128 x 9
-// 170 / 232, 64 x 16 135 / 116, 1 x 64 22.5 / 23.3, 32 x 64 254 / 173, 1 x 256 72 / 44, 8 x 2,048 2,126 / 1,226.
+// In a step whose long portions go by tiles (tiles_pay) those are the portions of at least ST_FROM tokens.
 constexpr int ST_FROM = 64;
 constexpr int ST_COLS = 16, ST_STAGE = 16, ST_THREADS = 128;
 
@@ -36,6 +33,44 @@ __device__ __forceinline__ int state_tile_entry(const int* __restrict__ qo_indpt
     count = min(step, count - k * step);
   }
   return first;
+}
+
+// What a token takes, us on a B200: ``chain`` in a portion's chain, ``rate`` times heads x rows of the instance x value columns when
+// the device is full.
+struct TokenCost {
+  double chain, rate;
+};
+
+// Whether a step is faster with its long portions by tiles.  Tiles have the shorter chain, 8 tokens in about a microsecond, but
+// one instance for all heads of up to 128 rows, a preparation, and a second kernel for the shorter portions; token loops have
+// instances for 32 and 64 rows.  So both are estimated, as the longer of a chain and the work of a full device.  The constants are
+// fitted to 594 measured steps (1 to 64 heads of 32 to 256, 1 to 64 requests of 1 to 8,192 tokens); where the choice is wrong the
+// other form is less than 5 us or a sixth faster.  By tokens / by tiles, us, delta rule and lightning attention:
+//   16 heads of 128 x 128: 1 x 64 19 / 14 and 18 / 15; 2,048 beside 24 decoded 666 / 388 and 853 / 358; 32 x 128 344 / 314 and 485 / 306
+//   16 heads of 64 x 64: 1 x 64 13 / 14; 32 x 64 53 / 90 and 61 / 88; 4 x 2,048 577 / 412 and 550 / 389
+//   64 heads of 64 x 64: 32 x 128 374 / 660 and 448 / 618; 2,048 beside 63 653 / 548 and 628 / 513; 128 beside 63 (lightning) 47 / 76
+//   32 heads of 32 x 32 (lightning): 32 x 64 40 / 97; 512 beside 63 88 / 76
+//   8 heads of 256 x 256: 32 x 64 354 / 315 and 733 / 262; 64 tokens beside twenty of 60, any heads: a loss, 119 / 137 at 16 x 128
+// (A step is what the estimate needs; a request's results differ by rounding between the two forms.)
+inline bool tiles_pay(int n, int n_entries, int shortest, int longest, int H, int dim, int vdim, TokenCost tokens, TokenCost tiles) {
+  if (longest < ST_FROM) return false;
+  const int least = shortest < 1 ? 1 : shortest;
+  const long long spare = (long long)n - longest - (long long)(n_entries - 1) * least;      // tokens above the others' least
+  const long long rest = spare < 0 ? 0 : spare;
+  long long tall = 1;                                                                       // the most portions that go by tiles
+  if (least >= ST_FROM) tall = n_entries;
+  else tall += rest / (ST_FROM - least) < n_entries - 1 ? rest / (ST_FROM - least) : n_entries - 1;
+  const double tiled = (double)n - (double)(n_entries - tall) * least;                      // tokens in them
+  const int rows = dim <= 32 ? 32 : (dim <= 64 ? 64 : (dim <= 128 ? 128 : 256));
+  const double token_work = (double)H * rows * vdim * tokens.rate, tile_work = (double)H * ((vdim + 15) / 16) * tiles.rate;
+  auto longer = [](double a, double b) { return a > b ? a : b; };
+  const double by_tokens = longer(longest * tokens.chain, n * token_work) + 4.0;
+  double by_tiles = longer(longest * tiles.chain, tiled * tile_work) + tiled * H * (0.5e-4 + 2e-6 * dim) + 7.5;
+  if (least < ST_FROM && n_entries > 1) {                                                   // the second kernel
+    const double s = least + rest < ST_FROM - 1 ? (double)(least + rest) : ST_FROM - 1;
+    by_tiles += 3.0 + longer(s * tokens.chain, (n - tiled) * token_work) + (double)(n_entries - 1) * H * dim * vdim / 3e6;
+  }
+  return by_tiles < by_tokens;
 }
 
 constexpr size_t state_tiles_smem(int dp) {

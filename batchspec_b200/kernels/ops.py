@@ -53,7 +53,7 @@ _SIGNATURES = {
     "bspec_lightning_recurrence": [c_void_p, c_longlong, c_int, c_int, c_int, c_void_p, c_void_p, c_longlong, c_void_p,
                                    c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_void_p,
                                    c_int, c_void_p, c_void_p, c_void_p],
-    "bspec_lightning_scratch": [c_int, c_int, c_int, c_int, c_int],
+    "bspec_lightning_scratch": [c_int] * 7,
     "bspec_branch_join": [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p,
                           c_float, c_void_p, c_longlong, c_int, c_int, c_void_p, c_void_p, c_float, c_void_p, c_int, c_int,
                           c_longlong, c_int, c_void_p],
@@ -80,7 +80,7 @@ _SIGNATURES = {
                             c_int, c_int, c_int, c_float, c_float, c_void_p],
     "bspec_delta_recurrence": [c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_longlong, c_longlong, c_void_p,
                                c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p],
-    "bspec_delta_scratch": [c_int, c_int, c_int, c_int],
+    "bspec_delta_scratch": [c_int] * 7,
     "bspec_gated_rmsnorm": [c_void_p, c_void_p, c_longlong, c_void_p, c_int, c_void_p, c_int, c_longlong, c_int, c_int, c_int,
                             c_float, c_int, c_void_p, c_float, c_void_p],
     "bspec_state_space": [c_void_p, c_longlong, c_void_p, c_void_p, c_longlong, c_void_p, c_void_p, c_void_p, c_void_p,
@@ -1009,7 +1009,7 @@ def delta_recurrence(mix: torch.Tensor, gates: torch.Tensor, proj: torch.Tensor,
     out = torch.empty((n, n_heads * v_dim), dtype=torch.float32, device=mix.device)
     lib = load_library()
     shortest, longest = _portion_bounds(ctx, n)
-    need = lib.bspec_delta_scratch(n, ctx.n_entries, longest, n_heads)
+    need = lib.bspec_delta_scratch(n, ctx.n_entries, shortest, longest, n_heads, dim, v_dim)
     scratch = torch.empty((need,), dtype=torch.float32, device=mix.device) if need else None
     _check(lib.bspec_delta_recurrence(
         mix.data_ptr(), gates.data_ptr(), proj.data_ptr(), proj.shape[1], state.data_ptr(), state.stride(0),
@@ -1122,7 +1122,7 @@ def lightning_recurrence(proj: torch.Tensor, q_off: int, k_off: int, v_off: int,
     out = torch.empty((n, n_heads * v_dim), dtype=torch.float32, device=proj.device)
     lib = load_library()
     shortest, longest = _portion_bounds(ctx, n)
-    need = lib.bspec_lightning_scratch(n, ctx.n_entries, longest, n_heads, dim)
+    need = lib.bspec_lightning_scratch(n, ctx.n_entries, shortest, longest, n_heads, dim, v_dim)
     scratch = torch.empty((need,), dtype=torch.float32, device=proj.device) if need else None
     _check(lib.bspec_lightning_recurrence(
         proj.data_ptr(), proj.stride(0), int(q_off), int(k_off), int(v_off), decay.data_ptr(), state.data_ptr(),

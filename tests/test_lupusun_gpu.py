@@ -555,7 +555,8 @@ def test_delta_prepare_takes_tokens_eight_at_a_time(ops, Hh, G, dk, dv):
             assert (got.double().cpu() - want).abs().max() <= 2e-6 * max(1.0, want.abs().max().item())
 
 
-@pytest.mark.parametrize("lens", [[64], [63, 71], [1, 9, 65, 80], [200, 3, 64], [1] * 20 + [1030] + [3] * 15 + [70, 2]])
+@pytest.mark.parametrize("lens", [[64], [63, 71], [1, 9, 65, 80], [200, 3, 64], [1] * 20 + [1030] + [3] * 15 + [70, 2], [265], [192, 329],
+                                  [1, 500, 6, 64]])
 @pytest.mark.parametrize("Hh,G,dk,dv", [(2, 1, 128, 40), (3, 3, 6, 16), (4, 2, 256, 17)])
 def test_delta_rule_tiles(ops, Hh, G, dk, dv, lens):
     """Portions of whole and partial tiles of eight tokens beside shorter ones that go token by token, keys that repeat (the tile's inverse at its largest),
@@ -597,6 +598,17 @@ def test_delta_rule_tiles(ops, Hh, G, dk, dv, lens):
         want = P.gated_delta_rule(q, k, m[:, 2 * G * dk:].view(T, Hh, dv), g[:, :Hh], g[:, Hh:]).reshape(T, -1)
         # the bound of the tests above
         assert (whole(outs) - want).abs().max() <= 2e-4 * max(1.0, want.abs().max().item()), e
+
+
+@pytest.mark.parametrize("lens,sizes,tiles", [
+    ([265], (2, 6, 16), True), ([1, 500, 6, 64], (3, 6, 16), True), ([192, 329], (2, 128, 40), True), ([2048], (16, 128, 128), True),
+    ([512] + [1] * 63, (16, 64, 64), True), ([512] + [1] * 63, (16, 128, 128), True), ([64], (16, 128, 128), True), ([63], (16, 128, 128), False),
+    ([64] * 32, (16, 64, 64), False), ([128] * 32, (64, 64, 64), False), ([64] + [60] * 20, (16, 128, 128), False), ([1] * 64, (16, 128, 128), False)])
+def test_portions_go_by_tiles_where_they_measured_faster(ops, lens, sizes, tiles):
+    """The choice by the step's portions and the heads' sizes, for both recurrences (and that the tests of the tiles reach them)."""
+    lib = ops.load_library()
+    for scratch in (lib.bspec_delta_scratch, lib.bspec_lightning_scratch):
+        assert (scratch(sum(lens), len(lens), min(lens), max(lens), *sizes) > 0) == tiles
 
 
 # ------------------------------------------------------------------------------------------- the engine

@@ -596,7 +596,7 @@ def test_tiles_are_found_among_many_requests(ops, first):
     """Long portions behind ``first`` decoded tokens, so that a tile's request is looked for among up to 1,104, against the same
     portions alone."""
     Hh, dk, dv = 2, 64, 16
-    lens = [1] * first + [90, 7, 64, 1]
+    lens = [1] * first + [400, 7, 64, 1]
     n, ld = sum(lens), Hh * (2 * dk + dv)
     gen = torch.Generator(device=DEV).manual_seed(first)
     proj, decay = torch.randn(n, ld, device=DEV, generator=gen), torch.tensor([0.9, 0.99], device=DEV)
@@ -619,7 +619,7 @@ def test_tiles_are_found_among_many_requests(ops, first):
 def test_lightning_attention_by_tiles(ops, Hh, dk, dv, act, scale):
     """Portions long enough to go by tiles (whole and partial last ones) beside ones that go token by token, states carried
     between them, against the plain recurrence; a request's last token being infinite changes nothing before it."""
-    steps = [dict(a=70, b=1, c=5), dict(a=64, c=63), dict(a=1, b=200, c=65)]
+    steps = [dict(a=70, b=1, c=5), dict(a=64, c=63), dict(a=1, b=300, c=65), dict(a=265, c=1), dict(a=200)]
     gen = torch.Generator(device=DEV).manual_seed(dk + dv)
     ld = 2 * Hh * dk + Hh * dv + 1
     k_off, v_off = Hh * dk, 2 * Hh * dk + 1
