@@ -715,12 +715,27 @@ BSPEC_API int bspec_scan_conv(const float* xz, long long ld, const void* conv, c
   return BSPEC_LAUNCH_CHECK();
 }
 
+// Few channels x requests: more lanes per channel, so that a lone prompt's chain is shorter and more SMs take part.
+static bool scan_few(int inner, int n_entries) { return (long long)((inner + SC_THREADS - 1) / SC_THREADS) * n_entries < 148; }
+
 // Floats of scratch for a step of n tokens: 0 where the portions go from end to end.  In segments where the longest chain is
-// long and the requests are so few that twice the arithmetic spread over the device takes less time than that chain.
-// Measured with 4,096 channels of 16 states, end to end / in segments, us: 1 x 256 tokens 83 / 91, 4 x 300 169 / 176,
-// 1 x 2,048 609 / 259.  More than 32 states spread over several lanes of a channel and go from end to end.
+// long and twice the arithmetic spread over the device takes less time than that chain.  Both are estimated, us on a B200: end
+// to end a chain whose tokens take longer the more blocks work beside it (those of n / max_q_len requests), in segments the work.
+// Measured, end to end / in segments: 4,096 channels of 16 states 1 x 256 tokens 83 / 91, 1 x 2,048 599 / 254, 4 x 512 276 / 254;
+// 8,192 channels 2 x 512 276 / 254, 3 x 512 340 / 359, 4 x 2,048 1,347 / 1,734, 2,048 tokens beside 3 1,337 / 482; 16,384 channels 1 x 512
+// 277 / 255, 2 x 512 340 / 460; 4,096 channels of 32 states 1 x 512 213 / 145, 2 x 512 233 / 308; 8,192 1 x 512 233 / 314.  More than
+// 32 states spread over several lanes of a channel and go from end to end.
 BSPEC_API long long bspec_scan_scratch(int n, int n_entries, int max_q_len, int inner, int N) {
   if (max_q_len < SC_SEG_MIN || n_entries > SC_SEG_ENTRIES || N > SC_SEG_MAX_N) return 0;
+  const double blocks = (double)((inner + SC_THREADS - 1) / SC_THREADS) * n / max_q_len, million = 1e-6 * n * inner;
+  double token;
+  if (scan_few(inner, n_entries)) {
+    const double x = blocks > 32 ? blocks - 32 : 0;
+    token = N <= 16 ? 0.29 * (1 + 0.0055 * x + 3e-5 * x * x) : 0.412 * (1 + 0.0003 * x + 8e-5 * x * x);
+  } else {
+    token = (N <= 16 ? 0.655 : 1.07) * (blocks > 300 ? blocks / 300 : 1);
+  }
+  if ((N <= 16 ? 50 + 25.2 * million : 30 + 55 * million) >= max_q_len * token) return 0;
   return (long long)(n / SC_SEG + n_entries + 1) * (N + 1) * inner;
 }
 
@@ -732,8 +747,7 @@ BSPEC_API int bspec_selective_scan(const float* xz, long long ld, const float* x
                                    int N, int taps, float* scratch, cudaStream_t stream) {
   if (n_entries <= 0) return 0;
   if (inner <= 0 || N <= 0 || N > SC_MAX_N || taps < 1 || n_entries > 65535) return (int)cudaErrorInvalidValue;
-  // few channels x requests: more lanes per channel, so that a lone prompt's chain is shorter and more SMs take part
-  const bool few = scratch == nullptr && (long long)((inner + SC_THREADS - 1) / SC_THREADS) * n_entries < 148;
+  const bool few = scratch == nullptr && scan_few(inner, n_entries);
   const int segs = scratch != nullptr ? (max_q_len + SC_SEG - 1) / SC_SEG : 1;
   if (segs > 65535) return (int)cudaErrorInvalidConfiguration;
   float* dt_sum = scratch != nullptr ? scratch + (size_t)(n / SC_SEG + n_entries + 1) * N * inner : nullptr;

@@ -689,6 +689,14 @@ def test_selective_scan_in_segments(ops, inner, N, taps, lens):
         assert torch.equal(state[slots[e], tail_off:].view(taps - 1, inner), kept), e
 
 
+@pytest.mark.parametrize("inner,N,lens,segments", [
+    (4096, 16, [2048], True), (4096, 16, [512] * 4, True), (8192, 16, [2048] * 4, False), (8192, 16, [2048, 1, 1, 1], True),
+    (16384, 16, [512] * 2, False), (4096, 32, [512], True), (4096, 32, [512] * 2, False), (8192, 32, [512], False), (64, 24, [511, 513, 1, 64], True),
+    (4096, 16, [511], False), (4096, 40, [2048], False)])
+def test_the_scan_goes_in_segments_where_they_measured_faster(ops, inner, N, lens, segments):
+    assert (ops.load_library().bspec_scan_scratch(sum(lens), len(lens), max(lens), inner, N) > 0) == segments
+
+
 @pytest.mark.parametrize("N", [16, 32])
 @pytest.mark.parametrize("size", [1e4, 1e5])
 def test_a_state_that_is_gone_leaves_no_rounding_behind_in_segments(ops, N, size):
