@@ -92,8 +92,8 @@ delta_prepare_kernel(const float* __restrict__ proj, int ld, int b_off, int a_of
 
 // The same for four taps and heads of up to 128 numbers that start on 16-byte boundaries: a lane holds four channels of the
 // warp's head with their weights, and the inputs of TT consecutive tokens and the three before them, so that an input is
-// read once for four uses.  Bound by memory: 3,207 tokens of 4,096 channels 92 -> 46 us, 2,048 of them 74 -> 45 us on a B200
-// (the bytes need 16 and 10).
+// read once for four uses.  Bound by memory: 6,144 channels (48 heads of 128), 2,048 tokens 83.8 -> 39.3 us on a B200, 8,192 tokens
+// 328 -> 144 us (the bytes need 16 and 62).
 template <int TT>
 __global__ void __launch_bounds__(DP_WARPS * 32)
 delta_prepare4_kernel(const float* __restrict__ proj, int n, int ld, int b_off, int a_off, const void* __restrict__ conv,
@@ -675,17 +675,24 @@ gated_rmsnorm_wide_kernel(const float* __restrict__ o, const float* __restrict__
 BSPEC_API int bspec_delta_prepare(const float* proj, int n, int ld, int b_off, int a_off, const void* conv,
                                   const void* a_log, const void* dt_bias, int w_dtype, const float* state,
                                   long long state_stride, long long tail_off, const int* qo_indptr,
-                                  const int* tok_entry, const int* state_slots, float* mix, float* gates, int H, int Gk,
-                                  int dim, int vdim, int taps, float q_scale, float unit_eps, cudaStream_t stream) {
+                                  const int* tok_entry, const int* state_slots, float* mix, float* gates, int n_entries,
+                                  int H, int Gk, int dim, int vdim, int taps, float q_scale, float unit_eps, cudaStream_t stream) {
   if (n <= 0) return 0;
   if (H <= 0 || Gk <= 0 || H % Gk != 0 || taps < 1) return (int)cudaErrorInvalidValue;
   if (dim > 256) return (int)cudaErrorInvalidValue;
   const dim3 grid(n, (2 * Gk + H + DP_WARPS - 1) / DP_WARPS);
   if (grid.y > 65535) return (int)cudaErrorInvalidConfiguration;
-  // Eight tokens per warp where that leaves two blocks an SM; fewer tokens (decode steps) keep a warp per token and head.
-  if (taps == 4 && dim <= 128 && vdim <= 128 && ((dim | vdim | ld) & 3) == 0 && ((state_stride | tail_off) & 3) == 0 &&
-      ((reinterpret_cast<uintptr_t>(proj) | reinterpret_cast<uintptr_t>(state) | reinterpret_cast<uintptr_t>(mix)) & 15) == 0 &&
-      (long long)(n / 8) * grid.y >= 2ll * bspec::sm_count()) {
+  // Eight tokens per warp where enough blocks are left, the more of them the more lanes heads of this size leave idle, and the
+  // portions are long enough to share inputs; else a warp per token and head.  One token / eight, us: 16 heads of 128 x 128, 300
+  // tokens 13.4 / 11.1, 200 tokens 9.8 / 10.7, 200 requests of four 32 / 21, 256 of one 12.1 / 14.8; 64 x 128, 512 tokens 16.3 / 14.8, 400
+  // 13.4 / 14.6, 200 requests of four 24 / 27; 8 heads of 96 x 96, 8,192 tokens 136 / 109, 2,048 33 / 36; 64 x 64 (half of the lanes)
+  // 2,048 tokens 31.5 / 35.9, 8,192 132 / 135; 32 x 32 2,048 tokens 10.1 / 21.0.
+  const long long lanes = 128ll * (2 * Gk + H), used = 2ll * Gk * dim + (long long)H * vdim, sms = bspec::sm_count();
+  const long long eights = (long long)(n / 8) * grid.y;
+  const bool pays = 10 * used >= 9 * lanes ? 10 * eights >= 27 * sms && n >= 3ll * n_entries
+                                           : 20 * used >= 13 * lanes && eights >= (max(dim, vdim) > 96 ? 5 : 20) * sms && n >= 8ll * n_entries;
+  if (pays && taps == 4 && dim <= 128 && vdim <= 128 && ((dim | vdim | ld) & 3) == 0 && ((state_stride | tail_off) & 3) == 0 &&
+      ((reinterpret_cast<uintptr_t>(proj) | reinterpret_cast<uintptr_t>(state) | reinterpret_cast<uintptr_t>(mix)) & 15) == 0) {
     BSPEC_LAUNCH((delta_prepare4_kernel<8>), dim3((n + 7) / 8, grid.y), DP_WARPS * 32, 0, stream, proj, n, ld, b_off, a_off, conv,
                  a_log, dt_bias, w_dtype, state, state_stride, tail_off, qo_indptr, tok_entry, state_slots, mix, gates, H, Gk, dim,
                  vdim, q_scale, unit_eps);

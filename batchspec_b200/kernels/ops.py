@@ -76,7 +76,7 @@ _SIGNATURES = {
                                c_longlong, c_float, c_int, c_void_p, c_longlong, c_longlong, c_float, c_int, c_void_p,
                                c_int, c_void_p, c_void_p, c_void_p, c_longlong, c_int, c_void_p],
     "bspec_delta_prepare": [c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_int, c_void_p,
-                            c_longlong, c_longlong, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int,
+                            c_longlong, c_longlong, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int,
                             c_int, c_int, c_int, c_float, c_float, c_void_p],
     "bspec_delta_recurrence": [c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_longlong, c_longlong, c_void_p,
                                c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p],
@@ -987,8 +987,8 @@ def delta_prepare(proj: torch.Tensor, b_off: int, a_off: int, conv: torch.Tensor
     _check(load_library().bspec_delta_prepare(
         proj.data_ptr(), n, ld, int(b_off), int(a_off), conv.data_ptr(), a_log.data_ptr(), dt_bias.data_ptr(),
         _dtype_code(conv.dtype), state.data_ptr(), state.stride(0), int(tail_off), ctx.qo_indptr.data_ptr(),
-        ctx.tok_entry.data_ptr(), ctx.state_slots.data_ptr(), mix.data_ptr(), gates.data_ptr(), n_heads, n_kv_heads,
-        dim, v_dim, taps, float(q_scale), float(unit_eps), _stream()), "delta_prepare")
+        ctx.tok_entry.data_ptr(), ctx.state_slots.data_ptr(), mix.data_ptr(), gates.data_ptr(),
+        getattr(ctx, "n_entries", 1), n_heads, n_kv_heads, dim, v_dim, taps, float(q_scale), float(unit_eps), _stream()), "delta_prepare")
     return mix, gates
 
 

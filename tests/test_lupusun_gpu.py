@@ -521,7 +521,7 @@ def test_delta_rule_recurrence_with_many_requests(ops, Hh, G, dk, dv, n_req):
         assert (torch.cat(got[i]).double().cpu() - want).abs().max() <= 2e-4 * max(1.0, want.abs().max().item()), i
 
 
-@pytest.mark.parametrize("Hh,G,dk,dv", [(16, 8, 128, 64), (8, 4, 36, 100)])
+@pytest.mark.parametrize("Hh,G,dk,dv", [(16, 8, 128, 64), (8, 4, 36, 100), (16, 8, 68, 100), (16, 8, 124, 116)])
 def test_delta_prepare_takes_tokens_eight_at_a_time(ops, Hh, G, dk, dv):
     """Enough tokens that a warp takes eight of them, requests of 1 to 60 that begin anywhere in the eight, against the plain
     convolution after the state's inputs, and against every request alone (a warp per token)."""
