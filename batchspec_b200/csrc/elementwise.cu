@@ -693,8 +693,9 @@ BSPEC_API int bspec_relu_squared(void* x, int dtype, long long total, cudaStream
 
 // ---------------------------------------------------------------- soft cap in place:  cap * tanh(x / cap)
 // Bound by memory: four quads per thread are on their way before the first is worked on (a number at a time took 148 us
-// for 2,048 x 32,000, where the bytes need 80; whole scoring passes of that size are 61 us shorter).  Lengths and pointers that
-// are no whole quads take the kernel of single numbers.
+// for 2,048 x 32,000, where the bytes need 80; 87 now).  Up to half a million numbers, where most of a thread's quads are not
+// there (100,000 1.5 us one by one, 1.8 in quads; 524,288 2.8 and 2.4), and lengths and pointers that are no whole quads
+// take the kernel of single numbers.
 __global__ void __launch_bounds__(256)
 tanh_softcap_vec_kernel(float4* __restrict__ x, size_t quads, float cap) {
   bspec::pdl_prologue(17);
@@ -722,7 +723,7 @@ BSPEC_API int bspec_tanh_softcap(float* x, long long total, float cap, cudaStrea
   if (total <= 0) return 0;
   const int threads = 256;
   const size_t cap_blocks = (size_t)bspec::sm_count() * 32;
-  if (total % 4 == 0 && ((uintptr_t)x & 15) == 0) {
+  if (total >= 1 << 19 && total % 4 == 0 && ((uintptr_t)x & 15) == 0) {
     const size_t want = ((size_t)total / 4 + threads - 1) / threads;
     BSPEC_LAUNCH((tanh_softcap_vec_kernel), (int)(want > cap_blocks ? cap_blocks : want), threads, 0, stream, (float4*)x,
                  (size_t)total / 4, cap);

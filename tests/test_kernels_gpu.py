@@ -154,7 +154,7 @@ def test_a_product_may_be_the_second_operand_of_the_next(ops, dtype, M):
     ops.check_status()
 
 
-@pytest.mark.parametrize("total", [4, 1028, 148 * 32 * 256 * 4 + 4, 148 * 32 * 256 * 20 + 8])
+@pytest.mark.parametrize("total", [4, 1028, (1 << 19) - 4, 1 << 19, 148 * 32 * 256 * 4 + 4, 148 * 32 * 256 * 20 + 8])
 def test_tanh_softcap_in_quads_and_one_by_one(ops, total):
     """Four numbers at a time, less and more than a thread's four quads, against the kernel of single numbers, which takes
     what begins off a 16-byte boundary."""
