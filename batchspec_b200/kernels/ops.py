@@ -992,6 +992,9 @@ def delta_prepare(proj: torch.Tensor, b_off: int, a_off: int, conv: torch.Tensor
     return mix, gates
 
 
+TILE_FROM = 64             # state_tiles.cuh's ST_FROM: in a step by tiles shorter portions take a third kernel
+
+
 def _portion_bounds(ctx, n: int):
     """Bounds of the step's portions: none is shorter than the first or longer than the second."""
     return getattr(ctx, "extras", {}).get("min_q_len", 1), getattr(ctx, "max_q_len", n)
@@ -1016,7 +1019,7 @@ def delta_recurrence(mix: torch.Tensor, gates: torch.Tensor, proj: torch.Tensor,
         int(tail_off), ctx.qo_indptr.data_ptr(), ctx.state_slots.data_ptr(), out.data_ptr(), n, ctx.n_entries,
         shortest, n_heads, n_kv_heads, dim, v_dim, taps, _ptr(scratch), _stream()), "delta_recurrence")
     if need:
-        count_launches(1)
+        count_launches(1 + int(shortest < TILE_FROM))
     return out
 
 
@@ -1131,7 +1134,7 @@ def lightning_recurrence(proj: torch.Tensor, q_off: int, k_off: int, v_off: int,
         int(rotary_dim), ctx.positions.data_ptr() if rotary_dim else None, _ptr(scratch), _stream()),
         "lightning_recurrence")
     if need:
-        count_launches(1)
+        count_launches(1 + int(shortest < TILE_FROM))
     return out
 
 
@@ -1433,6 +1436,8 @@ def _sgemm(x, w, out, M: int, N: int, K: int, lda: int, ldw: int, sa: int, sw: i
     scratch = torch.empty((need,), dtype=torch.float32, device=x.device) if need else None
     _check(lib.bspec_sgemm_tn_batched(x.data_ptr(), w.data_ptr(), out.data_ptr(), M, N, K, lda, ldw, N, sa, sw, M * N, batch,
                                       _ptr(scratch), int(w_is_parameter), _status_word(x.device).data_ptr(), _stream()), "sgemm_tn")
+    if need:
+        count_launches(1)
 
 
 # ---------------------------------------------------------------------------- latent attention

@@ -611,6 +611,33 @@ def test_portions_go_by_tiles_where_they_measured_faster(ops, lens, sizes, tiles
         assert (scratch(sum(lens), len(lens), min(lens), max(lens), *sizes) > 0) == tiles
 
 
+@pytest.mark.parametrize("lens,kernels", [([300], 2), ([300, 1], 3), ([40], 1), ([1, 1], 1)])
+def test_launches_of_the_recurrences_and_of_long_sums_are_counted(ops, lens, kernels):
+    """Against the kernels of the same call captured in a graph."""
+    runtime = pytest.importorskip("cuda.bindings.runtime")
+    n, E = sum(lens), len(lens)
+    ctx = SimpleNamespace(qo_indptr=_i32([0] + list(np.cumsum(lens))), n_entries=E, max_q_len=max(lens), state_slots=_i32(range(E)),
+                          extras={"min_q_len": min(lens)})
+    x, state, gates = torch.randn(n, 3 * 128, device=DEV), torch.zeros(E, 128 * 128, device=DEV), torch.rand(n, 2, device=DEV)
+    a, w, decay = torch.randn(40, 4096, device=DEV), torch.randn(64, 4096, device=DEV), torch.ones(1, device=DEV)
+    calls = [(lambda: ops.delta_recurrence(x, gates, x, state, state.shape[1], ctx, 1, 1, 128, 128, 1), kernels),
+             (lambda: ops.lightning_recurrence(x, 0, 128, 256, decay, state, ctx, 1, 128, 128), kernels),
+             (lambda: ops.linear(a, w), 2)]
+    for call, want in calls:
+        call()
+        torch.cuda.synchronize()
+        graph = torch.cuda.CUDAGraph(keep_graph=True)
+        before = ops.launch_count()
+        with torch.cuda.graph(graph):
+            call()
+        counted = ops.launch_count() - before
+        handle = runtime.cudaGraph_t(graph.raw_cuda_graph())
+        nodes = runtime.cudaGraphGetNodes(handle, runtime.cudaGraphGetNodes(handle)[2])[1]
+        kernel = runtime.cudaGraphNodeType.cudaGraphNodeTypeKernel
+        seen = sum(runtime.cudaGraphNodeGetType(node)[1] == kernel for node in nodes)
+        assert counted == want == seen
+
+
 # ------------------------------------------------------------------------------------------- the engine
 
 @pytest.mark.parametrize("dtype", DTYPES)
