@@ -1,11 +1,11 @@
-// Paged causal attention, generic path: any head_dim that is a multiple of 16 up
-// to 256, any number of heads and groups, any page size, float32 or bfloat16
-// storage, float32 arithmetic throughout.  A block holds R consecutive (query token, query head of the group) rows of one
-// request and kv head.  Keys are visited in chunks of 32 that start at multiples of 32 of the key index; chunk c goes to
-// warp c % W, which keeps a running softmax of its chunks for every row, and the warps' results are joined in their order
-// at the end.  (attn_row_kernel below: one warp per row, which takes the W shares of the chunks one after the other.)  So the order of every sum depends only on the query's own position (and the head sizes, which choose W),
-// not on how the request was cut into steps or on what else is in the batch: a key that a row does not see adds an
-// exact nothing.
+// Paged causal attention, generic path: any head_dim up to 256, any number of heads and groups, any page size, float32 or
+// bfloat16 storage, float32 arithmetic throughout.  A block holds R consecutive (query token, query head of the group) rows of
+// one request and kv head.  Keys are visited in chunks of 32 that start at multiples of 32 of the key index; chunk c belongs to
+// share c % W, which keeps a running softmax of its chunks for every row, and the shares' results are joined in their order at
+// the end.  A share is a warp's; attn_row_kernel below has one warp per row, which takes the shares one after the other.  So the
+// order of every sum depends only on the query's own position (and the head sizes, which choose W), not on how the request
+// was cut into steps, on what else is in the batch or on which of the two kernels runs: a key that a row does not see adds
+// an exact nothing.
 //
 // Cache layer layout: [pages][k: [Hkv][page_size][hd] | v: [Hkv][page_size][vd]] (vd = hd unless values have a size
 // of their own).

@@ -9,13 +9,15 @@
 //                     scale), beta = sigmoid(b), g = exp(-exp(A_log) softplus(a + dt_bias))
 //   delta_recurrence  per (request, head, 32 or 8 value columns): the token loop over the portion with the state in
 //                     registers (a column of S is spread over four or sixteen lanes), state read at the start and
-//                     written at the end; the request's blocks also move the convolutions' inputs on.  Where that is faster, portions
-//                     of ST_FROM tokens and more take delta_tiles_prepare and delta_tiles instead, which multiply the
-//                     rule out over tiles of eight tokens
+//                     written at the end; the request's blocks also move the convolutions' inputs on.  Where that is
+//                     faster (tiles_pay), portions of ST_FROM tokens and more take delta_tiles_prepare and delta_tiles
+//                     instead, which multiply the rule out over tiles of eight tokens
 //   gated_rmsnorm     per (token, head): o / rms(o) * w * silu(gate), with options other mixers use
 //
-// The order of every sum depends on the sizes alone, not on how a request was cut into portions or on what else is
-// in the step.
+// Which form runs depends on the portion's length and, through the estimates of their times, on the step's tokens, its requests
+// and the sizes: token loop or tiles, lanes per column of the token loop, one or eight tokens per warp of the preparation.
+// Within a form the order of every sum is fixed; between forms, so between ways to cut a request into portions and between
+// neighbours in a step, results differ by float32 rounding.
 #include "state_tiles.cuh"
 #include <math.h>
 using namespace bspec;

@@ -10,9 +10,11 @@
 //                              y_c = sum_n S[c, n] C_n + D_c x_c,  out_c = y_c silu(z_c),  dt = softplus(raw + bias),
 //                              A = -exp(A_log)
 //
-// A step holds portions of several requests (qo_indptr, state_slots); a portion of one token is a decode step.  Every
-// sum runs in an order fixed by the sizes alone, so a position's result does not depend on how the request was cut
-// or on what else is in the step.
+// A step holds portions of several requests (qo_indptr, state_slots); a portion of one token is a decode step.
+// Which form runs depends on the portion's length and, through the estimates of their times, on the step's tokens, its requests
+// and the sizes: lightning attention token by token or by tiles, the scan end to end or in segments, lanes per column or
+// channel.  Within a form the order of every sum is fixed; between forms, so between ways to cut a request into portions and
+// between neighbours in a step, results differ by float32 rounding.
 #include "state_tiles.cuh"
 #include <math.h>
 using namespace bspec;
@@ -430,11 +432,11 @@ constexpr int SC_MAX_N = 256;
 // LN lanes per channel; lane l keeps states l, l + LN, ... (NPL of them) of its channel in registers.  Tokens go
 // SC_TT at a time: the next batch's B and C rows and the channel's own x, dt and z are fetched into registers while
 // the recurrence runs over the current batch, and softplus and silu are taken once per batch outside the chain, so
-// what is left per token is one exponential and two multiply-adds per state.  Every token's arithmetic is the same
-// wherever it falls in a batch, so a position's result does not depend on where a portion was cut.
+// what is left per token is one exponential and two multiply-adds per state.  End to end, every token's arithmetic is the
+// same wherever it falls in a batch, so the result does not depend on where a portion was cut.
 //
 // A chain of 2,048 tokens takes 605 us whatever the device has free (4,096 channels of 16 states: 32 to 128 blocks).  So
-// long portions of few requests go in segments of SC_SEG tokens, all at once: MODE 1 runs every segment from a zero state
+// long portions go in segments of SC_SEG tokens, all at once, where that is faster (bspec_scan_scratch): MODE 1 runs every segment from a zero state
 // and leaves its end state and the sum of its dt; scan_segments_kernel carries the state from segment to segment,
 // S <- exp(A sum dt) S + end, leaving the state before each; MODE 2 runs every segment again from there and writes the
 // outputs.  Twice the arithmetic, but on all SMs.  MODE 0: the portion from end to end.
