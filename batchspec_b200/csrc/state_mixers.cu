@@ -771,7 +771,7 @@ BSPEC_API int bspec_selective_scan(const float* xz, long long ld, const float* x
   do {                                                                                                               \
     if (scratch != nullptr) {                                                                                        \
       if (N <= 16) LSS(T, 16); else LSS(T, 32);                                                                      \
-    } else if (few) {                                                                                                       \
+    } else if (few) {                                                                                                \
       if (N <= 16) LS(T, 4, 4); else if (N <= 32) LS(T, 8, 4); else if (N <= 64) LS(T, 8, 8);                        \
       else if (N <= 128) LS(T, 16, 8); else LS(T, 32, 8);                                                            \
     } else {                                                                                                         \

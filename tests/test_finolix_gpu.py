@@ -308,6 +308,8 @@ LATENT_WINDOW_SHAPES = [
     (4, 64, 16, 8, [33, 1], [33, 2049], None),           # a sink without a window
     (16, 512, 64, 16, [1, 1, 40], [700, 65, 300], 128),  # the widest latent the tensor-core kernel takes
     (128, 256, 64, 64, [1, 2], [700, 65], 500),
+    (16, 512, 64, 16, [1, 1, 1], [700, 65, 300], 128),   # decode on 16-row tiles, whose warps divide the numbers of an entry
+    (7, 256, 32, 8, [1, 1, 1], [40, 333, 96], None),
 ]
 
 

@@ -591,6 +591,28 @@ def test_interleaved_rotation_and_append_from_wider_rows(ops, dtype, Hq, G, hd, 
     assert int((cache != 0).sum()) <= n * entry
 
 
+@pytest.mark.parametrize("dk,rot", [(128, 64), (64, 64), (256, 18)])
+def test_tiles_rotate_queries_and_keys(ops, dk, rot):
+    """Portions by tiles with the rotation inside, against the same tokens in portions that go token by token."""
+    Hh, dv, n = 2, 32, 301
+    gen = torch.Generator(device=DEV).manual_seed(rot)
+    proj, decay = torch.randn(n, Hh * (2 * dk + dv), device=DEV, generator=gen), torch.tensor([0.9, 0.99], device=DEV)
+    table = ops.rope_frequency_table(10000.0 ** (-torch.arange(rot // 2, dtype=torch.float64) / (rot // 2)), DEV)
+
+    def run(cuts):
+        state, outs = torch.zeros(1, Hh * dk * dv, device=DEV), []
+        for a, b in zip(cuts[:-1], cuts[1:]):
+            ctx = SimpleNamespace(qo_indptr=_i32([0, b - a]), n_entries=1, max_q_len=b - a, state_slots=_i32([0]), positions=_i32(range(7 + a, 7 + b)))
+            outs.append(ops.lightning_recurrence(proj[a:b], 0, Hh * dk, 2 * Hh * dk, decay, state, ctx, Hh, dk, dv, "silu", 0.5, table, rot))
+        return torch.cat(outs), state
+
+    assert ops.load_library().bspec_lightning_scratch(n, 1, n, n, Hh, dk, dv) > 0
+    (out, state), (want, state_want) = run([0, n]), run([0, 60, 61, 120, 180, 240, 300, n])
+    # the bound of the tests above
+    assert (out - want).abs().max() <= 2e-5 * max(1.0, want.abs().max().item())
+    assert (state - state_want).abs().max() <= 2e-5 * max(1.0, state_want.abs().max().item())
+
+
 @pytest.mark.parametrize("first", [1, 36, 1100])
 def test_tiles_are_found_among_many_requests(ops, first):
     """Long portions behind ``first`` decoded tokens, so that a tile's request is looked for among up to 1,104, against the same
@@ -654,7 +676,7 @@ def test_lightning_attention_by_tiles(ops, Hh, dk, dv, act, scale):
 
 
 @pytest.mark.parametrize("lens", [[512], [511, 513, 1, 64], [1000, 3]])
-@pytest.mark.parametrize("inner,N,taps", [(64, 16, 4), (130, 5, 1), (33, 40, 3)])
+@pytest.mark.parametrize("inner,N,taps", [(64, 16, 4), (130, 5, 1), (33, 40, 3), (96, 24, 2), (64, 32, 4)])
 def test_selective_scan_in_segments(ops, inner, N, taps, lens):
     """Portions long enough to run in segments at once (whole ones, partial ones, requests of a token beside them), from a
     state that is not zero, against the recurrence in float64; states and the convolution's inputs are left as the

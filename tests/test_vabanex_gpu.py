@@ -255,6 +255,11 @@ LATENT_SHAPES = [
     (3, 80, 48, 16, [70], [70]),
     (2, 96, 16, 16, [1, 1, 1], [5, 130, 64]),          # decode with a latent of 3 x 32
     (32, 160, 32, 16, [1, 1], [300, 31]),
+    # decode on 16-row tiles, whose warps divide the numbers of an entry: 8 and 16 output tiles per warp
+    (16, 256, 64, 16, [1, 1, 1], [300, 33, 1]),
+    (16, 512, 64, 16, [1, 1, 1, 1], [700, 17, 64, 129]),
+    (5, 512, 64, 8, [1, 1], [95, 31]),
+    (8, 384, 32, 16, [1, 1, 1], [64, 250, 5]),
 ]
 
 
