@@ -134,6 +134,9 @@ _SIGNATURES = {
                           c_void_p, c_void_p, c_longlong, c_void_p],
     "bspec_sgemm_tn_batched": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_longlong, c_longlong, c_longlong,
                                c_longlong, c_longlong, c_longlong, c_int, c_void_p, c_int, c_void_p, c_void_p],
+    "bspec_sgemm_tc": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_longlong, c_longlong, c_void_p, c_void_p, c_void_p],
+    "bspec_sgemm_tc_scratch": [c_void_p, c_int, c_int, c_int, c_longlong],
+    "bspec_sgemm_tc_launches": [c_int, c_int, c_int],
     "bspec_sgemm_scratch": [c_void_p, c_void_p, c_int, c_int, c_int, c_longlong, c_longlong, c_longlong, c_longlong, c_int],
     "bspec_attention_generic": [c_void_p, c_longlong, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p,
                                 c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_int, c_longlong, c_void_p],
@@ -227,7 +230,7 @@ def set_pdl(on: bool) -> None:
 
 
 _TRACE_SETTERS = ["bspec_trace_set_attention_tcgen05", "bspec_trace_set_elementwise", "bspec_trace_set_attention_generic", "bspec_trace_set_attention_bf16",
-                  "bspec_trace_set_gemm_fp32", "bspec_trace_set_sampling", "bspec_trace_set_gemm_tcgen05", "bspec_trace_set_latent",
+                  "bspec_trace_set_gemm_fp32", "bspec_trace_set_gemm_fp32_tc", "bspec_trace_set_sampling", "bspec_trace_set_gemm_tcgen05", "bspec_trace_set_latent",
                   "bspec_trace_set_moe", "bspec_trace_set_latent_mma", "bspec_trace_set_delta",
                   "bspec_trace_set_state_mixers", "bspec_trace_set_streams", "bspec_trace_set_joins",
                   "bspec_trace_set_gated_states"]
@@ -1432,6 +1435,13 @@ def _sgemm(x, w, out, M: int, N: int, K: int, lda: int, ldw: int, sa: int, sw: i
     """``batch`` float32 products, operands sa / sw numbers apart; the K slices of small tiles meet in scratch that the
     stream's order protects."""
     lib = load_library()
+    split = lib.bspec_sgemm_tc_scratch(w.data_ptr(), M, N, K, ldw) if batch == 1 else 0
+    if split:
+        scratch = torch.empty((split,), dtype=torch.uint8, device=x.device)
+        _check(lib.bspec_sgemm_tc(x.data_ptr(), w.data_ptr(), out.data_ptr(), M, N, K, lda, ldw, scratch.data_ptr(),
+                                  _status_word(x.device).data_ptr(), _stream()), "sgemm_tc")
+        count_launches(lib.bspec_sgemm_tc_launches(M, N, K) - 1)
+        return
     need = lib.bspec_sgemm_scratch(x.data_ptr(), w.data_ptr(), M, N, K, lda, ldw, sa, sw, batch)
     scratch = torch.empty((need,), dtype=torch.float32, device=x.device) if need else None
     _check(lib.bspec_sgemm_tn_batched(x.data_ptr(), w.data_ptr(), out.data_ptr(), M, N, K, lda, ldw, N, sa, sw, M * N, batch,

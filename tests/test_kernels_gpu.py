@@ -118,6 +118,51 @@ def test_sgemm_sums_have_one_order_in_every_kernel(ops, N, K, batch):
     ops.check_status()
 
 
+@pytest.mark.parametrize("M,N,K", [(192, 1024, 1024), (193, 900, 1028), (257, 516, 2080), (320, 2052, 480), (1030, 388, 548),
+                                   (200, 20484, 36), (640, 128, 4100)])
+def test_sgemm_of_many_rows_on_the_tensor_cores(ops, M, N, K):
+    """Ragged tiles in every direction, K past the last 32 / 64 / 512, groups dealt to several CTAs and not.  The bound: a
+    span of 32 k rounds at most twice towards zero per 16 k and product (a unit each, of partial sums below the sum of
+    magnitudes), 16 spans and K / 512 groups add with half a unit each, 2^-25 of every product is left out."""
+    g = torch.Generator(device=DEV).manual_seed(M + K)
+    a = torch.randn(M, K + 4, device=DEV, generator=g)[:, :K]
+    w = torch.randn(N, K, device=DEV, generator=g)
+    lib = ops.load_library()
+    assert lib.bspec_sgemm_tc_scratch(w.data_ptr(), M, N, K, K) > 0
+    got = ops.linear(a, w)
+    want, mag = a.double() @ w.double().T, a.abs().double() @ w.abs().double().T
+    bound = 2.0 ** -24 * (2 * 4 + 16 + K / 512 + 2) * mag
+    assert bool(((got.double() - want).abs() <= bound).all())
+    whole = (got.double() - want).norm() / want.norm()
+    assert whole <= 2.0 ** -23, whole                      # as near to the exact sums as the chains of float32 numbers
+    part = ops.linear(a[M - 192:].contiguous(), w)          # another cut into tiles and along K: the same bits
+    assert lib.bspec_sgemm_tc_scratch(w.data_ptr(), 192, N, K, K) == 0 or torch.equal(part, got[M - 192:])
+    odd = torch.empty(M * (K + 1) + 1, device=DEV)[1:].view(M, K + 1)[:, :K]
+    assert torch.equal(ops.linear(odd.copy_(a), w), got)    # rows that begin off a 16-byte boundary
+    ops.check_status()
+
+
+def test_sgemm_on_the_tensor_cores_keeps_what_is_not_finite(ops):
+    """Infinities, NaN, and magnitudes up to the type's largest and below its smallest normal number."""
+    g = torch.Generator(device=DEV).manual_seed(9)
+    a, w = torch.randn(200, 2048, device=DEV, generator=g), torch.randn(512, 2048, device=DEV, generator=g)
+    a[3, 7], a[5, 9], w[11, 100] = math.inf, math.nan, -math.inf
+    a[100], a[101, 0], a[150] = 3e38, torch.finfo(torch.float32).max, 1e-42
+    w[20] = 0.0
+    w[20, 0] = 1.0                                             # row 101 x 20: the largest number itself
+    got, want = ops.linear(a, w), a.double() @ w.double().T
+    plain = torch.cat([ops.linear(a[i:i + 1], w) for i in range(200)])
+    assert torch.equal(torch.isnan(got), torch.isnan(plain)) and torch.equal(torch.isinf(got), torch.isinf(plain))
+    assert got[101, 20] == a[101, 0] and bool(torch.isinf(got[3, 0])) and bool(torch.isnan(got[5]).all())
+    rows, cols = torch.ones(200, dtype=torch.bool, device=DEV), torch.ones(512, dtype=torch.bool, device=DEV)
+    rows[[3, 5, 100, 101, 150]], cols[11] = False, False
+    err = (got.double() - want).abs()
+    assert err[rows][:, cols].max() <= 1e-6 * want[rows][:, cols].abs().max()
+    # 2,048 products of multiples of 2^-149, each rounded to one, and the sums' own rounding
+    assert bool((err[150][cols] <= 2048 * 2.0 ** -149 + 1e-6 * want[150][cols].abs()).all())
+    ops.check_status()
+
+
 def test_sgemm_takes_many_products_of_long_sums(ops):
     """2,000 products of one output column and 64 groups of k: as many K slices as a grid's z still takes."""
     B, M, K = 2000, 33, 65536
