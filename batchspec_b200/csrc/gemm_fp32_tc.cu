@@ -3,7 +3,7 @@
 // A float32 number is the sum of three bfloat16 numbers (8 significant bits each, rounded to nearest, every remainder
 // exact): x = x1 + x2 + x3.  Of the nine products of two such sums the six of at most 2^-16 of the whole are formed,
 // x1 y1 + (x1 y2 + x2 y1) + (x1 y3 + x2 y2 + x3 y1); each is exact in float32, and what is left out is below 2^-25 of
-// |x y|.  The tensor core's accumulator rounds towards zero, so it never carries a long sum: it takes SPAN numbers of K,
+// |x y|.  (The tensor core takes parts below the smallest normal number, 2^-126, as zero: numbers below 2^-102 lose digits.)  The tensor core's accumulator rounds towards zero, so it never carries a long sum: it takes SPAN numbers of K,
 // smallest products first, and what it has then is added in float32, rounded to nearest, by the threads that read it:
 //   span    32 k in the tensor core;
 //   group   512 k: its spans, added in order;
@@ -34,7 +34,7 @@ constexpr int TN = 128;                            // rows of W = accumulator ro
 constexpr int TT = 128;                            // rows of A = accumulator columns
 constexpr int KB = 64, SPAN = 32, GROUP = 512;
 constexpr int MIN_ROWS = 192;
-constexpr double MIN_WORK = 1 << 27;
+constexpr double MIN_WORK = 1 << 28;
 constexpr int B_STAGES = 3, W_STAGES = 4, A_STAGES = 4;
 constexpr int PLANE = TT * KB * 2;                 // bytes of one plane of a stage
 constexpr int B_BYTES = 3 * PLANE, W_BYTES = TN * SPAN * 4;
@@ -390,6 +390,9 @@ int tc_splits(int M, int N, int K) {
 
 // Which products come here.  From 33 rows on this kernel is the faster one (33 x 16,384 x 2,048 79 against 136 us); up to
 // 191 rows the chains of gemm_fp32.cu stay, so that a decode step, a short prompt and a portion give a row the same bits.
+// Small products do not pay for the taking apart and the pipeline's filling, us, multiply-adds / here: 512 x 512 x 512 20.5 / 28.5,
+// 2,048 x 256 x 256 18.5 / 21.5; 2^28 and more: 1,024 x 512 x 512 28.8 / 28.7, 256 x 512 x 2,048 33.8 / 32.7, 1,024^3 78 / 36,
+// 4,096 x 128 x 2,048 90 / 48, 192 x 2,048 x 2,048 71 / 35.
 bool takes(const float* W, int M, int N, int K, long long ldw) {
   return M >= MIN_ROWS && N % 4 == 0 && K >= SPAN && (ldw & 3) == 0 && ((uintptr_t)W & 15) == 0 &&
          (double)M * N * K >= MIN_WORK;
