@@ -77,7 +77,7 @@ latent_attn_mma_kernel(const __nv_bfloat16* __restrict__ ql, long long ql_row, l
                        const int* __restrict__ kv_indices, int H, int R, int P, int page_size, float scale,
                        int n_splits, float* __restrict__ o_part, float* __restrict__ ml_part, long long n_pages,
                        const float* __restrict__ inv_freq, float magnitude, int window,
-                       const float* __restrict__ sink) {
+                       const float* __restrict__ sink, int skip_from) {
   constexpr int BM = 16 * RG;
   constexpr int KW = BN / CH;                     // keys of a score tile per warp: 16 or 8
   constexpr int TPR = 2 * CH, KPT = BN / TPR;     // softmax: threads per row, keys per thread
@@ -96,6 +96,7 @@ latent_attn_mma_kernel(const __nv_bfloat16* __restrict__ ql, long long ql_row, l
 
   const int e = blockIdx.y, split = blockIdx.z;
   const int q_begin = qo_indptr[e], q_len = qo_indptr[e + 1] - q_begin;
+  if (q_len >= skip_from) return;                  // another kernel's portions
   const long long rows_total = (long long)q_len * H;
   const long long row0 = (long long)blockIdx.x * BM;
   if (row0 >= rows_total) return;
@@ -575,6 +576,7 @@ BSPEC_API int bspec_latent_attention_mma_rows(int max_q_len, int H, int R, int P
   return two_small_ctas(R, P) ? 32 : 64;
 }
 
+// ``skip_from``: portions of that many tokens and more are left alone (``max_q_len``: the longest of the others).
 BSPEC_API int bspec_latent_attention_mma(const void* ql, long long ql_row, long long ql_head, const void* qr,
                                          long long qr_row, long long qr_head, void* out, long long o_row,
                                          long long o_head, const void* cache, const int* qo_indptr,
@@ -582,7 +584,7 @@ BSPEC_API int bspec_latent_attention_mma(const void* ql, long long ql_row, long 
                                          int n_entries, int n_tokens, int max_q_len, int H, int R, int P,
                                          int page_size, float scale, int n_splits, float* o_part, float* ml_part,
                                          long long n_pages, const float* inv_freq, float magnitude, int window,
-                                         const float* sink, cudaStream_t stream) {
+                                         const float* sink, int skip_from, cudaStream_t stream) {
   const bool wide = prompt_mode() != 1;
   if (n_entries <= 0 || max_q_len <= 0) return 0;
   if (!bspec_latent_attention_mma_supported(R, P) || n_splits < 1 || (n_splits > 1 && (!o_part || !ml_part)))
@@ -605,7 +607,7 @@ BSPEC_API int bspec_latent_attention_mma(const void* ql, long long ql_row, long 
     BSPEC_LAUNCH((latent_attn_mma_kernel<RG, CH, N>), grid, 32 * RG * CH, smem, stream, (const __nv_bfloat16*)ql,    \
                  ql_row, ql_head, (const __nv_bfloat16*)qr, qr_row, qr_head, (__nv_bfloat16*)out, o_row, o_head,     \
                  (const __nv_bfloat16*)cache, qo_indptr, positions, kv_indptr, kv_indices, H, R, P, page_size,       \
-                 scale, n_splits, o_part, ml_part, n_pages, inv_freq, magnitude, window, sink); \
+                 scale, n_splits, o_part, ml_part, n_pages, inv_freq, magnitude, window, sink, skip_from); \
   } while (0)
 #define LMS(RG, CH, N, DS)                                                                                           \
   do {                                                                                                               \
@@ -613,7 +615,7 @@ BSPEC_API int bspec_latent_attention_mma(const void* ql, long long ql_row, long 
     BSPEC_LAUNCH((latent_attn_mma_kernel<RG, CH, N, 1, DS>), grid, 32 * RG * CH, smem, stream, (const __nv_bfloat16*)ql, \
                  ql_row, ql_head, (const __nv_bfloat16*)qr, qr_row, qr_head, (__nv_bfloat16*)out, o_row, o_head,     \
                  (const __nv_bfloat16*)cache, qo_indptr, positions, kv_indptr, kv_indices, H, R, P, page_size,       \
-                 scale, n_splits, o_part, ml_part, n_pages, inv_freq, magnitude, window, sink); \
+                 scale, n_splits, o_part, ml_part, n_pages, inv_freq, magnitude, window, sink, skip_from); \
   } while (0)
 #define LM1(RG, CH, N) LMS(RG, CH, N, false)
   if (small_pair) {

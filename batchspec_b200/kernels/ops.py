@@ -15,8 +15,10 @@ import ctypes
 import sys
 import threading
 from ctypes import c_float, c_int, c_longlong, c_ulonglong, c_void_p
+from dataclasses import dataclass
 from typing import Optional
 
+import numpy as np
 import torch
 
 _lib = None
@@ -117,7 +119,13 @@ _SIGNATURES = {
     "bspec_latent_attention_mma": [c_void_p, c_longlong, c_longlong, c_void_p, c_longlong, c_longlong, c_void_p,
                                    c_longlong, c_longlong, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int,
                                    c_int, c_int, c_int, c_int, c_int, c_float, c_int, c_void_p, c_void_p, c_longlong,
-                                   c_void_p, c_float, c_int, c_void_p, c_void_p],
+                                   c_void_p, c_float, c_int, c_void_p, c_int, c_void_p],
+    "bspec_latent_prompt_supported": [c_int, c_int, c_int, c_int],
+    "bspec_latent_gather": [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int,
+                            c_void_p, c_void_p, c_void_p, c_longlong, c_void_p],
+    "bspec_latent_prompt": [c_void_p, c_longlong, c_int, c_int, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_longlong,
+                            c_longlong, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_void_p,
+                            c_void_p, c_void_p],
     "bspec_gate_heads": [c_void_p, c_longlong, c_longlong, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int, c_void_p],
     "bspec_moe_route": [c_void_p, c_int, c_int, c_int, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_float,
                         c_void_p, c_void_p, c_void_p, c_longlong, c_int, c_void_p],
@@ -231,7 +239,7 @@ def set_pdl(on: bool) -> None:
 
 _TRACE_SETTERS = ["bspec_trace_set_attention_tcgen05", "bspec_trace_set_elementwise", "bspec_trace_set_attention_generic", "bspec_trace_set_attention_bf16",
                   "bspec_trace_set_gemm_fp32", "bspec_trace_set_gemm_fp32_tc", "bspec_trace_set_sampling", "bspec_trace_set_gemm_tcgen05", "bspec_trace_set_latent",
-                  "bspec_trace_set_moe", "bspec_trace_set_latent_mma", "bspec_trace_set_delta",
+                  "bspec_trace_set_moe", "bspec_trace_set_latent_mma", "bspec_trace_set_latent_prompt", "bspec_trace_set_delta",
                   "bspec_trace_set_state_mixers", "bspec_trace_set_streams", "bspec_trace_set_joins",
                   "bspec_trace_set_gated_states"]
 TRACE_KERNEL_NAMES = {1: "embed", 2: "add_rmsnorm", 3: "gather_rows_add", 4: "silu_mul", 5: "rope_kv_append",
@@ -1479,14 +1487,16 @@ FORCE_GENERIC_LATENT = False       # tests set this to compare the tensor-core k
 
 def latent_attention(q_lat: torch.Tensor, q_rot: torch.Tensor, out: torch.Tensor, cache: torch.Tensor, ctx, tables,
                      n_heads: int, kv_rank: int, rot_dim: int, scale: float, rotate=None, window: int = 0,
-                     sink: Optional[torch.Tensor] = None) -> None:
+                     sink: Optional[torch.Tensor] = None, others: Optional["LongPortions"] = None) -> None:
     """Causal softmax attention in the latent space over the paged entries [c | kr].  ``q_lat`` [H, n, kv_rank] and
     ``q_rot`` [n, H, rot_dim] are views with a dense last dim; ``out`` [H, n, kv_rank] receives sum_j p_j c_j per
     head.  ``rotate`` None: ``q_rot`` is already rotated.  ``rotate`` = (``rope_frequency_table``, magnitude):
     it is not, and is rotated by adjacent pairs on the way, inside the tensor-core kernel as it loads the queries,
     or in place by the rotation kernel before the generic one.  ``window`` > 0: a query sees its own entry and the
-    ``window - 1`` before it.  ``sink`` (float32 per head): exp(sink) joins the softmax denominator."""
+    ``window - 1`` before it.  ``sink`` (float32 per head): exp(sink) joins the softmax denominator.  ``others`` (from
+    ``latent_long_portions``, so on the tensor cores): those portions' rows of ``out`` are not written."""
     _require_cuda(q_lat, q_rot, out, cache, sink)
+    max_q_len = ctx.max_q_len if others is None else others.longest_other
     assert sink is None or (sink.dtype == torch.float32 and sink.numel() == n_heads and sink.is_contiguous())
     H, n, R = q_lat.shape
     assert H == n_heads and R == kv_rank and q_rot.shape == (n, H, rot_dim) and out.shape == (H, n, R)
@@ -1498,14 +1508,14 @@ def latent_attention(q_lat: torch.Tensor, q_rot: torch.Tensor, out: torch.Tensor
         # Few rows and many entries (decode): the key tiles of a request are cut into shares for more CTAs.  The
         # count depends on the step's shape alone (entries, longest portion, longest allowed request), so a
         # captured step keeps it; shares that get no tile leave at once.
-        rows = lib.bspec_latent_attention_mma_rows(ctx.max_q_len, n_heads, kv_rank, rot_dim)       # rows of a CTA's tile
-        row_tiles = -(-(ctx.max_q_len * n_heads) // rows)
+        rows = lib.bspec_latent_attention_mma_rows(max_q_len, n_heads, kv_rank, rot_dim)       # rows of a CTA's tile
+        row_tiles = -(-(max_q_len * n_heads) // rows)
         n_splits = 1
-        if ctx.max_q_len * n_heads <= 256:
+        if max_q_len * n_heads <= 256:
             # as many shares as fill the CTAs that are resident at once (one wave), at least 256 keys each
             smem = lib.bspec_latent_attention_mma_smem(rows, kv_rank, rot_dim, 0) + 1024
             slots = sm_count(q_lat.device) * max(1, min(4, (227 * 1024) // smem))
-            keys = min(ctx.max_kv_len, window + ctx.max_q_len) if window > 0 else ctx.max_kv_len
+            keys = min(ctx.max_kv_len, window + max_q_len) if window > 0 else ctx.max_kv_len
             n_splits = max(1, min(64, slots // (ctx.n_entries * row_tiles), -(-keys // 256)))
         o_part = ml_part = None
         if n_splits > 1:
@@ -1515,12 +1525,14 @@ def latent_attention(q_lat: torch.Tensor, q_rot: torch.Tensor, out: torch.Tensor
             q_lat.data_ptr(), q_lat.stride(1), q_lat.stride(0), q_rot.data_ptr(), q_rot.stride(0), q_rot.stride(1),
             out.data_ptr(), out.stride(1), out.stride(0), cache.data_ptr(), ctx.qo_indptr.data_ptr(),
             ctx.positions.data_ptr(), tables.kv_indptr.data_ptr(), tables.kv_indices.data_ptr(), ctx.n_entries, n,
-            ctx.max_q_len, n_heads, kv_rank, rot_dim, tables.page_size, float(scale), n_splits, _ptr(o_part),
+            max_q_len, n_heads, kv_rank, rot_dim, tables.page_size, float(scale), n_splits, _ptr(o_part),
             _ptr(ml_part), cache.shape[0], rotate[0].data_ptr() if rotate else None,
-            float(rotate[1]) if rotate else 1.0, int(window), _ptr(sink), _stream()), "latent_attention_mma")
+            float(rotate[1]) if rotate else 1.0, int(window), _ptr(sink),
+            others.at_least if others is not None else 2 ** 31 - 1, _stream()), "latent_attention_mma")
         if n_splits > 1:
             count_launches(1)
         return
+    assert others is None
     if rotate:
         rope_inplace(q_rot, ctx.positions, rotate[0], rot_dim, True, rotate[1])
     _check(lib.bspec_latent_attention_generic(
@@ -1529,6 +1541,69 @@ def latent_attention(q_lat: torch.Tensor, q_rot: torch.Tensor, out: torch.Tensor
         ctx.qo_indptr.data_ptr(), ctx.positions.data_ptr(), tables.kv_indptr.data_ptr(), tables.kv_indices.data_ptr(),
         ctx.n_entries, ctx.max_q_len, n_heads, kv_rank, rot_dim, tables.page_size, float(scale), cache.shape[0],
         int(window), _ptr(sink), _stream()), "latent_attention_generic")
+
+
+LATENT_PROMPT_FROM = 64            # tokens of a portion from which keys and values per head are formed
+LATENT_PROMPT_ROWS = 1 << 19       # at most this many rows of keys (600 MB of entries)
+LATENT_PROMPT_BYTES = 512 << 20    # keys and values of as many heads at a time as this holds
+
+
+@dataclass
+class LongPortions:
+    """The portions of a step that attend over keys and values per head."""
+    at_least: int                  # the shortest has this many tokens or more
+    rows: int                      # rows of keys, every portion's rounded up to 64
+    longest: int
+    longest_other: int             # 0: the step has no other portions
+
+
+def latent_long_portions(ctx, dtype: torch.dtype, kv_rank: int, dim: int, rot_dim: int, v_dim: int,
+                         window: int = 0) -> Optional[LongPortions]:
+    """The step's portions of at least ``LATENT_PROMPT_FROM`` tokens, None when there are none or ``latent_prompt`` does not
+    take these sizes.  Needs the lengths on the host: a captured step has none."""
+    host = getattr(ctx, "host", None)
+    if (host is None or ctx.max_q_len < LATENT_PROMPT_FROM or dtype != torch.bfloat16 or FORCE_GENERIC_LATENT
+            or not latent_mma_supported(kv_rank, rot_dim)
+            or not load_library().bspec_latent_prompt_supported(kv_rank, dim, rot_dim, v_dim)):
+        return None
+    lens = np.diff(host["qo_indptr"]).astype(np.int64)
+    kv = host["kv_len"].astype(np.int64)
+    first = np.maximum(kv - lens - window + 1, 0) // 64 * 64 if window > 0 else np.zeros_like(kv)
+    chosen = lens >= LATENT_PROMPT_FROM
+    rows = int(((kv - first + 63) // 64 * 64)[chosen].sum())
+    if rows > LATENT_PROMPT_ROWS:
+        return None
+    return LongPortions(LATENT_PROMPT_FROM, rows, int(lens[chosen].max()), int(lens[~chosen].max()) if not chosen.all() else 0)
+
+
+def latent_prompt(q: torch.Tensor, w_kv: torch.Tensor, out: torch.Tensor, cache: torch.Tensor, ctx, tables, long: LongPortions,
+                  n_heads: int, kv_rank: int, scale: float, window: int = 0, sink: Optional[torch.Tensor] = None) -> None:
+    """Causal softmax attention of the step's long portions over keys and values per head.  ``q`` [n, H, dim + rot_dim], the
+    rotated part rotated; ``w_kv`` [H, dim + v_dim, kv_rank], the rows that make a head's key and value parts of a latent;
+    ``out`` [H, n, v_dim], a view with a dense last dim, receives sum_j p_j v_j.  The other rows of ``out`` stay."""
+    _require_cuda(q, w_kv, out, cache, sink)
+    H, n, V = out.shape
+    R, width = int(kv_rank), w_kv.shape[1]
+    assert q.is_contiguous() and w_kv.is_contiguous() and cache.is_contiguous() and out.stride(2) == 1
+    assert q.shape[:2] == (n, H) and H == n_heads and w_kv.shape == (H, width, R) and cache.dtype == torch.bfloat16
+    assert sink is None or (sink.dtype == torch.float32 and sink.numel() == H and sink.is_contiguous())
+    lib, dev, T = load_library(), q.device, long.rows
+    entries = torch.empty((T, R), dtype=torch.bfloat16, device=dev)
+    rotated = torch.empty((T, q.shape[2] - (width - V)), dtype=torch.bfloat16, device=dev)
+    base = torch.empty((ctx.n_entries,), dtype=torch.int32, device=dev)
+    _check(lib.bspec_latent_gather(cache.data_ptr(), ctx.qo_indptr.data_ptr(), ctx.positions.data_ptr(), tables.kv_indptr.data_ptr(),
+                                   tables.kv_indices.data_ptr(), ctx.n_entries, R, tables.page_size, int(window), long.at_least, T,
+                                   entries.data_ptr(), rotated.data_ptr(), base.data_ptr(), cache.shape[0], _stream()),
+           "latent_gather")
+    step = max(1, min(H, LATENT_PROMPT_BYTES // (T * width * 2)))
+    for h in range(0, H, step):
+        w = w_kv[h:h + step]
+        kv = linear(entries, w.reshape(-1, R), w_is_parameter=True)
+        _check(lib.bspec_latent_prompt(q.data_ptr(), q.stride(0), n, H, kv.data_ptr(), rotated.data_ptr(), base.data_ptr(), T,
+                                       out.data_ptr(), out.stride(1), out.stride(0), ctx.qo_indptr.data_ptr(),
+                                       ctx.positions.data_ptr(), ctx.n_entries, long.longest, h, w.shape[0], int(window),
+                                       long.at_least, float(scale), _ptr(sink), _status_word(dev).data_ptr(), _stream()),
+               "latent_prompt")
 
 
 def latent_mma_supported(kv_rank: int, rot_dim: int) -> bool:

@@ -12,14 +12,17 @@ Options: ``gated`` False leaves the gate out; ``window`` W keeps the keys i - W 
 window has passed are given back); ``sink``: a learned logit per head that only enlarges the softmax's denominator
 (nothing is attended through it, and ``scale`` does not touch it).
 
-Only [c | rot(kr)] is cached (one tensor per token, ``kv_rank + rot_dim`` numbers).  The per-head keys and values
-are never formed: since q_h . (Wuk_h c) = (Wuk_h^T q_h) . c, the unrotated query is taken into the latent space
+Only [c | rot(kr)] is cached (one tensor per token, ``kv_rank + rot_dim`` numbers).  Decoded tokens and short portions
+never form per-head keys and values: since q_h . (Wuk_h c) = (Wuk_h^T q_h) . c, the unrotated query is taken into the latent space
 (one small product per head), attention runs there for all heads over the same entries, and the head's value
 up-projection is applied to its attended latent afterwards.  The step's launch sequence:
 
     one product for [Wdq; Wdkv; Wg] (float32 out) -> latent_prepare (both RMS norms in float32, rotation of kr,
     cache append) -> Wuq -> per-head Wuk^T -> latent attention (which rotates the queries' rotated parts as it
     loads them) -> per-head Wuv -> gate and regroup -> Wo
+
+Long portions (``ops.latent_long_portions``) do: [Wuk; Wuv] of the entries that they see in one product, a flash attention
+per head over the result (``ops.latent_prompt``), gate and Wo.
 """
 from __future__ import annotations
 
@@ -81,6 +84,8 @@ class LatentAttention(Mixer):
         # Wuk_h^T as the [N, K] operand of "x @ w^T": [H, kv_rank, head_dim]
         self.w_uk_t = params["uk"].view(H, self.head_dim, self.kv_rank).transpose(1, 2).contiguous()
         self.w_uv = params["uv"].view(H, self.v_dim, self.kv_rank).contiguous()
+        # per head [Wuk_h; Wuv_h], for portions that form keys and values
+        self.w_kv = torch.cat([params["uk"].view(H, self.head_dim, self.kv_rank), self.w_uv], dim=1).contiguous()
         self.w_o = params["o"].contiguous()
         self.n_q, self.n_kv = params["dq_norm"], params["dkv_norm"]
         if self.n_kv.dtype != self.n_q.dtype:
@@ -108,15 +113,28 @@ class LatentAttention(Mixer):
                                     tables.kv_indices, cache.kv, tables.page_size, write_kv=cache.owner)
         with bucket("attn.q_proj"):
             q = ops.linear(cq, self.w_uq, w_is_parameter=True).view(n, H, dh + P)
-        q_rot = q[:, :, dh:]                      # rotated on its way into the attention kernel
-        with bucket("attn.absorb"):
-            q_lat = ops.linear_batched(q[:, :, :dh].transpose(0, 1), self.w_uk_t, w_is_parameter=True)          # [H, n, R]
-        o_lat = torch.empty((H, n, R), dtype=x.dtype, device=x.device)
-        with bucket("attn.compute"):
-            ops.latent_attention(q_lat, q_rot, o_lat, cache.kv, ctx, tables, H, R, P, self.scale,
-                                 rotate=(pos.inv_freq, pos.magnitude), window=self.window, sink=self.sinks)
-        with bucket("attn.v_proj"):
-            v = ops.linear_batched(o_lat, self.w_uv, w_is_parameter=True)                                        # [H, n, v_dim]
+        q_rot = q[:, :, dh:]
+        long = ops.latent_long_portions(ctx, x.dtype, R, dh, P, self.v_dim, self.window)
+        v = None
+        if long is not None:
+            with bucket("attn.rotate"):
+                ops.rope_inplace(q_rot, ctx.positions, pos.inv_freq, P, True, pos.magnitude)
+        if long is None or long.longest_other:
+            with bucket("attn.absorb"):
+                q_lat = ops.linear_batched(q[:, :, :dh].transpose(0, 1), self.w_uk_t, w_is_parameter=True)      # [H, n, R]
+            o_lat = torch.empty((H, n, R), dtype=x.dtype, device=x.device)
+            with bucket("attn.compute"):          # (unless they are rotated already, the queries are on their way in)
+                ops.latent_attention(q_lat, q_rot, o_lat, cache.kv, ctx, tables, H, R, P, self.scale,
+                                     rotate=(pos.inv_freq, pos.magnitude) if long is None else None, window=self.window,
+                                     sink=self.sinks, others=long)
+            with bucket("attn.v_proj"):
+                v = ops.linear_batched(o_lat, self.w_uv, w_is_parameter=True)                                    # [H, n, v_dim]
+        if long is not None:
+            if v is None:
+                v = torch.empty((n, H, self.v_dim), dtype=x.dtype, device=x.device).transpose(0, 1)
+            with bucket("attn.compute"):
+                ops.latent_prompt(q, self.w_kv, v, cache.kv, ctx, tables, long, H, R, self.scale, window=self.window,
+                                  sink=self.sinks)
         heads = torch.empty((n, H * self.v_dim), dtype=x.dtype, device=x.device)
         with bucket("attn.gate"):
             if self.gated:

@@ -309,6 +309,112 @@ def test_latent_attention_rotates_the_queries_on_the_way(ops, dtype, generic):
     assert torch.equal(got, want)
 
 
+LONG_PORTIONS = [
+    # heads, latent, page, q_lens, kv_lens, window, sinks, heads at a time
+    (2, 64, 16, [64], [64], 0, False, 2),
+    (3, 48, 5, [65, 1, 300, 63], [65, 90, 301, 400], 0, True, 1),        # ragged rows, short portions between
+    (1, 512, 16, [128, 256, 257], [1000, 256, 257], 0, False, 1),         # tiles just full and one over
+    (5, 40, 8, [700], [733], 100, True, 2),                               # a window shorter than a block of rows
+    (2, 64, 64, [129, 70], [2500, 71], 1024, False, 2),
+    (40, 24, 16, [513, 600], [513, 640], 0, False, 40),                   # more items than SMs: CTAs take a second one
+]
+
+
+@pytest.mark.parametrize("heads,R,ps,q_lens,kv_lens,window,sinks,group", LONG_PORTIONS)
+def test_long_portions_over_keys_and_values_per_head(ops, heads, R, ps, q_lens, kv_lens, window, sinks, group, monkeypatch):
+    """Against a float64 softmax over the bfloat16 keys and values that the product gives.  Scores are sums of 192 float32
+    products (2^-17 of a weight at these sizes), weights carry 2^-17, the result is rounded to bfloat16.  Pages behind the
+    window are given back (page numbers that do not exist); rows of short portions are not written."""
+    dk, P_, V, D = 128, 64, 128, R + 64
+    g = torch.Generator(device=DEV).manual_seed(R + len(q_lens))
+    n, E = sum(q_lens), len(q_lens)
+    q = torch.randn(n, heads, dk + P_, device=DEV, generator=g).bfloat16()
+    w = (torch.randn(heads, dk + V, R, device=DEV, generator=g) * R ** -0.5).bfloat16()
+    ents = [torch.randn(L, D, device=DEV, generator=g).bfloat16() for L in kv_lens]
+    sink = torch.randn(heads, device=DEV, generator=g) if sinks else None
+    pages_per = [-(-L // ps) for L in kv_lens]
+    perm = torch.randperm(sum(pages_per) + 3, generator=torch.Generator().manual_seed(1))[:sum(pages_per)]
+    cache = torch.full((sum(pages_per) + 3, 1, ps * D), math.inf, device=DEV, dtype=torch.bfloat16)
+    indptr = [0] + list(np.cumsum(pages_per))
+    for e, L in enumerate(kv_lens):
+        padded = torch.full((pages_per[e] * ps, D), math.inf, device=DEV, dtype=torch.bfloat16)
+        padded[:L] = ents[e]
+        cache[perm[indptr[e]:indptr[e + 1]].to(DEV), 0] = padded.view(pages_per[e], ps * D)
+    table = perm.clone()
+    lows = [max(0, L - x - window + 1) if window else 0 for x, L in zip(q_lens, kv_lens)]
+    for e, low in enumerate(lows):
+        table[indptr[e]:indptr[e] + low // ps] = -1
+    qo = np.concatenate([[0], np.cumsum(q_lens)]).astype(np.int32)
+    pos = torch.cat([torch.arange(L - x, L) for x, L in zip(q_lens, kv_lens)]).to(DEV, torch.int32)
+    ctx = SimpleNamespace(qo_indptr=torch.from_numpy(qo).to(DEV), positions=pos, n_entries=E, n_tokens=n, max_q_len=max(q_lens),
+                          max_kv_len=max(kv_lens), host=dict(qo_indptr=qo, kv_len=np.asarray(kv_lens, np.int32)))
+    tables = SimpleNamespace(kv_indptr=torch.tensor(indptr, dtype=torch.int32, device=DEV),
+                             kv_indices=table.to(DEV, torch.int32), page_size=ps)
+    monkeypatch.setattr(ops, "latent_mma_supported", lambda *a: True)
+    long = ops.latent_long_portions(ctx, torch.bfloat16, R, dk, P_, V, window)
+    assert long.longest_other == max([x for x in q_lens if x < 64], default=0)
+    monkeypatch.setattr(ops, "LATENT_PROMPT_BYTES", group * long.rows * (dk + V) * 2)
+    out = torch.full((n, heads, V), 7.0, device=DEV, dtype=torch.bfloat16).transpose(0, 1)
+    scale = 0.1
+    ops.latent_prompt(q, w, out, cache, ctx, tables, long, heads, R, scale, window=window, sink=sink)
+    ops.check_status()
+    # the same rows of entries through the same products: keys and values of the same bits
+    firsts = [low // 64 * 64 for low in lows]
+    rows_in, at, r0 = torch.zeros(long.rows, R, device=DEV, dtype=torch.bfloat16), {}, 0
+    for e, (x, L) in enumerate(zip(q_lens, kv_lens)):
+        if x >= 64:
+            rows_in[r0 + lows[e] - firsts[e]:r0 + L - firsts[e]] = ents[e][lows[e]:, :R]
+            at[e] = r0
+            r0 += -(-(L - firsts[e]) // 64) * 64
+    assert r0 == long.rows
+    kv_all = torch.cat([ops.linear(rows_in, w[h:h + group].reshape(-1, R)) for h in range(0, heads, group)], 1)
+    for e, (x, L) in enumerate(zip(q_lens, kv_lens)):
+        rows = slice(int(qo[e]), int(qo[e + 1]))
+        if x < 64:
+            assert bool((out[:, rows] == 7.0).all())
+            continue
+        f = firsts[e]
+        kv = kv_all[at[e]:at[e] + L - f].view(L - f, heads, dk + V).double()
+        k = torch.cat([kv[:, :, :dk], ents[e][f:, None, R:].double().expand(L - f, heads, P_)], -1)
+        sc = torch.einsum("qhd,khd->hqk", q[rows].double(), k) * scale
+        i, j = torch.arange(L - x, L, device=DEV)[:, None], torch.arange(f, L, device=DEV)[None]
+        sc = sc.masked_fill((j > i) | ((j <= i - window) if window else (j < 0)), -math.inf)
+        if sinks:
+            sc = torch.cat([sc, sink.double()[:, None, None].expand(heads, x, 1)], -1)
+        p = torch.softmax(sc, -1)[:, :, :L - f]
+        want = torch.einsum("hqk,khv->hqv", p, kv[:, :, dk:])
+        most = torch.einsum("hqk,khv->hqv", p, kv[:, :, dk:].abs())
+        assert bool(((out[:, rows].double() - want).abs() <= 2.0 ** -8 * want.abs() + 2.0 ** -13 * most + 1e-30).all()), e
+
+
+def test_an_engine_step_of_long_and_short_portions_gives_what_short_ones_give(ops):
+    """The same prompts whole, in portions that are partly short, and beside a decoding request, at the head sizes that form
+    keys and values: the logits agree as two roundings of one model do."""
+    from batchspec_b200.config import config_from_json_dict
+    from batchspec_b200.engine import Engine, StepEntry
+    mix = _mixer(4, 128, 64, 128, 96, 64, 0.08, 10000.0, None)
+    cfg = dict(CFG_A, layers=[dict(type="latent_attention", mixer=mix, mlp=dict(kind="dense", ff=80, limit=0.7))] * 2)
+    prompts = [H.random_tokens(n, cfg["vocab"], 50 + n) for n in (300, 150, 20)]
+    got = []
+    for cuts in ((300, 150, 20), (40, 40, 20), (170, 63, 3)):
+        eng = Engine(dtype="bfloat16", device=DEV)
+        eng.load_model(config=config_from_json_dict(cfg), random_seed=3, draw_on_device=True)
+        eng.setup_caches(max_batch_size=3, max_seq_length=512, page_size=16, prefill_chunk_size=512)
+        eng.setup_sampling_params(temperature=0.0)
+        for r in range(3):
+            eng.admit(r)
+        done, last = [0, 0, 0], {}
+        while any(d < len(p) for d, p in zip(done, prompts)):
+            step = [(r, done[r], min(cuts[r], len(p) - done[r])) for r, p in enumerate(prompts) if done[r] < len(p)]
+            out = eng.step([StepEntry(r, prompts[r][a:a + c], want=(c - 1,)) for r, a, c in step])
+            for (r, a, c), row in zip(step, out):
+                done[r] += c
+                last[r] = row.float().clone()
+        got.append(torch.stack([last[r] for r in range(3)]))
+    for other in got[1:]:
+        assert (got[0] - other).norm() <= 0.03 * got[0].norm()
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("key", [0, 15, 16, 511, 512, 1023, 1500])
 def test_one_far_entry_among_hundreds_is_found(ops, dtype, key):
