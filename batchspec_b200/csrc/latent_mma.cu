@@ -15,9 +15,9 @@
 // Entries arrive by cp.async; the block-table lookup of a tile is made one tile before its copies.  A CTA holds
 // two tiles of entries (the next one arrives under the current one's products: the 64-row tiles) or one (32-row
 // tiles of prompt portions and the 16- and 32-row tiles of decoded tokens: two to four CTAs then share an SM and
-// cover each other's loads, which measured faster).  With n_splits > 1 (decode: few rows, many entries) CTA z takes
-// the z-th share of the key tiles and leaves (max, sum, unnormalised output) for the join kernel, which adds the
-// shares in their order.  How the tiles are cut into shares follows from the request's length, read on the device.
+// cover each other's loads, which measured faster).  In steps of few rows and many entries (decode) the requests' key
+// tiles are dealt to the CTAs in even shares (``deal``); a CTA leaves (max, sum, unnormalised output) of its share for the
+// join kernel, which adds a request's shares in their order.
 #include "common.cuh"
 #include <math.h>
 #include <stdlib.h>
@@ -60,6 +60,84 @@ __host__ __device__ inline size_t smem_bytes(int D, int BM, int stages = 2, int 
   return (size_t)(BM + stages * BN) * DP * 2 + (size_t)shares * BM * (BN + 8) * 4 + 2 * (size_t)BM * (BN + 8) * 2 + 3 * BM * 4;
 }
 
+// The work of a step of few rows, dealt evenly: the requests' key tiles are cut into shares of ``per`` tiles, about as many
+// shares in all as CTAs fit the device at once (a request has at least one, at most MAX_SHARES), and CTA z takes the z-th.
+// Every CTA finds that out for itself from the lengths, so a captured step follows them.  (With as many shares for every
+// request the longest request's were the kernel's time: 64 requests of 300 to 4,096 entries, 16 heads.)
+constexpr int MAX_SHARES = 64, MIN_TILES = 4;
+struct Share {
+  int e, split, first, count, per;       // request (-1: none), which of its shares, its first share and how many it has
+};
+template <int NT>
+__device__ __forceinline__ Share deal(int z, const int* __restrict__ qo_indptr, const int* __restrict__ positions, int n_entries,
+                                      int window, int skip_from, int want_shares) {
+  __shared__ int part[3][NT / 32], found[3];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  auto tiles_of = [&](int e) -> int {
+    if (e >= n_entries) return 0;
+    const int q0 = qo_indptr[e], q1 = qo_indptr[e + 1];
+    if (q1 <= q0 || q1 - q0 >= skip_from) return 0;
+    const int pos0 = positions[q0];
+    return (pos0 + q1 - q0 - 1) / BN + 1 - (window > 0 ? max(0, pos0 - window + 1) / BN : 0);
+  };
+  if (tid == 0) found[0] = -1;
+  const int own = tiles_of(tid);
+  int total = 0, most = 0;
+  for (int e0 = 0; e0 < n_entries; e0 += NT) {
+    const int t = e0 == 0 ? own : tiles_of(e0 + tid);
+    total += t;
+    most = max(most, t);
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    total += __shfl_xor_sync(0xffffffffu, total, o);
+    most = max(most, __shfl_xor_sync(0xffffffffu, most, o));
+  }
+  if (lane == 0) {
+    part[0][warp] = total;
+    part[1][warp] = most;
+  }
+  __syncthreads();
+  total = most = 0;
+#pragma unroll
+  for (int w = 0; w < NT / 32; ++w) {
+    total += part[0][w];
+    most = max(most, part[1][w]);
+  }
+  const int per = max(MIN_TILES, max((total + want_shares - 1) / want_shares, (most + MAX_SHARES - 1) / MAX_SHARES));
+  int before = 0;
+  for (int e0 = 0; e0 < n_entries; e0 += NT) {
+    const int n = ((e0 == 0 ? own : tiles_of(e0 + tid)) + per - 1) / per;
+    int sum = n;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int up = __shfl_up_sync(0xffffffffu, sum, o);
+      if (lane >= o) sum += up;
+    }
+    if (lane == 31) part[2][warp] = sum;
+    __syncthreads();
+    int first = before + sum - n;
+#pragma unroll
+    for (int w = 0; w < NT / 32; ++w) {
+      if (w < warp) first += part[2][w];
+      before += part[2][w];
+    }
+    if (n > 0 && z >= first && z < first + n) {
+      found[0] = e0 + tid;
+      found[1] = first;
+      found[2] = n;
+    }
+    __syncthreads();
+  }
+  Share s;
+  s.e = found[0];
+  s.first = found[1];
+  s.count = found[2];
+  s.split = z - found[1];
+  s.per = per;
+  return s;
+}
+
 // RG row groups x CH column groups of warps; NT: n-tiles (of 8 columns) of the output one warp may own,
 // R / (8 CH) <= NT.
 // ST: tiles of entries in shared memory: 2 (the next one arrives under the current one's products) or 1 (two CTAs
@@ -75,14 +153,19 @@ latent_attn_mma_kernel(const __nv_bfloat16* __restrict__ ql, long long ql_row, l
                        const __nv_bfloat16* __restrict__ cache, const int* __restrict__ qo_indptr,
                        const int* __restrict__ positions, const int* __restrict__ kv_indptr,
                        const int* __restrict__ kv_indices, int H, int R, int P, int page_size, float scale,
-                       int n_splits, float* __restrict__ o_part, float* __restrict__ ml_part, long long n_pages,
+                       float* __restrict__ o_part, float* __restrict__ ml_part, long long n_pages,
                        const float* __restrict__ inv_freq, float magnitude, int window,
-                       const float* __restrict__ sink, int skip_from) {
+                       const float* __restrict__ sink, int skip_from, int* __restrict__ plan, int n_entries,
+                       int rows_max, int want_shares) {
   constexpr int BM = 16 * RG;
   constexpr int KW = BN / CH;                     // keys of a score tile per warp: 16 or 8
   constexpr int TPR = 2 * CH, KPT = BN / TPR;     // softmax: threads per row, keys per thread
-  bspec::pdl_prologue(43);
   extern __shared__ __align__(16) unsigned char smem_raw[];
+  // (the step's lengths were uploaded before its first kernel: they may be read before the wait)
+  Share mine = {(int)blockIdx.y, 0, 0, 0, 0};
+  if (plan != nullptr) mine = deal<32 * RG * CH>(blockIdx.z, qo_indptr, positions, n_entries, window, skip_from, want_shares);
+  bspec::pdl_prologue(43);
+  if (mine.e < 0) return;
   const int D = R + P, DP = D + 8;
   constexpr int PP = BN + 8, SP = BN + 8;
   __nv_bfloat16* Qs = reinterpret_cast<__nv_bfloat16*>(smem_raw);
@@ -94,7 +177,11 @@ latent_attn_mma_kernel(const __nv_bfloat16* __restrict__ ql, long long ql_row, l
   float* row_l = row_m + BM;
   float* row_c = row_l + BM;
 
-  const int e = blockIdx.y, split = blockIdx.z;
+  const int e = mine.e, split = mine.split;
+  if (plan != nullptr && split == 0 && blockIdx.x == 0 && threadIdx.x == 0) {      // for the join
+    plan[2 * e] = mine.first;
+    plan[2 * e + 1] = mine.count;
+  }
   const int q_begin = qo_indptr[e], q_len = qo_indptr[e + 1] - q_begin;
   if (q_len >= skip_from) return;                  // another kernel's portions
   const long long rows_total = (long long)q_len * H;
@@ -110,8 +197,9 @@ latent_attn_mma_kernel(const __nv_bfloat16* __restrict__ ql, long long ql_row, l
   const int min_key = window > 0 ? max(0, pos0 + (int)(row0 / H) - window + 1) : 0;
   const int tile0 = min_key / BN;
   const int n_tiles = max_pos / BN + 1;
-  const int per = (n_tiles - tile0 + n_splits - 1) / n_splits;
-  const int t_begin = tile0 + split * per, t_end = min(n_tiles, t_begin + per);
+  const int per = plan != nullptr ? mine.per : n_tiles - tile0;
+  const int from = plan != nullptr ? (window > 0 ? max(0, pos0 - window + 1) / BN : 0) : tile0;      // the shares' first tile
+  const int t_begin = max(tile0, from + split * per), t_end = min(n_tiles, from + (split + 1) * per);
   const int* table = kv_indices + kv_indptr[e];
 
   // ---- queries: row r holds [ql | qr] of (token, head) = divmod(row0 + r, H); rows past the portion are zero.
@@ -465,7 +553,7 @@ latent_attn_mma_kernel(const __nv_bfloat16* __restrict__ ql, long long ql_row, l
     if (row >= rows_total) continue;
     const long long t = q_begin + row / H;
     const int h = (int)(row % H);
-    if (n_splits == 1) {
+    if (plan == nullptr) {
       const float inv = 1.f / row_l[r];
       __nv_bfloat16* op = out + t * o_row + h * o_head;
 #pragma unroll
@@ -476,7 +564,7 @@ latent_attn_mma_kernel(const __nv_bfloat16* __restrict__ ql, long long ql_row, l
               __floats2bfloat162_rn(o[nd][2 * half] * inv, o[nd][2 * half + 1] * inv);
         }
     } else {
-      const size_t slot = ((size_t)t * H + h) * n_splits + split;
+      const size_t slot = (size_t)(mine.first + split) * rows_max + (size_t)row;
       float* op = o_part + slot * R;
 #pragma unroll
       for (int nd = 0; nd < NT; ++nd)
@@ -494,19 +582,23 @@ latent_attn_mma_kernel(const __nv_bfloat16* __restrict__ ql, long long ql_row, l
 
 // out[row, :] = sum_s w_s O_s / sum_s w_s l_s with w_s = exp(m_s - max m), s ascending.  One block per (token, head):
 // the shares' weights are formed once (in parallel, into shared memory), then every thread adds its columns.
+// ``plan``: first share and number of shares per request, whose rows lie rows_max apart from share to share.
 __global__ void latent_attn_join_kernel(const float* __restrict__ o_part, const float* __restrict__ ml_part,
                                         __nv_bfloat16* __restrict__ out, long long o_row, long long o_head, int H,
-                                        int R, int n_splits) {
+                                        int R, const int* __restrict__ plan, const int* __restrict__ tok_entry,
+                                        const int* __restrict__ qo_indptr, int rows_max, int skip_from) {
   bspec::pdl_prologue(44);
-  __shared__ float w[64];
+  __shared__ float w[MAX_SHARES];
   __shared__ float inv_l;
-  const size_t row = blockIdx.x;
-  const long long t = row / H;
-  const int h = (int)(row % H);
+  const long long t = blockIdx.x / H;
+  const int h = (int)(blockIdx.x % H), e = tok_entry[t], q0 = qo_indptr[e];
+  if (qo_indptr[e + 1] - q0 >= skip_from) return;
+  const int n_shares = plan[2 * e + 1];
+  const size_t row = (size_t)plan[2 * e] * rows_max + (size_t)(t - q0) * H + h, step = rows_max;
   if (threadIdx.x < 32) {
     const int lane = threadIdx.x;
-    float m0 = lane < n_splits ? ml_part[2 * (row * n_splits + lane)] : -INFINITY;
-    float m1 = lane + 32 < n_splits ? ml_part[2 * (row * n_splits + lane + 32)] : -INFINITY;
+    float m0 = lane < n_shares ? ml_part[2 * (row + lane * step)] : -INFINITY;
+    float m1 = lane + 32 < n_shares ? ml_part[2 * (row + (lane + 32) * step)] : -INFINITY;
     const float M = warp_max(fmaxf(m0, m1));
     const float w0 = m0 == -INFINITY ? 0.f : expf(m0 - M), w1 = m1 == -INFINITY ? 0.f : expf(m1 - M);
     w[lane] = w0;
@@ -514,8 +606,8 @@ __global__ void latent_attn_join_kernel(const float* __restrict__ o_part, const 
     __syncwarp();
     if (lane == 0) {                 // the sum in the order of the shares
       float L = 0.f;
-      for (int s = 0; s < n_splits; ++s)
-        if (w[s] != 0.f) L += w[s] * ml_part[2 * (row * n_splits + s) + 1];
+      for (int s = 0; s < n_shares; ++s)
+        if (w[s] != 0.f) L += w[s] * ml_part[2 * (row + s * step) + 1];
       inv_l = 1.f / L;
     }
   }
@@ -524,8 +616,8 @@ __global__ void latent_attn_join_kernel(const float* __restrict__ o_part, const 
   for (int c = threadIdx.x; c < R; c += blockDim.x) {
     float acc = 0.f;
 #pragma unroll 4
-    for (int s = 0; s < n_splits; ++s) {
-      const float x = o_part[(row * n_splits + s) * R + c];
+    for (int s = 0; s < n_shares; ++s) {
+      const float x = o_part[(row + s * step) * R + c];
       if (w[s] != 0.f) acc += w[s] * x;
     }
     out[t * o_row + h * o_head + c] = __float2bfloat16_rn(acc * inv);
@@ -576,24 +668,31 @@ BSPEC_API int bspec_latent_attention_mma_rows(int max_q_len, int H, int R, int P
   return two_small_ctas(R, P) ? 32 : 64;
 }
 
+// ``plan`` (not null: 2 ints per request of scratch): the requests' keys are dealt in want_shares shares and at most one
+// more per request; o_part and ml_part then hold (want_shares + n_entries) * max_q_len * H rows of R and of 2 floats.
 // ``skip_from``: portions of that many tokens and more are left alone (``max_q_len``: the longest of the others).
 BSPEC_API int bspec_latent_attention_mma(const void* ql, long long ql_row, long long ql_head, const void* qr,
                                          long long qr_row, long long qr_head, void* out, long long o_row,
                                          long long o_head, const void* cache, const int* qo_indptr,
                                          const int* positions, const int* kv_indptr, const int* kv_indices,
                                          int n_entries, int n_tokens, int max_q_len, int H, int R, int P,
-                                         int page_size, float scale, int n_splits, float* o_part, float* ml_part,
+                                         int page_size, float scale, float* o_part, float* ml_part,
                                          long long n_pages, const float* inv_freq, float magnitude, int window,
-                                         const float* sink, int skip_from, cudaStream_t stream) {
+                                         const float* sink, int skip_from, int* plan, const int* tok_entry, int want_shares,
+                                         cudaStream_t stream) {
   const bool wide = prompt_mode() != 1;
   if (n_entries <= 0 || max_q_len <= 0) return 0;
-  if (!bspec_latent_attention_mma_supported(R, P) || n_splits < 1 || (n_splits > 1 && (!o_part || !ml_part)))
+  if (!bspec_latent_attention_mma_supported(R, P))
     return (int)cudaErrorInvalidValue;
   const int BM = bspec_latent_attention_mma_rows(max_q_len, H, R, P);
   const bool small_pair = BM == 32 && (long long)max_q_len * H > 32;     // prompt portions on 32-row tiles, one buffer
   const long long row_tiles = ((long long)max_q_len * H + BM - 1) / BM;
-  if ((long long)max_q_len * H > 2147483647ll || n_entries > 65535 || n_splits > 64) return (int)cudaErrorInvalidConfiguration;
-  dim3 grid((unsigned)row_tiles, n_entries, n_splits);
+  if ((long long)max_q_len * H > 2147483647ll || n_entries > 65535) return (int)cudaErrorInvalidConfiguration;
+  dim3 grid((unsigned)row_tiles, n_entries, 1);
+  if (plan != nullptr) {
+    if (want_shares < 1 || want_shares + n_entries > 65535 || !o_part || !ml_part || tok_entry == nullptr) return (int)cudaErrorInvalidValue;
+    grid = dim3((unsigned)row_tiles, 1, want_shares + n_entries);
+  }
   const bool one_stage = small_pair || (BM < 64 && decode_stages() == 1);
   // Shares of the numbers of an entry on 16-row tiles, where as many CTAs still share an SM with the larger score tiles (a
   // decode step of 64 requests through four layers, 16 heads, latent 512 + 64: 769 -> 738 us).  With 32 rows, prompt
@@ -607,7 +706,7 @@ BSPEC_API int bspec_latent_attention_mma(const void* ql, long long ql_row, long 
     BSPEC_LAUNCH((latent_attn_mma_kernel<RG, CH, N>), grid, 32 * RG * CH, smem, stream, (const __nv_bfloat16*)ql,    \
                  ql_row, ql_head, (const __nv_bfloat16*)qr, qr_row, qr_head, (__nv_bfloat16*)out, o_row, o_head,     \
                  (const __nv_bfloat16*)cache, qo_indptr, positions, kv_indptr, kv_indices, H, R, P, page_size,       \
-                 scale, n_splits, o_part, ml_part, n_pages, inv_freq, magnitude, window, sink, skip_from); \
+                 scale, o_part, ml_part, n_pages, inv_freq, magnitude, window, sink, skip_from, plan, n_entries, max_q_len * H, want_shares); \
   } while (0)
 #define LMS(RG, CH, N, DS)                                                                                           \
   do {                                                                                                               \
@@ -615,7 +714,7 @@ BSPEC_API int bspec_latent_attention_mma(const void* ql, long long ql_row, long 
     BSPEC_LAUNCH((latent_attn_mma_kernel<RG, CH, N, 1, DS>), grid, 32 * RG * CH, smem, stream, (const __nv_bfloat16*)ql, \
                  ql_row, ql_head, (const __nv_bfloat16*)qr, qr_row, qr_head, (__nv_bfloat16*)out, o_row, o_head,     \
                  (const __nv_bfloat16*)cache, qo_indptr, positions, kv_indptr, kv_indices, H, R, P, page_size,       \
-                 scale, n_splits, o_part, ml_part, n_pages, inv_freq, magnitude, window, sink, skip_from); \
+                 scale, o_part, ml_part, n_pages, inv_freq, magnitude, window, sink, skip_from, plan, n_entries, max_q_len * H, want_shares); \
   } while (0)
 #define LM1(RG, CH, N) LMS(RG, CH, N, false)
   if (small_pair) {
@@ -642,9 +741,9 @@ BSPEC_API int bspec_latent_attention_mma(const void* ql, long long ql_row, long 
 #undef LMS
 #undef LM
   int err = BSPEC_LAUNCH_CHECK();
-  if (err != 0 || n_splits == 1) return err;
+  if (err != 0 || plan == nullptr) return err;
   BSPEC_LAUNCH((latent_attn_join_kernel), (unsigned)((long long)n_tokens * H), R >= 256 ? 128 : 64, 0, stream, o_part,
-               ml_part, (__nv_bfloat16*)out, o_row, o_head, H, R, n_splits);
+               ml_part, (__nv_bfloat16*)out, o_row, o_head, H, R, (const int*)plan, tok_entry, qo_indptr, max_q_len * H, skip_from);
   return BSPEC_LAUNCH_CHECK();
 }
 

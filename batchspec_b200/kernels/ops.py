@@ -118,8 +118,8 @@ _SIGNATURES = {
     "bspec_latent_attention_mma_smem": [c_int, c_int, c_int, c_int],
     "bspec_latent_attention_mma": [c_void_p, c_longlong, c_longlong, c_void_p, c_longlong, c_longlong, c_void_p,
                                    c_longlong, c_longlong, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int,
-                                   c_int, c_int, c_int, c_int, c_int, c_float, c_int, c_void_p, c_void_p, c_longlong,
-                                   c_void_p, c_float, c_int, c_void_p, c_int, c_void_p],
+                                   c_int, c_int, c_int, c_int, c_int, c_float, c_void_p, c_void_p, c_longlong,
+                                   c_void_p, c_float, c_int, c_void_p, c_int, c_void_p, c_void_p, c_int, c_void_p],
     "bspec_latent_prompt_supported": [c_int, c_int, c_int, c_int],
     "bspec_latent_gather": [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int,
                             c_void_p, c_void_p, c_void_p, c_longlong, c_void_p],
@@ -1505,31 +1505,34 @@ def latent_attention(q_lat: torch.Tensor, q_rot: torch.Tensor, out: torch.Tensor
     lib = load_library()
     if (q_lat.dtype == torch.bfloat16 and not FORCE_GENERIC_LATENT and latent_mma_supported(kv_rank, rot_dim)
             and out.stride(2) == 1 and out.stride(1) % 2 == 0 and out.stride(0) % 2 == 0 and out.data_ptr() % 4 == 0):
-        # Few rows and many entries (decode): the key tiles of a request are cut into shares for more CTAs.  The
-        # count depends on the step's shape alone (entries, longest portion, longest allowed request), so a
-        # captured step keeps it; shares that get no tile leave at once.
+        # Few rows and many entries (decode): the requests' key tiles are dealt out in even shares, about as many as CTAs fit
+        # the device at once.  The count depends on the step's shape alone (entries, longest portion), so a captured step
+        # keeps it; the kernel makes the shares from the lengths on the device, and CTAs without one leave at once.
         rows = lib.bspec_latent_attention_mma_rows(max_q_len, n_heads, kv_rank, rot_dim)       # rows of a CTA's tile
         row_tiles = -(-(max_q_len * n_heads) // rows)
-        n_splits = 1
+        shares, plan = 0, None
+        o_part = ml_part = None
         if max_q_len * n_heads <= 256:
-            # as many shares as fill the CTAs that are resident at once (one wave), at least 256 keys each
             smem = lib.bspec_latent_attention_mma_smem(rows, kv_rank, rot_dim, 0) + 1024
             slots = sm_count(q_lat.device) * max(1, min(4, (227 * 1024) // smem))
+            # rounding gives the requests half a share each beyond their part
+            shares = max(slots // row_tiles - ctx.n_entries // 2, slots // (2 * row_tiles), 1)
+            part_rows = (shares + ctx.n_entries) * max_q_len * n_heads
             keys = min(ctx.max_kv_len, window + max_q_len) if window > 0 else ctx.max_kv_len
-            n_splits = max(1, min(64, slots // (ctx.n_entries * row_tiles), -(-keys // 256)))
-        o_part = ml_part = None
-        if n_splits > 1:
-            o_part = torch.empty((n * H * n_splits * R,), dtype=torch.float32, device=q_lat.device)
-            ml_part = torch.empty((n * H * n_splits * 2,), dtype=torch.float32, device=q_lat.device)
+            if keys > 256 and part_rows * kv_rank <= LATENT_PART_FLOATS:
+                plan = torch.empty((2 * ctx.n_entries,), dtype=torch.int32, device=q_lat.device)
+                o_part = torch.empty((part_rows * kv_rank,), dtype=torch.float32, device=q_lat.device)
+                ml_part = torch.empty((part_rows * 2,), dtype=torch.float32, device=q_lat.device)
         _check(lib.bspec_latent_attention_mma(
             q_lat.data_ptr(), q_lat.stride(1), q_lat.stride(0), q_rot.data_ptr(), q_rot.stride(0), q_rot.stride(1),
             out.data_ptr(), out.stride(1), out.stride(0), cache.data_ptr(), ctx.qo_indptr.data_ptr(),
             ctx.positions.data_ptr(), tables.kv_indptr.data_ptr(), tables.kv_indices.data_ptr(), ctx.n_entries, n,
-            max_q_len, n_heads, kv_rank, rot_dim, tables.page_size, float(scale), n_splits, _ptr(o_part),
+            max_q_len, n_heads, kv_rank, rot_dim, tables.page_size, float(scale), _ptr(o_part),
             _ptr(ml_part), cache.shape[0], rotate[0].data_ptr() if rotate else None,
             float(rotate[1]) if rotate else 1.0, int(window), _ptr(sink),
-            others.at_least if others is not None else 2 ** 31 - 1, _stream()), "latent_attention_mma")
-        if n_splits > 1:
+            others.at_least if others is not None else 2 ** 31 - 1, _ptr(plan), ctx.tok_entry.data_ptr(), shares,
+            _stream()), "latent_attention_mma")
+        if plan is not None:
             count_launches(1)
         return
     assert others is None
@@ -1543,6 +1546,7 @@ def latent_attention(q_lat: torch.Tensor, q_rot: torch.Tensor, out: torch.Tensor
         int(window), _ptr(sink), _stream()), "latent_attention_generic")
 
 
+LATENT_PART_FLOATS = 64 << 20      # partial results of steps of few rows, at most
 LATENT_PROMPT_FROM = 64            # tokens of a portion from which keys and values per head are formed
 LATENT_PROMPT_ROWS = 1 << 19       # at most this many rows of keys (600 MB of entries)
 LATENT_PROMPT_BYTES = 512 << 20    # keys and values of as many heads at a time as this holds
