@@ -12,10 +12,10 @@
 //
 // A step holds portions of several requests (qo_indptr, state_slots); a portion of one token is a decode step.
 // Which form runs depends on the portion's length and, through the estimates of their times, on the step's tokens, its requests
-// and the sizes: lightning attention token by token or by tiles, the scan end to end or in segments, lanes per column or
+// and the sizes: lightning attention token by token, by tiles or by chunks, the scan end to end or in segments, lanes per column or
 // channel.  Within a form the order of every sum is fixed; between forms, so between ways to cut a request into portions and
 // between neighbours in a step, results differ by float32 rounding.
-#include "state_tiles.cuh"
+#include "state_chunks.cuh"
 #include <math.h>
 using namespace bspec;
 
@@ -270,6 +270,7 @@ lightning_tiles_prepare_kernel(const float* __restrict__ proj, long long ld, int
       row[dim + d] = ks[t][d];
     }
   }
+  if (coef == nullptr) return;                                 // (chunks: q and k are all that is wanted)
   // a warp takes two t, eight lanes a dot (four s at a time)
 #pragma unroll
   for (int u = 0; u < ST_B / 2; ++u) {
@@ -342,6 +343,210 @@ int launch_lightning_tiles(dim3 grid, cudaStream_t stream, const float* proj, lo
   BSPEC_LAUNCH_SERIALIZED((lightning_tiles_kernel<R>), grid, ST_THREADS, state_tiles_smem(16 * R), stream, proj, ld, v_off, qk, coef,
                           state, state_stride, qo_indptr, state_slots, out, H, dim, vdim, act);
   return BSPEC_LAUNCH_CHECK();
+}
+
+// ---------------------------------------------------------------- lightning attention, chunks at once
+// With a fixed decay what a chunk of 64 tokens adds to S does not depend on S, so only the decayed sum over the chunks is a
+// chain; everything else is products of whole chunks, formed by all SMs at once:
+//   lightning_chunk_sums   U_c = sum_t d^(cnt-1-t) k_t v_t^T                    [value columns x key rows] per chunk and head
+//   lightning_chunk_scan   S_c = d^cnt S_(c-1) + U_(c-1), over a head's chunks; S_c takes U_c's place
+//   lightning_chunk_out    o_t = d^(t+1) S_c^T q_t + sum_(s <= t) d^(t-s) (q_t . k_s) v_s
+// Float32 throughout, in packed multiply-adds; bound by them (3.1 million per chunk and head of 128 x 128).  q and k come
+// prepared, as for the tiles.
+constexpr long long CH_SCRATCH = 64ll << 20;         // floats of the chunks' sums at most
+constexpr int CH_SUM_SMEM = 2 * CH * CH_W * 4;
+constexpr int CH_OUT_SMEM = (2 * CH * CH_LD + CH * CH_AT + CH_W * (CH_SL + 4) + CH + 1) * 4;
+
+// d^u, formed in float64
+__device__ __forceinline__ float power_of(float d, int u) {
+  double r = 1.0, b = d;
+  for (; u > 0; u >>= 1, b *= b)
+    if (u & 1) r *= b;
+  return (float)r;
+}
+
+// Block: one chunk and head; thread (tx, ty): rows 4 tx + {0..3} and 64 more, columns 4 ty + {0..3} and 64 more.
+__global__ void __launch_bounds__(CH_THREADS, 2)
+lightning_chunk_sums_kernel(const float* __restrict__ proj, long long ld, int v_off, const float* __restrict__ qk,
+                            const float* __restrict__ decay, const int* __restrict__ qo_indptr, int n_entries, float* __restrict__ sums,
+                            int H, int dim, int vdim, int act) {
+  bspec::pdl_prologue(65);
+  extern __shared__ __align__(16) float smem_f[];
+  float *ks = smem_f, *vs = smem_f + CH * CH_W;
+  __shared__ float pw[CH];                           // powers of the decay
+  const int h = blockIdx.y, e = chunk_entry(qo_indptr, n_entries, blockIdx.x);
+  const int q_begin = qo_indptr[e], n = qo_indptr[e + 1] - q_begin, i = blockIdx.x - (int)chunk_slot(q_begin, e, 0);
+  if (n < ST_FROM || i * CH >= n) return;
+  const int cnt = min(CH, n - i * CH), t0 = q_begin + i * CH, tid = threadIdx.x;
+  if (tid < CH) pw[tid] = power_of(decay[h], tid);
+  __syncthreads();
+  for (int x = tid; x < CH * CH_W; x += CH_THREADS) {
+    const int t = x / CH_W, c = x % CH_W;
+    float k = 0.f, v = 0.f;
+    if (t < cnt && c < dim) k = pw[cnt - 1 - t] * qk[((size_t)(t0 + t) * H + h) * 2 * dim + dim + c];
+    if (t < cnt && c < vdim) {
+      v = proj[(size_t)(t0 + t) * ld + v_off + (size_t)h * vdim + c];
+      if (act) v = silu_f(v);
+    }
+    ks[x] = k;
+    vs[x] = v;
+  }
+  __syncthreads();
+  const int tx = tid & 15, ty = tid >> 4;
+  unsigned long long acc[4][8];                      // [pair of rows][column]
+#pragma unroll
+  for (int a = 0; a < 4; ++a)
+#pragma unroll
+    for (int b = 0; b < 8; ++b) acc[a][b] = 0ull;
+#pragma unroll 2
+  for (int t = 0; t < cnt; ++t) {
+    const ulonglong2 k0 = *reinterpret_cast<const ulonglong2*>(ks + t * CH_W + 4 * tx);
+    const ulonglong2 k1 = *reinterpret_cast<const ulonglong2*>(ks + t * CH_W + 64 + 4 * tx);
+    const float4 v0 = *reinterpret_cast<const float4*>(vs + t * CH_W + 4 * ty), v1 = *reinterpret_cast<const float4*>(vs + t * CH_W + 64 + 4 * ty);
+    const float v[8] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y, v1.z, v1.w};
+    const unsigned long long k[4] = {k0.x, k0.y, k1.x, k1.y};
+#pragma unroll
+    for (int b = 0; b < 8; ++b) {
+      const unsigned long long vb = pair_of(v[b], v[b]);
+#pragma unroll
+      for (int a = 0; a < 4; ++a) fma_pair(acc[a][b], k[a], vb);
+    }
+  }
+  float* dst = sums + ((size_t)blockIdx.x * H + h) * vdim * dim;
+#pragma unroll
+  for (int b = 0; b < 8; ++b) {
+    const int j = (b < 4 ? 0 : 64) + 4 * ty + (b & 3);
+    if (j >= vdim) continue;
+#pragma unroll
+    for (int a = 0; a < 2; ++a) {
+      const int r = 64 * a + 4 * tx;
+      if (r < dim) {
+        float4 o;
+        halves_of(acc[2 * a][b], o.x, o.y);
+        halves_of(acc[2 * a + 1][b], o.z, o.w);
+        *reinterpret_cast<float4*>(dst + (size_t)j * dim + r) = o;
+      }
+    }
+  }
+}
+
+// A thread takes one number of one head's S through the chunks of a portion, eight chunks' sums asked for at a time.
+__global__ void __launch_bounds__(256)
+lightning_chunk_scan_kernel(float* __restrict__ sums, const float* __restrict__ decay, float* __restrict__ state, long long state_stride,
+                            const int* __restrict__ qo_indptr, const int* __restrict__ state_slots, int H, int numbers) {
+  bspec::pdl_prologue(65);
+  const int e = blockIdx.z, h = blockIdx.y, x = blockIdx.x * 256 + threadIdx.x;
+  const int q_begin = qo_indptr[e], n = qo_indptr[e + 1] - q_begin;
+  if (n < ST_FROM || x >= numbers) return;
+  const int chunks = (n + CH - 1) / CH, last = n - (chunks - 1) * CH;
+  const float d = decay[h], whole = power_of(d, CH), rest = power_of(d, last);
+  float* sp = state + (size_t)state_slots[e] * state_stride + (size_t)h * numbers + x;
+  float* up = sums + (chunk_slot(q_begin, e, 0) * H + h) * numbers + x;
+  const size_t step = (size_t)H * numbers;
+  float s = *sp;
+  for (int c0 = 0; c0 < chunks; c0 += 8) {
+    float u[8];
+#pragma unroll
+    for (int c = 0; c < 8; ++c) u[c] = c0 + c < chunks ? up[(c0 + c) * step] : 0.f;
+#pragma unroll
+    for (int c = 0; c < 8; ++c)
+      if (c0 + c < chunks) {
+        up[(c0 + c) * step] = s;
+        s = fmaf(c0 + c == chunks - 1 ? rest : whole, s, u[c]);
+      }
+  }
+  *sp = s;
+}
+
+// Block: one chunk and head, 64 tokens x 128 value columns.  First the chunk's own q . k (thread (tx, ty): tokens ty + 16 a
+// against tx + 16 b), kept as at[s][t]; then per warp eight tokens, per lane columns lane + 32 b: S_c^T q over slices of 32 key
+// rows, then the values' sum.
+__global__ void __launch_bounds__(CH_THREADS, 2)
+lightning_chunk_out_kernel(const float* __restrict__ proj, long long ld, int v_off, const float* __restrict__ qk,
+                           const float* __restrict__ decay, const int* __restrict__ qo_indptr, int n_entries,
+                           const float* __restrict__ sums, float* __restrict__ out, int H, int dim, int vdim, int act) {
+  bspec::pdl_prologue(65);
+  extern __shared__ __align__(16) float smem_f[];
+  float* qs = smem_f;                                // [CH][CH_LD]
+  float* kv = qs + CH * CH_LD;                       // [CH][CH_LD] k, then v
+  float* at = kv + CH * CH_LD;                       // [CH s][CH_AT t]
+  float* ss = at + CH * CH_AT;                       // [CH_W columns][CH_SL + 4 rows]
+  float* pw = ss + CH_W * (CH_SL + 4);               // [CH + 1] powers of the decay
+  const int h = blockIdx.y, e = chunk_entry(qo_indptr, n_entries, blockIdx.x);
+  const int q_begin = qo_indptr[e], n = qo_indptr[e + 1] - q_begin, i = blockIdx.x - (int)chunk_slot(q_begin, e, 0);
+  if (n < ST_FROM || i * CH >= n) return;
+  const int cnt = min(CH, n - i * CH), t0 = q_begin + i * CH, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  if (tid <= CH) pw[tid] = power_of(decay[h], tid);
+  for (int x = tid; x < CH * (CH_W / 4); x += CH_THREADS) {
+    const int t = x / (CH_W / 4), c = x % (CH_W / 4) * 4;
+    float4 q = make_float4(0.f, 0.f, 0.f, 0.f), k = q;
+    if (t < cnt && c < dim) {                        // dim is a multiple of 4
+      const float* row = qk + ((size_t)(t0 + t) * H + h) * 2 * dim + c;
+      q = *reinterpret_cast<const float4*>(row);
+      k = *reinterpret_cast<const float4*>(row + dim);
+    }
+    *reinterpret_cast<float4*>(qs + t * CH_LD + c) = q;
+    *reinterpret_cast<float4*>(kv + t * CH_LD + c) = k;
+  }
+  __syncthreads();
+  {
+    const int tx = tid & 15, ty = tid >> 4;
+    unsigned long long acc[4][4];
+#pragma unroll
+    for (int a = 0; a < 4; ++a)
+#pragma unroll
+      for (int b = 0; b < 4; ++b) acc[a][b] = 0ull;
+    for (int c = 0; c < dim; c += 4) {
+      ulonglong2 q[4], k[4];
+#pragma unroll
+      for (int a = 0; a < 4; ++a) q[a] = *reinterpret_cast<const ulonglong2*>(qs + (ty + 16 * a) * CH_LD + c);
+#pragma unroll
+      for (int b = 0; b < 4; ++b) k[b] = *reinterpret_cast<const ulonglong2*>(kv + (tx + 16 * b) * CH_LD + c);
+#pragma unroll
+      for (int a = 0; a < 4; ++a)
+#pragma unroll
+        for (int b = 0; b < 4; ++b) {
+          fma_pair(acc[a][b], q[a].x, k[b].x);
+          fma_pair(acc[a][b], q[a].y, k[b].y);
+        }
+    }
+#pragma unroll
+    for (int a = 0; a < 4; ++a)
+#pragma unroll
+      for (int b = 0; b < 4; ++b) {
+        const int t = ty + 16 * a, s = tx + 16 * b;
+        float x, y;
+        halves_of(acc[a][b], x, y);
+        at[s * CH_AT + t] = s <= t ? pw[t - s] * (x + y) : 0.f;
+      }
+  }
+  __syncthreads();                                   // everybody is done with k
+  for (int x = tid; x < CH * CH_W; x += CH_THREADS) {
+    const int t = x / CH_W, c = x % CH_W;
+    float v = 0.f;
+    if (t < cnt && c < vdim) {
+      v = proj[(size_t)(t0 + t) * ld + v_off + (size_t)h * vdim + c];
+      if (act) v = silu_f(v);
+    }
+    kv[t * CH_LD + c] = v;
+  }
+  const float* S = sums + ((size_t)blockIdx.x * H + h) * vdim * dim;
+  const int tb = 8 * warp;                           // this warp's tokens
+  unsigned long long acc[8][4];
+  chunk_read_state(acc, qs, ss, S, dim, vdim, tb, lane);
+  bspec::pdl_launch_dependents();
+  unsigned long long o[4][4];                        // [pair of tokens][column]
+#pragma unroll
+  for (int a = 0; a < 4; ++a)
+#pragma unroll
+    for (int b = 0; b < 4; ++b) {
+      float x0, y0, x1, y1;
+      halves_of(acc[2 * a][b], x0, y0);
+      halves_of(acc[2 * a + 1][b], x1, y1);
+      o[a][b] = pair_of(pw[tb + 2 * a + 1] * (x0 + y0), pw[tb + 2 * a + 2] * (x1 + y1));
+    }
+  chunk_below(o, at, tb, [&](int s, int b) { return kv[s * CH_LD + lane + 32 * b]; });
+  chunk_write(o, out + ((size_t)t0 * H + h) * vdim, (long long)H * vdim, vdim, cnt, tb, lane);
 }
 
 // ---------------------------------------------------------------- selective scan
@@ -630,9 +835,10 @@ scan_segments_kernel(const float* __restrict__ xz, long long ld, const float* __
 }
 }  // namespace
 
-// Floats of scratch for a step of n tokens in portions of min_q_len to max_q_len: the tiles' coefficients and prepared q and k
-// (as large as the step's q and k columns), or 0 where no portion goes by tiles.
-BSPEC_API long long bspec_lightning_scratch(int n, int n_entries, int min_q_len, int max_q_len, int H, int dim, int vdim) {
+// How the portions of ST_FROM tokens and more of a step of n tokens in portions of min_q_len to max_q_len go: 0 token by token,
+// 1 by tiles, 2 by chunks.  Chunks where tiles pay and the heads fill most of the 128 x 128 numbers that a chunk's products are
+// laid out for, from a portion's length on at which the chain of tiles is the longer one.
+static int lightning_form(int n, int n_entries, int min_q_len, int max_q_len, int H, int dim, int vdim) {
   if (n <= 0 || n_entries <= 0 || H <= 0 || dim <= 0 || vdim <= 0) return 0;
   // (the token loop's time per unit of work falls with the blocks that share the device)
   const long long blocks = (long long)((vdim + LT_COLS - 1) / LT_COLS) * H * n_entries, sms = bspec::sm_count();
@@ -640,13 +846,28 @@ BSPEC_API long long bspec_lightning_scratch(int n, int n_entries, int min_q_len,
   const bspec::TokenCost tokens = {dim <= 32 ? 0.165 : (dim <= 64 ? 0.19 : (dim <= 128 ? 0.25 : 0.38)), rate};
   const bspec::TokenCost tiles = {dim <= 128 ? 0.115 : 0.165, dim <= 128 ? 6.0e-4 : 9e-4};
   if (!bspec::tiles_pay(n, n_entries, min_q_len, max_q_len, H, dim, vdim, tokens, tiles)) return 0;
-  return bspec::state_tile_slots(n, n_entries) * H * ST_CO + (long long)n * H * 2 * dim;
+  const bool fits = chunk_sizes(dim, vdim) && chunk_slots(n, n_entries) * H * dim * vdim <= CH_SCRATCH;
+  return fits && max_q_len >= CH_FROM ? 2 : 1;
+}
+
+// Floats of scratch: the tiles' coefficients or the chunks' sums, and prepared q and k (as large as the step's q and k columns);
+// 0 where no portion goes by either.
+BSPEC_API long long bspec_lightning_scratch(int n, int n_entries, int min_q_len, int max_q_len, int H, int dim, int vdim) {
+  const int form = lightning_form(n, n_entries, min_q_len, max_q_len, H, dim, vdim);
+  if (form == 0) return 0;
+  const long long qk = (long long)n * H * 2 * dim;
+  return qk + (form == 2 ? chunk_slots(n, n_entries) * H * dim * vdim : bspec::state_tile_slots(n, n_entries) * H * ST_CO);
+}
+// Kernels that a step launches.
+BSPEC_API int bspec_lightning_launches(int n, int n_entries, int min_q_len, int max_q_len, int H, int dim, int vdim) {
+  const int form = lightning_form(n, n_entries, min_q_len, max_q_len, H, dim, vdim);
+  return form == 0 ? 1 : (form == 2 ? 4 : 2) + (min_q_len < ST_FROM ? 1 : 0);
 }
 
 BSPEC_API int bspec_lightning_recurrence(const float* proj, long long ld, int q_off, int k_off, int v_off,
                                          const float* decay, float* state, long long state_stride,
                                          const int* qo_indptr, const int* state_slots, float* out, int n, int n_entries,
-                                         int min_q_len, int H, int dim, int vdim, int act, float k_scale,
+                                         int min_q_len, int max_q_len, int H, int dim, int vdim, int act, float k_scale,
                                          const float* inv_freq, int rot, const int* positions, float* scratch,
                                          cudaStream_t stream) {
   if (n_entries <= 0) return 0;
@@ -654,7 +875,30 @@ BSPEC_API int bspec_lightning_recurrence(const float* proj, long long ld, int q_
     return (int)cudaErrorInvalidValue;
   if (dim <= 0 || dim > 256 || vdim <= 0 || H <= 0 || H > 65535 || n_entries > 65535)
     return (int)cudaErrorInvalidValue;
-  if (scratch != nullptr) {
+  const int form = scratch != nullptr ? lightning_form(n, n_entries, min_q_len, max_q_len, H, dim, vdim) : 0;
+  if (form == 2) {
+    float* qk = scratch + chunk_slots(n, n_entries) * H * dim * vdim;
+    static bool set[bspec::kMaxDevices] = {};
+    bool& done = set[bspec::current_device()];
+    if (!done) {
+      cudaError_t e = cudaFuncSetAttribute(lightning_chunk_sums_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, CH_SUM_SMEM);
+      if (e == cudaSuccess) e = cudaFuncSetAttribute(lightning_chunk_out_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, CH_OUT_SMEM);
+      if (e != cudaSuccess) return (int)e;
+      done = true;
+    }
+    BSPEC_LAUNCH(lightning_tiles_prepare_kernel, dim3((unsigned)bspec::state_tile_slots(n, n_entries), H), 128, 0, stream, proj, ld,
+                 q_off, k_off, decay, qo_indptr, n_entries, qk, (float*)nullptr, H, dim, act, k_scale, inv_freq, rot, positions);
+    const dim3 chunks((unsigned)chunk_slots(n, n_entries), H);
+    BSPEC_LAUNCH(lightning_chunk_sums_kernel, chunks, CH_THREADS, CH_SUM_SMEM, stream, proj, ld, v_off, (const float*)qk, decay, qo_indptr,
+                 n_entries, scratch, H, dim, vdim, act);
+    BSPEC_LAUNCH(lightning_chunk_scan_kernel, dim3((dim * vdim + 255) / 256, H, n_entries), 256, 0, stream, scratch, decay, state,
+                 state_stride, qo_indptr, state_slots, H, dim * vdim);
+    BSPEC_LAUNCH(lightning_chunk_out_kernel, chunks, CH_THREADS, CH_OUT_SMEM, stream, proj, ld, v_off, (const float*)qk, decay, qo_indptr,
+                 n_entries, (const float*)scratch, out, H, dim, vdim, act);
+    const int err = BSPEC_LAUNCH_CHECK();
+    if (err != 0 || min_q_len >= ST_FROM) return err;
+  }
+  if (form == 1) {
     float* qk = scratch + bspec::state_tile_slots(n, n_entries) * H * ST_CO;
     BSPEC_LAUNCH(lightning_tiles_prepare_kernel, dim3((unsigned)bspec::state_tile_slots(n, n_entries), H), 128, 0, stream, proj, ld,
                  q_off, k_off, decay, qo_indptr, n_entries, qk, scratch, H, dim, act, k_scale, inv_freq, rot, positions);
@@ -667,7 +911,7 @@ BSPEC_API int bspec_lightning_recurrence(const float* proj, long long ld, int q_
                                                   state_slots, out, H, dim, vdim, act);
     if (tiled != 0 || min_q_len >= ST_FROM) return tiled;
   }
-  const int below = scratch != nullptr ? ST_FROM : 0x7fffffff;           // the portions left for the token loop
+  const int below = form != 0 ? ST_FROM : 0x7fffffff;           // the portions left for the token loop
   const dim3 grid((vdim + LT_COLS - 1) / LT_COLS, H, n_entries);
   // few blocks (a lone prompt): 32 lanes per column, so that an SM holds 16 warps of its one block; many blocks
   // (a decode batch): 8 lanes with more rows each, and the SMs fill with blocks

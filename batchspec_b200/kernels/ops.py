@@ -53,9 +53,10 @@ _SIGNATURES = {
     "bspec_scale": [c_void_p, c_longlong, c_float, c_void_p],
     "bspec_gate_mul": [c_void_p, c_void_p, c_longlong, c_void_p, c_longlong, c_int, c_int, c_int, c_float, c_void_p],
     "bspec_lightning_recurrence": [c_void_p, c_longlong, c_int, c_int, c_int, c_void_p, c_void_p, c_longlong, c_void_p,
-                                   c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_void_p,
+                                   c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_void_p,
                                    c_int, c_void_p, c_void_p, c_void_p],
     "bspec_lightning_scratch": [c_int] * 7,
+    "bspec_lightning_launches": [c_int] * 7,
     "bspec_branch_join": [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p,
                           c_float, c_void_p, c_longlong, c_int, c_int, c_void_p, c_void_p, c_float, c_void_p, c_int, c_int,
                           c_longlong, c_int, c_void_p],
@@ -1140,12 +1141,12 @@ def lightning_recurrence(proj: torch.Tensor, q_off: int, k_off: int, v_off: int,
     scratch = torch.empty((need,), dtype=torch.float32, device=proj.device) if need else None
     _check(lib.bspec_lightning_recurrence(
         proj.data_ptr(), proj.stride(0), int(q_off), int(k_off), int(v_off), decay.data_ptr(), state.data_ptr(),
-        state.stride(0), ctx.qo_indptr.data_ptr(), ctx.state_slots.data_ptr(), out.data_ptr(), n, ctx.n_entries, shortest,
+        state.stride(0), ctx.qo_indptr.data_ptr(), ctx.state_slots.data_ptr(), out.data_ptr(), n, ctx.n_entries, shortest, longest,
         n_heads, dim, v_dim, int(activation == "silu"), float(k_scale), _ptr(inv_freq) if rotary_dim else None,
         int(rotary_dim), ctx.positions.data_ptr() if rotary_dim else None, _ptr(scratch), _stream()),
         "lightning_recurrence")
     if need:
-        count_launches(1 + int(shortest < TILE_FROM))
+        count_launches(lib.bspec_lightning_launches(n, ctx.n_entries, shortest, longest, n_heads, dim, v_dim) - 1)
     return out
 
 

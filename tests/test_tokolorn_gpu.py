@@ -613,6 +613,59 @@ def test_tiles_rotate_queries_and_keys(ops, dk, rot):
     assert (state - state_want).abs().max() <= 2e-5 * max(1.0, state_want.abs().max().item())
 
 
+@pytest.mark.parametrize("Hh,dk,dv,act,scale,rot", [(2, 128, 128, "silu", 1.0, 0), (3, 100, 96, None, 0.25, 36),
+                                                    (1, 96, 128, "silu", 0.5, 0), (4, 128, 75, None, 0.125, 128)])
+def test_lightning_attention_by_chunks(ops, Hh, dk, dv, act, scale, rot):
+    """Steps whose longest portion goes by chunks of 64 tokens (whole and partial last ones, a lone chunk, shorter portions token
+    by token beside it), states carried between them, against the recurrence in float64: sums of dk products over a memory of
+    some hundred tokens, 2e-5 of the largest as in the tests above.  A portion's last token being infinite changes nothing
+    before it."""
+    lens = [1, 600, 64, 5, 256, 65, 127]
+    n, E = sum(lens), len(lens)
+    gen = torch.Generator(device=DEV).manual_seed(dk + dv)
+    ld = 2 * Hh * dk + Hh * dv + 1
+    k_off, v_off = Hh * dk, 2 * Hh * dk + 1
+    decay = torch.tensor([0.99, 0.5, 1.0, 0.9][:Hh], device=DEV)
+    proj = torch.randn(n, ld, device=DEV, generator=gen)
+    state0 = torch.randn(E + 1, Hh * dv * dk, device=DEV, generator=gen)
+    slots, qo = [4, 0, 7, 2, 1, 5, 6], [0] + list(np.cumsum(lens))
+    freqs = 10000.0 ** (-torch.arange(rot // 2, dtype=torch.float64) / max(1, rot // 2))
+    pos = torch.cat([torch.arange(9, 9 + x) for x in lens])
+    assert ops.load_library().bspec_lightning_launches(n, E, 1, 600, Hh, dk, dv) == 5
+
+    def run(x):
+        state = state0.clone()
+        ctx = SimpleNamespace(qo_indptr=_i32(qo), n_entries=E, max_q_len=max(lens), state_slots=_i32(slots), positions=pos.to(DEV, torch.int32),
+                              extras={"min_q_len": 1})
+        args = (ops.rope_frequency_table(freqs, DEV), rot) if rot else ()
+        return ops.lightning_recurrence(x, 0, k_off, v_off, decay, state, ctx, Hh, dk, dv, act, scale, *args), state
+
+    out, state = run(proj)
+    x = proj.double()
+    f = (lambda t: t * torch.sigmoid(t)) if act else (lambda t: t)
+    q, k, v = f(x[:, :Hh * dk]).view(n, Hh, dk), f(x[:, k_off:k_off + Hh * dk]).view(n, Hh, dk) * scale, f(x[:, v_off:v_off + Hh * dv]).view(n, Hh, dv)
+    if rot:
+        ang = pos[:, None].double() * freqs
+        c, s = torch.cos(ang).to(DEV)[:, None], torch.sin(ang).to(DEV)[:, None]
+        half = rot // 2
+        q, k = (torch.cat([u[..., :half] * c - u[..., half:rot] * s, u[..., half:rot] * c + u[..., :half] * s, u[..., rot:]], -1) for u in (q, k))
+    for e, (a, b) in enumerate(zip(qo[:-1], qo[1:])):
+        S = state0[slots[e]].double().view(Hh, dv, dk)
+        want = torch.empty(b - a, Hh, dv, device=DEV, dtype=torch.float64)
+        for t in range(a, b):
+            S = decay.double()[:, None, None] * S + v[t][:, :, None] * k[t][:, None, :]
+            want[t - a] = torch.einsum("hjd,hd->hj", S, q[t])
+        assert (out[a:b].view(b - a, Hh, dv) - want).abs().max() <= 2e-5 * max(1.0, want.abs().max().item()), e
+        assert (state[slots[e]].view(Hh, dv, dk) - S).abs().max() <= 2e-5 * max(1.0, S.abs().max().item()), e
+    untouched = [i for i in range(E + 1) if i not in slots]
+    assert torch.equal(state[untouched], state0[untouched])
+    spoilt, last = proj.clone(), torch.tensor(qo[1:], device=DEV) - 1
+    spoilt[last] = float("inf")
+    keep = torch.ones(n, dtype=torch.bool, device=DEV)
+    keep[last] = False
+    assert torch.equal(run(spoilt)[0][keep], out[keep])
+
+
 @pytest.mark.parametrize("first", [1, 36, 1100])
 def test_tiles_are_found_among_many_requests(ops, first):
     """Long portions behind ``first`` decoded tokens, so that a tile's request is looked for among up to 1,104, against the same
