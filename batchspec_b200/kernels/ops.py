@@ -6,8 +6,9 @@ functions raise.
 
 Matrix products in bfloat16 go to the vendor library through ``torch.mm`` (the
 reference's ``nn.Linear`` does the same, batchspec/models/modules/attention/base.py:32-39);
-float32 products use this package's own FFMA kernel so that no reduced-precision
-mode can slip in.
+float32 products use this package's own kernels so that no reduced-precision mode
+can slip in: multiply-adds on the CUDA cores, or, with many rows, every number as the
+sum of three bfloat16 numbers on the tensor cores (csrc/gemm_fp32_tc.cu).
 """
 from __future__ import annotations
 
