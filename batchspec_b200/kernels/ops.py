@@ -1530,8 +1530,8 @@ def latent_attention(q_lat: torch.Tensor, q_rot: torch.Tensor, out: torch.Tensor
             max_q_len, n_heads, kv_rank, rot_dim, tables.page_size, float(scale), _ptr(o_part),
             _ptr(ml_part), cache.shape[0], rotate[0].data_ptr() if rotate else None,
             float(rotate[1]) if rotate else 1.0, int(window), _ptr(sink),
-            others.at_least if others is not None else 2 ** 31 - 1, _ptr(plan), ctx.tok_entry.data_ptr(), shares,
-            _stream()), "latent_attention_mma")
+            others.at_least if others is not None else 2 ** 31 - 1, _ptr(plan),
+            ctx.tok_entry.data_ptr() if plan is not None else None, shares, _stream()), "latent_attention_mma")
         if plan is not None:
             count_launches(1)
         return

@@ -309,6 +309,18 @@ def test_latent_attention_rotates_the_queries_on_the_way(ops, dtype, generic):
     assert torch.equal(got, want)
 
 
+@pytest.mark.parametrize("heads,R,Pd,q_lens,kv_lens", [
+    (16, 64, 16, [1] * 140, [1 + 37 * i % 400 for i in range(139)] + [2500]),       # more requests than threads, one far longer
+    (3, 96, 16, [2, 1, 3, 1], [1700, 1, 300, 33]),                                   # rows of a portion in one share
+    (24, 64, 32, [1, 4, 2], [5000, 700, 2]),                                         # several row tiles, as many shares as there are
+])
+def test_decoded_tokens_are_dealt_in_even_shares(ops, heads, R, Pd, q_lens, kv_lens):
+    """Against the plain attention (as test_latent_attention) where requests of very different lengths share the CTAs."""
+    got, want = _latent_case(ops, torch.bfloat16, heads, R, Pd, 16, q_lens, kv_lens)
+    assert not torch.isnan(got).any()
+    assert (got - want).abs().max() <= 2.5e-2
+
+
 LONG_PORTIONS = [
     # heads, latent, page, q_lens, kv_lens, window, sinks, heads at a time
     (2, 64, 16, [64], [64], 0, False, 2),
