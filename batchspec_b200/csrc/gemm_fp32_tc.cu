@@ -373,7 +373,9 @@ join_groups_kernel(const float* __restrict__ part, float* __restrict__ C, long l
 
 long long plane_bytes(int M, int K) { return (3ll * M * ((K + KB - 1) / KB * KB) * 2 + 255) / 256 * 256; }
 
-// CTAs along K: whole groups each, so that the last wave of CTAs is well filled.
+// CTAs along K: whole groups each, so that the last wave of CTAs is well filled.  In units of a group's time in a CTA, about
+// 16 us; the groups' sums, written and read again at some 5 TB/s, are what it costs (967 x 2,048 x 8,192, 128 tiles of 16 groups,
+// each sum apart: 335 us against some 270).
 int tc_splits(int M, int N, int K) {
   const long long tiles = (long long)((M + TT - 1) / TT) * ((N + TN - 1) / TN);
   const int groups = (K + GROUP - 1) / GROUP;
@@ -382,7 +384,7 @@ int tc_splits(int M, int N, int K) {
   for (int s = 1; s <= groups; ++s) {
     const int per = (groups + s - 1) / s;
     const long long waves = (tiles * s + bspec::sm_count() - 1) / bspec::sm_count();
-    const double cost = (double)waves * per + (s > 1 ? 0.75 : 0.0);
+    const double cost = (double)waves * per + (s > 1 ? 0.3 + 8.0 * groups * M * N / 80e6 : 0.0);
     if (cost < best_cost - 1e-9) { best_cost = cost; best = s; }
   }
   return best;
