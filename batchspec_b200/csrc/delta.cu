@@ -11,15 +11,14 @@
 //                     registers (a column of S is spread over four or sixteen lanes), state read at the start and
 //                     written at the end; the request's blocks also move the convolutions' inputs on.  Where that is
 //                     faster (tiles_pay), portions of ST_FROM tokens and more take delta_tiles_prepare and delta_tiles
-//                     instead, which multiply the rule out over tiles of eight tokens, or delta_chunk_prepare, _chain and
-//                     _out, over chunks of 64
+//                     instead, which multiply the rule out over tiles of eight tokens
 //   gated_rmsnorm     per (token, head): o / rms(o) * w * silu(gate), with options other mixers use
 //
 // Which form runs depends on the portion's length and, through the estimates of their times, on the step's tokens, its requests
-// and the sizes: token loop, tiles or chunks, lanes per column of the token loop, one or eight tokens per warp of the preparation.
+// and the sizes: token loop or tiles, lanes per column of the token loop, one or eight tokens per warp of the preparation.
 // Within a form the order of every sum is fixed; between forms, so between ways to cut a request into portions and between
 // neighbours in a step, results differ by float32 rounding.
-#include "state_chunks.cuh"
+#include "state_tiles.cuh"
 #include <math.h>
 using namespace bspec;
 
@@ -526,392 +525,6 @@ int launch_delta_tiles(dim3 grid, cudaStream_t stream, const float* mix, const f
   return BSPEC_LAUNCH_CHECK();
 }
 
-// ---------------------------------------------------------------- portions of chunks
-// The same multiplied out over chunks of C = 64 tokens.  u = T diag(beta) V - W S with W = T diag(beta c) K, so that only
-//     u = U - W S (U = T diag(beta) V),      S <- c_C S + K^T diag(y(., C)) u
-// goes from chunk to chunk; T, W, U and the factors A_ts = y(s, t) (k_s . q_t) of u in the outputs are formed for all chunks at
-// once before, and o = diag(c) Q S + A u after:
-//   delta_chunk_prepare  per (chunk, head): T by forward substitution (a thread per column), W, U, A, c and y(., C)
-//   delta_chunk_chain    per (request, head, 16 value columns): the chain; leaves u in U's place and the S that each chunk starts from
-//   delta_chunk_out      per (chunk, head): the outputs
-constexpr long long DC_SCRATCH = 128ll << 20;        // floats of scratch at most
-constexpr int DC_COLS = 16, DC_US = DC_COLS + 4, DC_SC = 192;              // columns of a chain; floats of a chunk's c, y(., C) and c_C
-constexpr int DC_PREP_SMEM = (2 * CH * CH_LD + 2 * CH * CH_AT + 3 * CH) * 4;
-constexpr int DC_CHAIN_SMEM = (4 * CH * CH_LD + 2 * CH * DC_COLS + DC_COLS * CH_LD + CH * DC_US + 128 * 16 + 2 * 80) * 4;
-constexpr int DC_OUT_SMEM = (2 * CH * CH_LD + CH * CH_AT + CH_W * (CH_SL + 4) + CH) * 4;
-
-struct DeltaChunks {                                 // per (chunk, head)
-  float *w, *u, *a, *s, *c;                          // [CH][dim], [CH][vdim], [s][t], [vdim][dim], [c 64 | y(., C) 64 | c_C ..]
-};
-inline long long delta_chunk_floats(int dim, int vdim) { return (long long)CH * (dim + vdim) + CH * CH + (long long)dim * vdim + DC_SC; }
-inline DeltaChunks delta_chunk_parts(float* scratch, long long items, int dim, int vdim) {
-  DeltaChunks p;
-  p.w = scratch;
-  p.u = p.w + items * CH * dim;
-  p.a = p.u + items * CH * vdim;
-  p.s = p.a + items * CH * CH;
-  p.c = p.s + items * dim * vdim;
-  return p;
-}
-
-__global__ void __launch_bounds__(CH_THREADS, 2)
-delta_chunk_prepare_kernel(const float* __restrict__ mix, const float* __restrict__ gates, const int* __restrict__ qo_indptr,
-                           int n_entries, const DeltaChunks out, int H, int Gk, int dim, int vdim) {
-  bspec::pdl_prologue(60);
-  extern __shared__ __align__(16) float smem_f[];
-  float* ks = smem_f;                                // [CH][CH_LD]
-  float* qv = ks + CH * CH_LD;                       // [CH][CH_LD] q, then v
-  float* low = qv + CH * CH_LD;                      // [t][CH_AT] L, then T by columns
-  float* inv = low + CH * CH_AT;                     // [t][CH_AT] T; before that y(s, t) as [s][CH_AT]
-  float *be = inv + CH * CH_AT, *g = be + CH, *bc = g + CH;
-  const int h = blockIdx.y, e = chunk_entry(qo_indptr, n_entries, blockIdx.x);
-  const int q_begin = qo_indptr[e], n = qo_indptr[e + 1] - q_begin, i = blockIdx.x - (int)chunk_slot(q_begin, e, 0);
-  if (n < ST_FROM || i * CH >= n) return;
-  const int cnt = min(CH, n - i * CH), t0 = q_begin + i * CH, C = 2 * Gk * dim + H * vdim, kh = h / (H / Gk);
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const size_t item = (size_t)blockIdx.x * H + h;
-  for (int x = tid; x < CH * (CH_W / 4); x += CH_THREADS) {
-    const int t = x / (CH_W / 4), c = x % (CH_W / 4) * 4;
-    float4 q = make_float4(0.f, 0.f, 0.f, 0.f), k = q;
-    if (t < cnt && c < dim) {
-      const float* row = mix + (size_t)(t0 + t) * C + c;
-      q = *reinterpret_cast<const float4*>(row + kh * dim);
-      k = *reinterpret_cast<const float4*>(row + (Gk + kh) * dim);
-    }
-    *reinterpret_cast<float4*>(qv + t * CH_LD + c) = q;
-    *reinterpret_cast<float4*>(ks + t * CH_LD + c) = k;
-  }
-  if (tid < CH) {
-    const float* gr = gates + (size_t)(t0 + min(tid, cnt - 1)) * 2 * H + h;
-    be[tid] = tid < cnt ? gr[0] : 0.f;
-    g[tid] = tid < cnt ? gr[H] : 1.f;
-  }
-  __syncthreads();
-  float* y = inv;
-  if (tid < CH) {
-    float a = 1.f;
-    y[tid * CH_AT + tid] = 1.f;
-    for (int t = tid + 1; t < CH; ++t) y[tid * CH_AT + t] = a *= g[t];
-  }
-  __syncthreads();
-  if (tid < CH) {
-    const float c = g[0] * y[tid];
-    float* sc = out.c + item * DC_SC;
-    bc[tid] = be[tid] * c;
-    sc[tid] = c;
-    sc[CH + tid] = y[tid * CH_AT + CH - 1];
-    if (tid == CH - 1) sc[2 * CH] = c;
-  }
-  {
-    const int tx = tid & 15, ty = tid >> 4;          // tokens t = tx + 16 a against s = ty + 16 b
-#pragma unroll 1
-    for (int pass = 0; pass < 2; ++pass) {
-      const float* rows = pass == 0 ? ks : qv;
-      unsigned long long acc[4][4];
-#pragma unroll
-      for (int a = 0; a < 4; ++a)
-#pragma unroll
-        for (int b = 0; b < 4; ++b) acc[a][b] = 0ull;
-      for (int c = 0; c < dim; c += 4) {
-        ulonglong2 r[4], k[4];
-#pragma unroll
-        for (int a = 0; a < 4; ++a) r[a] = *reinterpret_cast<const ulonglong2*>(rows + (tx + 16 * a) * CH_LD + c);
-#pragma unroll
-        for (int b = 0; b < 4; ++b) k[b] = *reinterpret_cast<const ulonglong2*>(ks + (ty + 16 * b) * CH_LD + c);
-#pragma unroll
-        for (int a = 0; a < 4; ++a)
-#pragma unroll
-          for (int b = 0; b < 4; ++b) {
-            fma_pair(acc[a][b], r[a].x, k[b].x);
-            fma_pair(acc[a][b], r[a].y, k[b].y);
-          }
-      }
-#pragma unroll
-      for (int a = 0; a < 4; ++a)
-#pragma unroll
-        for (int b = 0; b < 4; ++b) {
-          const int t = tx + 16 * a, s = ty + 16 * b;
-          float x0, x1;
-          halves_of(acc[a][b], x0, x1);
-          if (pass == 0) low[t * CH_AT + s] = s < t ? be[t] * y[s * CH_AT + t] * (x0 + x1) : 0.f;
-          else out.a[item * CH * CH + s * CH + t] = s <= t ? y[s * CH_AT + t] * (x0 + x1) : 0.f;
-        }
-    }
-  }
-  __syncthreads();                                   // y and q have been used
-  for (int x = tid; x < CH * (CH_W / 4); x += CH_THREADS) {
-    const int t = x / (CH_W / 4), c = x % (CH_W / 4) * 4;
-    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (t < cnt && c < vdim) v = *reinterpret_cast<const float4*>(mix + (size_t)(t0 + t) * C + 2 * Gk * dim + (size_t)h * vdim + c);
-    *reinterpret_cast<float4*>(qv + t * CH_LD + c) = v;
-  }
-  if (tid < CH) {                                    // column tid of T; its rows above the diagonal are zero
-    for (int t = 0; t < CH; ++t) {
-      float a[4] = {t == tid ? 1.f : 0.f, 0.f, 0.f, 0.f};
-      int r = tid & ~3;
-      for (; r + 4 <= t; r += 4) {
-        const float4 l = *reinterpret_cast<const float4*>(low + t * CH_AT + r);
-        a[0] = fmaf(-l.x, r >= tid ? inv[r * CH_AT + tid] : 0.f, a[0]);
-        a[1] = fmaf(-l.y, r + 1 >= tid ? inv[(r + 1) * CH_AT + tid] : 0.f, a[1]);
-        a[2] = fmaf(-l.z, r + 2 >= tid ? inv[(r + 2) * CH_AT + tid] : 0.f, a[2]);
-        a[3] = fmaf(-l.w, inv[(r + 3) * CH_AT + tid], a[3]);
-      }
-      for (; r < t; ++r)
-        if (r >= tid) a[0] = fmaf(-low[t * CH_AT + r], inv[r * CH_AT + tid], a[0]);
-      inv[t * CH_AT + tid] = t >= tid ? (a[0] + a[1]) + (a[2] + a[3]) : 0.f;
-    }
-  }
-  __syncthreads();
-  for (int x = tid; x < CH * CH; x += CH_THREADS) low[(x % CH) * CH_AT + x / CH] = inv[(x / CH) * CH_AT + x % CH];
-  __syncthreads();
-  const int tb = 8 * warp;
-  unsigned long long o[4][4];
-#pragma unroll
-  for (int part = 0; part < 2; ++part) {
-#pragma unroll
-    for (int a = 0; a < 4; ++a)
-#pragma unroll
-      for (int b = 0; b < 4; ++b) o[a][b] = 0ull;
-    if (part == 0) {
-      chunk_below(o, low, tb, [&](int s, int b) { return bc[s] * ks[s * CH_LD + lane + 32 * b]; });
-      chunk_write(o, out.w + item * CH * dim, dim, dim, CH, tb, lane);
-    } else {
-      chunk_below(o, low, tb, [&](int s, int b) { return be[s] * qv[s * CH_LD + lane + 32 * b]; });
-      chunk_write(o, out.u + item * CH * vdim, vdim, vdim, CH, tb, lane);
-    }
-  }
-}
-
-// The chain of one request's chunks for 16 value columns of a head; S in shared memory, W, K and U of the next chunk copied under
-// the current one.  W S: a thread takes 4 tokens x 4 columns over a quarter of the key rows (rows 16 x + 4 (lane % 4) ..), the
-// quarters are joined over neighbouring lanes; K^T u: 4 key rows x 4 columns over half of the tokens, the halves joined through
-// shared memory.  Both read two or three 16-byte operands of shared memory for sixteen multiply-adds.
-__global__ void __launch_bounds__(CH_THREADS, 1)
-delta_chunk_chain_kernel(const float* __restrict__ mix, const float* __restrict__ proj, const DeltaChunks ch, int ld,
-                         float* __restrict__ state, long long state_stride, long long tail_off, const int* __restrict__ qo_indptr,
-                         const int* __restrict__ state_slots, int H, int Gk, int dim, int vdim, int taps) {
-  bspec::pdl_prologue_late(61);
-  extern __shared__ __align__(16) float smem_f[];
-  float* wb = smem_f;                                // [2][CH][CH_LD]
-  float* kb = wb + 2 * CH * CH_LD;                   // [2][CH][CH_LD]
-  float* ub = kb + 2 * CH * CH_LD;                   // [2][CH][DC_COLS]
-  float* S = ub + 2 * CH * DC_COLS;                  // [DC_COLS][CH_LD]
-  float* us = S + DC_COLS * CH_LD;                   // [CH][DC_US] y(., C) u
-  float* part = us + CH * DC_US;                     // [4][128] quads
-  float* sc = part + 128 * 16;                       // [2][80] y(., C), c_C
-  const int e = blockIdx.z, h = blockIdx.y, j0 = blockIdx.x * DC_COLS;
-  const int q_begin = qo_indptr[e], n = qo_indptr[e + 1] - q_begin;
-  const int C = 2 * Gk * dim + H * vdim, kh = h / (H / Gk);
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  float* srow = state + (size_t)state_slots[e] * state_stride;
-  if (n < ST_FROM) return;
-  if (taps > 1) {                                              // as in delta_recurrence_kernel
-    float* tail = srow + tail_off;
-    const int share = blockIdx.y * gridDim.x + blockIdx.x, shares = gridDim.y * gridDim.x;
-    for (int c = share * CH_THREADS + tid; c < C; c += shares * CH_THREADS)
-      for (int s = 0; s < taps - 1; ++s) {
-        const int rel = n + s - (taps - 1);
-        tail[(size_t)s * C + c] = rel >= 0 ? proj[(size_t)(q_begin + rel) * ld + c] : tail[(size_t)(s + n) * C + c];
-      }
-  }
-  const int chunks = (n + CH - 1) / CH;
-  const size_t first = chunk_slot(q_begin, e, 0) * H + h;
-  for (int x = tid; x < 4 * CH * CH_LD; x += CH_THREADS) wb[x] = 0.f;              // W's and K's pads stay zero
-  for (int x = tid; x < DC_COLS * CH_LD; x += CH_THREADS) S[x] = 0.f;
-  __syncthreads();
-  float* sp = srow + ((size_t)h * vdim + j0) * dim;
-  for (int x = tid; x < DC_COLS * dim; x += CH_THREADS)
-    if (j0 + x / dim < vdim) S[x / dim * CH_LD + x % dim] = sp[x];
-  auto load = [&](int c, int buf) {
-    const size_t item = first + (size_t)c * H;
-    const int cnt = min(CH, n - c * CH), quads = dim / 4;
-    for (int x = tid; x < CH * quads; x += CH_THREADS) {
-      const int t = x / quads, r = x % quads * 4;
-      __pipeline_memcpy_async(wb + (buf * CH + t) * CH_LD + r, ch.w + item * CH * dim + t * dim + r, 16);
-      float* kd = kb + (buf * CH + t) * CH_LD + r;
-      if (t < cnt) __pipeline_memcpy_async(kd, mix + (size_t)(q_begin + c * CH + t) * C + (Gk + kh) * dim + r, 16);
-      else *reinterpret_cast<float4*>(kd) = make_float4(0.f, 0.f, 0.f, 0.f);
-    }
-    {
-      const int t = tid / 4, j = tid % 4 * 4;
-      float* ud = ub + (buf * CH + t) * DC_COLS + j;
-      if (j0 + j < vdim) __pipeline_memcpy_async(ud, ch.u + item * CH * vdim + t * vdim + j0 + j, 16);
-      else *reinterpret_cast<float4*>(ud) = make_float4(0.f, 0.f, 0.f, 0.f);
-    }
-    if (tid < 17) __pipeline_memcpy_async(sc + buf * 80 + 4 * tid, ch.c + item * DC_SC + CH + 4 * tid, 16);
-    __pipeline_commit();
-  };
-  load(0, 0);
-  for (int c = 0; c < chunks; ++c) {
-    const int buf = c & 1;
-    const size_t item = first + (size_t)c * H;
-    __pipeline_wait_prior(0);
-    __syncthreads();                                 // the chunk is there, S is complete, and everybody is done with the other half
-    if (c + 1 < chunks) load(c + 1, buf ^ 1);
-    for (int x = tid; x < DC_COLS * (dim / 4); x += CH_THREADS) {
-      const int j = x / (dim / 4), r = x % (dim / 4) * 4;
-      if (j0 + j < vdim)
-        *reinterpret_cast<float4*>(ch.s + item * dim * vdim + (size_t)(j0 + j) * dim + r) = *reinterpret_cast<const float4*>(S + j * CH_LD + r);
-    }
-    {
-      const int quarter = lane & 3, j = 4 * ((lane >> 2) & 3), t = 8 * warp + 4 * (lane >> 4);
-      unsigned long long acc[4][4];
-#pragma unroll
-      for (int a = 0; a < 4; ++a)
-#pragma unroll
-        for (int b = 0; b < 4; ++b) acc[a][b] = 0ull;
-      const float* wr = wb + (buf * CH + t) * CH_LD + 4 * quarter;
-      const float* sr = S + j * CH_LD + 4 * quarter;
-#pragma unroll 2
-      for (int r = 0; r < dim; r += 16) {            // (rows past dim are zero)
-        ulonglong2 w[4], s[4];
-#pragma unroll
-        for (int a = 0; a < 4; ++a) w[a] = *reinterpret_cast<const ulonglong2*>(wr + a * CH_LD + r);
-#pragma unroll
-        for (int b = 0; b < 4; ++b) s[b] = *reinterpret_cast<const ulonglong2*>(sr + b * CH_LD + r);
-#pragma unroll
-        for (int a = 0; a < 4; ++a)
-#pragma unroll
-          for (int b = 0; b < 4; ++b) {
-            fma_pair(acc[a][b], w[a].x, s[b].x);
-            fma_pair(acc[a][b], w[a].y, s[b].y);
-          }
-      }
-      float f[4][4];
-#pragma unroll
-      for (int a = 0; a < 4; ++a)
-#pragma unroll
-        for (int b = 0; b < 4; ++b) {
-          float x0, x1;
-          halves_of(acc[a][b], x0, x1);
-          f[a][b] = x0 + x1;
-        }
-      const bool b0 = lane & 1, b1 = lane & 2;       // this lane finishes token t + 2 b0 + b1
-      float f2[2][4], f3[4];
-#pragma unroll
-      for (int a = 0; a < 2; ++a)
-#pragma unroll
-        for (int b = 0; b < 4; ++b)
-          f2[a][b] = (b0 ? f[2 + a][b] : f[a][b]) + __shfl_xor_sync(0xffffffffu, b0 ? f[a][b] : f[2 + a][b], 1);
-#pragma unroll
-      for (int b = 0; b < 4; ++b) f3[b] = (b1 ? f2[1][b] : f2[0][b]) + __shfl_xor_sync(0xffffffffu, b1 ? f2[0][b] : f2[1][b], 2);
-      const int tt = t + 2 * (lane & 1) + ((lane >> 1) & 1);
-      const float4 u0 = *reinterpret_cast<const float4*>(ub + (buf * CH + tt) * DC_COLS + j);
-      const float4 u = make_float4(u0.x - f3[0], u0.y - f3[1], u0.z - f3[2], u0.w - f3[3]);
-      if (j0 + j < vdim) *reinterpret_cast<float4*>(ch.u + item * CH * vdim + tt * vdim + j0 + j) = u;
-      const float yc = sc[buf * 80 + tt];
-      *reinterpret_cast<float4*>(us + tt * DC_US + j) = make_float4(yc * u.x, yc * u.y, yc * u.z, yc * u.w);
-    }
-    __syncthreads();
-    const int r = 4 * ((warp & 3) * 8 + (lane & 7)), j = 4 * (lane >> 3), half = warp >> 2, tile = (warp & 3) * 32 + lane;
-    unsigned long long acc[2][4];                    // [pair of rows][column]
-#pragma unroll
-    for (int a = 0; a < 2; ++a)
-#pragma unroll
-      for (int b = 0; b < 4; ++b) acc[a][b] = 0ull;
-#pragma unroll 4
-    for (int t = 32 * half; t < 32 * half + 32; ++t) {
-      const ulonglong2 k = *reinterpret_cast<const ulonglong2*>(kb + (buf * CH + t) * CH_LD + r);
-      const float4 u = *reinterpret_cast<const float4*>(us + t * DC_US + j);
-      const float uu[4] = {u.x, u.y, u.z, u.w};
-#pragma unroll
-      for (int b = 0; b < 4; ++b) {
-        const unsigned long long u2 = pair_of(uu[b], uu[b]);
-        fma_pair(acc[0][b], k.x, u2);
-        fma_pair(acc[1][b], k.y, u2);
-      }
-    }
-    float4 add[4];
-#pragma unroll
-    for (int b = 0; b < 4; ++b) {
-      halves_of(acc[0][b], add[b].x, add[b].y);
-      halves_of(acc[1][b], add[b].z, add[b].w);
-      if (half == 1) *reinterpret_cast<float4*>(part + (b * 128 + tile) * 4) = add[b];
-    }
-    __syncthreads();
-    if (half == 0) {
-      const float cc = sc[buf * 80 + CH];
-#pragma unroll
-      for (int b = 0; b < 4; ++b) {
-        float4* at = reinterpret_cast<float4*>(S + (j + b) * CH_LD + r);
-        const float4 p = *reinterpret_cast<const float4*>(part + (b * 128 + tile) * 4);
-        float4 s = *at;
-        s.x = fmaf(cc, s.x, add[b].x + p.x), s.y = fmaf(cc, s.y, add[b].y + p.y);
-        s.z = fmaf(cc, s.z, add[b].z + p.z), s.w = fmaf(cc, s.w, add[b].w + p.w);
-        *at = s;
-      }
-    }
-  }
-  bspec::pdl_launch_dependents();
-  __syncthreads();
-  for (int x = tid; x < DC_COLS * dim; x += CH_THREADS)
-    if (j0 + x / dim < vdim) sp[x] = S[x / dim * CH_LD + x % dim];
-}
-
-__global__ void __launch_bounds__(CH_THREADS, 2)
-delta_chunk_out_kernel(const float* __restrict__ mix, const DeltaChunks ch, const int* __restrict__ qo_indptr, int n_entries,
-                       float* __restrict__ out, int H, int Gk, int dim, int vdim) {
-  bspec::pdl_prologue(61);
-  extern __shared__ __align__(16) float smem_f[];
-  float* qs = smem_f;                                // [CH][CH_LD]
-  float* us = qs + CH * CH_LD;                       // [CH][CH_LD]
-  float* at = us + CH * CH_LD;                       // [CH s][CH_AT t]
-  float* ss = at + CH * CH_AT;                       // [CH_W columns][CH_SL + 4 rows]
-  float* cs = ss + CH_W * (CH_SL + 4);               // [CH]
-  const int h = blockIdx.y, e = chunk_entry(qo_indptr, n_entries, blockIdx.x);
-  const int q_begin = qo_indptr[e], n = qo_indptr[e + 1] - q_begin, i = blockIdx.x - (int)chunk_slot(q_begin, e, 0);
-  if (n < ST_FROM || i * CH >= n) return;
-  const int cnt = min(CH, n - i * CH), t0 = q_begin + i * CH, C = 2 * Gk * dim + H * vdim, kh = h / (H / Gk);
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, tb = 8 * warp;
-  const size_t item = (size_t)blockIdx.x * H + h;
-  for (int x = tid; x < CH * (CH_W / 4); x += CH_THREADS) {
-    const int t = x / (CH_W / 4), c = x % (CH_W / 4) * 4;
-    float4 q = make_float4(0.f, 0.f, 0.f, 0.f), u = q;
-    if (t < cnt && c < dim) q = *reinterpret_cast<const float4*>(mix + (size_t)(t0 + t) * C + kh * dim + c);
-    if (t < cnt && c < vdim) u = *reinterpret_cast<const float4*>(ch.u + item * CH * vdim + t * vdim + c);
-    *reinterpret_cast<float4*>(qs + t * CH_LD + c) = q;
-    *reinterpret_cast<float4*>(us + t * CH_LD + c) = u;
-  }
-  for (int x = tid; x < CH * (CH / 4); x += CH_THREADS)
-    *reinterpret_cast<float4*>(at + x / (CH / 4) * CH_AT + x % (CH / 4) * 4) = *reinterpret_cast<const float4*>(ch.a + item * CH * CH + 4 * x);
-  if (tid < CH) cs[tid] = ch.c[item * DC_SC + tid];
-  unsigned long long acc[8][4];
-  chunk_read_state(acc, qs, ss, ch.s + item * dim * vdim, dim, vdim, tb, lane);
-  unsigned long long o[4][4];                        // [pair of tokens][column]
-#pragma unroll
-  for (int a = 0; a < 4; ++a)
-#pragma unroll
-    for (int b = 0; b < 4; ++b) {
-      float x0, y0, x1, y1;
-      halves_of(acc[2 * a][b], x0, y0);
-      halves_of(acc[2 * a + 1][b], x1, y1);
-      o[a][b] = pair_of(cs[tb + 2 * a] * (x0 + y0), cs[tb + 2 * a + 1] * (x1 + y1));
-    }
-  chunk_below(o, at, tb, [&](int s, int b) { return us[s * CH_LD + lane + 32 * b]; });
-  chunk_write(o, out + ((size_t)t0 * H + h) * vdim, (long long)H * vdim, vdim, cnt, tb, lane);
-}
-
-int launch_delta_chunks(cudaStream_t stream, const float* mix, const float* gates, const float* proj, int ld, float* state,
-                        long long state_stride, long long tail_off, const int* qo_indptr, const int* state_slots, float* out, int n,
-                        int n_entries, int H, int Gk, int dim, int vdim, int taps, float* scratch) {
-  static bool set[bspec::kMaxDevices] = {};
-  bool& done = set[bspec::current_device()];
-  if (!done) {
-    cudaError_t err = cudaFuncSetAttribute(delta_chunk_prepare_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, DC_PREP_SMEM);
-    if (err == cudaSuccess) err = cudaFuncSetAttribute(delta_chunk_chain_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, DC_CHAIN_SMEM);
-    if (err == cudaSuccess) err = cudaFuncSetAttribute(delta_chunk_out_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, DC_OUT_SMEM);
-    if (err != cudaSuccess) return (int)err;
-    done = true;
-  }
-  const dim3 grid((unsigned)chunk_slots(n, n_entries), H);
-  const DeltaChunks parts = delta_chunk_parts(scratch, chunk_slots(n, n_entries) * H, dim, vdim);
-  BSPEC_LAUNCH(delta_chunk_prepare_kernel, grid, CH_THREADS, DC_PREP_SMEM, stream, mix, gates, qo_indptr, n_entries, parts, H, Gk, dim, vdim);
-  BSPEC_LAUNCH_SERIALIZED(delta_chunk_chain_kernel, dim3((vdim + DC_COLS - 1) / DC_COLS, H, n_entries), CH_THREADS, DC_CHAIN_SMEM, stream, mix,
-                          proj, parts, ld, state, state_stride, tail_off, qo_indptr, state_slots, H, Gk, dim, vdim, taps);
-  BSPEC_LAUNCH(delta_chunk_out_kernel, grid, CH_THREADS, DC_OUT_SMEM, stream, mix, parts, qo_indptr, n_entries, out, H, Gk, dim, vdim);
-  return BSPEC_LAUNCH_CHECK();
-}
-
 // out[t, h*V + j] = x / sqrt(mean_j x^2 + eps) * w[j] * act(gate[t, h*V + j]) * out_scale with x = o[t, h, j], or
 // o[t, h, j] / den[t, h] when ``den`` is given; w null: no weight.  ``flags``: bit 0 act = sigmoid (else silu), bit 1 the
 // gate comes before the norm (x is multiplied by act(gate) and normed then), bit 2 w has a number for every column
@@ -1093,46 +706,26 @@ BSPEC_API int bspec_delta_prepare(const float* proj, int n, int ld, int b_off, i
   return BSPEC_LAUNCH_CHECK();
 }
 
-// How the portions of ST_FROM tokens and more of a step of n tokens in portions of min_q_len to max_q_len go: 0 token by token,
-// 1 by tiles, 2 by chunks: where tiles pay, the heads fill most of the 128 x 128 numbers that a chunk's products are laid out for,
-// and a portion is long enough for its chain of tiles to be what counts.
-static int delta_form(int n, int n_entries, int min_q_len, int max_q_len, int H, int dim, int vdim) {
+// Floats of scratch for a step of n tokens in portions of min_q_len to max_q_len: the tiles' coefficients, or 0 where no
+// portion goes by tiles.
+BSPEC_API long long bspec_delta_scratch(int n, int n_entries, int min_q_len, int max_q_len, int H, int dim, int vdim) {
   if (n <= 0 || n_entries <= 0 || H <= 0 || dim <= 0 || vdim <= 0) return 0;
   // (the token loop's blocks of 8 columns, chosen where 32 would leave SMs idle, do less per microsecond)
   const bool narrow = (long long)((vdim + 31) / 32) * H * n_entries < 2ll * bspec::sm_count();
   const bspec::TokenCost tokens = {dim <= 64 ? 0.165 : (dim <= 128 ? 0.225 : 0.38), (narrow ? 0.9e-6 : 0.34e-6) * (dim <= 32 ? 1.8 : 1.0)};
   const bspec::TokenCost tiles = {dim <= 128 ? 0.118 : 0.2, dim <= 128 ? 6.2e-4 : 1.13e-3};
   if (!bspec::tiles_pay(n, n_entries, min_q_len, max_q_len, H, dim, vdim, tokens, tiles)) return 0;
-  const bool fits = chunk_sizes(dim, vdim) && vdim % 4 == 0 && chunk_slots(n, n_entries) * H * delta_chunk_floats(dim, vdim) <= DC_SCRATCH;
-  return fits && max_q_len >= CH_FROM ? 2 : 1;
-}
-
-// Floats of scratch: the tiles' coefficients or the chunks' parts; 0 where no portion goes by either.
-BSPEC_API long long bspec_delta_scratch(int n, int n_entries, int min_q_len, int max_q_len, int H, int dim, int vdim) {
-  const int form = delta_form(n, n_entries, min_q_len, max_q_len, H, dim, vdim);
-  if (form == 2) return chunk_slots(n, n_entries) * H * delta_chunk_floats(dim, vdim);
-  return form == 1 ? bspec::state_tile_slots(n, n_entries) * H * ST_CO : 0;
-}
-// Kernels that a step launches.
-BSPEC_API int bspec_delta_launches(int n, int n_entries, int min_q_len, int max_q_len, int H, int dim, int vdim) {
-  const int form = delta_form(n, n_entries, min_q_len, max_q_len, H, dim, vdim);
-  return form == 0 ? 1 : (form == 2 ? 3 : 2) + (min_q_len < ST_FROM ? 1 : 0);
+  return bspec::state_tile_slots(n, n_entries) * H * ST_CO;
 }
 
 BSPEC_API int bspec_delta_recurrence(const float* mix, const float* gates, const float* proj, int ld, float* state,
                                      long long state_stride, long long tail_off, const int* qo_indptr,
-                                     const int* state_slots, float* out, int n, int n_entries, int min_q_len, int max_q_len, int H, int Gk,
+                                     const int* state_slots, float* out, int n, int n_entries, int min_q_len, int H, int Gk,
                                      int dim, int vdim, int taps, float* scratch, cudaStream_t stream) {
   if (n_entries <= 0) return 0;
   if (dim <= 0 || dim > MAX_DIM || H % Gk != 0 || n_entries > 65535 || H > 65535)
     return (int)cudaErrorInvalidValue;
-  const int form = scratch != nullptr ? delta_form(n, n_entries, min_q_len, max_q_len, H, dim, vdim) : 0;
-  if (form == 2) {                                             // (rows of mix are whole quads: the sizes are multiples of four)
-    const int err = launch_delta_chunks(stream, mix, gates, proj, ld, state, state_stride, tail_off, qo_indptr, state_slots, out, n,
-                                        n_entries, H, Gk, dim, vdim, taps, scratch);
-    if (err != 0 || min_q_len >= ST_FROM) return err;
-  }
-  if (form == 1) {
+  if (scratch != nullptr) {
     BSPEC_LAUNCH(delta_tiles_prepare_kernel, dim3((unsigned)bspec::state_tile_slots(n, n_entries), H), 128, 0, stream, mix, gates,
                  qo_indptr, n_entries, scratch, H, Gk, dim, vdim);
     const int err = BSPEC_LAUNCH_CHECK();
@@ -1144,7 +737,7 @@ BSPEC_API int bspec_delta_recurrence(const float* mix, const float* gates, const
                                               state_slots, out, H, Gk, dim, vdim, taps);
     if (tiled != 0 || min_q_len >= ST_FROM) return tiled;
   }
-  const int below = form != 0 ? ST_FROM : 0x7fffffff;           // the portions left for the token loop
+  const int below = scratch != nullptr ? ST_FROM : 0x7fffffff;           // the portions left for the token loop
   // 32 value columns of 4 lanes per block; 8 columns of 16 lanes when that would leave most of the device idle
   const bool narrow = (long long)((vdim + 31) / 32) * H * n_entries < 2ll * bspec::sm_count();
   const int cols = narrow ? 8 : 32;

@@ -83,9 +83,8 @@ _SIGNATURES = {
                             c_longlong, c_longlong, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int,
                             c_int, c_int, c_int, c_float, c_float, c_void_p],
     "bspec_delta_recurrence": [c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_longlong, c_longlong, c_void_p,
-                               c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p],
+                               c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p],
     "bspec_delta_scratch": [c_int] * 7,
-    "bspec_delta_launches": [c_int] * 7,
     "bspec_gated_rmsnorm": [c_void_p, c_void_p, c_longlong, c_void_p, c_int, c_void_p, c_int, c_longlong, c_int, c_int, c_int,
                             c_float, c_int, c_void_p, c_float, c_void_p],
     "bspec_state_space": [c_void_p, c_longlong, c_void_p, c_void_p, c_longlong, c_void_p, c_void_p, c_void_p, c_void_p,
@@ -1006,6 +1005,9 @@ def delta_prepare(proj: torch.Tensor, b_off: int, a_off: int, conv: torch.Tensor
     return mix, gates
 
 
+TILE_FROM = 64             # state_tiles.cuh's ST_FROM: in a step by tiles shorter portions take a third kernel
+
+
 def _portion_bounds(ctx, n: int):
     """Bounds of the step's portions: none is shorter than the first or longer than the second."""
     return getattr(ctx, "extras", {}).get("min_q_len", 1), getattr(ctx, "max_q_len", n)
@@ -1028,9 +1030,9 @@ def delta_recurrence(mix: torch.Tensor, gates: torch.Tensor, proj: torch.Tensor,
     _check(lib.bspec_delta_recurrence(
         mix.data_ptr(), gates.data_ptr(), proj.data_ptr(), proj.shape[1], state.data_ptr(), state.stride(0),
         int(tail_off), ctx.qo_indptr.data_ptr(), ctx.state_slots.data_ptr(), out.data_ptr(), n, ctx.n_entries,
-        shortest, longest, n_heads, n_kv_heads, dim, v_dim, taps, _ptr(scratch), _stream()), "delta_recurrence")
+        shortest, n_heads, n_kv_heads, dim, v_dim, taps, _ptr(scratch), _stream()), "delta_recurrence")
     if need:
-        count_launches(lib.bspec_delta_launches(n, ctx.n_entries, shortest, longest, n_heads, dim, v_dim) - 1)
+        count_launches(1 + int(shortest < TILE_FROM))
     return out
 
 

@@ -600,57 +600,6 @@ def test_delta_rule_tiles(ops, Hh, G, dk, dv, lens):
         assert (whole(outs) - want).abs().max() <= 2e-4 * max(1.0, want.abs().max().item()), e
 
 
-@pytest.mark.parametrize("lens", [[513], [1, 600, 64, 127, 9], [576, 700]])
-@pytest.mark.parametrize("Hh,G,dk,dv", [(2, 1, 128, 128), (4, 2, 100, 96), (3, 3, 128, 76)])
-def test_delta_rule_chunks(ops, Hh, G, dk, dv, lens):
-    """As test_delta_rule_tiles, for steps whose longest portion goes by chunks of 64 tokens (whole and partial ones, a lone chunk,
-    shorter portions token by token beside it), with the states that are left."""
-    C = 2 * G * dk + Hh * dv
-    gen = torch.Generator(device=DEV).manual_seed(dk + sum(lens))
-    n, E = sum(lens), len(lens)
-    state = torch.randn(E + 1, Hh * dv * dk + 3, device=DEV, generator=gen)          # (rows off 16-byte boundaries)
-    first = state.clone()
-    slots, qo = list(range(E, 0, -1)), [0] + list(np.cumsum(lens))
-    ctx = SimpleNamespace(qo_indptr=_i32(qo), n_entries=E, max_q_len=max(lens), state_slots=_i32(slots), extras={"min_q_len": min(lens)})
-    assert ops.load_library().bspec_delta_launches(n, E, min(lens), max(lens), Hh, dk, dv) == 3 + (min(lens) < 64)
-    outs, mixes, gate = [], [], []
-    for part in range(2):
-        k = torch.randn(n, G, dk, device=DEV, generator=gen)
-        if part:
-            k[1:] = k[:1].clone()                                  # one key for all tokens
-        k /= k.norm(dim=-1, keepdim=True)
-        qv = torch.randn(n, G * dk + Hh * dv, device=DEV, generator=gen) * 0.5
-        mix = torch.cat([qv[:, :G * dk], k.reshape(n, -1), qv[:, G * dk:]], 1).contiguous()
-        gates = torch.rand(n, 2 * Hh, device=DEV, generator=gen)
-        gates[:, Hh:] = gates[:, Hh:] ** 0.05                      # a memory of some tens of tokens
-        gates[::5, :Hh], gates[1::5, :Hh], gates[2::7, Hh:], gates[3::97, Hh:] = 1.0, 0.0, 1.0, 0.0
-        before = state.clone()
-        outs.append(ops.delta_recurrence(mix, gates, mix, state, Hh * dv * dk, ctx, Hh, G, dk, dv, 1))
-        mixes.append(mix)
-        gate.append(gates)
-        spoilt = mix.clone()
-        spoilt[[e - 1 for e in qo[1:]]] = float("inf")
-        other = ops.delta_recurrence(spoilt, gates, spoilt, before, Hh * dv * dk, ctx, Hh, G, dk, dv, 1)
-        keep = torch.ones(n, dtype=torch.bool, device=DEV)
-        keep[[e - 1 for e in qo[1:]]] = False
-        assert torch.equal(other[keep], outs[-1][keep])
-    assert torch.equal(state[0], first[0])
-    for e in range(E):
-        S = first[slots[e], :Hh * dv * dk].double().view(Hh, dv, dk)
-        for m, g, o in zip(mixes, gate, outs):
-            q, k = (m[:, a:a + G * dk].double().view(n, G, dk).repeat_interleave(Hh // G, dim=1) for a in (0, G * dk))
-            v, want = m[:, 2 * G * dk:].double().view(n, Hh, dv), []
-            for t in range(qo[e], qo[e + 1]):
-                S = g[t, Hh:].double()[:, None, None] * S
-                u = g[t, :Hh].double()[:, None] * (v[t] - torch.einsum("hjd,hd->hj", S, k[t]))
-                S = S + u[:, :, None] * k[t][:, None, :]
-                want.append(torch.einsum("hjd,hd->hj", S, q[t]).reshape(-1))
-            want = torch.stack(want)
-            # the bound of the tests above
-            assert (o[qo[e]:qo[e + 1]] - want).abs().max() <= 2e-4 * max(1.0, want.abs().max().item()), e
-        assert (state[slots[e], :Hh * dv * dk].view(Hh, dv, dk) - S).abs().max() <= 2e-4 * max(1.0, S.abs().max().item()), e
-
-
 @pytest.mark.parametrize("lens,sizes,tiles", [
     ([265], (2, 6, 16), True), ([1, 500, 6, 64], (3, 6, 16), True), ([192, 329], (2, 128, 40), True), ([2048], (16, 128, 128), True),
     ([512] + [1] * 63, (16, 64, 64), True), ([512] + [1] * 63, (16, 128, 128), True), ([64], (16, 128, 128), True), ([63], (16, 128, 128), False),
