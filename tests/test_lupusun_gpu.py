@@ -264,6 +264,38 @@ def test_float32_attention_rows_have_the_same_bits_in_every_portion(ops, Hq, G, 
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("Hq,G,hd,vd,ps", [(8, 2, 64, 64, 16), (6, 1, 40, 20, 7), (5, 5, 36, 128, 16), (4, 2, 100, 30, 8), (2, 1, 256, 192, 16)])
+@pytest.mark.parametrize("options", [{}, {"window": 70, "softcap": 3.0}, {"chunk": 96, "slopes": True}, {"window": 40, "first": 33}, {"scale": 40.0}])
+def test_attention_rows_have_the_same_bits_in_portions_and_decoded(ops, dtype, Hq, G, hd, vd, ps, options):
+    """Portions against the same tokens decoded one by one (another kernel): the same bits with every mask, and where weights are
+    zero beside values that are not finite (scores far apart, and keys that no row sees)."""
+    lens = [3, 64, 97, 290]
+    ks, vs, cache, ctx, tables, fill, qo = _paged(ops, dtype, Hq, G, hd, vd, ps, lens, lens, hd + vd)
+    cache.fill_(float("inf"))
+    fill()
+    opts = dict(options)
+    scale, first = opts.pop("scale", 0.2), opts.pop("first", 0)
+    if opts.pop("slopes", None):
+        opts["slopes"] = torch.linspace(0.01, 0.3, Hq, device=DEV)
+    if first:
+        opts["pooled"] = (-first, cache, tables)
+    n = sum(lens)
+    q = torch.randn(n, Hq * hd, device=DEV, generator=torch.Generator(device=DEV).manual_seed(3)).to(dtype)
+    whole, one = (torch.empty(n, Hq * vd, device=DEV, dtype=dtype) for _ in range(2))
+    ops.masked_attention(q, whole, cache, ctx, tables, Hq, G, hd, vd, scale, **opts)
+    assert torch.isfinite(whole.float()).all()
+    for e, L in enumerate(lens):
+        tab = SimpleNamespace(kv_indptr=tables.kv_indptr[e:e + 2].contiguous(), kv_indices=tables.kv_indices, page_size=ps)
+        if first:
+            opts["pooled"] = (-first, cache, tab)
+        for t in sorted({0, L // 2, L - 2, L - 1}):
+            r = qo[e] + t
+            ctx1 = SimpleNamespace(qo_indptr=_i32([0, 1]), positions=ctx.positions[r:r + 1], n_entries=1, max_q_len=1)
+            ops.masked_attention(q[r:r + 1], one[r:r + 1], cache, ctx1, tab, Hq, G, hd, vd, scale, **opts)
+            assert torch.equal(one[r], whole[r]), (e, t)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("Hq,G,hd,n_req", [(32, 32, 64, 40), (48, 48, 128, 200), (16, 4, 96, 300), (6, 6, 256, 250), (20, 1, 40, 60)])
 def test_attention_rows_have_the_same_bits_in_full_and_idle_grids(ops, dtype, Hq, G, hd, n_req):
     """Decode steps of many requests, of which the smallest and the largest take a warp per row, against each request alone,
