@@ -270,7 +270,6 @@ lightning_tiles_prepare_kernel(const float* __restrict__ proj, long long ld, int
       row[dim + d] = ks[t][d];
     }
   }
-  if (coef == nullptr) return;                                 // (chunks: q and k are all that is wanted)
   // a warp takes two t, eight lanes a dot (four s at a time)
 #pragma unroll
   for (int u = 0; u < ST_B / 2; ++u) {
@@ -351,8 +350,9 @@ int launch_lightning_tiles(dim3 grid, cudaStream_t stream, const float* proj, lo
 //   lightning_chunk_sums   U_c = sum_t d^(cnt-1-t) k_t v_t^T                    [value columns x key rows] per chunk and head
 //   lightning_chunk_scan   S_c = d^cnt S_(c-1) + U_(c-1), over a head's chunks; S_c takes U_c's place
 //   lightning_chunk_out    o_t = d^(t+1) S_c^T q_t + sum_(s <= t) d^(t-s) (q_t . k_s) v_s
-// Float32 throughout, in packed multiply-adds; bound by them (3.1 million per chunk and head of 128 x 128).  q and k come
-// prepared, as for the tiles.
+// Float32 throughout, in packed multiply-adds; bound by them (3.1 million per chunk and head of 128 x 128).  q and k are
+// prepared (activation, scale, rotation) where they are loaded: a kernel of its own for that took 25 us a layer at 2,048 tokens
+// and 16 heads, and their memory.
 constexpr long long CH_SCRATCH = 64ll << 20;         // floats of the chunks' sums at most
 constexpr int CH_SUM_SMEM = 2 * CH * CH_W * 4;
 constexpr int CH_OUT_SMEM = (2 * CH * CH_LD + CH * CH_AT + CH_W * (CH_SL + 4) + CH + 1) * 4;
@@ -365,11 +365,58 @@ __device__ __forceinline__ float power_of(float d, int u) {
   return (float)r;
 }
 
+// A lane's quad of eight rows of a chunk (rows warp + 8 u, columns 4 lane ..): zeros past ``cnt`` and ``width``.
+struct ChunkQuads {
+  float4 v[CH / 8];
+  __device__ __forceinline__ void load(const float* __restrict__ src, long long ld, int cnt, int width, bool vec) {
+    const int c = 4 * (threadIdx.x & 31);
+#pragma unroll
+    for (int u = 0; u < CH / 8; ++u) {
+      const int t = (threadIdx.x >> 5) + 8 * u;
+      const float* p = src + (size_t)t * ld + c;
+      v[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (t < cnt && c < width) {
+        if (vec) v[u] = *reinterpret_cast<const float4*>(p);
+        else v[u] = make_float4(p[0], c + 1 < width ? p[1] : 0.f, c + 2 < width ? p[2] : 0.f, c + 3 < width ? p[3] : 0.f);
+      }
+    }
+  }
+  // to rows of ``lds`` floats; silu(0) = 0
+  __device__ __forceinline__ void store(float* dst, int lds, int act, float scale) const {
+#pragma unroll
+    for (int u = 0; u < CH / 8; ++u) {
+      float4 o = v[u];
+      if (act) o = make_float4(silu_f(o.x), silu_f(o.y), silu_f(o.z), silu_f(o.w));
+      *reinterpret_cast<float4*>(dst + ((threadIdx.x >> 5) + 8 * u) * lds + 4 * (threadIdx.x & 31)) =
+          make_float4(o.x * scale, o.y * scale, o.z * scale, o.w * scale);
+    }
+  }
+};
+// The rotation of a chunk's prepared rows, in place.
+template <int N>
+__device__ __forceinline__ void chunk_rotate(float* const (&rows)[N], int lds, int cnt, const float* __restrict__ inv_freq, int rot,
+                                             const int* __restrict__ positions) {
+  const int half = rot / 2;
+  for (int x = threadIdx.x; x < cnt * half; x += CH_THREADS) {
+    const int t = x / half, d = x - t * half;
+    float sn, c;
+    rotation_sincos(positions[t], inv_freq, half, d, &sn, &c);
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+      float* r = rows[i] + t * lds + d;
+      const float u = r[0], v = r[half];
+      r[0] = u * c - v * sn;
+      r[half] = v * c + u * sn;
+    }
+  }
+  __syncthreads();
+}
+
 // Block: one chunk and head; thread (tx, ty): rows 4 tx + {0..3} and 64 more, columns 4 ty + {0..3} and 64 more.
 __global__ void __launch_bounds__(CH_THREADS, 2)
-lightning_chunk_sums_kernel(const float* __restrict__ proj, long long ld, int v_off, const float* __restrict__ qk,
-                            const float* __restrict__ decay, const int* __restrict__ qo_indptr, int n_entries, float* __restrict__ sums,
-                            int H, int dim, int vdim, int act) {
+lightning_chunk_sums_kernel(const float* __restrict__ proj, long long ld, int k_off, int v_off, const float* __restrict__ decay,
+                            const int* __restrict__ qo_indptr, int n_entries, float* __restrict__ sums, int H, int dim, int vdim, int act,
+                            float k_scale, const float* __restrict__ inv_freq, int rot, const int* __restrict__ positions, int vec) {
   bspec::pdl_prologue(65);
   extern __shared__ __align__(16) float smem_f[];
   float *ks = smem_f, *vs = smem_f + CH * CH_W;
@@ -379,19 +426,25 @@ lightning_chunk_sums_kernel(const float* __restrict__ proj, long long ld, int v_
   if (n < ST_FROM || i * CH >= n) return;
   const int cnt = min(CH, n - i * CH), t0 = q_begin + i * CH, tid = threadIdx.x;
   if (tid < CH) pw[tid] = power_of(decay[h], tid);
+  const float* first = proj + (size_t)t0 * ld;
+  ChunkQuads k, v;
+  k.load(first + k_off + (size_t)h * dim, ld, cnt, dim, vec);
+  v.load(first + v_off + (size_t)h * vdim, ld, cnt, vdim, vec);
   __syncthreads();
-  for (int x = tid; x < CH * CH_W; x += CH_THREADS) {
-    const int t = x / CH_W, c = x % CH_W;
-    float k = 0.f, v = 0.f;
-    if (t < cnt && c < dim) k = pw[cnt - 1 - t] * qk[((size_t)(t0 + t) * H + h) * 2 * dim + dim + c];
-    if (t < cnt && c < vdim) {
-      v = proj[(size_t)(t0 + t) * ld + v_off + (size_t)h * vdim + c];
-      if (act) v = silu_f(v);
-    }
-    ks[x] = k;
-    vs[x] = v;
+  k.store(ks, CH_W, act, k_scale);
+#pragma unroll
+  for (int u = 0; u < CH / 8; ++u) {                 // the powers go to the values
+    const int t = (tid >> 5) + 8 * u;
+    const float p = pw[max(cnt - 1 - t, 0)];
+    float4 o = v.v[u];
+    if (act) o = make_float4(silu_f(o.x), silu_f(o.y), silu_f(o.z), silu_f(o.w));
+    *reinterpret_cast<float4*>(vs + t * CH_W + 4 * (tid & 31)) = make_float4(p * o.x, p * o.y, p * o.z, p * o.w);
   }
   __syncthreads();
+  if (rot > 0) {
+    float* const rows[1] = {ks};
+    chunk_rotate(rows, CH_W, cnt, inv_freq, rot, positions + t0);
+  }
   const int tx = tid & 15, ty = tid >> 4;
   unsigned long long acc[4][8];                      // [pair of rows][column]
 #pragma unroll
@@ -462,9 +515,10 @@ lightning_chunk_scan_kernel(float* __restrict__ sums, const float* __restrict__ 
 // against tx + 16 b), kept as at[s][t]; then per warp eight tokens, per lane columns lane + 32 b: S_c^T q over slices of 32 key
 // rows, then the values' sum.
 __global__ void __launch_bounds__(CH_THREADS, 2)
-lightning_chunk_out_kernel(const float* __restrict__ proj, long long ld, int v_off, const float* __restrict__ qk,
-                           const float* __restrict__ decay, const int* __restrict__ qo_indptr, int n_entries,
-                           const float* __restrict__ sums, float* __restrict__ out, int H, int dim, int vdim, int act) {
+lightning_chunk_out_kernel(const float* __restrict__ proj, long long ld, int q_off, int k_off, int v_off, const float* __restrict__ decay,
+                           const int* __restrict__ qo_indptr, int n_entries, const float* __restrict__ sums, float* __restrict__ out, int H,
+                           int dim, int vdim, int act, float k_scale, const float* __restrict__ inv_freq, int rot,
+                           const int* __restrict__ positions, int vec) {
   bspec::pdl_prologue(65);
   extern __shared__ __align__(16) float smem_f[];
   float* qs = smem_f;                                // [CH][CH_LD]
@@ -477,18 +531,19 @@ lightning_chunk_out_kernel(const float* __restrict__ proj, long long ld, int v_o
   if (n < ST_FROM || i * CH >= n) return;
   const int cnt = min(CH, n - i * CH), t0 = q_begin + i * CH, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   if (tid <= CH) pw[tid] = power_of(decay[h], tid);
-  for (int x = tid; x < CH * (CH_W / 4); x += CH_THREADS) {
-    const int t = x / (CH_W / 4), c = x % (CH_W / 4) * 4;
-    float4 q = make_float4(0.f, 0.f, 0.f, 0.f), k = q;
-    if (t < cnt && c < dim) {                        // dim is a multiple of 4
-      const float* row = qk + ((size_t)(t0 + t) * H + h) * 2 * dim + c;
-      q = *reinterpret_cast<const float4*>(row);
-      k = *reinterpret_cast<const float4*>(row + dim);
-    }
-    *reinterpret_cast<float4*>(qs + t * CH_LD + c) = q;
-    *reinterpret_cast<float4*>(kv + t * CH_LD + c) = k;
+  const float* first = proj + (size_t)t0 * ld;
+  {
+    ChunkQuads q, k;
+    q.load(first + q_off + (size_t)h * dim, ld, cnt, dim, vec);
+    k.load(first + k_off + (size_t)h * dim, ld, cnt, dim, vec);
+    q.store(qs, CH_LD, act, 1.f);
+    k.store(kv, CH_LD, act, k_scale);
   }
   __syncthreads();
+  if (rot > 0) {
+    float* const rows[2] = {qs, kv};
+    chunk_rotate(rows, CH_LD, cnt, inv_freq, rot, positions + t0);
+  }
   {
     const int tx = tid & 15, ty = tid >> 4;
     unsigned long long acc[4][4];
@@ -521,14 +576,10 @@ lightning_chunk_out_kernel(const float* __restrict__ proj, long long ld, int v_o
       }
   }
   __syncthreads();                                   // everybody is done with k
-  for (int x = tid; x < CH * CH_W; x += CH_THREADS) {
-    const int t = x / CH_W, c = x % CH_W;
-    float v = 0.f;
-    if (t < cnt && c < vdim) {
-      v = proj[(size_t)(t0 + t) * ld + v_off + (size_t)h * vdim + c];
-      if (act) v = silu_f(v);
-    }
-    kv[t * CH_LD + c] = v;
+  {
+    ChunkQuads v;
+    v.load(first + v_off + (size_t)h * vdim, ld, cnt, vdim, vec);
+    v.store(kv, CH_LD, act, 1.f);
   }
   const float* S = sums + ((size_t)blockIdx.x * H + h) * vdim * dim;
   const int tb = 8 * warp;                           // this warp's tokens
@@ -850,18 +901,17 @@ static int lightning_form(int n, int n_entries, int min_q_len, int max_q_len, in
   return fits && max_q_len >= CH_FROM ? 2 : 1;
 }
 
-// Floats of scratch: the tiles' coefficients or the chunks' sums, and prepared q and k (as large as the step's q and k columns);
+// Floats of scratch: the tiles' coefficients with prepared q and k (as large as the step's q and k columns), or the chunks' sums;
 // 0 where no portion goes by either.
 BSPEC_API long long bspec_lightning_scratch(int n, int n_entries, int min_q_len, int max_q_len, int H, int dim, int vdim) {
   const int form = lightning_form(n, n_entries, min_q_len, max_q_len, H, dim, vdim);
   if (form == 0) return 0;
-  const long long qk = (long long)n * H * 2 * dim;
-  return qk + (form == 2 ? chunk_slots(n, n_entries) * H * dim * vdim : bspec::state_tile_slots(n, n_entries) * H * ST_CO);
+  return form == 2 ? chunk_slots(n, n_entries) * H * dim * vdim : (long long)n * H * 2 * dim + bspec::state_tile_slots(n, n_entries) * H * ST_CO;
 }
 // Kernels that a step launches.
 BSPEC_API int bspec_lightning_launches(int n, int n_entries, int min_q_len, int max_q_len, int H, int dim, int vdim) {
   const int form = lightning_form(n, n_entries, min_q_len, max_q_len, H, dim, vdim);
-  return form == 0 ? 1 : (form == 2 ? 4 : 2) + (min_q_len < ST_FROM ? 1 : 0);
+  return form == 0 ? 1 : (form == 2 ? 3 : 2) + (min_q_len < ST_FROM ? 1 : 0);
 }
 
 BSPEC_API int bspec_lightning_recurrence(const float* proj, long long ld, int q_off, int k_off, int v_off,
@@ -877,7 +927,7 @@ BSPEC_API int bspec_lightning_recurrence(const float* proj, long long ld, int q_
     return (int)cudaErrorInvalidValue;
   const int form = scratch != nullptr ? lightning_form(n, n_entries, min_q_len, max_q_len, H, dim, vdim) : 0;
   if (form == 2) {
-    float* qk = scratch + chunk_slots(n, n_entries) * H * dim * vdim;
+    const int vec = ((ld | q_off | k_off | v_off | dim | vdim) & 3) == 0 && ((uintptr_t)proj & 15) == 0;
     static bool set[bspec::kMaxDevices] = {};
     bool& done = set[bspec::current_device()];
     if (!done) {
@@ -886,15 +936,13 @@ BSPEC_API int bspec_lightning_recurrence(const float* proj, long long ld, int q_
       if (e != cudaSuccess) return (int)e;
       done = true;
     }
-    BSPEC_LAUNCH(lightning_tiles_prepare_kernel, dim3((unsigned)bspec::state_tile_slots(n, n_entries), H), 128, 0, stream, proj, ld,
-                 q_off, k_off, decay, qo_indptr, n_entries, qk, (float*)nullptr, H, dim, act, k_scale, inv_freq, rot, positions);
     const dim3 chunks((unsigned)chunk_slots(n, n_entries), H);
-    BSPEC_LAUNCH(lightning_chunk_sums_kernel, chunks, CH_THREADS, CH_SUM_SMEM, stream, proj, ld, v_off, (const float*)qk, decay, qo_indptr,
-                 n_entries, scratch, H, dim, vdim, act);
+    BSPEC_LAUNCH(lightning_chunk_sums_kernel, chunks, CH_THREADS, CH_SUM_SMEM, stream, proj, ld, k_off, v_off, decay, qo_indptr, n_entries,
+                 scratch, H, dim, vdim, act, k_scale, inv_freq, rot, positions, vec);
     BSPEC_LAUNCH(lightning_chunk_scan_kernel, dim3((dim * vdim + 255) / 256, H, n_entries), 256, 0, stream, scratch, decay, state,
                  state_stride, qo_indptr, state_slots, H, dim * vdim);
-    BSPEC_LAUNCH(lightning_chunk_out_kernel, chunks, CH_THREADS, CH_OUT_SMEM, stream, proj, ld, v_off, (const float*)qk, decay, qo_indptr,
-                 n_entries, (const float*)scratch, out, H, dim, vdim, act);
+    BSPEC_LAUNCH(lightning_chunk_out_kernel, chunks, CH_THREADS, CH_OUT_SMEM, stream, proj, ld, q_off, k_off, v_off, decay, qo_indptr,
+                 n_entries, (const float*)scratch, out, H, dim, vdim, act, k_scale, inv_freq, rot, positions, vec);
     const int err = BSPEC_LAUNCH_CHECK();
     if (err != 0 || min_q_len >= ST_FROM) return err;
   }
