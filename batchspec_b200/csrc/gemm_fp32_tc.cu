@@ -374,8 +374,8 @@ join_groups_kernel(const float* __restrict__ part, float* __restrict__ C, long l
 long long plane_bytes(int M, int K) { return (3ll * M * ((K + KB - 1) / KB * KB) * 2 + 255) / 256 * 256; }
 
 // CTAs along K: whole groups each, so that the last wave of CTAs is well filled.  In units of a group's time in a CTA, about
-// 16 us; the groups' sums, written and read again at some 5 TB/s, are what it costs (967 x 2,048 x 8,192, 128 tiles of 16 groups,
-// each sum apart: 335 us against some 270).
+// 16 us; the groups' sums, written and read again at some 5 TB/s, are what it costs (967 x 2,048 x 8,192, 128 tiles of 16 groups:
+// sliced: 336 us, whole: 279).
 int tc_splits(int M, int N, int K) {
   const long long tiles = (long long)((M + TT - 1) / TT) * ((N + TN - 1) / TN);
   const int groups = (K + GROUP - 1) / GROUP;
