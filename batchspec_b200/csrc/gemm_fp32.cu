@@ -225,13 +225,17 @@ sgemm_join_kernel(const float* __restrict__ part, float* __restrict__ C, int M, 
 // the kernel when the tokens' 256-byte slices were such copies: 347 us against 20x at 128,256 x 2,048 and 8 tokens).  Rows
 // and slices are padded by 4 floats: a quarter warp's 16-byte loads fall into different banks.  64 consumer threads:
 // rows tid % 8 and tid % 8 + 8, slice tid / 8 of the stage; two rows per thread halve the loads of the tokens' numbers,
-// which bound the kernel at 8 tokens.  Two blocks per SM keep at least 128 KB of W in flight on an SM.
+// which bound the kernel at 8 tokens.  Two blocks per SM keep at least 128 KB of W in flight on an SM; where there is a tile per
+// SM or less (``deep``), one block keeps that much.  4 tokens, us, two stages / five: 2,048 x 8,192 24.9 / 21.1, 2,048 x 16,384
+// 47.1 / 39.7, 1,024 x 4,096 12.5 / 10.8; 8 tokens, two / four: 2,048 x 8,192 37.5 / 30.4, 2,048 x 2,048 11.9 / 10.5; 1 and 2 tokens,
+// whose rings have three stages, 19.9 / 20.4 and 23.1 / 22.9: not.  (Two more consumer warps, and the tokens' copies by a warp of
+// their own, changed little: 23.1 and 20.6.)
 constexpr int RT = 16, KC = 512, SL = KC / SLICE, LDR = KC + 4, LDX = SLICE + 4, ROW_THREADS = 96;
 
 constexpr int rows_stage_floats(int mt) { return RT * LDR + mt * SL * LDX; }
-constexpr int rows_stages(int mt) { return mt >= 4 ? 2 : 3; }
-constexpr int rows_smem(int mt) {
-  return rows_stages(mt) * rows_stage_floats(mt) * 4 + 2 * SL * RT * mt * 4 + 2 * rows_stages(mt) * 8 + 16;
+constexpr int rows_stages(int mt, bool deep) { return deep ? (mt >= 8 ? 4 : 5) : (mt >= 4 ? 2 : 3); }
+constexpr int rows_smem(int mt, bool deep) {
+  return rows_stages(mt, deep) * rows_stage_floats(mt) * 4 + 2 * SL * RT * mt * 4 + 2 * rows_stages(mt, deep) * 8 + 16;
 }
 
 __device__ __forceinline__ void bulk_copy(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
@@ -239,11 +243,11 @@ __device__ __forceinline__ void bulk_copy(void* dst, const void* src, uint32_t b
                ::"r"(s32(dst)), "l"(src), "r"(bytes), "r"(s32(bar)) : "memory");
 }
 
-template <int MT>
+template <int MT, bool DEEP>
 __global__ void __launch_bounds__(ROW_THREADS)
 sgemm_rows_kernel(const float* __restrict__ A, const float* __restrict__ W, float* __restrict__ C, int M, int N, int K,
                   long long lda, long long ldw, long long ldc, long long sa, long long sw, long long sc, int w_ahead, int* status) {
-  constexpr int STAGES = rows_stages(MT), SF = rows_stage_floats(MT);
+  constexpr int STAGES = rows_stages(MT, DEEP), SF = rows_stage_floats(MT);
   extern __shared__ __align__(128) float smem_f[];
   float* red = smem_f + STAGES * SF;                                  // [2][SL][RT][MT] slice values
   uint64_t* full = reinterpret_cast<uint64_t*>(red + 2 * SL * RT * MT);
@@ -376,21 +380,30 @@ sgemm_rows_kernel(const float* __restrict__ A, const float* __restrict__ W, floa
   }
 }
 
-template <int MT>
-int launch_rows(const float* A, const float* W, float* C, int M, int N, int K, long long lda, long long ldw, long long ldc,
+template <int MT, bool DEEP>
+int launch_rows_ring(const float* A, const float* W, float* C, int M, int N, int K, long long lda, long long ldw, long long ldc,
                 long long sa, long long sw, long long sc, int batch, int w_ahead, int* status, cudaStream_t stream) {
   static bool set[bspec::kMaxDevices] = {};
   bool& done = set[bspec::current_device()];
   if (!done) {
-    const cudaError_t e = cudaFuncSetAttribute(sgemm_rows_kernel<MT>, cudaFuncAttributeMaxDynamicSharedMemorySize, rows_smem(MT));
+    const cudaError_t e = cudaFuncSetAttribute(sgemm_rows_kernel<MT, DEEP>, cudaFuncAttributeMaxDynamicSharedMemorySize, rows_smem(MT, DEEP));
     if (e != cudaSuccess) return (int)e;
     done = true;
   }
   const int tiles = (N + RT - 1) / RT * ((M + MT - 1) / MT);
   const int fit = max(1, 2 * bspec::sm_count() / batch);
-  BSPEC_LAUNCH((sgemm_rows_kernel<MT>), dim3(min(tiles, fit), 1, batch), ROW_THREADS, rows_smem(MT), stream, A, W, C, M, N, K, lda,
+  BSPEC_LAUNCH((sgemm_rows_kernel<MT, DEEP>), dim3(min(tiles, fit), 1, batch), ROW_THREADS, rows_smem(MT, DEEP), stream, A, W, C, M, N, K, lda,
                ldw, ldc, sa, sw, sc, w_ahead, status);
   return BSPEC_LAUNCH_CHECK();
+}
+
+template <int MT>
+int launch_rows(const float* A, const float* W, float* C, int M, int N, int K, long long lda, long long ldw, long long ldc,
+                long long sa, long long sw, long long sc, int batch, int w_ahead, int* status, cudaStream_t stream) {
+  if constexpr (MT >= 4)
+    if ((long long)((N + RT - 1) / RT) * ((M + MT - 1) / MT) * batch <= bspec::sm_count())
+      return launch_rows_ring<MT, true>(A, W, C, M, N, K, lda, ldw, ldc, sa, sw, sc, batch, w_ahead, status, stream);
+  return launch_rows_ring<MT, false>(A, W, C, M, N, K, lda, ldw, ldc, sa, sw, sc, batch, w_ahead, status, stream);
 }
 
 template <int BM, bool VEC>
