@@ -1550,6 +1550,10 @@ def latent_attention(q_lat: torch.Tensor, q_rot: torch.Tensor, out: torch.Tensor
 
 LATENT_PART_FLOATS = 64 << 20      # partial results of steps of few rows, at most
 LATENT_PROMPT_FROM = 64            # tokens of a portion from which keys and values per head are formed
+# ... if one of them sees this many keys, or they have this many (token, key) pairs together: below, a step waits for its launches,
+# of which this form has more.  A portion on four layers of 16 heads, whole step, us, per head / in the latent space: 0 + 512 tokens
+# 1,341 / 1,170, 512 + 256 1,313 / 1,163, 512 + 512 1,347 / 1,432, 2,048 + 64 1,322 / 1,648, 8,192 + 64 1,900 / 4,352
+LATENT_PROMPT_KEYS, LATENT_PROMPT_PAIRS = 1024, 1 << 19
 LATENT_PROMPT_ROWS = 1 << 19       # at most this many rows of keys (600 MB of entries)
 LATENT_PROMPT_BYTES = 512 << 20    # keys and values of as many heads at a time as this holds
 
@@ -1576,7 +1580,10 @@ def latent_long_portions(ctx, dtype: torch.dtype, kv_rank: int, dim: int, rot_di
     kv = host["kv_len"].astype(np.int64)
     first = np.maximum(kv - lens - window + 1, 0) // 64 * 64 if window > 0 else np.zeros_like(kv)
     chosen = lens >= LATENT_PROMPT_FROM
-    rows = int(((kv - first + 63) // 64 * 64)[chosen].sum())
+    spans = (kv - first)[chosen]
+    if int(spans.max()) < LATENT_PROMPT_KEYS and int((lens[chosen] * spans).sum()) < LATENT_PROMPT_PAIRS:
+        return None
+    rows = int(((spans + 63) // 64 * 64).sum())
     if rows > LATENT_PROMPT_ROWS:
         return None
     return LongPortions(LATENT_PROMPT_FROM, rows, int(lens[chosen].max()), int(lens[~chosen].max()) if not chosen.all() else 0)

@@ -332,6 +332,16 @@ LONG_PORTIONS = [
 ]
 
 
+@pytest.mark.parametrize("q_lens,kv_lens,window,rows", [
+    ([64], [1023], 0, None), ([64], [1024], 0, 1024), ([63], [4096], 0, None), ([512], [512], 0, None), ([700], [900], 0, 960),
+    ([1, 400, 70], [5000, 400, 1500], 0, 448 + 1536), ([300] * 5, [300] * 5, 0, None), ([300] * 6, [300] * 6, 0, 1920), ([100], [5000], 256, None),
+    ([1000], [9000], 600, 1664)])
+def test_which_portions_go_by_keys_and_values_per_head(ops, q_lens, kv_lens, window, rows):
+    ctx = SimpleNamespace(max_q_len=max(q_lens), host=dict(qo_indptr=np.concatenate([[0], np.cumsum(q_lens)]), kv_len=np.asarray(kv_lens)))
+    long = ops.latent_long_portions(ctx, torch.bfloat16, 512, 128, 64, 128, window)
+    assert (long.rows if long is not None else None) == rows
+
+
 @pytest.mark.parametrize("heads,R,ps,q_lens,kv_lens,window,sinks,group", LONG_PORTIONS)
 def test_long_portions_over_keys_and_values_per_head(ops, heads, R, ps, q_lens, kv_lens, window, sinks, group, monkeypatch):
     """Against a float64 softmax over the bfloat16 keys and values that the product gives.  Scores are sums of 192 float32
@@ -363,6 +373,7 @@ def test_long_portions_over_keys_and_values_per_head(ops, heads, R, ps, q_lens, 
     tables = SimpleNamespace(kv_indptr=torch.tensor(indptr, dtype=torch.int32, device=DEV),
                              kv_indices=table.to(DEV, torch.int32), page_size=ps)
     monkeypatch.setattr(ops, "latent_mma_supported", lambda *a: True)
+    monkeypatch.setattr(ops, "LATENT_PROMPT_KEYS", 0)                 # (these portions are small)
     long = ops.latent_long_portions(ctx, torch.bfloat16, R, dk, P_, V, window)
     assert long.longest_other == max([x for x in q_lens if x < 64], default=0)
     monkeypatch.setattr(ops, "LATENT_PROMPT_BYTES", group * long.rows * (dk + V) * 2)
