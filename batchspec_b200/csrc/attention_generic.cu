@@ -4,7 +4,7 @@
 // share c % W, which keeps a running softmax of its chunks for every row, and the shares' results are joined in their order at
 // the end.  A share is a warp's; attn_row_kernel below has one warp per row, which takes the shares one after the other.  So the
 // order of every sum depends only on the query's own position (and the head sizes, which choose W), not on how the request
-// was cut into steps, on what else is in the batch or on which of the two kernels runs: a key that a row does not see adds
+// was cut into steps, on what else is in the batch or on which of the kernels runs: a key that a row does not see adds
 // an exact nothing.
 //
 // Cache layer layout: [pages][k: [Hkv][page_size][hd] | v: [Hkv][page_size][vd]] (vd = hd unless values have a size
