@@ -373,7 +373,7 @@ __global__ void silu_mul_kernel(const T* __restrict__ u, T* __restrict__ m, int 
 }
 
 // the same, four float32 per thread (I, and the group if any, multiples of 4), without a division of 64 bits per number, which
-// bound it: with the products' slices (gemm_fp32_tc.cu) 1.1 of 23.3 ms at 967 tokens of 16 layers of 8,192
+// bound it: 4,000 x 8,192 106 -> 58 us, with groups of 8 141 -> 60
 __global__ void silu_mul_f32x4_kernel(const float* __restrict__ u, float* __restrict__ m, int inter, int n, int group, int act) {
   bspec::pdl_prologue(4);
   const int col = 4 * (blockIdx.x * blockDim.x + threadIdx.x);

@@ -11,8 +11,7 @@
 // Two kernels:
 //   sgemm_rows_kernel  few rows (decode steps): bound by reading W once.  W streams through a ring of shared-memory
 //                      stages by bulk copies, a thread owns one output number and one slice at a time.
-//   sgemm_tile_kernel  everything else that gemm_fp32_tc.cu does not take (from 192 rows and 2^28 multiply-adds on, in an order of
-//                      its own): bound by the multiply-adds.  BM x 64 tiles, 8 x 4 outputs per thread; 32 x 32 tiles
+//   sgemm_tile_kernel  everything else: bound by the multiply-adds.  BM x 64 tiles, 8 x 4 outputs per thread; 32 x 32 tiles
 //                      where those would leave most of the device idle.
 #include "tma.cuh"
 

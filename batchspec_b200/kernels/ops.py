@@ -6,9 +6,8 @@ functions raise.
 
 Matrix products in bfloat16 go to the vendor library through ``torch.mm`` (the
 reference's ``nn.Linear`` does the same, batchspec/models/modules/attention/base.py:32-39);
-float32 products use this package's own kernels so that no reduced-precision mode
-can slip in: multiply-adds on the CUDA cores, or, with many rows, every number as the
-sum of three bfloat16 numbers on the tensor cores (csrc/gemm_fp32_tc.cu).
+float32 products use this package's own FFMA kernel so that no reduced-precision
+mode can slip in.
 """
 from __future__ import annotations
 
@@ -144,9 +143,6 @@ _SIGNATURES = {
                           c_void_p, c_void_p, c_longlong, c_void_p],
     "bspec_sgemm_tn_batched": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_longlong, c_longlong, c_longlong,
                                c_longlong, c_longlong, c_longlong, c_int, c_void_p, c_int, c_void_p, c_void_p],
-    "bspec_sgemm_tc": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_longlong, c_longlong, c_void_p, c_void_p, c_void_p],
-    "bspec_sgemm_tc_scratch": [c_void_p, c_int, c_int, c_int, c_longlong],
-    "bspec_sgemm_tc_launches": [c_int, c_int, c_int],
     "bspec_sgemm_scratch": [c_void_p, c_void_p, c_int, c_int, c_int, c_longlong, c_longlong, c_longlong, c_longlong, c_int],
     "bspec_attention_generic": [c_void_p, c_longlong, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p,
                                 c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_int, c_longlong, c_void_p],
@@ -240,7 +236,7 @@ def set_pdl(on: bool) -> None:
 
 
 _TRACE_SETTERS = ["bspec_trace_set_attention_tcgen05", "bspec_trace_set_elementwise", "bspec_trace_set_attention_generic", "bspec_trace_set_attention_bf16",
-                  "bspec_trace_set_gemm_fp32", "bspec_trace_set_gemm_fp32_tc", "bspec_trace_set_sampling", "bspec_trace_set_gemm_tcgen05", "bspec_trace_set_latent",
+                  "bspec_trace_set_gemm_fp32", "bspec_trace_set_sampling", "bspec_trace_set_gemm_tcgen05", "bspec_trace_set_latent",
                   "bspec_trace_set_moe", "bspec_trace_set_latent_mma", "bspec_trace_set_latent_prompt", "bspec_trace_set_delta",
                   "bspec_trace_set_state_mixers", "bspec_trace_set_streams", "bspec_trace_set_joins",
                   "bspec_trace_set_gated_states"]
@@ -1445,13 +1441,6 @@ def _sgemm(x, w, out, M: int, N: int, K: int, lda: int, ldw: int, sa: int, sw: i
     """``batch`` float32 products, operands sa / sw numbers apart; the K slices of small tiles meet in scratch that the
     stream's order protects."""
     lib = load_library()
-    split = lib.bspec_sgemm_tc_scratch(w.data_ptr(), M, N, K, ldw) if batch == 1 else 0
-    if split:
-        scratch = torch.empty((split,), dtype=torch.uint8, device=x.device)
-        _check(lib.bspec_sgemm_tc(x.data_ptr(), w.data_ptr(), out.data_ptr(), M, N, K, lda, ldw, scratch.data_ptr(),
-                                  _status_word(x.device).data_ptr(), _stream()), "sgemm_tc")
-        count_launches(lib.bspec_sgemm_tc_launches(M, N, K) - 1)
-        return
     need = lib.bspec_sgemm_scratch(x.data_ptr(), w.data_ptr(), M, N, K, lda, ldw, sa, sw, batch)
     scratch = torch.empty((need,), dtype=torch.float32, device=x.device) if need else None
     _check(lib.bspec_sgemm_tn_batched(x.data_ptr(), w.data_ptr(), out.data_ptr(), M, N, K, lda, ldw, N, sa, sw, M * N, batch,

@@ -312,6 +312,29 @@ def test_preemption_under_page_pressure_changes_nothing(tmp_path):
     assert outs[0] == outs[1]
 
 
+def test_float32_logits_do_not_depend_on_the_cut_or_the_neighbours(tmp_path):
+    """Layers of real widths, whose products of a prompt of 300 tokens are large ones: every logit has the same bits whether the
+    prompt is run whole, in portions, or beside another one."""
+    from batchspec_b200.engine import StepEntry
+    folder = H.make_folder(tmp_path, H.WIDE, 6, dtype=torch.float32)
+    prompt, other = (H.random_tokens(n, H.WIDE["vocab_size"], n) for n in (300, 210))
+    outs = []
+    for cuts, beside in (((300,), False), ((100, 1, 199), False), ((250, 50), True)):
+        eng = engine_for(folder, "float32", 16, max_seq=512)
+        eng.admit("x")
+        eng.admit("y")
+        at, rows = 0, []
+        for c in cuts:
+            step = [StepEntry("x", prompt[at:at + c], want=range(c))]
+            if beside and at == 0:
+                step.insert(0, StepEntry("y", other))
+            rows.append(eng.step(step).clone())
+            at += c
+        outs.append(torch.cat(rows))
+        del eng
+    assert torch.equal(outs[0], outs[1]) and torch.equal(outs[0], outs[2])
+
+
 def test_everything_at_once_gives_the_same_tokens(tmp_path):
     """Many requests of random lengths and limits, sampled, some ending on end-of-sequence tokens, more than fit at
     once, through a pool so small that requests are preempted: the tokens are those of a roomy engine without
