@@ -1557,11 +1557,12 @@ class LongPortions:
 
 
 def latent_long_portions(ctx, dtype: torch.dtype, kv_rank: int, dim: int, rot_dim: int, v_dim: int,
-                         window: int = 0) -> Optional[LongPortions]:
+                         window: int = 0, scale: float = 1.0) -> Optional[LongPortions]:
     """The step's portions of at least ``LATENT_PROMPT_FROM`` tokens, None when there are none or ``latent_prompt`` does not
-    take these sizes.  Needs the lengths on the host: a captured step has none."""
+    take these sizes or this ``scale`` of the scores (it finds a row's maximum before scaling, so only positive ones).  Needs
+    the lengths on the host: a captured step has none."""
     host = getattr(ctx, "host", None)
-    if (host is None or ctx.max_q_len < LATENT_PROMPT_FROM or dtype != torch.bfloat16 or FORCE_GENERIC_LATENT
+    if (host is None or ctx.max_q_len < LATENT_PROMPT_FROM or dtype != torch.bfloat16 or FORCE_GENERIC_LATENT or not scale > 0
             or not latent_mma_supported(kv_rank, rot_dim)
             or not load_library().bspec_latent_prompt_supported(kv_rank, dim, rot_dim, v_dim)):
         return None

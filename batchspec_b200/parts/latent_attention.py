@@ -114,7 +114,7 @@ class LatentAttention(Mixer):
         with bucket("attn.q_proj"):
             q = ops.linear(cq, self.w_uq, w_is_parameter=True).view(n, H, dh + P)
         q_rot = q[:, :, dh:]
-        long = ops.latent_long_portions(ctx, x.dtype, R, dh, P, self.v_dim, self.window)
+        long = ops.latent_long_portions(ctx, x.dtype, R, dh, P, self.v_dim, self.window, self.scale)
         v = None
         if long is not None:
             with bucket("attn.rotate"):

@@ -438,6 +438,28 @@ def test_an_engine_step_of_long_and_short_portions_gives_what_short_ones_give(op
         assert (got[0] - other).norm() <= 0.03 * got[0].norm()
 
 
+@pytest.mark.parametrize("scale", [-0.06, 0.0])
+def test_long_portions_run_with_scales_that_are_not_positive(ops, scale):
+    """A prompt of 1,100 tokens, whole and in portions too short for keys and values per head (whose kernel takes positive
+    scales only): the logits agree as two roundings of one model do."""
+    from batchspec_b200.config import config_from_json_dict
+    from batchspec_b200.engine import Engine, StepEntry
+    mix = _mixer(4, 128, 64, 128, 96, 64, scale, 10000.0, None)
+    cfg = dict(CFG_A, layers=[dict(type="latent_attention", mixer=mix, mlp=dict(kind="dense", ff=80, limit=0.7))] * 2)
+    eng = Engine(dtype="bfloat16", device=DEV)
+    eng.load_model(config=config_from_json_dict(cfg), random_seed=3, draw_on_device=True)
+    eng.setup_caches(max_batch_size=1, max_seq_length=1200, page_size=16, prefill_chunk_size=512)
+    prompt = H.random_tokens(1100, cfg["vocab"], 8)
+    got = []
+    for cut in (1100, 60):
+        eng.admit("x")
+        for a in range(0, 1100, cut):
+            out = eng.step([StepEntry("x", prompt[a:a + cut], want=(len(prompt[a:a + cut]) - 1,))])
+        got.append(out[0].float().clone())
+        eng.release("x")
+    assert not torch.isnan(got[0]).any() and (got[0] - got[1]).norm() <= 0.03 * got[0].norm()
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("key", [0, 15, 16, 511, 512, 1023, 1500])
 def test_one_far_entry_among_hundreds_is_found(ops, dtype, key):
