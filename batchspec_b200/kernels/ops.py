@@ -1231,6 +1231,24 @@ def _status_word(device) -> torch.Tensor:
     return _status[device]
 
 
+# What a kernel that gave up a bounded wait leaves in the status word: (first code, last code, meaning).
+WAIT_CODES = ((1, 1, "GEMM: stage never freed"), (2, 2, "GEMM: operands never arrived"),
+              (3, 3, "GEMM: accumulator never completed"),
+              (11, 11, "decode attention: stage never freed"), (12, 12, "decode attention: keys never arrived"),
+              (13, 13, "decode attention: stage never freed"), (14, 14, "decode attention: keys never arrived"),
+              (21, 21, "prompt attention: stage never freed"), (22, 22, "prompt attention: keys never arrived"),
+              (31, 41, "a role of the tensor-core prompt attention"),
+              (61, 63, "latent attention of long portions: a Q, key or value stage never freed"),
+              (64, 68, "latent attention of long portions: operands, weights or a free accumulator never came"),
+              (69, 71, "latent attention of long portions: scores or sums never completed"),
+              (91, 91, "float32 product of few rows: stage never freed"),
+              (92, 92, "float32 product of few rows: operands never arrived"))
+
+
+def wait_meaning(code: int) -> str:
+    return next((text for first, last, text in WAIT_CODES if first <= code <= last), "unknown")
+
+
 def _raise_status(dev, code: int) -> None:
     with torch.inference_mode():          # the words may have been made inside inference mode (by a step)
         _status[dev].zero_()
@@ -1239,11 +1257,7 @@ def _raise_status(dev, code: int) -> None:
                 b.zero_()
         for b in _work_counters.values():
             b.zero_()
-    raise KernelError(f"a kernel on {dev} gave up a bounded wait (code {code}: GEMM 1 = stage never freed, "
-                      f"2 = operands never arrived, 3 = accumulator never completed; decode attention 11/13 = stage "
-                      f"never freed, 12/14 = keys never arrived; prompt attention 21/22 the same, 31-41 = a role of "
-                      f"the tensor-core prompt kernel; float32 product of few rows 91 = stage never freed, 92 = operands "
-                      f"never arrived).  The results of the steps "
+    raise KernelError(f"a kernel on {dev} gave up a bounded wait (code {code}: {wait_meaning(code)}).  The results of the steps "
                       f"since the last check are not valid.")
 
 
@@ -1259,8 +1273,8 @@ def check_status() -> None:
 
 _BOUNDS_REPORTS = ["bspec_bounds_report_state_mixers", "bspec_bounds_report_elementwise", "bspec_bounds_report_gemm_tcgen05",
                    "bspec_bounds_report_attention_generic", "bspec_bounds_report_attention_bf16",
-                   "bspec_bounds_report_latent", "bspec_bounds_report_latent_mma", "bspec_bounds_report_delta",
-                   "bspec_bounds_report_streams", "bspec_bounds_report_joins"]
+                   "bspec_bounds_report_latent", "bspec_bounds_report_latent_mma", "bspec_bounds_report_latent_prompt",
+                   "bspec_bounds_report_delta", "bspec_bounds_report_streams", "bspec_bounds_report_joins"]
 BOUNDS_CODES = {101: "token id (embedding)", 102: "row (gather)", 103: "block-table slot (rotary + cache append)",
                 104: "page id (rotary + cache append)", 105: "block-table slot (q/k/v product's epilogue)",
                 106: "page id (q/k/v product's epilogue)", 107: "page id (attention over plain loads)",

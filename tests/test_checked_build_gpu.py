@@ -134,6 +134,23 @@ assert len(rep) == 1 and rep[0][0] == "attention_bf16" and rep[0][2:4] == (6, 5)
 # (the skipped keys are read as zeros here, not left out: a wrong result, reported, and no access outside)
 assert bool(torch.isfinite(out16.float()).all())
 print("bf16 attention ok")
+
+# 6. latent attention over keys and values per head: an entry on a page beyond the declared ones is read as zeros, and reported
+R, ps = 32, 16
+backing = torch.randn(8, 1, ps * (R + 64), device=dev).bfloat16()
+backing[6] = float("inf")
+q = torch.randn(64, 1, 192, device=dev).bfloat16()
+w_kv = (torch.randn(1, 256, R, device=dev) * 0.1).bfloat16()
+latent = torch.empty(64, 1, 128, device=dev, dtype=torch.bfloat16)
+long_ctx = SimpleNamespace(qo_indptr=i32([0, 64]), positions=i32(list(range(64))), n_entries=1, n_tokens=64, max_q_len=64,
+                           max_kv_len=64)
+tables = SimpleNamespace(kv_indptr=i32([0, 4]), kv_indices=i32([1, 4, 6, 0]), page_size=ps)
+ops.latent_prompt(q, w_kv, latent.transpose(0, 1), backing[:5], long_ctx, tables, ops.LongPortions(64, 64, 64, 0), 1, R, 0.1)
+torch.cuda.synchronize()
+rep = ops.bounds_reports()
+assert len(rep) == 1 and rep[0][0] == "latent_prompt" and rep[0][1].startswith("page id") and rep[0][2:4] == (6, 5), rep
+assert bool(torch.isfinite(latent.float()).all())
+print("latent prompt ok")
 try:
     ops.gather_rows_add(resid[:4], None, i32([1, 5]), out.new_empty(2, 48))
     ops.check_status()
