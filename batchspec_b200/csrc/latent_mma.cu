@@ -60,19 +60,22 @@ __host__ __device__ inline size_t smem_bytes(int D, int BM, int stages = 2, int 
   return (size_t)(BM + stages * BN) * DP * 2 + (size_t)shares * BM * (BN + 8) * 4 + 2 * (size_t)BM * (BN + 8) * 2 + 3 * BM * 4;
 }
 
-// The work of a step of few rows, dealt evenly: the requests' key tiles are cut into shares of ``per`` tiles, about as many
-// shares in all as CTAs fit the device at once (a request has at least one, at most MAX_SHARES), and CTA z takes the z-th.
-// Every CTA finds that out for itself from the lengths, so a captured step follows them.  (With as many shares for every
-// request the longest request's were the kernel's time: 64 requests of 300 to 4,096 entries, 16 heads,
-// 88 us, and 51 dealt evenly.)
-constexpr int MAX_SHARES = 64, MIN_TILES = 4;
+// The work of a step of few rows, dealt evenly: the requests' key tiles are cut into shares of ``per`` tiles, as many in all as CTAs
+// fit the device at once (a request has at least one, at most MAX_SHARES), and CTA z takes the z-th.  Every CTA finds that out
+// for itself from the lengths, so a captured step follows them.  ``per`` is the least of TRY lengths from the even share up, each up
+// to a sixteenth longer than the one before (then a quarter of the even share), whose shares all fit: a request's last share is
+// shorter than the others, and a share more than fit runs after all others.  64 requests of 300 to
+// 4,096 entries, 16 heads: 100 us with as many shares for each as for the longest, 55 dealt; requests of one length lose nothing
+// by it: 64 of 4,096 entries 117 / 111 (141 where a few shares ran in a second wave), 64 of 1,000 43 / 41 (57), 256 of 300, a
+// share each, 54 / 54 (73).  At latents of 128 and 256 the dealing itself shows, 256 of 300 26 / 29.
+constexpr int MAX_SHARES = 64, MIN_TILES = 4, TRY = 16, OWN = 4;
 struct Share {
   int e, split, first, count, per;       // request (-1: none), which of its shares, its first share and how many it has
 };
 template <int NT>
 __device__ __forceinline__ Share deal(int z, const int* __restrict__ qo_indptr, const int* __restrict__ positions, int n_entries,
                                       int window, int skip_from, int want_shares) {
-  __shared__ int part[3][NT / 32], found[3];
+  __shared__ int part[3][NT / 32], tried[TRY][NT / 32], found[3];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   auto tiles_of = [&](int e) -> int {
     if (e >= n_entries) return 0;
@@ -82,18 +85,28 @@ __device__ __forceinline__ Share deal(int z, const int* __restrict__ qo_indptr, 
     return (pos0 + q1 - q0 - 1) / BN + 1 - (window > 0 ? max(0, pos0 - window + 1) / BN : 0);
   };
   if (tid == 0) found[0] = -1;
-  const int own = tiles_of(tid);
-  int total = 0, most = 0;
-  for (int e0 = 0; e0 < n_entries; e0 += NT) {
-    const int t = e0 == 0 ? own : tiles_of(e0 + tid);
-    total += t;
-    most = max(most, t);
-  }
+  int own[OWN];                                    // this thread's requests among the first NT * OWN, asked for at once
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    total += __shfl_xor_sync(0xffffffffu, total, o);
-    most = max(most, __shfl_xor_sync(0xffffffffu, most, o));
-  }
+  for (int k = 0; k < OWN; ++k) own[k] = tiles_of(tid * OWN + k);
+  auto each = [&](auto visit) {                    // visit(this thread's first request, its OWN requests' tiles), for all requests
+    visit(tid * OWN, own);
+    for (int e0 = NT * OWN; e0 < n_entries; e0 += NT * OWN) {
+      int more[OWN];
+#pragma unroll
+      for (int k = 0; k < OWN; ++k) more[k] = tiles_of(e0 + tid * OWN + k);
+      visit(e0 + tid * OWN, more);
+    }
+  };
+  int total = 0, most = 0;
+  each([&](int, const int (&t)[OWN]) {
+#pragma unroll
+    for (int k = 0; k < OWN; ++k) {
+      total += t[k];
+      most = max(most, t[k]);
+    }
+  });
+  total = __reduce_add_sync(0xffffffffu, total);
+  most = __reduce_max_sync(0xffffffffu, most);
   if (lane == 0) {
     part[0][warp] = total;
     part[1][warp] = most;
@@ -105,11 +118,46 @@ __device__ __forceinline__ Share deal(int z, const int* __restrict__ qo_indptr, 
     total += part[0][w];
     most = max(most, part[1][w]);
   }
-  const int per = max(MIN_TILES, max((total + want_shares - 1) / want_shares, (most + MAX_SHARES - 1) / MAX_SHARES));
+  const int even = max(MIN_TILES, max((total + want_shares - 1) / want_shares, (most + MAX_SHARES - 1) / MAX_SHARES));
+  auto length = [&](int i) -> int { return even + (i <= 8 ? (even * i + 15) / 16 : (even * (i - 6) + 3) / 4); };
+  int per = even;
+  if (n_entries <= want_shares) {                  // (else in waves)
+    int shares[TRY];
+    float inverse[TRY];                              // (a share more or less by rounding only moves the choice)
+#pragma unroll
+    for (int i = 0; i < TRY; ++i) {
+      shares[i] = 0;
+      inverse[i] = __fdividef(1.f, (float)length(i));
+    }
+    each([&](int, const int (&t)[OWN]) {
+#pragma unroll
+      for (int k = 0; k < OWN; ++k)
+        if (t[k] > 0)
+#pragma unroll
+          for (int i = 0; i < TRY; ++i) shares[i] += __float2int_ru((float)t[k] * inverse[i] - 1e-3f);
+    });
+#pragma unroll
+    for (int i = 0; i < TRY; ++i) {
+      const int sum = __reduce_add_sync(0xffffffffu, shares[i]);
+      if (lane == i) tried[i][warp] = sum;
+    }
+    __syncthreads();
+    bool fits = false;
+    if (lane < TRY) {
+      int sum = 0;
+#pragma unroll
+      for (int w = 0; w < NT / 32; ++w) sum += tried[lane][w];
+      fits = sum <= want_shares;
+    }
+    const unsigned first_fit = __ballot_sync(0xffffffffu, fits);
+    if (first_fit != 0) per = length(__ffs(first_fit) - 1);
+  }
   int before = 0;
-  for (int e0 = 0; e0 < n_entries; e0 += NT) {
-    const int n = ((e0 == 0 ? own : tiles_of(e0 + tid)) + per - 1) / per;
-    int sum = n;
+  each([&](int e, const int (&t)[OWN]) {
+    int n[OWN], mine = 0;
+#pragma unroll
+    for (int k = 0; k < OWN; ++k) mine += n[k] = (t[k] + per - 1) / per;
+    int sum = mine;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
       const int up = __shfl_up_sync(0xffffffffu, sum, o);
@@ -117,19 +165,23 @@ __device__ __forceinline__ Share deal(int z, const int* __restrict__ qo_indptr, 
     }
     if (lane == 31) part[2][warp] = sum;
     __syncthreads();
-    int first = before + sum - n;
+    int first = before + sum - mine;
 #pragma unroll
     for (int w = 0; w < NT / 32; ++w) {
       if (w < warp) first += part[2][w];
       before += part[2][w];
     }
-    if (n > 0 && z >= first && z < first + n) {
-      found[0] = e0 + tid;
-      found[1] = first;
-      found[2] = n;
+#pragma unroll
+    for (int k = 0; k < OWN; ++k) {
+      if (z >= first && z < first + n[k]) {
+        found[0] = e + k;
+        found[1] = first;
+        found[2] = n[k];
+      }
+      first += n[k];
     }
     __syncthreads();
-  }
+  });
   Share s;
   s.e = found[0];
   s.first = found[1];
@@ -179,11 +231,10 @@ latent_attn_mma_kernel(const __nv_bfloat16* __restrict__ ql, long long ql_row, l
   float* row_c = row_l + BM;
 
   const int e = mine.e, split = mine.split;
-  if (plan != nullptr && split == 0 && blockIdx.x == 0 && threadIdx.x == 0) {      // for the join
-    plan[2 * e] = mine.first;
-    plan[2 * e + 1] = mine.count;
-  }
   const int q_begin = qo_indptr[e], q_len = qo_indptr[e + 1] - q_begin;
+  if (plan != nullptr && split == 0 && blockIdx.x == 0)                            // for the join
+    for (int t = threadIdx.x; t < q_len; t += 32 * RG * CH)
+      *reinterpret_cast<int2*>(plan + 2 * (q_begin + t)) = make_int2(mine.first * rows_max + t * H, mine.count);
   if (q_len >= skip_from) return;                  // another kernel's portions
   const long long rows_total = (long long)q_len * H;
   const long long row0 = (long long)blockIdx.x * BM;
@@ -554,7 +605,7 @@ latent_attn_mma_kernel(const __nv_bfloat16* __restrict__ ql, long long ql_row, l
     if (row >= rows_total) continue;
     const long long t = q_begin + row / H;
     const int h = (int)(row % H);
-    if (plan == nullptr) {
+    if (mine.count <= 1) {                         // the whole request is this CTA's
       const float inv = 1.f / row_l[r];
       __nv_bfloat16* op = out + t * o_row + h * o_head;
 #pragma unroll
@@ -581,48 +632,64 @@ latent_attn_mma_kernel(const __nv_bfloat16* __restrict__ ql, long long ql_row, l
   }
 }
 
-// out[row, :] = sum_s w_s O_s / sum_s w_s l_s with w_s = exp(m_s - max m), s ascending.  One block per (token, head):
-// the shares' weights are formed once (in parallel, into shared memory), then every thread adds its columns.
-// ``plan``: first share and number of shares per request, whose rows lie rows_max apart from share to share.
-__global__ void latent_attn_join_kernel(const float* __restrict__ o_part, const float* __restrict__ ml_part,
-                                        __nv_bfloat16* __restrict__ out, long long o_row, long long o_head, int H,
-                                        int R, const int* __restrict__ plan, const int* __restrict__ tok_entry,
-                                        const int* __restrict__ qo_indptr, int rows_max, int skip_from) {
+// out[row, :] = sum_s w_s O_s / sum_s w_s l_s with w_s = exp(m_s - max m), s ascending.  A block takes ``per_block`` (token, head)
+// rows, one after the other, and goes on: the shares' weights are formed once (in parallel, into shared memory), then every
+// thread adds its four columns, eight shares' numbers asked for at a time (one number each, four at a time: 0.5 us per share).
+// Several rows where there are many: most then have a single share, and blocks that only see that took their launch's time (256
+// requests of 128 heads: 17 us).
+// ``plan``: per token the row of its first head in its request's first share and the number of shares, whose rows lie rows_max
+// apart from share to share; a single share has left its result where it belongs, a portion of another kernel has none.
+__global__ void __launch_bounds__(128)
+latent_attn_join_kernel(const float* __restrict__ o_part, const float* __restrict__ ml_part, __nv_bfloat16* __restrict__ out,
+                        long long o_row, long long o_head, int H, int R, const int* __restrict__ plan, int rows_max, int rows,
+                        int per_block) {
   bspec::pdl_prologue(44);
-  __shared__ float w[MAX_SHARES];
+  __shared__ float w[MAX_SHARES], l[MAX_SHARES];
   __shared__ float inv_l;
-  const long long t = blockIdx.x / H;
-  const int h = (int)(blockIdx.x % H), e = tok_entry[t], q0 = qo_indptr[e];
-  if (qo_indptr[e + 1] - q0 >= skip_from) return;
-  const int n_shares = plan[2 * e + 1];
-  const size_t row = (size_t)plan[2 * e] * rows_max + (size_t)(t - q0) * H + h, step = rows_max;
-  if (threadIdx.x < 32) {
-    const int lane = threadIdx.x;
-    float m0 = lane < n_shares ? ml_part[2 * (row + lane * step)] : -INFINITY;
-    float m1 = lane + 32 < n_shares ? ml_part[2 * (row + (lane + 32) * step)] : -INFINITY;
-    const float M = warp_max(fmaxf(m0, m1));
-    const float w0 = m0 == -INFINITY ? 0.f : expf(m0 - M), w1 = m1 == -INFINITY ? 0.f : expf(m1 - M);
-    w[lane] = w0;
-    w[lane + 32] = w1;
-    __syncwarp();
-    if (lane == 0) {                 // the sum in the order of the shares
-      float L = 0.f;
-      for (int s = 0; s < n_shares; ++s)
-        if (w[s] != 0.f) L += w[s] * ml_part[2 * (row + s * step) + 1];
-      inv_l = 1.f / L;
+  for (int r0 = blockIdx.x * per_block; r0 < rows; r0 += gridDim.x * per_block)
+    for (int r = r0; r < min(rows, r0 + per_block); ++r) {
+      const int t = r / H, h = r - t * H;
+      const int2 from = *reinterpret_cast<const int2*>(plan + 2 * t);
+      const int n_shares = from.y;
+      if (n_shares <= 1) continue;
+      const size_t row = (size_t)from.x + h, step = rows_max;
+      __syncthreads();                             // the row before is done with w
+      if (threadIdx.x < 32) {
+        const int lane = threadIdx.x;
+        const float2 none = make_float2(-INFINITY, 0.f);
+        const float2* ml = reinterpret_cast<const float2*>(ml_part) + row;
+        const float2 a = lane < n_shares ? ml[lane * step] : none, b = lane + 32 < n_shares ? ml[(lane + 32) * step] : none;
+        const float M = warp_max(fmaxf(a.x, b.x));
+        w[lane] = a.x == -INFINITY ? 0.f : expf(a.x - M);
+        w[lane + 32] = b.x == -INFINITY ? 0.f : expf(b.x - M);
+        l[lane] = a.y;
+        l[lane + 32] = b.y;
+        __syncwarp();
+        if (lane == 0) {             // the sum in the order of the shares
+          float L = 0.f;
+#pragma unroll 8
+          for (int s = 0; s < n_shares; ++s) {
+            const float ws = w[s], ls = l[s];
+            L = ws != 0.f ? fmaf(ws, ls, L) : L;
+          }
+          inv_l = 1.f / L;
+        }
+      }
+      __syncthreads();
+      const float inv = inv_l;
+      for (int c = 4 * threadIdx.x; c < R; c += 512) {
+        float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 8
+        for (int s = 0; s < n_shares; ++s) {
+          const float4 x = *reinterpret_cast<const float4*>(o_part + (row + s * step) * R + c);
+          const float ws = w[s];
+          if (ws != 0.f) acc.x = fmaf(ws, x.x, acc.x), acc.y = fmaf(ws, x.y, acc.y), acc.z = fmaf(ws, x.z, acc.z), acc.w = fmaf(ws, x.w, acc.w);
+        }
+        __nv_bfloat162* to = reinterpret_cast<__nv_bfloat162*>(out + t * o_row + h * o_head + c);
+        to[0] = __floats2bfloat162_rn(acc.x * inv, acc.y * inv);
+        to[1] = __floats2bfloat162_rn(acc.z * inv, acc.w * inv);
+      }
     }
-  }
-  __syncthreads();
-  const float inv = inv_l;
-  for (int c = threadIdx.x; c < R; c += blockDim.x) {
-    float acc = 0.f;
-#pragma unroll 4
-    for (int s = 0; s < n_shares; ++s) {
-      const float x = o_part[(row + s * step) * R + c];
-      if (w[s] != 0.f) acc += w[s] * x;
-    }
-    out[t * o_row + h * o_head + c] = __float2bfloat16_rn(acc * inv);
-  }
 }
 
 }  // namespace
@@ -669,8 +736,8 @@ BSPEC_API int bspec_latent_attention_mma_rows(int max_q_len, int H, int R, int P
   return two_small_ctas(R, P) ? 32 : 64;
 }
 
-// ``plan`` (not null: 2 ints per request of scratch): the requests' keys are dealt in want_shares shares and at most one
-// more per request; o_part and ml_part then hold (want_shares + n_entries) * max_q_len * H rows of R and of 2 floats.
+// ``plan`` (not null: 2 ints per token of scratch, zeros where portions are left alone): the requests' keys are dealt in want_shares shares or, with more requests
+// than half of that, at most one more per request; o_part and ml_part then hold (want_shares + n_entries) * max_q_len * H rows of R and of 2 floats.
 // ``skip_from``: portions of that many tokens and more are left alone (``max_q_len``: the longest of the others).
 BSPEC_API int bspec_latent_attention_mma(const void* ql, long long ql_row, long long ql_head, const void* qr,
                                          long long qr_row, long long qr_head, void* out, long long o_row,
@@ -679,7 +746,7 @@ BSPEC_API int bspec_latent_attention_mma(const void* ql, long long ql_row, long 
                                          int n_entries, int n_tokens, int max_q_len, int H, int R, int P,
                                          int page_size, float scale, float* o_part, float* ml_part,
                                          long long n_pages, const float* inv_freq, float magnitude, int window,
-                                         const float* sink, int skip_from, int* plan, const int* tok_entry, int want_shares,
+                                         const float* sink, int skip_from, int* plan, int want_shares,
                                          cudaStream_t stream) {
   const bool wide = prompt_mode() != 1;
   if (n_entries <= 0 || max_q_len <= 0) return 0;
@@ -691,7 +758,7 @@ BSPEC_API int bspec_latent_attention_mma(const void* ql, long long ql_row, long 
   if ((long long)max_q_len * H > 2147483647ll || n_entries > 65535) return (int)cudaErrorInvalidConfiguration;
   dim3 grid((unsigned)row_tiles, n_entries, 1);
   if (plan != nullptr) {
-    if (want_shares < 1 || want_shares + n_entries > 65535 || !o_part || !ml_part || tok_entry == nullptr) return (int)cudaErrorInvalidValue;
+    if (want_shares < 1 || want_shares + n_entries > 65535 || !o_part || !ml_part) return (int)cudaErrorInvalidValue;
     grid = dim3((unsigned)row_tiles, 1, want_shares + n_entries);
   }
   const bool one_stage = small_pair || (BM < 64 && decode_stages() == 1);
@@ -743,8 +810,11 @@ BSPEC_API int bspec_latent_attention_mma(const void* ql, long long ql_row, long 
 #undef LM
   int err = BSPEC_LAUNCH_CHECK();
   if (err != 0 || plan == nullptr) return err;
-  BSPEC_LAUNCH((latent_attn_join_kernel), (unsigned)((long long)n_tokens * H), R >= 256 ? 128 : 64, 0, stream, o_part,
-               ml_part, (__nv_bfloat16*)out, o_row, o_head, H, R, (const int*)plan, tok_entry, qo_indptr, max_q_len * H, skip_from);
+  const long long rows = (long long)n_tokens * H, fit = 16ll * bspec::sm_count();
+  if (rows > 2147483647ll) return (int)cudaErrorInvalidConfiguration;
+  const int per_block = rows <= fit ? 1 : 4;
+  BSPEC_LAUNCH((latent_attn_join_kernel), (unsigned)min((rows + per_block - 1) / per_block, fit), 128, 0, stream, o_part, ml_part,
+               (__nv_bfloat16*)out, o_row, o_head, H, R, (const int*)plan, max_q_len * H, (int)rows, per_block);
   return BSPEC_LAUNCH_CHECK();
 }
 

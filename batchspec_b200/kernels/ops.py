@@ -120,7 +120,7 @@ _SIGNATURES = {
     "bspec_latent_attention_mma": [c_void_p, c_longlong, c_longlong, c_void_p, c_longlong, c_longlong, c_void_p,
                                    c_longlong, c_longlong, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int,
                                    c_int, c_int, c_int, c_int, c_int, c_float, c_void_p, c_void_p, c_longlong,
-                                   c_void_p, c_float, c_int, c_void_p, c_int, c_void_p, c_void_p, c_int, c_void_p],
+                                   c_void_p, c_float, c_int, c_void_p, c_int, c_void_p, c_int, c_void_p],
     "bspec_latent_prompt_supported": [c_int, c_int, c_int, c_int],
     "bspec_latent_gather": [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int,
                             c_void_p, c_void_p, c_void_p, c_longlong, c_void_p],
@@ -1510,8 +1510,8 @@ def latent_attention(q_lat: torch.Tensor, q_rot: torch.Tensor, out: torch.Tensor
     lib = load_library()
     if (q_lat.dtype == torch.bfloat16 and not FORCE_GENERIC_LATENT and latent_mma_supported(kv_rank, rot_dim)
             and out.stride(2) == 1 and out.stride(1) % 2 == 0 and out.stride(0) % 2 == 0 and out.data_ptr() % 4 == 0):
-        # Few rows and many entries (decode): the requests' key tiles are dealt out in even shares, about as many as CTAs fit
-        # the device at once.  The count depends on the step's shape alone (entries, longest portion), so a captured step
+        # Few rows and many entries (decode): the requests' key tiles are dealt out in even shares, as many as CTAs fit the
+        # device at once.  The count depends on the step's shape alone (entries, longest portion), so a captured step
         # keeps it; the kernel makes the shares from the lengths on the device, and CTAs without one leave at once.
         rows = lib.bspec_latent_attention_mma_rows(max_q_len, n_heads, kv_rank, rot_dim)       # rows of a CTA's tile
         row_tiles = -(-(max_q_len * n_heads) // rows)
@@ -1519,13 +1519,13 @@ def latent_attention(q_lat: torch.Tensor, q_rot: torch.Tensor, out: torch.Tensor
         o_part = ml_part = None
         if max_q_len * n_heads <= 256:
             smem = lib.bspec_latent_attention_mma_smem(rows, kv_rank, rot_dim, 0) + 1024
-            slots = sm_count(q_lat.device) * max(1, min(4, (227 * 1024) // smem))
-            # rounding gives the requests half a share each beyond their part
-            shares = max(slots // row_tiles - ctx.n_entries // 2, slots // (2 * row_tiles), 1)
+            # (the registers of a block, 128 or 256 threads, let four or two share an SM)
+            slots = sm_count(q_lat.device) * max(1, min(4 if rows == 16 else 2, (227 * 1024) // smem))
+            shares = max(slots // row_tiles, 1)
             part_rows = (shares + ctx.n_entries) * max_q_len * n_heads
             keys = min(ctx.max_kv_len, window + max_q_len) if window > 0 else ctx.max_kv_len
             if keys > 256 and part_rows * kv_rank <= LATENT_PART_FLOATS:
-                plan = torch.empty((2 * ctx.n_entries,), dtype=torch.int32, device=q_lat.device)
+                plan = (torch.empty if others is None else torch.zeros)((2 * n,), dtype=torch.int32, device=q_lat.device)
                 o_part = torch.empty((part_rows * kv_rank,), dtype=torch.float32, device=q_lat.device)
                 ml_part = torch.empty((part_rows * 2,), dtype=torch.float32, device=q_lat.device)
         _check(lib.bspec_latent_attention_mma(
@@ -1535,8 +1535,7 @@ def latent_attention(q_lat: torch.Tensor, q_rot: torch.Tensor, out: torch.Tensor
             max_q_len, n_heads, kv_rank, rot_dim, tables.page_size, float(scale), _ptr(o_part),
             _ptr(ml_part), cache.shape[0], rotate[0].data_ptr() if rotate else None,
             float(rotate[1]) if rotate else 1.0, int(window), _ptr(sink),
-            others.at_least if others is not None else 2 ** 31 - 1, _ptr(plan),
-            ctx.tok_entry.data_ptr() if plan is not None else None, shares, _stream()), "latent_attention_mma")
+            others.at_least if others is not None else 2 ** 31 - 1, _ptr(plan), shares, _stream()), "latent_attention_mma")
         if plan is not None:
             count_launches(1)
         return

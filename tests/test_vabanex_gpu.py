@@ -187,7 +187,7 @@ def test_yarn_frequencies_and_rotation_of_strided_heads(ops):
         assert (q[:, :, wide - 16:].double().cpu() - want).abs().max() <= (1e-5 if dtype == torch.float32 else 2e-2)
 
 
-def _latent_case(ops, dtype, H_, R, Pd, ps, q_lens, kv_lens, spike=None, seed=0, generic=False):
+def _latent_case(ops, dtype, H_, R, Pd, ps, q_lens, kv_lens, spike=None, seed=0, generic=False, others=None):
     """Random queries and entries, pages in scrambled order; returns (got, want) [n, H, R]."""
     g = torch.Generator(device=DEV).manual_seed(seed)
     n = sum(q_lens)
@@ -224,7 +224,7 @@ def _latent_case(ops, dtype, H_, R, Pd, ps, q_lens, kv_lens, spike=None, seed=0,
     scale = 0.5 / math.sqrt(R + Pd)
     ops.FORCE_GENERIC_LATENT = generic
     try:
-        ops.latent_attention(ql, qr, out, cache, ctx, tables, H_, R, Pd, scale)
+        ops.latent_attention(ql, qr, out, cache, ctx, tables, H_, R, Pd, scale, others=others)
         torch.cuda.synchronize()
         ops.check_status()
     finally:
@@ -313,12 +313,28 @@ def test_latent_attention_rotates_the_queries_on_the_way(ops, dtype, generic):
     (16, 64, 16, [1] * 140, [1 + 37 * i % 400 for i in range(139)] + [2500]),       # more requests than threads, one far longer
     (3, 96, 16, [2, 1, 3, 1], [1700, 1, 300, 33]),                                   # rows of a portion in one share
     (24, 64, 32, [1, 4, 2], [5000, 700, 2]),                                         # several row tiles, as many shares as there are
+    (16, 64, 16, [1] * 40, [257] * 40),                                              # one length: shares that all fit at once
+    (16, 64, 16, [1] * 560, [1 + 7 * i % 60 for i in range(559)] + [900]),           # more requests than a block looks at at once
+    (40, 64, 16, [1] * 250, [40] * 248 + [700, 300]),                                # more requests than CTAs: nearly all in one share
 ])
 def test_decoded_tokens_are_dealt_in_even_shares(ops, heads, R, Pd, q_lens, kv_lens):
     """Against the plain attention (as test_latent_attention) where requests of very different lengths share the CTAs."""
     got, want = _latent_case(ops, torch.bfloat16, heads, R, Pd, 16, q_lens, kv_lens)
     assert not torch.isnan(got).any()
     assert (got - want).abs().max() <= 2.5e-2
+
+
+@pytest.mark.parametrize("heads,q_lens,kv_lens", [
+    (3, [1, 70, 2, 64, 1], [300, 400, 33, 64, 700]),              # shares of decoded tokens beside two long portions
+    (16, [1, 64, 1], [600, 64, 20]), (16, [63, 200, 5], [90, 333, 400]),     # ... and portions that go in one piece
+])
+def test_portions_of_another_kernel_are_left_alone(ops, heads, q_lens, kv_lens):
+    """Portions of 64 tokens and more beside others: their rows are not written, the others' are as ever."""
+    others = ops.LongPortions(64, 0, max(q_lens), max(x for x in q_lens if x < 64))
+    got, want = _latent_case(ops, torch.bfloat16, heads, 64, 16, 16, q_lens, kv_lens, others=others)
+    long = torch.cat([torch.full((x,), x >= 64) for x in q_lens]).to(DEV)
+    assert torch.isnan(got[long]).all() and not torch.isnan(got[~long]).any()
+    assert (got - want)[~long].abs().max() <= 2.5e-2
 
 
 LONG_PORTIONS = [
