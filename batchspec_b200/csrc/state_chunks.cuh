@@ -9,7 +9,7 @@
 namespace bspec {
 
 constexpr int CH = 64, CH_W = 128, CH_LD = CH_W + 4, CH_AT = CH + 4, CH_SL = 32, CH_THREADS = 256;     // tokens; numbers of a head at most
-constexpr int CH_FROM = 512;                         // tokens of a step's longest portion from which its long ones go by chunks
+constexpr int CH_FROM = 512;                         // no chunks in steps whose longest portion is shorter
 
 // Where chunk i of entry e has its scratch (times heads): chunks of different entries never meet.
 __host__ __device__ __forceinline__ size_t chunk_slot(int q_begin, int e, int i) { return (size_t)(q_begin / CH + e + i); }

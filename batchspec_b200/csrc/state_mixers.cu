@@ -483,32 +483,42 @@ lightning_chunk_sums_kernel(const float* __restrict__ proj, long long ld, int k_
   }
 }
 
-// A thread takes one number of one head's S through the chunks of a portion, eight chunks' sums asked for at a time.
+// A thread takes four numbers of one head's S through the chunks of a portion, eight chunks' sums asked for at a time; the blocks go
+// over the requests, of which at most n / ST_FROM have chunks.  (One number per thread and blocks for every request: beside 31
+// decoded requests of 64 heads 131,000 blocks: a step of 512 tokens and those 363 us, and 226 now.)
 __global__ void __launch_bounds__(256)
 lightning_chunk_scan_kernel(float* __restrict__ sums, const float* __restrict__ decay, float* __restrict__ state, long long state_stride,
-                            const int* __restrict__ qo_indptr, const int* __restrict__ state_slots, int H, int numbers) {
+                            const int* __restrict__ qo_indptr, const int* __restrict__ state_slots, int n_entries, int H, int numbers,
+                            int vec) {
   bspec::pdl_prologue(65);
-  const int e = blockIdx.z, h = blockIdx.y, x = blockIdx.x * 256 + threadIdx.x;
-  const int q_begin = qo_indptr[e], n = qo_indptr[e + 1] - q_begin;
-  if (n < ST_FROM || x >= numbers) return;
-  const int chunks = (n + CH - 1) / CH, last = n - (chunks - 1) * CH;
-  const float d = decay[h], whole = power_of(d, CH), rest = power_of(d, last);
-  float* sp = state + (size_t)state_slots[e] * state_stride + (size_t)h * numbers + x;
-  float* up = sums + (chunk_slot(q_begin, e, 0) * H + h) * numbers + x;
+  const int h = blockIdx.y, x = 4 * (blockIdx.x * 256 + threadIdx.x);
+  if (x >= numbers) return;
+  const float d = decay[h], whole = power_of(d, CH);
   const size_t step = (size_t)H * numbers;
-  float s = *sp;
-  for (int c0 = 0; c0 < chunks; c0 += 8) {
-    float u[8];
+  for (int e = blockIdx.z; e < n_entries; e += gridDim.z) {
+    const int q_begin = qo_indptr[e], n = qo_indptr[e + 1] - q_begin;
+    if (n < ST_FROM) continue;
+    const int chunks = (n + CH - 1) / CH;
+    const float rest = power_of(d, n - (chunks - 1) * CH);
+    float* sp = state + (size_t)state_slots[e] * state_stride + (size_t)h * numbers + x;
+    float* up = sums + (chunk_slot(q_begin, e, 0) * H + h) * numbers + x;
+    float4 s = vec ? *reinterpret_cast<const float4*>(sp) : make_float4(sp[0], sp[1], sp[2], sp[3]);
+    for (int c0 = 0; c0 < chunks; c0 += 8) {
+      float4 u[8];
 #pragma unroll
-    for (int c = 0; c < 8; ++c) u[c] = c0 + c < chunks ? up[(c0 + c) * step] : 0.f;
+      for (int c = 0; c < 8; ++c)
+        u[c] = c0 + c < chunks ? *reinterpret_cast<const float4*>(up + (c0 + c) * step) : make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-    for (int c = 0; c < 8; ++c)
-      if (c0 + c < chunks) {
-        up[(c0 + c) * step] = s;
-        s = fmaf(c0 + c == chunks - 1 ? rest : whole, s, u[c]);
-      }
+      for (int c = 0; c < 8; ++c)
+        if (c0 + c < chunks) {
+          *reinterpret_cast<float4*>(up + (c0 + c) * step) = s;
+          const float f = c0 + c == chunks - 1 ? rest : whole;
+          s = make_float4(fmaf(f, s.x, u[c].x), fmaf(f, s.y, u[c].y), fmaf(f, s.z, u[c].z), fmaf(f, s.w, u[c].w));
+        }
+    }
+    if (vec) *reinterpret_cast<float4*>(sp) = s;
+    else sp[0] = s.x, sp[1] = s.y, sp[2] = s.z, sp[3] = s.w;
   }
-  *sp = s;
 }
 
 // Block: one chunk and head, 64 tokens x 128 value columns.  First the chunk's own q . k (thread (tx, ty): tokens ty + 16 a
@@ -887,8 +897,16 @@ scan_segments_kernel(const float* __restrict__ xz, long long ld, const float* __
 }  // namespace
 
 // How the portions of ST_FROM tokens and more of a step of n tokens in portions of min_q_len to max_q_len go: 0 token by token,
-// 1 by tiles, 2 by chunks.  Chunks where tiles pay and the heads fill most of the 128 x 128 numbers that a chunk's products are
-// laid out for, from a portion's length on at which the chain of tiles is the longer one.
+// 1 by tiles, 2 by chunks.  Chunks where tiles pay, the heads fill most of the 128 x 128 numbers that a chunk's products are
+// laid out for, and an estimate of both says so.  Tiles: the longest portion's chain, slower where an SM holds two heads' blocks, or
+// the work of a full device, to the last of its blocks' rounds.  Chunks: the products of all chunks, partial ones like whole ones,
+// and every further portion's states.  Fitted to 160 steps (1 to 64 heads of 96 to 128, 1 to 101 requests); the choice is at most 3 %
+// slower than tiles, and leaves up to 17 % in a few steps of several portions.  Tiles / chunks, us, heads of 128 x 128:
+//   16 heads: 512 66 / 67; 1,000 124 / 74; 2,048 254 / 144; 2,048 beside 31 decoded 360 / 167; eight of 600 391 / 388; 512 beside twenty
+//   of 64 142 / 178; 2,048 beside twenty of 200 460 / 582; 520 beside a hundred of 70 590 / 1,484
+//   4 heads: 512 63 / 56; 2,048 231 / 73; 512 beside twenty of 64 74 / 73; 520 beside a hundred of 70 163 / 302
+//   64 heads: 512 207 / 143; 2,048 724 / 575; 512 beside four of 300 498 / 558; 512 beside twenty of 64 522 / 953
+//   16 heads of 96 x 96: 512 65 / 81; 1,000 122 / 84; three of 512 98 / 134; 32 of 512 876 / 1,223
 static int lightning_form(int n, int n_entries, int min_q_len, int max_q_len, int H, int dim, int vdim) {
   if (n <= 0 || n_entries <= 0 || H <= 0 || dim <= 0 || vdim <= 0) return 0;
   // (the token loop's time per unit of work falls with the blocks that share the device)
@@ -897,8 +915,16 @@ static int lightning_form(int n, int n_entries, int min_q_len, int max_q_len, in
   const bspec::TokenCost tokens = {dim <= 32 ? 0.165 : (dim <= 64 ? 0.19 : (dim <= 128 ? 0.25 : 0.38)), rate};
   const bspec::TokenCost tiles = {dim <= 128 ? 0.115 : 0.165, dim <= 128 ? 6.0e-4 : 9e-4};
   if (!bspec::tiles_pay(n, n_entries, min_q_len, max_q_len, H, dim, vdim, tokens, tiles)) return 0;
-  const bool fits = chunk_sizes(dim, vdim) && chunk_slots(n, n_entries) * H * dim * vdim <= CH_SCRATCH;
-  return fits && max_q_len >= CH_FROM ? 2 : 1;
+  if (max_q_len < CH_FROM || !chunk_sizes(dim, vdim) || chunk_slots(n, n_entries) * H * dim * vdim > CH_SCRATCH) return 1;
+  const bspec::Tall t = bspec::tall_portions(n, n_entries, min_q_len, max_q_len);
+  const double per = (double)((vdim + LT_COLS - 1) / LT_COLS) * H, all = per * t.count;        // blocks of a portion, of all
+  const double rounds = all < 4.0 * sms ? (double)(((long long)all + sms - 1) / sms * sms) / all : 1.0;
+  const double by_tiles = max(max_q_len * (all <= sms ? 0.118 : 0.175), t.tokens * per * 5.5e-4 * rounds) +
+                          t.tokens * H * (0.5e-4 + 2e-6 * dim) + 7.5;
+  const double parts = ((max_q_len + CH - 1) / CH + (t.tokens - max_q_len) / CH + 0.5 * (t.count - 1)) * H;
+  const bool whole = dim == CH_W && vdim == CH_W;
+  const double by_chunks = max((whole ? 48.0 : 70.0) + 0.1 * parts, (whole ? 0.27 : 0.31) * parts) + 0.33 * (t.count - 1) * H;
+  return by_chunks < 0.96 * by_tiles ? 2 : 1;
 }
 
 // Floats of scratch: the tiles' coefficients with prepared q and k (as large as the step's q and k columns), or the chunks' sums;
@@ -939,8 +965,9 @@ BSPEC_API int bspec_lightning_recurrence(const float* proj, long long ld, int q_
     const dim3 chunks((unsigned)chunk_slots(n, n_entries), H);
     BSPEC_LAUNCH(lightning_chunk_sums_kernel, chunks, CH_THREADS, CH_SUM_SMEM, stream, proj, ld, k_off, v_off, decay, qo_indptr, n_entries,
                  scratch, H, dim, vdim, act, k_scale, inv_freq, rot, positions, vec);
-    BSPEC_LAUNCH(lightning_chunk_scan_kernel, dim3((dim * vdim + 255) / 256, H, n_entries), 256, 0, stream, scratch, decay, state,
-                 state_stride, qo_indptr, state_slots, H, dim * vdim);
+    BSPEC_LAUNCH(lightning_chunk_scan_kernel, dim3((dim * vdim + 1023) / 1024, H, min(n_entries, n / ST_FROM)), 256, 0, stream, scratch,
+                 decay, state, state_stride, qo_indptr, state_slots, n_entries, H, dim * vdim,
+                 (int)(state_stride % 4 == 0 && ((uintptr_t)state & 15) == 0));
     BSPEC_LAUNCH(lightning_chunk_out_kernel, chunks, CH_THREADS, CH_OUT_SMEM, stream, proj, ld, q_off, k_off, v_off, decay, qo_indptr,
                  n_entries, (const float*)scratch, out, H, dim, vdim, act, k_scale, inv_freq, rot, positions, vec);
     const int err = BSPEC_LAUNCH_CHECK();

@@ -41,6 +41,24 @@ struct TokenCost {
   double chain, rate;
 };
 
+struct Tall {                    // the most portions of ST_FROM tokens and more, the tokens in them, what the others than the longest have beyond ``least`` each
+  long long count;
+  double tokens;
+  long long rest;
+  int least;
+};
+inline Tall tall_portions(int n, int n_entries, int shortest, int longest) {
+  Tall t;
+  t.least = shortest < 1 ? 1 : shortest;
+  const long long spare = (long long)n - longest - (long long)(n_entries - 1) * t.least;
+  t.rest = spare < 0 ? 0 : spare;
+  t.count = 1;
+  if (t.least >= ST_FROM) t.count = n_entries;
+  else t.count += t.rest / (ST_FROM - t.least) < n_entries - 1 ? t.rest / (ST_FROM - t.least) : n_entries - 1;
+  t.tokens = (double)n - (double)(n_entries - t.count) * t.least;
+  return t;
+}
+
 // Whether a step is faster with its long portions by tiles.  Tiles have the shorter chain, 8 tokens in about a microsecond, but
 // one instance for all heads of up to 128 rows, a preparation, and a second kernel for the shorter portions; token loops have
 // instances for 32 and 64 rows.  So both are estimated, as the longer of a chain and the work of a full device.  The constants are
@@ -54,13 +72,10 @@ struct TokenCost {
 // (A step is what the estimate needs; a request's results differ by rounding between the two forms.)
 inline bool tiles_pay(int n, int n_entries, int shortest, int longest, int H, int dim, int vdim, TokenCost tokens, TokenCost tiles) {
   if (longest < ST_FROM) return false;
-  const int least = shortest < 1 ? 1 : shortest;
-  const long long spare = (long long)n - longest - (long long)(n_entries - 1) * least;      // tokens above the others' least
-  const long long rest = spare < 0 ? 0 : spare;
-  long long tall = 1;                                                                       // the most portions that go by tiles
-  if (least >= ST_FROM) tall = n_entries;
-  else tall += rest / (ST_FROM - least) < n_entries - 1 ? rest / (ST_FROM - least) : n_entries - 1;
-  const double tiled = (double)n - (double)(n_entries - tall) * least;                      // tokens in them
+  const Tall t = tall_portions(n, n_entries, shortest, longest);
+  const int least = t.least;
+  const long long rest = t.rest;
+  const double tiled = t.tokens;
   const int rows = dim <= 32 ? 32 : (dim <= 64 ? 64 : (dim <= 128 ? 128 : 256));
   const double token_work = (double)H * rows * vdim * tokens.rate, tile_work = (double)H * ((vdim + 15) / 16) * tiles.rate;
   auto longer = [](double a, double b) { return a > b ? a : b; };

@@ -613,6 +613,17 @@ def test_tiles_rotate_queries_and_keys(ops, dk, rot):
     assert (state - state_want).abs().max() <= 2e-5 * max(1.0, state_want.abs().max().item())
 
 
+@pytest.mark.parametrize("lens,heads,size,chunks", [
+    ([640], 4, 128, True), ([1000], 16, 128, True), ([2048] + [1] * 31, 16, 128, True), ([600] * 8, 16, 128, False),
+    ([512] + [64] * 20, 16, 128, False), ([2048] + [200] * 20, 16, 128, False), ([520] + [70] * 100, 4, 128, False), ([512], 4, 128, True),
+    ([2048] * 8, 4, 128, True), ([512] + [64] * 20, 64, 128, False), ([512], 64, 128, True), ([512], 16, 96, False), ([2048], 16, 96, True),
+    ([512] * 3, 16, 96, False), ([500], 1, 128, False), ([2048], 16, 64, False)])
+def test_portions_go_by_chunks_where_they_measured_faster(ops, lens, heads, size, chunks):
+    """The choice by the step's portions and the heads' sizes: three kernels (and one for portions under 64 tokens) instead of two."""
+    got = ops.load_library().bspec_lightning_launches(sum(lens), len(lens), min(lens), max(lens), heads, size, size)
+    assert got == (3 if chunks else 2) + (min(lens) < 64)
+
+
 @pytest.mark.parametrize("Hh,dk,dv,act,scale,rot", [(2, 128, 128, "silu", 1.0, 0), (3, 100, 96, None, 0.25, 36),
                                                     (1, 96, 128, "silu", 0.5, 0), (4, 128, 75, None, 0.125, 128)])
 def test_lightning_attention_by_chunks(ops, Hh, dk, dv, act, scale, rot):
@@ -620,7 +631,7 @@ def test_lightning_attention_by_chunks(ops, Hh, dk, dv, act, scale, rot):
     by token beside it), states carried between them, against the recurrence in float64: sums of dk products over a memory of
     some hundred tokens, 2e-5 of the largest as in the tests above.  A portion's last token being infinite changes nothing
     before it."""
-    lens = [1, 600, 64, 5, 256, 65, 127]
+    lens = [1, 1000, 64, 5, 256, 65, 127]
     n, E = sum(lens), len(lens)
     gen = torch.Generator(device=DEV).manual_seed(dk + dv)
     ld = 2 * Hh * dk + Hh * dv + 1
@@ -631,7 +642,7 @@ def test_lightning_attention_by_chunks(ops, Hh, dk, dv, act, scale, rot):
     slots, qo = [4, 0, 7, 2, 1, 5, 6], [0] + list(np.cumsum(lens))
     freqs = 10000.0 ** (-torch.arange(rot // 2, dtype=torch.float64) / max(1, rot // 2))
     pos = torch.cat([torch.arange(9, 9 + x) for x in lens])
-    assert ops.load_library().bspec_lightning_launches(n, E, 1, 600, Hh, dk, dv) == 4
+    assert ops.load_library().bspec_lightning_launches(n, E, 1, 1000, Hh, dk, dv) == 4
 
     def run(x):
         state = state0.clone()
