@@ -83,6 +83,20 @@ def test_silu_mul(ops, dtype, n, inter):
     torch.testing.assert_close(out.float(), (gate * torch.sigmoid(gate) * up).to(dtype).float(), **tol(dtype))
 
 
+@pytest.mark.parametrize("n,inter,group", [(2048, 64, 0), (2100, 64, 8), (33000, 4, 4), (9, 16384, 0), (373, 352, 8), (130, 1020, 0)])
+@pytest.mark.parametrize("act", ["silu_mul", "relu_mul", "gelu_tanh_mul"])
+def test_gated_products_of_many_float32_numbers(ops, n, inter, group, act):
+    """Four numbers per thread from 2^17 numbers on, rows narrower and wider than a block: the bits of a few rows alone."""
+    g = torch.Generator(device=DEV).manual_seed(inter)
+    u = torch.randn(n, 2 * inter, device=DEV, generator=g) * 4
+    out, part = torch.full((n, inter), math.nan, device=DEV), torch.empty(7, inter, device=DEV)
+    getattr(ops, act)(u, out, group)
+    for r in (0, (n - 7) // 2, n - 7):
+        getattr(ops, act)(u[r:r + 7], part, group)
+        assert torch.equal(out[r:r + 7], part), r
+    assert not out.isnan().any()
+
+
 @pytest.mark.parametrize("M,N,K", [(1, 5, 3), (7, 130, 96), (64, 64, 16), (65, 1000, 257), (300, 33, 1024)])
 def test_sgemm_is_true_float32(ops, M, N, K):
     g = torch.Generator(device=DEV).manual_seed(4)
