@@ -224,10 +224,11 @@ sgemm_join_kernel(const float* __restrict__ part, float* __restrict__ C, int M, 
 // the kernel when the tokens' 256-byte slices were such copies: 347 us against 20x at 128,256 x 2,048 and 8 tokens).  Rows
 // and slices are padded by 4 floats: a quarter warp's 16-byte loads fall into different banks.  64 consumer threads:
 // rows tid % 8 and tid % 8 + 8, slice tid / 8 of the stage; two rows per thread halve the loads of the tokens' numbers,
-// which bound the kernel at 8 tokens.  Two blocks per SM keep at least 128 KB of W in flight on an SM; where there is a tile per
-// SM or less (``deep``), one block keeps that much.  4 tokens, us, two stages / five: 2,048 x 8,192 24.9 / 21.1, 2,048 x 16,384
+// which bound the kernel at 8 tokens.  Two blocks per SM keep at least 128 KB of W in flight on an SM; where there are
+// fewer tiles than SMs (``deep``), one block keeps that much.  4 tokens, us, two stages / five: 2,048 x 8,192 24.9 / 21.1, 2,048 x 16,384
 // 47.1 / 39.7, 1,024 x 4,096 12.5 / 10.8; 8 tokens, two / four: 2,048 x 8,192 37.5 / 30.4, 2,048 x 2,048 11.9 / 10.5; 1 and 2 tokens,
-// whose rings have three stages, 19.9 / 20.4 and 23.1 / 22.9: not.  (Two more consumer warps, and the tokens' copies by a warp of
+// whose rings have three stages, 19.9 / 20.4 and 23.1 / 22.9: not; a tile on every SM leaves the next kernel's blocks no room
+// beside, 2,368 x 4,096 12.2 / 13.0: not.  (Two more consumer warps, and the tokens' copies by a warp of
 // their own, changed little: 23.1 and 20.6.)
 constexpr int RT = 16, KC = 512, SL = KC / SLICE, LDR = KC + 4, LDX = SLICE + 4, ROW_THREADS = 96;
 
@@ -400,7 +401,7 @@ template <int MT>
 int launch_rows(const float* A, const float* W, float* C, int M, int N, int K, long long lda, long long ldw, long long ldc,
                 long long sa, long long sw, long long sc, int batch, int w_ahead, int* status, cudaStream_t stream) {
   if constexpr (MT >= 4)
-    if ((long long)((N + RT - 1) / RT) * ((M + MT - 1) / MT) * batch <= bspec::sm_count())
+    if ((long long)((N + RT - 1) / RT) * ((M + MT - 1) / MT) * batch < bspec::sm_count())
       return launch_rows_ring<MT, true>(A, W, C, M, N, K, lda, ldw, ldc, sa, sw, sc, batch, w_ahead, status, stream);
   return launch_rows_ring<MT, false>(A, W, C, M, N, K, lda, ldw, ldc, sa, sw, sc, batch, w_ahead, status, stream);
 }
