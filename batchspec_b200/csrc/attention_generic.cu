@@ -300,7 +300,11 @@ attn_generic_kernel(const T* __restrict__ q, long long q_row_stride, T* __restri
 // are there.  128 registers keep two blocks of eight warps on an SM where the 168 of the layout above kept one.  Measured at the 1B
 // sizes in float32 (32 heads of 64 over 8 kv heads, prompts of 61, 207 and 700 tokens): 371 -> 169 us a layer, the pass 22.25 ->
 // 18.95 ms.  Bound by the multiply-adds, the exponentials and the latency of a chunk's two copies: a warp has at most three chunks
-// there.  Decoded tokens keep the layout above: its rows are few, and its next keys come under the values' sum.
+// there.  Other sizes, us, layout above / this one: float32, 24/8 x 128 the same prompts 393 / 255, 64 tokens beside 63 decoded ones of
+// 2,000 keys 877 / 444, 16/4 x 256 861 / 551 and 1,384 / 504; bfloat16, whose values this one has to convert on their way, 32/8 x 64
+// 381 / 204, 24/8 x 128 488 / 415, 12/2 x 80 213 / 160, but 16/4 x 256 1,197 / 1,218 and 8/8 x 256, 16 tokens beside 7 decoded ones,
+// 283 / 296: bfloat16 heads above 128 numbers keep the layout above.  So do decoded tokens: their rows are few, and the next keys
+// come under the values' sum.
 constexpr int LDP = 40;                                     // a row of weights: four rows of a quad lie in different banks
 
 constexpr int attn_tile_smem(int nd, int r) {
@@ -742,7 +746,7 @@ int launch_sizes(int width, int n_entries, int max_rows, int max_q_len, int Hkv,
   if (max_q_len > 1) {
     if (width <= 64) return launch_tiles<T, 2, 16>(n_entries, max_rows, Hkv, stream, args...);
     if (width <= 128) return launch_tiles<T, 4, 16>(n_entries, max_rows, Hkv, stream, args...);
-    return launch_tiles<T, 8, 8>(n_entries, max_rows, Hkv, stream, args...);
+    if constexpr (sizeof(T) == 4) return launch_tiles<T, 8, 8>(n_entries, max_rows, Hkv, stream, args...);
   }
   if (width <= 64) return launch_shape<T, 2, 16>(n_entries, max_rows, Hkv, stream, args...);
   if (width <= 128) return launch_shape<T, 4, 16>(n_entries, max_rows, Hkv, stream, args...);
