@@ -1438,13 +1438,14 @@ def linear(x: torch.Tensor, w: torch.Tensor, out_dtype: Optional[torch.dtype] = 
 
 def linear_batched(x: torch.Tensor, w: torch.Tensor, w_is_parameter: bool = False) -> torch.Tensor:
     """x [B, M, K] (rows and batches may be strided, K dense) times w [B, N, K]^T -> [B, M, N] contiguous: one product
-    per head.  bfloat16 on the vendor library's batched product, float32 on this package's FFMA kernels.
+    per head.  bfloat16 on the vendor library's batched product (``w`` may be a view), float32 on this package's FFMA kernels.
     ``w_is_parameter`` as in ``linear``."""
     _require_cuda(x, w)
     B, M, K = x.shape
     N = w.shape[1]
-    assert w.shape == (B, N, K) and x.dtype == w.dtype and x.stride(2) == 1 and w.is_contiguous()
+    assert w.shape == (B, N, K) and x.dtype == w.dtype and x.stride(2) == 1
     if x.dtype == torch.float32:
+        assert w.is_contiguous()
         out = torch.empty((B, M, N), dtype=torch.float32, device=x.device)
         _sgemm(x, w, out, M, N, K, x.stride(1), K, x.stride(0), N * K, B, w_is_parameter)
         return out
@@ -1551,45 +1552,58 @@ def latent_attention(q_lat: torch.Tensor, q_rot: torch.Tensor, out: torch.Tensor
 
 
 LATENT_PART_FLOATS = 64 << 20      # partial results of steps of few rows, at most
-LATENT_PROMPT_FROM = 64            # tokens of a portion from which keys and values per head are formed
-# ... if one of them sees this many keys, or they have this many (token, key) pairs together: below, a step waits for its launches,
-# of which this form has more.  A portion on four layers of 16 heads, whole step, us, per head / in the latent space: 0 + 512 tokens
-# 1,341 / 1,170, 512 + 256 1,313 / 1,163, 512 + 512 1,347 / 1,432, 2,048 + 64 1,322 / 1,648, 8,192 + 64 1,900 / 4,352
-LATENT_PROMPT_KEYS, LATENT_PROMPT_PAIRS = 1024, 1 << 19
-LATENT_PROMPT_ROWS = 1 << 19       # at most this many rows of keys (600 MB of entries)
-LATENT_PROMPT_BYTES = 512 << 20    # keys and values of as many heads at a time as this holds
+# Tokens of a portion from which keys and values per head are formed, and (token, head) rows from which on: fewer are dealt in shares
+# in the latent space.  The choice follows from the portion's own length, so that neither its context nor its neighbours in the step
+# change its rounding.  Device time of a step of four layers, us, per head / in the latent space: 16 heads 0 + 64 tokens 396 / 396,
+# 0 + 256 459 / 516, 2,048 + 64 632 / 1,277, 0 + 1,024 814 / 1,466; 128 heads 0 + 64 541 / 516, 0 + 256 679 / 1,074; 4 heads, 256 rows,
+# 2,048 + 64 636 / 516; a window of 64 keys 512 + 256 490 / 464, 0 + 2,048 1,156 / 1,439
+LATENT_PROMPT_FROM, LATENT_PROMPT_ROWS = 64, 256
+LATENT_PROMPT_KEYS = 1 << 17       # rows of keys that portions share a gather for (150 MB of entries); a longer one has its own
+LATENT_PROMPT_BYTES = 256 << 20    # keys and values of as many heads at a time as this holds
 
 
 @dataclass
 class LongPortions:
     """The portions of a step that attend over keys and values per head."""
     at_least: int                  # the shortest has this many tokens or more
-    rows: int                      # rows of keys, every portion's rounded up to 64
+    groups: tuple                  # (first request, request behind the last, rows of keys: every portion's rounded up to 64)
     longest: int
     longest_other: int             # 0: the step has no other portions
 
 
-def latent_long_portions(ctx, dtype: torch.dtype, kv_rank: int, dim: int, rot_dim: int, v_dim: int,
-                         window: int = 0, scale: float = 1.0) -> Optional[LongPortions]:
-    """The step's portions of at least ``LATENT_PROMPT_FROM`` tokens, None when there are none or ``latent_prompt`` does not
-    take these sizes or this ``scale`` of the scores (it finds a row's maximum before scaling, so only positive ones).  Needs
-    the lengths on the host: a captured step has none."""
-    host = getattr(ctx, "host", None)
-    if (host is None or ctx.max_q_len < LATENT_PROMPT_FROM or dtype != torch.bfloat16 or FORCE_GENERIC_LATENT or not scale > 0
-            or not latent_mma_supported(kv_rank, rot_dim)
-            or not load_library().bspec_latent_prompt_supported(kv_rank, dim, rot_dim, v_dim)):
+def latent_prompt_takes(dtype: torch.dtype, kv_rank: int, dim: int, rot_dim: int, v_dim: int) -> bool:
+    """Whether ``latent_prompt`` takes heads of these sizes."""
+    return (dtype == torch.bfloat16 and latent_mma_supported(kv_rank, rot_dim)
+            and bool(load_library().bspec_latent_prompt_supported(kv_rank, dim, rot_dim, v_dim)))
+
+
+def latent_long_portions(ctx, dtype: torch.dtype, kv_rank: int, dim: int, rot_dim: int, v_dim: int, window: int = 0,
+                         scale: float = 1.0, n_heads: int = 16) -> Optional[LongPortions]:
+    """The step's portions of at least ``LATENT_PROMPT_FROM`` tokens and more than ``LATENT_PROMPT_ROWS`` rows, None when there
+    are none or ``latent_prompt`` does not take these sizes or this ``scale`` of the scores (it finds a row's maximum before
+    scaling, so only positive ones).  Needs the lengths on the host: a captured step has none."""
+    host, extras = getattr(ctx, "host", None), getattr(ctx, "extras", {})
+    if host is None:
         return None
-    lens = np.diff(host["qo_indptr"]).astype(np.int64)
-    kv = host["kv_len"].astype(np.int64)
-    first = np.maximum(kv - lens - window + 1, 0) // 64 * 64 if window > 0 else np.zeros_like(kv)
-    chosen = lens >= LATENT_PROMPT_FROM
-    spans = (kv - first)[chosen]
-    if int(spans.max()) < LATENT_PROMPT_KEYS and int((lens[chosen] * spans).sum()) < LATENT_PROMPT_PAIRS:
-        return None
-    rows = int(((spans + 63) // 64 * 64).sum())
-    if rows > LATENT_PROMPT_ROWS:
-        return None
-    return LongPortions(LATENT_PROMPT_FROM, rows, int(lens[chosen].max()), int(lens[~chosen].max()) if not chosen.all() else 0)
+    key = ("long portions", dtype, kv_rank, dim, rot_dim, v_dim, window, scale > 0, n_heads, FORCE_GENERIC_LATENT)
+    if key not in extras:                 # the same for every layer of a step
+        extras[key] = None
+        at_least = max(LATENT_PROMPT_FROM, LATENT_PROMPT_ROWS // n_heads + 1)
+        if (ctx.max_q_len >= at_least and scale > 0 and not FORCE_GENERIC_LATENT
+                and latent_prompt_takes(dtype, kv_rank, dim, rot_dim, v_dim)):
+            lens = np.diff(host["qo_indptr"]).tolist()
+            groups, rows, first = [], 0, 0
+            for e, (n, kv) in enumerate(zip(lens, host["kv_len"].tolist())):
+                if n < at_least:
+                    continue
+                span = kv - (max(kv - n - window + 1, 0) // 64 * 64 if window > 0 else 0)
+                if rows and rows + span > LATENT_PROMPT_KEYS:
+                    groups.append((first, e, rows))
+                    rows, first = 0, e
+                rows += (span + 63) // 64 * 64
+            groups.append((first, len(lens), rows))
+            extras[key] = LongPortions(at_least, tuple(groups), max(lens), max((n for n in lens if n < at_least), default=0))
+    return extras[key]
 
 
 def latent_prompt(q: torch.Tensor, w_kv: torch.Tensor, out: torch.Tensor, cache: torch.Tensor, ctx, tables, long: LongPortions,
@@ -1603,23 +1617,25 @@ def latent_prompt(q: torch.Tensor, w_kv: torch.Tensor, out: torch.Tensor, cache:
     assert q.is_contiguous() and w_kv.is_contiguous() and cache.is_contiguous() and out.stride(2) == 1
     assert q.shape[:2] == (n, H) and H == n_heads and w_kv.shape == (H, width, R) and cache.dtype == torch.bfloat16
     assert sink is None or (sink.dtype == torch.float32 and sink.numel() == H and sink.is_contiguous())
-    lib, dev, T = load_library(), q.device, long.rows
-    entries = torch.empty((T, R), dtype=torch.bfloat16, device=dev)
-    rotated = torch.empty((T, q.shape[2] - (width - V)), dtype=torch.bfloat16, device=dev)
-    base = torch.empty((ctx.n_entries,), dtype=torch.int32, device=dev)
-    _check(lib.bspec_latent_gather(cache.data_ptr(), ctx.qo_indptr.data_ptr(), ctx.positions.data_ptr(), tables.kv_indptr.data_ptr(),
-                                   tables.kv_indices.data_ptr(), ctx.n_entries, R, tables.page_size, int(window), long.at_least, T,
-                                   entries.data_ptr(), rotated.data_ptr(), base.data_ptr(), cache.shape[0], _stream()),
-           "latent_gather")
-    step = max(1, min(H, LATENT_PROMPT_BYTES // (T * width * 2)))
-    for h in range(0, H, step):
-        w = w_kv[h:h + step]
-        kv = linear(entries, w.reshape(-1, R), w_is_parameter=True)
-        _check(lib.bspec_latent_prompt(q.data_ptr(), q.stride(0), n, H, kv.data_ptr(), rotated.data_ptr(), base.data_ptr(), T,
-                                       out.data_ptr(), out.stride(1), out.stride(0), ctx.qo_indptr.data_ptr(),
-                                       ctx.positions.data_ptr(), ctx.n_entries, long.longest, h, w.shape[0], int(window),
-                                       long.at_least, float(scale), _ptr(sink), _status_word(dev).data_ptr(), _stream()),
-               "latent_prompt")
+    lib, dev, P = load_library(), q.device, q.shape[2] - (width - V)
+    for first, end, T in long.groups:
+        count, at = end - first, 4 * first
+        # one block: entries [T, R], rotated parts [T, P], the first row of every request
+        block = torch.empty((T * (R + P) + 2 * count,), dtype=torch.bfloat16, device=dev)
+        entries = block[:T * R].view(T, R)
+        rotated = block.data_ptr() + 2 * T * R
+        base, qo = rotated + 2 * T * P, ctx.qo_indptr.data_ptr() + at
+        _check(lib.bspec_latent_gather(cache.data_ptr(), qo, ctx.positions.data_ptr(), tables.kv_indptr.data_ptr() + at,
+                                       tables.kv_indices.data_ptr(), count, R, tables.page_size, int(window), long.at_least, T,
+                                       block.data_ptr(), rotated, base, cache.shape[0], _stream()), "latent_gather")
+        step = max(1, min(H, LATENT_PROMPT_BYTES // (T * width * 2)))
+        for h in range(0, H, step):
+            w = w_kv[h:h + step]
+            kv = linear(entries, w.reshape(-1, R), w_is_parameter=True)
+            _check(lib.bspec_latent_prompt(q.data_ptr(), q.stride(0), n, H, kv.data_ptr(), rotated, base, T, out.data_ptr(),
+                                           out.stride(1), out.stride(0), qo, ctx.positions.data_ptr(), count, long.longest, h,
+                                           w.shape[0], int(window), long.at_least, float(scale), _ptr(sink),
+                                           _status_word(dev).data_ptr(), _stream()), "latent_prompt")
 
 
 def latent_mma_supported(kv_rank: int, rot_dim: int) -> bool:

@@ -12,7 +12,7 @@ Options: ``gated`` False leaves the gate out; ``window`` W keeps the keys i - W 
 window has passed are given back); ``sink``: a learned logit per head that only enlarges the softmax's denominator
 (nothing is attended through it, and ``scale`` does not touch it).
 
-Only [c | rot(kr)] is cached (one tensor per token, ``kv_rank + rot_dim`` numbers).  Decoded tokens and short portions
+Only [c | rot(kr)] is cached (one tensor per token, ``kv_rank + rot_dim`` numbers).  Decoded tokens and portions under 64 tokens
 never form per-head keys and values: since q_h . (Wuk_h c) = (Wuk_h^T q_h) . c, the unrotated query is taken into the latent space
 (one small product per head), attention runs there for all heads over the same entries, and the head's value
 up-projection is applied to its attended latent afterwards.  The step's launch sequence:
@@ -21,8 +21,9 @@ up-projection is applied to its attended latent afterwards.  The step's launch s
     cache append) -> Wuq -> per-head Wuk^T -> latent attention (which rotates the queries' rotated parts as it
     loads them) -> per-head Wuv -> gate and regroup -> Wo
 
-Long portions (``ops.latent_long_portions``) do: [Wuk; Wuv] of the entries that they see in one product, a flash attention
-per head over the result (``ops.latent_prompt``), gate and Wo.
+Portions of 64 tokens and more (``ops.latent_long_portions``, bfloat16, heads of 128 + 64 / 128 numbers) do: [Wuk; Wuv] of the
+entries that they see in one product, a flash attention per head over the result (``ops.latent_prompt``), gate and Wo.  A head's
+keys and values are then rounded to bfloat16 where the queries' and the outputs' latents are otherwise.
 """
 from __future__ import annotations
 
@@ -81,11 +82,15 @@ class LatentAttention(Mixer):
         rows = [params["dq"], params["dkv"]] + ([params["g"]] if self.gated else [])
         self.w_down = torch.cat(rows, dim=0).contiguous()                  # [q_rank + kv_rank + rot_dim (+ H), dim]
         self.w_uq = params["uq"].contiguous()
+        uk, uv = params["uk"].view(H, self.head_dim, self.kv_rank), params["uv"].view(H, self.v_dim, self.kv_rank)
+        self.w_kv = None
+        if uk.is_cuda and ops.latent_prompt_takes(uk.dtype, self.kv_rank, self.head_dim, self.rot_dim, self.v_dim):
+            # per head [Wuk_h; Wuv_h], for portions that form keys and values; the other products read views of it
+            self.w_kv = torch.cat([uk, uv], dim=1)
+            uk, uv = self.w_kv[:, :self.head_dim], self.w_kv[:, self.head_dim:]
         # Wuk_h^T as the [N, K] operand of "x @ w^T": [H, kv_rank, head_dim]
-        self.w_uk_t = params["uk"].view(H, self.head_dim, self.kv_rank).transpose(1, 2).contiguous()
-        self.w_uv = params["uv"].view(H, self.v_dim, self.kv_rank).contiguous()
-        # per head [Wuk_h; Wuv_h], for portions that form keys and values
-        self.w_kv = torch.cat([params["uk"].view(H, self.head_dim, self.kv_rank), self.w_uv], dim=1).contiguous()
+        self.w_uk_t = uk.transpose(1, 2) if self.w_kv is not None else uk.transpose(1, 2).contiguous()
+        self.w_uv = uv if self.w_kv is not None else uv.contiguous()
         self.w_o = params["o"].contiguous()
         self.n_q, self.n_kv = params["dq_norm"], params["dkv_norm"]
         if self.n_kv.dtype != self.n_q.dtype:
@@ -114,7 +119,7 @@ class LatentAttention(Mixer):
         with bucket("attn.q_proj"):
             q = ops.linear(cq, self.w_uq, w_is_parameter=True).view(n, H, dh + P)
         q_rot = q[:, :, dh:]
-        long = ops.latent_long_portions(ctx, x.dtype, R, dh, P, self.v_dim, self.window, self.scale)
+        long = ops.latent_long_portions(ctx, x.dtype, R, dh, P, self.v_dim, self.window, self.scale, H)
         v = None
         if long is not None:
             with bucket("attn.rotate"):

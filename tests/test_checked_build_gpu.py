@@ -145,7 +145,7 @@ latent = torch.empty(64, 1, 128, device=dev, dtype=torch.bfloat16)
 long_ctx = SimpleNamespace(qo_indptr=i32([0, 64]), positions=i32(list(range(64))), n_entries=1, n_tokens=64, max_q_len=64,
                            max_kv_len=64)
 tables = SimpleNamespace(kv_indptr=i32([0, 4]), kv_indices=i32([1, 4, 6, 0]), page_size=ps)
-ops.latent_prompt(q, w_kv, latent.transpose(0, 1), backing[:5], long_ctx, tables, ops.LongPortions(64, 64, 64, 0), 1, R, 0.1)
+ops.latent_prompt(q, w_kv, latent.transpose(0, 1), backing[:5], long_ctx, tables, ops.LongPortions(64, ((0, 1, 64),), 64, 0), 1, R, 0.1)
 torch.cuda.synchronize()
 rep = ops.bounds_reports()
 assert len(rep) == 1 and rep[0][0] == "latent_prompt" and rep[0][1].startswith("page id") and rep[0][2:4] == (6, 5), rep

@@ -330,7 +330,7 @@ def test_decoded_tokens_are_dealt_in_even_shares(ops, heads, R, Pd, q_lens, kv_l
 ])
 def test_portions_of_another_kernel_are_left_alone(ops, heads, q_lens, kv_lens):
     """Portions of 64 tokens and more beside others: their rows are not written, the others' are as ever."""
-    others = ops.LongPortions(64, 0, max(q_lens), max(x for x in q_lens if x < 64))
+    others = ops.LongPortions(64, (), max(q_lens), max(x for x in q_lens if x < 64))
     got, want = _latent_case(ops, torch.bfloat16, heads, 64, 16, 16, q_lens, kv_lens, others=others)
     long = torch.cat([torch.full((x,), x >= 64) for x in q_lens]).to(DEV)
     assert torch.isnan(got[long]).all() and not torch.isnan(got[~long]).any()
@@ -348,14 +348,17 @@ LONG_PORTIONS = [
 ]
 
 
-@pytest.mark.parametrize("q_lens,kv_lens,window,rows", [
-    ([64], [1023], 0, None), ([64], [1024], 0, 1024), ([63], [4096], 0, None), ([512], [512], 0, None), ([700], [900], 0, 960),
-    ([1, 400, 70], [5000, 400, 1500], 0, 448 + 1536), ([300] * 5, [300] * 5, 0, None), ([300] * 6, [300] * 6, 0, 1920), ([100], [5000], 256, None),
-    ([1000], [9000], 600, 1664)])
-def test_which_portions_go_by_keys_and_values_per_head(ops, q_lens, kv_lens, window, rows):
+@pytest.mark.parametrize("q_lens,kv_lens,window,heads,groups", [
+    ([64], [64], 0, 16, [(0, 1, 64)]), ([63], [4096], 0, 16, None), ([700, 1], [900, 50], 0, 16, [(0, 2, 960)]),
+    ([1, 400, 70], [5000, 400, 1500], 0, 16, [(0, 2, 448), (2, 3, 1536)]), ([1000], [9000], 600, 16, [(0, 1, 1664)]),
+    ([64, 65], [2000, 65], 0, 4, [(0, 2, 128)]), ([128], [128], 0, 2, None), ([257], [300], 0, 1, [(0, 1, 320)]),      # more than 256 rows
+    ([64, 1, 64, 64], [1000, 7, 2000, 100], 0, 16, [(0, 2, 1024), (2, 3, 2048), (3, 4, 128)]),                           # at most 1,500 keys together
+    ([64] * 3, [200, 1000, 640], 0, 16, [(0, 2, 1280), (2, 3, 640)])])
+def test_which_portions_go_by_keys_and_values_per_head(ops, q_lens, kv_lens, window, heads, groups, monkeypatch):
+    monkeypatch.setattr(ops, "LATENT_PROMPT_KEYS", 1500)
     ctx = SimpleNamespace(max_q_len=max(q_lens), host=dict(qo_indptr=np.concatenate([[0], np.cumsum(q_lens)]), kv_len=np.asarray(kv_lens)))
-    long = ops.latent_long_portions(ctx, torch.bfloat16, 512, 128, 64, 128, window)
-    assert (long.rows if long is not None else None) == rows
+    long = ops.latent_long_portions(ctx, torch.bfloat16, 512, 128, 64, 128, window, 0.1, heads)
+    assert (list(long.groups) if long is not None else None) == groups
 
 
 @pytest.mark.parametrize("heads,R,ps,q_lens,kv_lens,window,sinks,group", LONG_PORTIONS)
@@ -389,24 +392,29 @@ def test_long_portions_over_keys_and_values_per_head(ops, heads, R, ps, q_lens, 
     tables = SimpleNamespace(kv_indptr=torch.tensor(indptr, dtype=torch.int32, device=DEV),
                              kv_indices=table.to(DEV, torch.int32), page_size=ps)
     monkeypatch.setattr(ops, "latent_mma_supported", lambda *a: True)
-    monkeypatch.setattr(ops, "LATENT_PROMPT_KEYS", 0)                 # (these portions are small)
+    monkeypatch.setattr(ops, "LATENT_PROMPT_KEYS", 1000)              # (several of them share no gather)
     long = ops.latent_long_portions(ctx, torch.bfloat16, R, dk, P_, V, window)
     assert long.longest_other == max([x for x in q_lens if x < 64], default=0)
-    monkeypatch.setattr(ops, "LATENT_PROMPT_BYTES", group * long.rows * (dk + V) * 2)
+    total = sum(rows for _, _, rows in long.groups)
+    monkeypatch.setattr(ops, "LATENT_PROMPT_BYTES", group * max(rows for _, _, rows in long.groups) * (dk + V) * 2)
     out = torch.full((n, heads, V), 7.0, device=DEV, dtype=torch.bfloat16).transpose(0, 1)
     scale = 0.1
     ops.latent_prompt(q, w, out, cache, ctx, tables, long, heads, R, scale, window=window, sink=sink)
     ops.check_status()
     # the same rows of entries through the same products: keys and values of the same bits
     firsts = [low // 64 * 64 for low in lows]
-    rows_in, at, r0 = torch.zeros(long.rows, R, device=DEV, dtype=torch.bfloat16), {}, 0
+    rows_in, at, r0 = torch.zeros(total, R, device=DEV, dtype=torch.bfloat16), {}, 0
     for e, (x, L) in enumerate(zip(q_lens, kv_lens)):
         if x >= 64:
             rows_in[r0 + lows[e] - firsts[e]:r0 + L - firsts[e]] = ents[e][lows[e]:, :R]
             at[e] = r0
             r0 += -(-(L - firsts[e]) // 64) * 64
-    assert r0 == long.rows
-    kv_all = torch.cat([ops.linear(rows_in, w[h:h + group].reshape(-1, R)) for h in range(0, heads, group)], 1)
+    assert r0 == total
+    kv_all = []
+    for rows in rows_in.split([rows for _, _, rows in long.groups]):
+        step = max(1, min(heads, ops.LATENT_PROMPT_BYTES // (rows.shape[0] * (dk + V) * 2)))
+        kv_all.append(torch.cat([ops.linear(rows, w[h:h + step].reshape(-1, R)) for h in range(0, heads, step)], 1))
+    kv_all = torch.cat(kv_all)
     for e, (x, L) in enumerate(zip(q_lens, kv_lens)):
         rows = slice(int(qo[e]), int(qo[e + 1]))
         if x < 64:
@@ -426,16 +434,24 @@ def test_long_portions_over_keys_and_values_per_head(ops, heads, R, ps, q_lens, 
         assert bool(((out[:, rows].double() - want).abs() <= 2.0 ** -8 * want.abs() + 2.0 ** -13 * most + 1e-30).all()), e
 
 
-def test_an_engine_step_of_long_and_short_portions_gives_what_short_ones_give(ops):
-    """The same prompts whole, in portions that are partly short, and beside a decoding request, at the head sizes that form
-    keys and values: the logits agree as two roundings of one model do."""
+def test_an_engine_step_of_long_and_short_portions_gives_what_short_ones_give(ops, monkeypatch):
+    """The same prompts whole, in portions that are all short or partly, and beside a request that decodes, at the head sizes that
+    form keys and values: the logits agree as two roundings of one model do."""
     from batchspec_b200.config import config_from_json_dict
     from batchspec_b200.engine import Engine, StepEntry
     mix = _mixer(4, 128, 64, 128, 96, 64, 0.08, 10000.0, None)
     cfg = dict(CFG_A, layers=[dict(type="latent_attention", mixer=mix, mlp=dict(kind="dense", ff=80, limit=0.7))] * 2)
     prompts = [H.random_tokens(n, cfg["vocab"], 50 + n) for n in (300, 150, 20)]
+    calls, prompt, attention = [], ops.latent_prompt, ops.latent_attention
+    monkeypatch.setattr(ops, "latent_prompt", lambda *a, **k: (calls.append(("long", a[6].longest)), prompt(*a, **k)))
+    monkeypatch.setattr(ops, "latent_attention", lambda *a, **k: (calls.append(("other", k["others"] and k["others"].longest_other)),
+                                                                  attention(*a, **k)))
     got = []
-    for cuts in ((300, 150, 20), (40, 40, 20), (170, 63, 3)):
+    for cuts, want in ((([300], [150], [20]), [("other", 20), ("long", 300)]),
+                       (([40] * 8, [40] * 4, [20]), [("other", None)]),
+                       (([170, 130], [63] * 3, [3] * 7), [("other", 63), ("long", 170), ("long", 130)]),
+                       (([170, 130], [149, 1], [20]), [("other", 20), ("long", 170), ("other", 1), ("long", 130)])):
+        calls.clear()
         eng = Engine(dtype="bfloat16", device=DEV)
         eng.load_model(config=config_from_json_dict(cfg), random_seed=3, draw_on_device=True)
         eng.setup_caches(max_batch_size=3, max_seq_length=512, page_size=16, prefill_chunk_size=512)
@@ -443,12 +459,13 @@ def test_an_engine_step_of_long_and_short_portions_gives_what_short_ones_give(op
         for r in range(3):
             eng.admit(r)
         done, last = [0, 0, 0], {}
-        while any(d < len(p) for d, p in zip(done, prompts)):
-            step = [(r, done[r], min(cuts[r], len(p) - done[r])) for r, p in enumerate(prompts) if done[r] < len(p)]
+        for i in range(max(len(c) for c in cuts)):
+            step = [(r, done[r], min(c[i], len(prompts[r]) - done[r])) for r, c in enumerate(cuts) if i < len(c)]
             out = eng.step([StepEntry(r, prompts[r][a:a + c], want=(c - 1,)) for r, a, c in step])
             for (r, a, c), row in zip(step, out):
                 done[r] += c
                 last[r] = row.float().clone()
+        assert done == [300, 150, 20] and set(want) <= set(calls) and (any(c[0] == "long" for c in calls) == any(c[0] == "long" for c in want))
         got.append(torch.stack([last[r] for r in range(3)]))
     for other in got[1:]:
         assert (got[0] - other).norm() <= 0.03 * got[0].norm()
