@@ -28,8 +28,7 @@
 // tokens that stay visible when the window has passed them are such a source too, in the tokens' own pages.
 // With a distance bias an item walks its key tiles from the last to the first: the bias grows towards the query, by tens
 // of units a tile for the steep heads, so in ascending order nearly every tile would move the maximum and rescale O.
-#include "common.cuh"
-#include "tma.cuh"
+#include "umma.cuh"
 #include <math.h>
 using namespace bspec;
 
@@ -46,105 +45,6 @@ constexpr int SUBQ = ROWS * 64;      // elements of a [128][64] sub-tile (16 KB)
 constexpr int SUBK = KT * 64;        // elements of a [64][64] sub-tile (8 KB): K and V halves
 constexpr int QTILE = 2 * SUBQ;      // [128][128] Q tile
 constexpr int KTILE = 2 * SUBK;      // [64][128] K (or V) tile
-
-__device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tc_commit(uint64_t* bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(s32(bar)) : "memory");
-}
-__device__ __forceinline__ void tc_mma(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accum) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-      ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accum) : "memory");
-}
-// the A operand read from tensor memory (rows on the lanes, two bfloat16 per 32-bit column)
-__device__ __forceinline__ void tc_mma_a_tmem(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc, uint32_t accum) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
-      ::"r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accum) : "memory");
-}
-__device__ __forceinline__ void tc_ld32(uint32_t taddr, uint32_t (&v)[32]) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-      "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
-      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]),
-        "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]), "=r"(v[16]),
-        "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]), "=r"(v[24]),
-        "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
-      : "r"(taddr) : "memory");
-}
-__device__ __forceinline__ void tc_st32(uint32_t taddr, const uint32_t (&v)[32]) {
-  asm volatile(
-      "tcgen05.st.sync.aligned.32x32b.x32.b32 [%32], "
-      "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31};"
-      ::"r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]), "r"(v[9]),
-        "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15]), "r"(v[16]), "r"(v[17]), "r"(v[18]),
-        "r"(v[19]), "r"(v[20]), "r"(v[21]), "r"(v[22]), "r"(v[23]), "r"(v[24]), "r"(v[25]), "r"(v[26]), "r"(v[27]),
-        "r"(v[28]), "r"(v[29]), "r"(v[30]), "r"(v[31]), "r"(taddr)
-      : "memory");
-}
-__device__ __forceinline__ void tc_st16(uint32_t taddr, const uint32_t* v) {
-  asm volatile(
-      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%16], "
-      "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15};"
-      ::"r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]), "r"(v[9]),
-        "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15]), "r"(taddr)
-      : "memory");
-}
-__device__ __forceinline__ void tc_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
-__device__ __forceinline__ void tc_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
-__device__ __forceinline__ float ex2(float x) {          // 2^x on the special-function unit; 2^-inf = 0
-  float y;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
-}
-// Two float32 operations per instruction (sm_100 has packed forms of add, mul and fma) and a maximum of three:
-// the softmax is bound by the number of instructions it issues, not by the arithmetic pipes.
-__device__ __forceinline__ uint64_t pack2(float a, float b) {
-  uint64_t r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
-  return r;
-}
-__device__ __forceinline__ void unpack2(uint64_t v, float& a, float& b) {
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
-}
-__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
-  uint64_t d;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-  return d;
-}
-__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
-  uint64_t d;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-  return d;
-}
-__device__ __forceinline__ float max3(float a, float b, float c) {
-  float d;
-  asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
-  return d;
-}
-__device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
-
-// K-major operand tile: rows of 128 bytes, 128-byte swizzle, 8-row groups 1024 bytes apart.
-__device__ __forceinline__ uint64_t desc_kmajor(const void* tile) {
-  const uint64_t addr = (uint64_t)((s32(tile) & 0x3FFFFu) >> 4);
-  return addr | (1ull << 16) | (64ull << 32) | (1ull << 46) | (2ull << 61);
-}
-// MN-major operand (V: rows = keys = K dimension, 64 contiguous head dims per 128-byte row): the next block of 64
-// head dims is one sub-tile (8 KB) further, 8-key groups are 1024 bytes apart.
-__device__ __forceinline__ uint64_t desc_mnmajor(const void* tile) {
-  const uint64_t addr = (uint64_t)((s32(tile) & 0x3FFFFu) >> 4);
-  return addr | ((uint64_t)((SUBK * 2) >> 4) << 16) | (64ull << 32) | (1ull << 46) | (2ull << 61);
-}
-// float32 accumulator, bfloat16 operands, M = 128, N = n; b_mn: B operand is MN-major.
-__device__ __forceinline__ uint32_t idesc(int n, bool b_mn) {
-  return (1u << 4) | (1u << 7) | (1u << 10) | (b_mn ? (1u << 16) : 0u) | ((uint32_t)(n >> 3) << 17) |
-         ((uint32_t)(128 >> 4) << 24);
-}
 
 struct Geom {
   int q_begin, q_len, pos0, G, rows_total;
@@ -418,8 +318,8 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap kv_map, const __grid_
     // Q tile now has its own issuing thread (in different warps); the tensor core takes from both.
     const int tt = warp == 1 ? 0 : 1;
     if (lane == 0) {
-      const uint32_t id_s = idesc(KT, false), id_o = idesc(HD, true);
-      const uint64_t qdesc = desc_kmajor(Qs + tt * QTILE);
+      const uint32_t id_s = instr_desc(KT), id_o = instr_desc(HD, true);
+      const uint64_t qdesc = smem_desc(Qs + tt * QTILE);
       uint32_t kv_base = 0;      // key tiles of the items before this one (all of them pass through the ring)
       uint32_t sq = 0;           // key tiles of this Q tile before this item: the S buffers (and P in them) alternate with it
       uint32_t n_mine = 0;       // items before this one in which this Q tile had rows
@@ -437,7 +337,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap kv_map, const __grid_
           // announced P of that tile, and this thread has seen that announcement (it issued that tile's P V,
           // also across the end of an item): no wait here.
           tc_fence_after();
-          const uint64_t kdesc = desc_kmajor(KV + (size_t)st * 2 * KTILE);
+          const uint64_t kdesc = smem_desc(KV + (size_t)st * 2 * KTILE);
           const uint32_t d = tmem + (uint32_t)(tt * 128) + bf * 64u;
 #pragma unroll
           for (int ks = 0; ks < HD / 16; ++ks) {
@@ -473,7 +373,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap kv_map, const __grid_
           }
           tc_fence_after();
           const uint32_t p_tmem = tmem + (uint32_t)(tt * 128) + bf * 64u;     // P: the first 32 columns of its S buffer
-          const uint64_t vdesc = desc_mnmajor(KV + (size_t)st * 2 * KTILE + KTILE);
+          const uint64_t vdesc = desc_mnmajor(KV + (size_t)st * 2 * KTILE + KTILE, 2 * SUBK);
           const uint32_t d = tmem + (uint32_t)(256 + tt * 128);
 #pragma unroll
           for (int kk = 0; kk < KT / 16; ++kk)          // 16 keys: 8 columns of P, 16 rows of V

@@ -131,6 +131,17 @@ __device__ __forceinline__ bool in_range(long long v, long long n, int code) {
 #else
 __device__ __forceinline__ bool in_range(long long, long long, int) { return true; }
 #endif
+// Pairs of float32 numbers in 64 bits, for packed multiply-adds.
+__device__ __forceinline__ unsigned long long pair_of(float a, float b) {
+  unsigned long long r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ void halves_of(unsigned long long v, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
+__device__ __forceinline__ void fma_pair(unsigned long long& acc, unsigned long long a, unsigned long long b) {
+  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b));
+}
+
 __device__ __forceinline__ void pdl_prologue(int kid = 0) {
   const unsigned long long t0 = g_trace_buf != nullptr ? global_timer() : 0ull;
   pdl_launch_dependents();

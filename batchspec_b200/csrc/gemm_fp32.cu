@@ -21,13 +21,10 @@ namespace {
 
 constexpr int SLICE = 64, GROUP = 1024;
 
-__device__ __forceinline__ void fma2(unsigned long long& acc, unsigned long long a, unsigned long long b) {
-  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b));
-}
 // the slice's value: its even chain plus its odd chain
 __device__ __forceinline__ float fold2(unsigned long long acc) {
   float lo, hi;
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(acc));
+  halves_of(acc, lo, hi);
   return lo + hi;
 }
 
@@ -149,9 +146,9 @@ sgemm_tile_kernel(const float* __restrict__ A, const float* __restrict__ W, floa
       for (int i = 0; i < TI; ++i) {
         const ulonglong2 a = *reinterpret_cast<const ulonglong2*>(a_ + RM * i * LDT + k);
 #pragma unroll
-        for (int j = 0; j < TJ; ++j) fma2(acc[i][j], a.x, b[j].x);
+        for (int j = 0; j < TJ; ++j) fma_pair(acc[i][j], a.x, b[j].x);
 #pragma unroll
-        for (int j = 0; j < TJ; ++j) fma2(acc[i][j], a.y, b[j].y);
+        for (int j = 0; j < TJ; ++j) fma_pair(acc[i][j], a.y, b[j].y);
       }
     }
     const int done = (t + 1) * BK;

@@ -4,7 +4,10 @@
 // dim + rot_dim + 2 vdim = 448 multiply-adds (the weights enter the product with the values as two bfloat16 numbers, the
 // rounded weight and the rounding's remainder) where attention in the latent space takes rank + rot_dim + 2 rank = 1,600,
 // and a head's accumulator fits tensor memory twice.  The products per entry cost what the queries' way into the latent
-// space and the outputs' way out of it cost per token otherwise, so it pays as soon as a portion has some tens of tokens.
+// space and the outputs' way out of it cost per token otherwise, so it pays as soon as a portion has some tens of tokens
+// (a step of four layers of 16 heads, latent 512, us, here / in the latent space: 64 tokens 396 / 396, 256 459 / 516, 1,024
+// 814 / 1,466; 64 after 2,048 632 / 1,277).  Keys and values per head are rounded to bfloat16 here, the queries' and outputs' latents
+// there; both are as far from 64 bits.  Heads of 128 + 64 / 128 numbers only; others stay in the latent space.
 //
 //   latent_gather_kernel   pages -> rows: cbuf [T, R], krbuf [T, P].  A portion's rows begin at a multiple of 64 and are
 //                          filled up to one with zeros, T rows in all; base[e] is the first row of entry e.
@@ -18,7 +21,6 @@
 //   Tensor memory: 2 x 2 S buffers of 64 columns, 2 O accumulators of 128.  Every wait is bounded.
 // Bound by the softmax between the two products.  2,048 tokens of 16 heads: 66 us, 325 TFLOP/s (455 with the weights' second part);
 // latent_attn_mma for the same 636 us.
-#include "tma.cuh"
 #include "umma.cuh"
 #include <math.h>
 
@@ -32,22 +34,6 @@ constexpr int MMA_WARP_1 = 2 + 4 * QT, THREADS = 32 * (3 + 4 * QT);
 constexpr int SUBQ = ROWS * 64 * 2, SUBK = KT * 64 * 2;               // bytes of 64 columns of a Q and of a key tile
 constexpr int Q_BYTES = 3 * SUBQ, K_BYTES = 3 * SUBK, V_BYTES = 2 * SUBK;
 constexpr int SMEM = 1024 + QT * Q_BYTES + STAGES * (K_BYTES + V_BYTES) + 256;
-
-__device__ __forceinline__ float ex2(float x) {
-  float y;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
-}
-__device__ __forceinline__ float max3(float a, float b, float c) {
-  float d;
-  asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
-  return d;
-}
-// V: rows = keys = the product's K, 64 contiguous numbers per 128-byte row; the next 64 are one sub-tile further
-__device__ __forceinline__ uint64_t desc_mnmajor(const void* tile) {
-  const uint64_t addr = (uint64_t)((s32(tile) & 0x3FFFFu) >> 4);
-  return addr | ((uint64_t)(SUBK >> 4) << 16) | (64ull << 32) | (1ull << 46) | (2ull << 61);
-}
 
 // What is asked of entry e: its tokens, the first key its tokens see (down to a multiple of 64), how many rows of keys.
 struct Span {
@@ -285,7 +271,7 @@ latent_prompt_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_con
     // ------------------------------------------------------------------ products, one thread per Q tile
     const int tt = warp == 1 ? 0 : 1;
     if (lane == 0) {
-      const uint32_t id_s = instr_desc(KT), id_o = instr_desc(DV) | (1u << 16);          // B = V is MN-major
+      const uint32_t id_s = instr_desc(KT), id_o = instr_desc(DV, true);
       const uint64_t qdesc = smem_desc(Qs + tt * Q_BYTES);
       uint32_t base_no = 0, sq = 0, n_mine = 0;
       bool ok = true;
@@ -332,7 +318,7 @@ latent_prompt_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_con
           if (!ok) break;
           tc_fence_after();
           const uint32_t p_tmem = tmem + (uint32_t)(tt * 128) + bf * 64u;
-          const uint64_t vdesc = desc_mnmajor(Vs + st * V_BYTES);
+          const uint64_t vdesc = desc_mnmajor(Vs + st * V_BYTES, SUBK);
           const uint32_t d = tmem + (uint32_t)(256 + tt * 128);
 #pragma unroll
           for (int part = 1; part >= 0; --part)                       // the remainders, then the rounded weights

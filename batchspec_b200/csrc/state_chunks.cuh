@@ -26,16 +26,6 @@ __device__ __forceinline__ int chunk_entry(const int* __restrict__ qo_indptr, in
 // Heads that fill most of the 128 x 128 numbers which the products are laid out for.
 inline bool chunk_sizes(int dim, int vdim) { return dim <= CH_W && vdim <= CH_W && dim % 4 == 0 && dim * vdim >= 96 * 96; }
 
-__device__ __forceinline__ unsigned long long pair_of(float a, float b) {
-  unsigned long long r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
-  return r;
-}
-__device__ __forceinline__ void halves_of(unsigned long long v, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
-__device__ __forceinline__ void fma_pair(unsigned long long& acc, unsigned long long a, unsigned long long b) {
-  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b));
-}
-
 // acc[a][b] = (even, odd) parts of S^T q for tokens tb + a (a < 8: a warp's) and columns lane + 32 b.  qs [CH][CH_LD] queries, S
 // [vdim][dim] in memory, ss [CH_W][CH_SL + 4] shared memory for a slice of 32 key rows.  All threads of the block.
 __device__ __forceinline__ void chunk_read_state(unsigned long long (&acc)[8][4], const float* qs, float* ss, const float* __restrict__ S,

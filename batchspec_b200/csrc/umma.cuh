@@ -1,6 +1,6 @@
-// tcgen05 (5th-generation tensor core) helpers shared by the matrix-product kernels: fences, commit, the MMA
-// itself for bfloat16 operands in shared memory with a float32 accumulator in tensor memory, accumulator loads,
-// and the shared-memory and instruction descriptors of K-major 128-byte-swizzled tiles with 128 accumulator rows.
+// tcgen05 (5th-generation tensor core) helpers shared by the matrix-product and prompt attention kernels: fences, commit, the MMA
+// itself for bfloat16 operands (A in shared or tensor memory) with a float32 accumulator in tensor memory, loads and stores of
+// tensor memory, packed arithmetic, and the descriptors of 128-byte-swizzled tiles with 128 accumulator rows.
 #pragma once
 #include "common.cuh"
 #include "tma.cuh"
@@ -61,7 +61,7 @@ __device__ __forceinline__ void tc_st32(uint32_t taddr, const uint32_t (&v)[32])
         "r"(v[28]), "r"(v[29]), "r"(v[30]), "r"(v[31]), "r"(taddr)
       : "memory");
 }
-__device__ __forceinline__ void tc_st16(uint32_t taddr, const uint32_t (&v)[16]) {
+__device__ __forceinline__ void tc_st16(uint32_t taddr, const uint32_t* v) {
   asm volatile(
       "tcgen05.st.sync.aligned.32x32b.x16.b32 [%16], "
       "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15};"
@@ -70,7 +70,14 @@ __device__ __forceinline__ void tc_st16(uint32_t taddr, const uint32_t (&v)[16])
       : "memory");
 }
 __device__ __forceinline__ void tc_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
-// two float32 operations per instruction
+__device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
+__device__ __forceinline__ float ex2(float x) {          // 2^x on the special-function unit; 2^-inf = 0
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+// Two float32 operations per instruction (sm_100 has packed forms of add, mul and fma) and a maximum of three:
+// a softmax is bound by the number of instructions it issues, not by the arithmetic pipes.
 __device__ __forceinline__ uint64_t pack2(float a, float b) {
   uint64_t r;
   asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
@@ -88,14 +95,26 @@ __device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
   return d;
 }
 
+__device__ __forceinline__ float max3(float a, float b, float c) {
+  float d;
+  asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+  return d;
+}
+
 // Shared-memory matrix descriptor: K-major tile, rows of 128 bytes, 128-byte swizzle, 8-row groups 1024 bytes apart.
 __device__ __forceinline__ uint64_t smem_desc(const void* tile) {
   const uint64_t addr = (uint64_t)((s32(tile) & 0x3FFFFu) >> 4);
   return addr | (1ull << 16) | (64ull << 32) | (1ull << 46) | (2ull << 61);
 }
-// Instruction descriptor: float32 accumulator, bfloat16 A and B, both K-major, M = 128, N = bn.
-__device__ __forceinline__ uint32_t instr_desc(int bn) {
-  return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(bn >> 3) << 17) | ((uint32_t)(UMMA_M >> 4) << 24);
+// MN-major operand (V: rows = keys = the product's K, 64 contiguous numbers per 128-byte row): the next 64 numbers are ``sub``
+// bytes further, 8-key groups 1024.
+__device__ __forceinline__ uint64_t desc_mnmajor(const void* tile, int sub) {
+  const uint64_t addr = (uint64_t)((s32(tile) & 0x3FFFFu) >> 4);
+  return addr | ((uint64_t)(sub >> 4) << 16) | (64ull << 32) | (1ull << 46) | (2ull << 61);
+}
+// Instruction descriptor: float32 accumulator, bfloat16 A and B, A K-major, B too or MN-major, M = 128, N = bn.
+__device__ __forceinline__ uint32_t instr_desc(int bn, bool b_mn = false) {
+  return (1u << 4) | (1u << 7) | (1u << 10) | (b_mn ? 1u << 16 : 0u) | ((uint32_t)(bn >> 3) << 17) | ((uint32_t)(UMMA_M >> 4) << 24);
 }
 
 }  // namespace bspec
