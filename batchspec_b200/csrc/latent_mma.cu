@@ -67,8 +67,10 @@ __host__ __device__ inline size_t smem_bytes(int D, int BM, int stages = 2, int 
 // shorter than the others, and a share more than fit runs after all others.  64 requests of 300 to
 // 4,096 entries, 16 heads: 100 us with as many shares for each as for the longest, 55 dealt; requests of one length lose nothing
 // by it: 64 of 4,096 entries 117 / 111 (141 where a few shares ran in a second wave), 64 of 1,000 43 / 41 (57), 256 of 300, a
-// share each, 54 / 54 (73).  At latents of 128 and 256 the dealing itself shows, 256 of 300 26 / 29.
-constexpr int MAX_SHARES = 64, MIN_TILES = 4, TRY = 16, OWN = 4;
+// share each, 54 / 54 (73).  At latents of 128 and 256 the dealing itself shows, 256 of 300 26 / 29.  Shares of at least two tiles: a
+// captured step whose bound is 4,608 entries, 5 requests of 100 16.6 us (of four tiles, all in one share, 20.2), 2 of 2,000 23.7 (of
+// one tile, 40 shares to join, 28.9).
+constexpr int MAX_SHARES = 64, MIN_TILES = 2, TRY = 16, OWN = 4;
 struct Share {
   int e, split, first, count, per;       // request (-1: none), which of its shares, its first share and how many it has
 };
